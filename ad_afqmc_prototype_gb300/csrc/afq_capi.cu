@@ -118,6 +118,7 @@ struct StepWS {
     double2* fb;        // W*G
     double2* xs;        // W*G
     double2* V;         // Wc*n*n
+    OzScratch oz;       // digit products
     // mixed form
     __nv_bfloat16* Ag;  // 2W x Kt_F
     float* fbm;         // 2W x G
@@ -137,7 +138,28 @@ struct StepWS {
 // (7 norb 2^12 < 2^24).
 static bool oz_supported(const afq_dims* d) { return d->nocc <= 32 && d->norb <= 584; }
 
-static StepWS layout_step(Arena& a, const afq_dims* d, int n_chunks) {
+static size_t max3(size_t a, size_t b, size_t c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
+
+// Scratch of the binary64 form's digit products (one region, used by one at a time).
+static OzScratch take_oz(Arena& a, size_t bytes, int* status) {
+    OzScratch z;
+    z.p = a.take<char>(bytes);
+    z.err = status;
+    return z;
+}
+static size_t fb_oz_bytes(const afq_dims* d) {
+    return zgemm_oz_scratch(d->n_walkers, d->nchol, d->nocc * d->norb);
+}
+static size_t trotter_oz_bytes(const afq_dims* d, int n_chunks) {
+    const int n = d->norb, wc = chunk_size(d->n_walkers, n_chunks);
+    const size_t v = zgemm_oz_scratch(wc, n * n, d->nchol), t = trotter_oz_scratch(wc, n, d->nocc, 1);
+    return v > t ? v : t;
+}
+static size_t energy_oz_bytes(const afq_dims* d) {
+    return energy_oz_scratch(d->n_walkers, d->norb, d->nocc, d->nchol);
+}
+
+static StepWS layout_step(Arena& a, const afq_dims* d, int n_chunks, size_t oz_bytes = 0) {
     const size_t W = d->n_walkers, n = d->norb, o = d->nocc, G = d->nchol;
     const size_t Wc = chunk_size(d->n_walkers, n_chunks);
     StepWS s = {};
@@ -167,6 +189,7 @@ static StepWS layout_step(Arena& a, const afq_dims* d, int n_chunks) {
         s.fb = a.take<double2>(W * G);
         s.xs = a.take<double2>(W * G);
         s.V = a.take<double2>(Wc * n * n);
+        s.oz = take_oz(a, max3(oz_bytes, fb_oz_bytes(d), trotter_oz_bytes(d, n_chunks)), s.status);
     }
     return s;
 }
@@ -206,7 +229,7 @@ struct BlockWS {
 
 static BlockWS layout_block(Arena& a, const afq_dims* d, int n_chunks) {
     BlockWS b = {};
-    b.step = layout_step(a, d, n_chunks);
+    b.step = layout_step(a, d, n_chunks, is_mixed(d->precision) ? 0 : energy_oz_bytes(d));
     const size_t W = d->n_walkers;
     b.green = is_mixed(d->precision) ? a.take<double2>(W * d->nocc * d->norb) : b.step.green;
     b.energy = a.take<double2>(W);
@@ -240,26 +263,26 @@ static BlockWS layout_block(Arena& a, const afq_dims* d, int n_chunks) {
 
 // ------------------------------------------------------------ step pieces
 static int force_bias_from_green(const afq_dims* d, const double2* green, const double* rot_chol,
-                                 double2* fb, cudaStream_t s) {
+                                 double2* fb, const OzScratch& oz, cudaStream_t s) {
     const int on = d->nocc * d->norb;
-    return launch_zgemm(d->n_walkers, d->nchol, on, 2.0, green, on, rot_chol, on, !d->trial_is_real, true, fb,
-                        d->nchol, s);
+    return launch_zgemm_auto(d->n_walkers, d->nchol, on, 2.0, green, on, rot_chol, on, !d->trial_is_real, true, fb,
+                             d->nchol, oz, s);
 }
 
 static int trotter_chunked(const afq_dims* d, int n_terms, double sqrt_dt, int n_chunks, const double* chol,
                            const double* E, const double2* win, const double2* xs, double2* wout, double2* V,
-                           cudaStream_t s) {
+                           const OzScratch& oz, cudaStream_t s) {
     const int W = d->n_walkers, n = d->norb, o = d->nocc, G = d->nchol;
     const int Wc = chunk_size(W, n_chunks);
     for (int w0 = 0; w0 < W; w0 += Wc) {
         const int wc = W - w0 < Wc ? W - w0 : Wc;
         // V (wc x n^2) = x~ (wc x G) . chol (G x n^2)   (prop/chol_afqmc_ops.py:70-74)
         { AFQ_PHASE("vbuild_gemm", s);
-        AFQ_TRY(launch_zgemm(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, V,
-                             (int64_t)n * n, s)); }
+        AFQ_TRY(launch_zgemm_auto(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, V,
+                                  (int64_t)n * n, oz, s)); }
         { AFQ_PHASE("trotter", s);
-        AFQ_TRY(launch_trotter(wc, n, o, n_terms, sqrt_dt, E, V, win + (size_t)w0 * n * o,
-                               wout + (size_t)w0 * n * o, s)); }
+        AFQ_TRY(launch_trotter_auto(wc, n, o, n_terms, sqrt_dt, E, V, win + (size_t)w0 * n * o,
+                                    wout + (size_t)w0 * n * o, 1, oz, s)); }
     }
     return AFQ_OK;
 }
@@ -391,7 +414,7 @@ static int energy_impl(const afq_problem* pb, const afq_state* st, const BlockWS
     AFQ_PHASE("energy", s);
     if (!is_mixed(d->precision))
         return launch_energy(W, n, o, G, pb->h0, ws.green, pb->rot_chol, d->trial_is_real,
-                             (const double2*)pb->rot_h1, ws.partial, ws.energy, s);
+                             (const double2*)pb->rot_h1, ws.partial, ws.energy, ws.step.oz, s);
     const LowpDims L = lowp_dims(d);
     Arena la((void*)pb->lowp, (size_t)-1);
     const LowpBufs lb = layout_lowp(la, d);
@@ -454,14 +477,14 @@ static int step_impl(const afq_problem* pb, const afq_params* p, const afq_state
     if (is_mixed(d->precision)) return step_mixed(pb, p, st, fields, ws, green_ready, s, green_out);
     // force bias (prop/afqmc.py:90-95)
     { AFQ_PHASE("green", s); AFQ_TRY(launch_green(W, n, o, mo, d->trial_is_real, walk, nullptr, ws.green, s)); }
-    { AFQ_PHASE("fb_gemm", s); AFQ_TRY(force_bias_from_green(d, ws.green, pb->rot_chol, ws.fb, s)); }
+    { AFQ_PHASE("fb_gemm", s); AFQ_TRY(force_bias_from_green(d, ws.green, pb->rot_chol, ws.fb, ws.oz, s)); }
     // shifts (prop/afqmc.py:97-101)
     { AFQ_PHASE("field_shift", s);
     AFQ_TRY(launch_field_shift(W, G, pb->sqrt_dt, fields, ws.fb, (const double2*)pb->mf_shifts, ws.xs,
                                ws.shift_term, ws.fb_term, s)); }
     // propagation (prop/afqmc.py:103-110)
     AFQ_TRY(trotter_chunked(d, p->n_exp_terms, pb->sqrt_dt, p->n_chunks, pb->chol, pb->exp_h1_half, walk, ws.xs,
-                            walk, ws.V, s));
+                            walk, ws.V, ws.oz, s));
     // overlaps (prop/afqmc.py:112-114)
     { AFQ_PHASE("overlap", s); AFQ_TRY(launch_green(W, n, o, mo, d->trial_is_real, walk, ws.ovl_new, nullptr, s)); }
     AFQ_PHASE("weight_update", s);
@@ -683,6 +706,7 @@ size_t afq_force_bias_workspace(const afq_dims* d) {
     Arena a;
     a.take<int>(64);  // status word: offset 0 of every workspace
     a.take<double2>((size_t)d->n_walkers * d->nocc * d->norb);
+    a.take<char>(fb_oz_bytes(d));
     return a.used;
 }
 
@@ -692,13 +716,14 @@ int afq_force_bias(const afq_dims* d, const double* mo_coeff, const double* rot_
     AFQ_NOTNULL(mo_coeff); AFQ_NOTNULL(rot_chol); AFQ_NOTNULL(walkers); AFQ_NOTNULL(force_bias);
     AFQ_NOTNULL(workspace);
     Arena a(workspace, workspace_bytes);
-    a.take<int>(64);  // status word: offset 0 of every workspace
+    int* status = a.take<int>(64);  // status word: offset 0 of every workspace
     double2* green = a.take<double2>((size_t)d->n_walkers * d->nocc * d->norb);
+    const OzScratch oz = take_oz(a, fb_oz_bytes(d), status);
     AFQ_TRY(check_ws(a, workspace_bytes));
     cudaStream_t s = as_stream(stream);
     AFQ_TRY(launch_green(d->n_walkers, d->norb, d->nocc, (const double2*)mo_coeff, d->trial_is_real,
                          (const double2*)walkers, nullptr, green, s));
-    return force_bias_from_green(d, green, rot_chol, (double2*)force_bias, s);
+    return force_bias_from_green(d, green, rot_chol, (double2*)force_bias, oz, s);
 }
 
 size_t afq_energy_workspace(const afq_dims* d) {
@@ -707,6 +732,7 @@ size_t afq_energy_workspace(const afq_dims* d) {
     a.take<int>(64);  // status word: offset 0 of every workspace
     a.take<double2>((size_t)d->n_walkers * d->nocc * d->norb);
     a.take<double2>(energy_partial_count(d->n_walkers, d->nocc, d->nchol));
+    a.take<char>(energy_oz_bytes(d));
     return a.used;
 }
 
@@ -716,15 +742,16 @@ int afq_energy(const afq_dims* d, double h0, const double* mo_coeff, const doubl
     AFQ_NOTNULL(mo_coeff); AFQ_NOTNULL(rot_h1); AFQ_NOTNULL(rot_chol); AFQ_NOTNULL(walkers); AFQ_NOTNULL(energy);
     AFQ_NOTNULL(workspace);
     Arena a(workspace, workspace_bytes);
-    a.take<int>(64);  // status word: offset 0 of every workspace
+    int* status = a.take<int>(64);  // status word: offset 0 of every workspace
     double2* green = a.take<double2>((size_t)d->n_walkers * d->nocc * d->norb);
     double* partial = (double*)a.take<double2>(energy_partial_count(d->n_walkers, d->nocc, d->nchol));
+    const OzScratch oz = take_oz(a, energy_oz_bytes(d), status);
     AFQ_TRY(check_ws(a, workspace_bytes));
     cudaStream_t s = as_stream(stream);
     AFQ_TRY(launch_green(d->n_walkers, d->norb, d->nocc, (const double2*)mo_coeff, d->trial_is_real,
                          (const double2*)walkers, nullptr, green, s));
     return launch_energy(d->n_walkers, d->norb, d->nocc, d->nchol, h0, green, rot_chol, d->trial_is_real,
-                         (const double2*)rot_h1, partial, (double2*)energy, s);
+                         (const double2*)rot_h1, partial, (double2*)energy, oz, s);
 }
 
 size_t afq_apply_trotter_workspace(const afq_dims* d, int32_t n_chunks) {
@@ -732,6 +759,7 @@ size_t afq_apply_trotter_workspace(const afq_dims* d, int32_t n_chunks) {
     Arena a;
     a.take<int>(64);  // status word: offset 0 of every workspace
     a.take<double2>((size_t)chunk_size(d->n_walkers, n_chunks) * d->norb * d->norb);
+    a.take<char>(trotter_oz_bytes(d, n_chunks));
     return a.used;
 }
 
@@ -743,11 +771,12 @@ int afq_apply_trotter(const afq_dims* d, int32_t n_terms, double sqrt_dt, int32_
     AFQ_NOTNULL(walkers_out); AFQ_NOTNULL(workspace);
     if (n_terms < 0) return fail(AFQ_E_INVALID_ARGUMENT, "n_terms=%d < 0", n_terms);
     Arena a(workspace, workspace_bytes);
-    a.take<int>(64);  // status word: offset 0 of every workspace
+    int* status = a.take<int>(64);  // status word: offset 0 of every workspace
     double2* V = a.take<double2>((size_t)chunk_size(d->n_walkers, n_chunks) * d->norb * d->norb);
+    const OzScratch oz = take_oz(a, trotter_oz_bytes(d, n_chunks), status);
     AFQ_TRY(check_ws(a, workspace_bytes));
     return trotter_chunked(d, n_terms, sqrt_dt, n_chunks, chol, exp_h1_half, (const double2*)walkers,
-                           (const double2*)shifted_fields, (double2*)walkers_out, V, as_stream(stream));
+                           (const double2*)shifted_fields, (double2*)walkers_out, V, oz, as_stream(stream));
 }
 
 int afq_orthogonalize(const afq_dims* d, const double* walkers, double* walkers_out, double* det_r, void* stream) {

@@ -13,6 +13,7 @@
 // Fields and comb uniforms are regenerated from the Philox stream, never
 // stored.  dL/dE_half and the one-body energy term are accumulated over the
 // run and turned into dL/dh1 at the end (launch_h1bar).
+#include <algorithm>
 #include <utility>
 
 #include "afq_internal.cuh"
@@ -66,6 +67,7 @@ struct GradWS {
     BlockSnap snap;  // ck blocks, n_ops slots each (energy: ck x W; V: ck x n_prop_steps when kept)
     bool keep_v;     // the replay keeps each step's V for the adjoint (no V-build recomputation)
     double2* zpart;  // split-K layers of the adjoint's FP64 GEMMs
+    OzScratch oz;    // digit products
     // adjoint state (two copies for the comb's scatter)
     double2 *wk, *wk2, *ob, *ob2;
     double *wb, *wb2, *pb, *wsum;
@@ -116,6 +118,11 @@ GradWS layout_grad(Arena& a, const afq_dims* d, const afq_params* p, int ck) {
         const size_t z1 = (size_t)zgemm_splits((int)W, (int)G, (int)(n * n)) * W * G;
         const size_t z2 = (size_t)zgemm_splits((int)W, (int)no, (int)G) * W * no;
         g.zpart = a.take<double2>(z1 > z2 ? z1 : z2);
+        const int Wi = (int)W, Gi = (int)G, n2 = (int)(n * n), noi = (int)no, oi = (int)o, ni = (int)n, wo = (int)(wc * o);
+        g.oz.p = a.take<char>(std::max({zgemm_oz_scratch(Wi, Gi, noi), zgemm_oz_scratch(Wi, n2, Gi),
+                                        zgemm_oz_scratch(Wi, Gi, n2), zgemm_oz_scratch(Wi, noi, Gi),
+                                        zgemm_oz_scratch(wo, Gi * oi, ni), zgemm_oz_scratch(wo, ni, Gi * oi)}));
+        g.oz.err = g.status;
     }
     g.wk = a.take<double2>(W * no);
     g.wk2 = a.take<double2>(W * no);
@@ -188,6 +195,14 @@ struct Ctx {
 template <class T>
 T* slot(T* base, size_t per, int k) { return base + (size_t)k * per; }
 
+// C (M x N) by digits where that pays, else split over K on the binary64 pipe.
+int zgemm_adj(const GradWS& g, int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B,
+              int64_t ldb, bool b_trans, double2* C, cudaStream_t s) {
+    if (zgemm_oz_pays(M, N, K))
+        return launch_zgemm_oz(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, N, g.oz.p, g.oz.err, s);
+    return launch_zgemm_splitk(M, N, K, alpha, A, lda, B, ldb, false, b_trans, C, g.zpart, s);
+}
+
 // Adjoint of step st_i of a block, whose input state is snapshot slot op.
 int step_adjoint(const Ctx& c, const BlockSnap& sn, int op, int st_i, uint64_t counter) {
     const afq_problem* pb = c.pb;
@@ -203,15 +218,15 @@ int step_adjoint(const Ctx& c, const BlockSnap& sn, int op, int st_i, uint64_t c
         AFQ_PHASE("adj_recompute", s);
         AFQ_TRY(launch_philox((int64_t)W * G, c.seed, counter, 1, g.fields, s));
         AFQ_TRY(launch_green(W, n, o, mo, 1, Wpre, nullptr, g.green, s));
-        AFQ_TRY(launch_zgemm(W, G, no, 2.0, g.green, no, pb->rot_chol, no, false, true, g.fb, G, s));
+        AFQ_TRY(launch_zgemm_auto(W, G, no, 2.0, g.green, no, pb->rot_chol, no, false, true, g.fb, G, g.oz, s));
         AFQ_TRY(launch_field_shift(W, G, pb->sqrt_dt, g.fields, g.fb, (const double2*)pb->mf_shifts, g.xs,
                                    g.shift_term, g.fb_term, s));
     }
     const double2* V = sn.V ? sn.V + (size_t)st_i * W * n * n : g.V;
     if (!sn.V) {
         AFQ_PHASE("adj_vbuild_gemm", s);
-        AFQ_TRY(launch_zgemm(W, n * n, G, 1.0, g.xs, G, pb->chol, (int64_t)n * n, false, false, g.V,
-                             (int64_t)n * n, s));
+        AFQ_TRY(launch_zgemm_auto(W, n * n, G, 1.0, g.xs, G, pb->chol, (int64_t)n * n, false, false, g.V,
+                             (int64_t)n * n, g.oz, s));
     }
     { AFQ_PHASE("adj_taylor_tape", s);
       AFQ_TRY(launch_taylor_tape(W, n, o, K, pb->sqrt_dt, pb->exp_h1_half, V, Wpre, g.terms, g.w2, s)); }
@@ -233,12 +248,11 @@ int step_adjoint(const Ctx& c, const BlockSnap& sn, int op, int st_i, uint64_t c
     // V = sum_g x~_g L_g: x~b = Vb . L^T
     { AFQ_PHASE("adj_vbar", s); AFQ_TRY(launch_vbar(W, n, o, K, pb->sqrt_dt, g.tbar, g.terms, g.V, s)); }
     { AFQ_PHASE("adj_xbar_gemm", s);
-      AFQ_TRY(launch_zgemm_splitk(W, G, n * n, 1.0, g.V, (int64_t)n * n, pb->chol, (int64_t)n * n, false, true,
-                                  g.xtb, g.zpart, s)); }
+      AFQ_TRY(zgemm_adj(g, W, G, n * n, 1.0, g.V, (int64_t)n * n, pb->chol, (int64_t)n * n, true, g.xtb, s)); }
     // field shifts, then the force bias fb = 2 L~ vec(G_half)
     AFQ_TRY(launch_fs_adj(W, G, pb->sqrt_dt, g.fields, g.fb, (const double2*)pb->mf_shifts, g.fbt_bar, g.shift_bar,
                           g.xtb, s));
-    AFQ_TRY(launch_zgemm_splitk(W, no, G, 2.0, g.xtb, G, pb->rot_chol, no, false, false, g.gbar, g.zpart, s));
+    AFQ_TRY(zgemm_adj(g, W, no, G, 2.0, g.xtb, G, pb->rot_chol, no, false, g.gbar, s));
     return launch_green_adj(W, n, o, mo, Wpre, g.gbar, nullptr, nullptr, g.wk, g.status, s);
 }
 
@@ -267,17 +281,17 @@ int block_adjoint(const Ctx& c, const BlockSnap& sn, const TapeLayout& t, int b,
                                g.pb, g.wb, g.ebar_w, s));
     // local energies -> G_half of the measured walkers
     AFQ_TRY(launch_green(W, n, o, mo, 1, Wm, nullptr, g.green, s));
-    AFQ_TRY(launch_zgemm(W, G, no, 1.0, g.green, no, pb->rot_chol, no, false, true, g.xtb, G, s));   // c_g
-    AFQ_TRY(launch_zgemm(W, no, G, 1.0, g.xtb, G, pb->rot_chol, no, false, false, g.cl, no, s));     // sum c_g L~_g
+    AFQ_TRY(launch_zgemm_auto(W, G, no, 1.0, g.green, no, pb->rot_chol, no, false, true, g.xtb, G, g.oz, s));   // c_g
+    AFQ_TRY(launch_zgemm_auto(W, no, G, 1.0, g.xtb, G, pb->rot_chol, no, false, false, g.cl, no, g.oz, s));     // sum c_g L~_g
     const int wc = grad_energy_chunk(d);
     for (int w0 = 0; w0 < W; w0 += wc) {
         const int nw = W - w0 < wc ? W - w0 : wc;
         // F[(w, q), (g, p)] = f_g[p, q];  y[(w, p), j] = sum_{g, q} f_g[p, q] L~_g[q, j]
-        AFQ_TRY(launch_zgemm(nw * o, G * o, n, 1.0, g.green + (size_t)w0 * no, n, pb->rot_chol, n, false, true, g.F,
-                             (int64_t)G * o, s));
+        AFQ_TRY(launch_zgemm_auto(nw * o, G * o, n, 1.0, g.green + (size_t)w0 * no, n, pb->rot_chol, n, false, true, g.F,
+                             (int64_t)G * o, g.oz, s));
         AFQ_TRY(launch_block_transpose(nw, o, G, g.F, g.Ft, s));
-        AFQ_TRY(launch_zgemm(nw * o, n, G * o, 1.0, g.Ft, (int64_t)G * o, pb->rot_chol, n, false, false,
-                             g.y + (size_t)w0 * no, n, s));
+        AFQ_TRY(launch_zgemm_auto(nw * o, n, G * o, 1.0, g.Ft, (int64_t)G * o, pb->rot_chol, n, false, false,
+                             g.y + (size_t)w0 * no, n, g.oz, s));
     }
     AFQ_TRY(launch_energy_gbar(W, no, g.ebar_w, (const double2*)pb->rot_h1, g.cl, g.y, g.gbar, s));
     AFQ_TRY(launch_sg_accum(W, no, g.ebar_w, g.green, g.sg_part, s));

@@ -290,6 +290,34 @@ int zgemm_splits(int M, int N, int K);
 int launch_zgemm_splitk(int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B,
                         int64_t ldb, bool b_complex, bool b_trans, double2* C, double2* part, cudaStream_t s);
 
+// k_ozgemm.cu : the binary64 form's contractions from integer digits on the
+// tensor cores.  Scratch of a call: *_oz_scratch bytes, 256-byte aligned; a
+// bounded wait that expires sets *err.
+struct OzScratch {
+    void* p = nullptr;
+    int* err = nullptr;
+};
+bool zgemm_oz_pays(int M, int N, int K);
+size_t zgemm_oz_scratch(int M, int N, int K);
+// launch_zgemm with a real right operand; alpha a power of two
+int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
+                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s);
+bool trotter_oz_pays(int W, int n, int o, int n_terms);
+size_t trotter_oz_scratch(int W, int n, int o, int vdiv);
+int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
+                      const double2* win, double2* wout, int vdiv, void* scratch, int* err, cudaStream_t s);
+bool energy_oz_pays(int W, int n, int o, int G);
+size_t energy_oz_scratch(int W, int n, int o, int G);
+int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, const double* rot_chol,
+                             double* partial, void* scratch, int* err, cudaStream_t s);
+// the product by digits where that pays, else on the binary64 pipe
+int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B, int64_t ldb,
+                      bool b_complex, bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s);
+int launch_trotter_auto(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
+                        const double2* win, double2* wout, int vdiv, const OzScratch& oz, cudaStream_t s);
+int launch_energy_partial_auto(int W, int n, int o, int G, const double2* green, const void* rot_chol, int trial_real,
+                               double* partial, const OzScratch& oz, cudaStream_t s);
+
 // k_walker.cu
 int launch_green(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
                  double2* ovlp_out, double2* green_out, cudaStream_t s);
@@ -308,7 +336,7 @@ int launch_weight_update(int W, const afq_params* p, double sqrt_dt, double dt,
                          int* status = nullptr);  // status: a workspace's status word, counts non-finite walkers
 int launch_energy(int W, int n, int o, int G, double h0, const double2* green,
                   const void* rot_chol, int trial_real, const double2* rot_h1,
-                  double* partial, double2* energy, cudaStream_t s);
+                  double* partial, double2* energy, const OzScratch& oz, cudaStream_t s);
 int launch_qr(int W, int n, int o, const double2* win, double2* wout, double2* det_r,
               cudaStream_t s);
 int launch_sr_scan(int W, const double* weights, double zeta, double* levels, int32_t* idx,
@@ -350,6 +378,7 @@ int launch_green_det(int W, int n, int o, const double2* mo, int trial_real, con
                      double2* det_out, double2* green_out, cudaStream_t s);
 // the energy's per-chunk partials (sum c^2, sum exchange) without the finish
 int energy_partial_chunks(int o, int G);
+bool energy_partial_fits(int o, int G, int trial_real);
 int launch_energy_partial(int W, int n, int o, int G, const double2* green, const void* rot_chol, int trial_real,
                           double* partial, cudaStream_t s);
 size_t energy_partial_count(int W, int o, int G);

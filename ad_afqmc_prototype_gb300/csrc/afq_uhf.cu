@@ -16,6 +16,9 @@
 //              + [sum_g (c_up + c_dn)_g^2 - exc_up - exc_dn] / 2
 //   Trotter    the same V_w on both spins
 //   QR         per spin;  comb: one set of indices for both spins.
+#include <algorithm>
+#include <initializer_list>
+
 #include "afq_internal.cuh"
 
 namespace afq {
@@ -84,6 +87,8 @@ int launch_spin_sum(long long count, const double2* green, double2* g, cudaStrea
     return AFQ_OK;
 }
 
+size_t oz_most(std::initializer_list<size_t> v) { return std::max(v); }
+
 int chunk_of(int W, int n_chunks) { return n_chunks <= 1 ? W : (W + n_chunks - 1) / n_chunks; }
 
 struct UWS {
@@ -96,6 +101,7 @@ struct UWS {
     double2* xs;         // W G
     double2 *shift_term, *fb_term, *det, *ov_new;  // W, W, 2W, W
     double2* V;          // Wc n n
+    OzScratch oz;        // digit products
     double* partial;     // energy partials of 2W spin-walkers
     double2* energy;     // W
     double* levels;
@@ -119,7 +125,13 @@ UWS layout_u(Arena& a, const afq_dims* d, int n_chunks) {
     u.fb_term = a.take<double2>(W);
     u.det = a.take<double2>(2 * W);
     u.ov_new = a.take<double2>(W);
-    u.V = a.take<double2>((size_t)chunk_of(d->n_walkers, n_chunks) * n * n);
+    const int wc = chunk_of(d->n_walkers, n_chunks);
+    u.V = a.take<double2>((size_t)wc * n * n);
+    u.oz.p = a.take<char>(oz_most({zgemm_oz_scratch(2 * d->n_walkers, d->nchol, (int)no),
+                                   zgemm_oz_scratch(wc, (int)(n * n), d->nchol),
+                                   trotter_oz_scratch(wc, d->norb, d->nocc, 1),
+                                   energy_oz_scratch(2 * d->n_walkers, d->norb, d->nocc, d->nchol)}));
+    u.oz.err = u.status;
     u.partial = (double*)a.take<double2>(energy_partial_count(2 * d->n_walkers, d->nocc, d->nchol));
     u.energy = a.take<double2>(W);
     u.levels = a.take<double>(sr_levels_size(d->n_walkers));
@@ -153,23 +165,24 @@ int overlap_u(const afq_dims* d, const double2* mo, const double2* walk, double2
 int force_bias_u(const afq_dims* d, const double* rot_chol, const UWS& u, double2* fb, cudaStream_t s) {
     const int W = d->n_walkers, on = d->norb * d->nocc;
     AFQ_TRY(launch_spin_sum((long long)W * on, u.green, u.gsum, s));
-    return launch_zgemm(W, d->nchol, on, 1.0, u.gsum, on, rot_chol, on, !d->trial_is_real, true, fb, d->nchol, s);
+    return launch_zgemm_auto(W, d->nchol, on, 1.0, u.gsum, on, rot_chol, on, !d->trial_is_real, true, fb, d->nchol,
+                             u.oz, s);
 }
 
 int trotter_u(const afq_dims* d, int n_terms, double sqrt_dt, int n_chunks, const double* chol, const double* E,
-              const double2* win, const double2* xs, double2* wout, double2* V, cudaStream_t s) {
+              const double2* win, const double2* xs, double2* wout, double2* V, const OzScratch& oz, cudaStream_t s) {
     const int W = d->n_walkers, n = d->norb, o = d->nocc, G = d->nchol;
     const size_t half = (size_t)W * n * o;
     const int Wc = chunk_of(W, n_chunks);
     for (int w0 = 0; w0 < W; w0 += Wc) {
         const int wc = W - w0 < Wc ? W - w0 : Wc;
         { AFQ_PHASE("vbuild_gemm", s);
-          AFQ_TRY(launch_zgemm(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, V,
-                               (int64_t)n * n, s)); }
+          AFQ_TRY(launch_zgemm_auto(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, V,
+                                    (int64_t)n * n, oz, s)); }
         AFQ_PHASE("trotter", s);
         for (int spin = 0; spin < 2; ++spin)
-            AFQ_TRY(launch_trotter(wc, n, o, n_terms, sqrt_dt, E, V, win + spin * half + (size_t)w0 * n * o,
-                                   wout + spin * half + (size_t)w0 * n * o, s));
+            AFQ_TRY(launch_trotter_auto(wc, n, o, n_terms, sqrt_dt, E, V, win + spin * half + (size_t)w0 * n * o,
+                                        wout + spin * half + (size_t)w0 * n * o, 1, oz, s));
     }
     return AFQ_OK;
 }
@@ -180,8 +193,9 @@ int energy_u(const afq_problem* pb, const UWS& u, cudaStream_t s) {
     const int W = d->n_walkers, n = d->norb, o = d->nocc, G = d->nchol, on = n * o;
     AFQ_PHASE("energy", s);
     AFQ_TRY(launch_spin_sum((long long)W * on, u.green, u.gsum, s));
-    AFQ_TRY(launch_zgemm(2 * W, G, on, 1.0, u.green, on, pb->rot_chol, on, !d->trial_is_real, true, u.c, G, s));
-    AFQ_TRY(launch_energy_partial(2 * W, n, o, G, u.green, pb->rot_chol, d->trial_is_real, u.partial, s));
+    AFQ_TRY(launch_zgemm_auto(2 * W, G, on, 1.0, u.green, on, pb->rot_chol, on, !d->trial_is_real, true, u.c, G, u.oz,
+                              s));
+    AFQ_TRY(launch_energy_partial_auto(2 * W, n, o, G, u.green, pb->rot_chol, d->trial_is_real, u.partial, u.oz, s));
     k_energy_finish_u<<<(W + 7) / 8, 256, 0, s>>>(W, on, G, energy_partial_chunks(o, G), pb->h0, u.gsum,
                                                   (const double2*)pb->rot_h1, u.c, (const double2*)u.partial,
                                                   u.energy);
@@ -207,7 +221,7 @@ int step_u(const afq_problem* pb, const afq_params* p, const afq_state* st, cons
       AFQ_TRY(launch_field_shift(W, G, pb->sqrt_dt, fields, u.fb, (const double2*)pb->mf_shifts, u.xs, u.shift_term,
                                  u.fb_term, s)); }
     AFQ_TRY(trotter_u(d, p->n_exp_terms, pb->sqrt_dt, p->n_chunks, pb->chol, pb->exp_h1_half, walk, u.xs, walk, u.V,
-                      s));
+                      u.oz, s));
     { AFQ_PHASE("overlap", s); AFQ_TRY(overlap_u(d, mo, walk, u.ov_new, nullptr, u, s)); }
     AFQ_PHASE("weight_update", s);
     return launch_weight_update(W, p, pb->sqrt_dt, pb->dt, make_double2(pb->h0_prop_re, pb->h0_prop_im),
@@ -273,6 +287,7 @@ struct GWS {
     double2* green;  // W x 2o x 2n
     double2* gsum;   // W x o x n
     double2* V;      // Wc x n x n
+    OzScratch oz;    // digit products
 };
 
 GWS layout_g(Arena& a, const afq_dims* d, int n_chunks) {
@@ -282,7 +297,12 @@ GWS layout_g(Arena& a, const afq_dims* d, int n_chunks) {
     g.cg = a.take<double2>(4 * n * o);
     g.green = a.take<double2>(W * 4 * o * n);
     g.gsum = a.take<double2>(W * o * n);
-    g.V = a.take<double2>((size_t)chunk_of(d->n_walkers, n_chunks) * n * n);
+    const int wc = chunk_of(d->n_walkers, n_chunks);
+    g.V = a.take<double2>((size_t)wc * n * n);
+    g.oz.p = a.take<char>(oz_most({zgemm_oz_scratch(d->n_walkers, d->nchol, (int)(n * o)),
+                                   zgemm_oz_scratch(wc, (int)(n * n), d->nchol),
+                                   trotter_oz_scratch(2 * wc, d->norb, 2 * d->nocc, 2)}));
+    g.oz.err = g.status;
     return g;
 }
 
@@ -346,8 +366,8 @@ int afq_force_bias_g(const afq_dims* d, const double* mo_coeff, const double* ro
     if (blocks > 152 * 32) blocks = 152 * 32;
     k_fold_g<<<(unsigned)blocks, 256, 0, s>>>(W, n, o, g.green, g.gsum);
     AFQ_LAUNCHED("k_fold_g");
-    return launch_zgemm(W, d->nchol, on, 1.0, g.gsum, on, rot_chol, on, !d->trial_is_real, true,
-                        (double2*)force_bias, d->nchol, s);
+    return launch_zgemm_auto(W, d->nchol, on, 1.0, g.gsum, on, rot_chol, on, !d->trial_is_real, true,
+                             (double2*)force_bias, d->nchol, g.oz, s);
 }
 
 int afq_apply_trotter_g(const afq_dims* d, int32_t n_terms, double sqrt_dt, int32_t n_chunks, const double* chol,
@@ -366,12 +386,12 @@ int afq_apply_trotter_g(const afq_dims* d, int32_t n_terms, double sqrt_dt, int3
     const double2* xs = (const double2*)shifted_fields;
     for (int w0 = 0; w0 < W; w0 += Wc) {
         const int wc = W - w0 < Wc ? W - w0 : Wc;
-        AFQ_TRY(launch_zgemm(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, g.V,
-                             (int64_t)n * n, s));
+        AFQ_TRY(launch_zgemm_auto(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, g.V,
+                                  (int64_t)n * n, g.oz, s));
         // the top and bottom n x 2o halves of each walker, both with the walker's V
-        AFQ_TRY(launch_trotter(2 * wc, n, 2 * o, n_terms, sqrt_dt, exp_h1_half, g.V,
-                               (const double2*)walkers + (size_t)w0 * 4 * n * o,
-                               (double2*)walkers_out + (size_t)w0 * 4 * n * o, s, 2));
+        AFQ_TRY(launch_trotter_auto(2 * wc, n, 2 * o, n_terms, sqrt_dt, exp_h1_half, g.V,
+                                    (const double2*)walkers + (size_t)w0 * 4 * n * o,
+                                    (double2*)walkers_out + (size_t)w0 * 4 * n * o, 2, g.oz, s));
     }
     return AFQ_OK;
 }
@@ -440,7 +460,7 @@ int afq_apply_trotter_u(const afq_dims* d, int32_t n_terms, double sqrt_dt, int3
     const UWS u = layout_u(a, d, n_chunks);
     if (!a.ok()) return fail(AFQ_E_WORKSPACE, "workspace: %zu bytes < %zu", workspace_bytes, a.used);
     return trotter_u(d, n_terms, sqrt_dt, n_chunks, chol, exp_h1_half, (const double2*)walkers,
-                     (const double2*)shifted_fields, (double2*)walkers_out, u.V, as_stream(stream));
+                     (const double2*)shifted_fields, (double2*)walkers_out, u.V, u.oz, as_stream(stream));
 }
 
 int afq_stochastic_reconfiguration_u(const afq_dims* d, const double* weights, double zeta, const double* walkers,

@@ -1,0 +1,1066 @@
+// Binary64 products of a real and a complex operand on the bf16 tensor cores,
+// for the binary64 form's contractions:
+//   V-build     V (W x n^2)    = x~ (W x G) . L (G x n^2)      (prop/chol_afqmc_ops.py:70-74)
+//   force bias  fb (W x G)     = 2 G_half (W x o n) . L~^T     (meas/rhf.py:27-33)
+//   exchange    f_g (o x o)    = L~_g G_half^T                 (meas/rhf.py:36-50)
+//   Taylor      T_k            = (i sqrt_dt / k) V_w T_{k-1}   (prop/utils.py:20-31)
+// and the adjoint's GEMMs.  GB300's binary64 pipe gives two FMAs a clock an
+// SM (1.2 TFLOP/s a GPU), the bf16 tensor cores 2 PFLOP/s: cutting both
+// operands into exact integer digits (the integer slicing of Ozaki, Ogita,
+// Oishi and Rump, 2012) costs 34 bf16 products a binary64 one and is still
+// tens of times faster.
+//
+// Digits.  Each operand row r (K contiguous) is scaled by a power of two E_r
+// above its largest entry and rounded to 55 bits: X = x 2^(7 - E_r) is
+// seven signed base-256 digits X = sum_s a_s 2^(-8 s), |a_s| <= 128, stored as
+// bf16 (a_s 2^(-8 s), exact).  A digit array is stored as the MMAs read it: for
+// each 32 k and digit a (rows x 64 bytes) plane with the 64-byte swizzle, so
+// that a tile is one contiguous bulk copy (tensor-map copies of 64-byte rows
+// moved 18-25 bytes a clock an SM) and rows past the end are never copied.  The product of two rows is
+// sum_{s,t} 2^(-8 (s + t)) sum_k a_s b_t; the pairs s + t <= 7 are kept.  What
+// is dropped is below the rounding to 55 bits (with s + t <= 6 it is eight
+// times that, and the error of a force bias passes the binary64 chain's).
+// Pairs of one s + t = d share a tensor-memory accumulator (d = 5, 6, 7 share
+// one): their sum is an integer multiple of 2^(-8 d), at most 2^14 (d + 1) of
+// them a product, which the fp32 accumulator holds exactly below 2^24, that is
+// for 256 products at d = 2, 3 and 512 at d = 0, 1, where it is drained.  d =
+// 4 and the last one (drained every 512) pass 2^24 only in sums of hundreds of
+// extremal digits of one sign; what truncation loses there is below 2^-45 of
+// such a sum's value and nothing otherwise.  The drained values are summed in
+// 64-bit integers (d <= 4; units of 2^-46 of the largest product, so that
+// 2^17 of them cannot overflow) and in fp32 (the last accumulator), and
+// converted once to binary64.  Rows holding inf or nan give nan.
+//
+// Kernel: persistent CTAs with 128 x 64 tiles, so that all six accumulators
+// stay in tensor memory and each digit tile is read once for its 34 products.
+// The digit tiles of a 32-k stage arrive as seven units (A_{6-j}, B_j) in the
+// order in which the rows of products A_s B_0 .. A_s B_{6-s}, s = 6 .. 0,
+// need them (s + t = 7 included); an A tile is released after its row, the B tiles after the
+// stage, so that copies run more than two stages ahead (two whole stages in
+// flight, released at once, waited on the copies: 120 clocks an MMA at a
+// V-build of 1000 x 40000 x 1024 walkers).  A row's MMAs keep A_s in the tensor
+// core's collector buffer: 35 clocks an MMA of 128 x 64 x 16 against 48 (the
+// operands' shared-memory reads), as issued from resident operands.
+#include "afq_internal.cuh"
+#include "tc_common.cuh"
+
+namespace afq {
+
+namespace {
+
+using namespace tc;
+
+constexpr int OZ_S = 7;                   // digits
+constexpr int OZ_ROWS = 128;              // real-operand rows a tile (tensor-memory lanes)
+constexpr int OZ_BK = 32;                 // K a stage: one 64-byte swizzle row
+constexpr int OZ_TN = 64;                 // complex-operand digit rows a tile
+constexpr int OZ_CHUNK = 8;               // stages (256 k) between drains of d = 2, 3 (16 for the others)
+constexpr int OZ_EW = 16;                 // epilogue warps
+constexpr int OZ_GT = 64 + 32 * OZ_EW;    // threads
+constexpr int OZ_CW = OZ_TN * 4 / OZ_EW;  // columns an epilogue thread
+constexpr int OZ_STG = 2;                 // stages in shared memory
+constexpr int OZ_A_SL = OZ_ROWS * OZ_BK * 2, OZ_B_SL = OZ_TN * OZ_BK * 2;
+constexpr int OZ_GSMEM = OZ_STG * OZ_S * (OZ_A_SL + OZ_B_SL) + 1024 + 512;
+// tensor-memory slot of an accumulator; d = 2 and 3 alternate between two
+enum { OZ_D5, OZ_D4, OZ_D1, OZ_D0, OZ_D3, OZ_D2 = 6, OZ_SLOTS = 8 };
+constexpr uint32_t OZ_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_TN >> 3) << 17) |
+                              ((uint32_t)(OZ_ROWS >> 4) << 24);
+static_assert(OZ_GSMEM <= 227 * 1024, "digit GEMM shared memory");
+constexpr int OZ_NAN = 0x7fffffff;        // scale of a row holding inf or nan
+
+__device__ __forceinline__ void oz_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"((unsigned long long)src), "r"(bytes), "r"(bar)
+                 : "memory");
+}
+
+// K-major tile of 64-byte rows, 64-byte swizzle: 8-row atoms 512 bytes apart.
+__device__ __forceinline__ uint64_t desc_k64(uint32_t saddr) {
+    uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(512 >> 4) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)4 << 61;
+    return d;
+}
+
+// (acc 2^-32 + tail) 2^ex in binary64, rounded to nearest even, by integer
+// operations (the binary64 pipe converts two a clock an SM): acc is shifted up
+// until it or the tail's last bits fill 62 bits, and the tail added there.
+__device__ __forceinline__ double oz_to_double(long long acc, float tail, int ex) {
+    const unsigned long long am = acc < 0 ? 0ull - (unsigned long long)acc : (unsigned long long)acc;
+    const int te = (int)((__float_as_uint(tail) >> 23) & 255u) - 127;  // |tail| < 2^(te + 1)
+    const int sh = min(am ? __clzll((long long)am) - 2 : 62, 29 - te);
+    const long long v = (long long)((unsigned long long)acc << sh) + __float2ll_rn(tail * __int_as_float((127 + 32 + sh) << 23));
+    const unsigned long long sign = (unsigned long long)v & 0x8000000000000000ull;
+    const unsigned long long mag = sign ? 0ull - (unsigned long long)v : (unsigned long long)v;
+    if (mag == 0) return 0.0;
+    const int lz = __clzll((long long)mag);
+    const unsigned long long nrm = mag << lz;
+    const unsigned long long m = (nrm >> 11) + (((nrm & 0x7ffull) + ((nrm >> 11) & 1ull)) > 0x400ull ? 1ull : 0ull);
+    const int e = 63 - lz + ex - 32 - sh + 1023;
+    if (e <= 0) return __longlong_as_double((long long)sign);
+    const unsigned long long bits = ((unsigned long long)(e - 1) << 52) + m;  // m carries its leading bit
+    if (e >= 2047) return __longlong_as_double((long long)(sign | 0x7ff0000000000000ull));
+    return __longlong_as_double((long long)(sign | bits));
+}
+
+// Where output (row r, complex column m) of batch b goes: C[b bs + (m / md)
+// ms1 + (m % md) ms0 + r rs], times 2^aexp, plus the same entry of add.
+struct OzOut {
+    double2* C;
+    long long bs, ms1, ms0, rs;
+    int md, aexp;
+    const double2* add;
+};
+
+struct OzArgs {
+    const uint8_t *da, *db;   // digit arrays of the real and the complex operand
+    int r8a, r8b;             // their plane rows
+    int rows, cols, K;        // cols: digit rows of the complex operand (re, im interleaved)
+    int batch, adiv;          // batch b takes real-operand plane b / adiv (adiv 0: the one plane)
+    int gn;                   // column tiles a group of the tile order
+    int splits, cps;          // K splits, 256-k chunks a split
+    const int *ea, *eb;       // row scales
+    long long* raw;           // splits > 1: integer sums (splits x cols x rows), and the tails
+    float* rawt;
+    int* err;
+    OzOut out;
+};
+
+__device__ __forceinline__ void oz_tile(const OzArgs& a, int t, int mt, int nt, int& z, int& mb, int& nb) {
+    z = t / (mt * nt);
+    const int r = t - z * (mt * nt), g = r / (a.gn * mt), rr = r - g * a.gn * mt, gs = min(a.gn, nt - g * a.gn);
+    mb = rr / gs;
+    nb = g * a.gn + rr % gs;
+}
+
+// One MMA, issued by the warp's elected lane (the whole warp calls, so that
+// descriptors stay warp-uniform).  H: 0 no collector hint, 1 A is read into
+// the collector, 2 used from it, 3 used for the last time.
+template <int H>
+__device__ __forceinline__ void oz_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t acc) {
+#define AFQ_OZ_MMA(HINT)                                                                                      \
+    asm volatile(                                                                                             \
+        "{\n\t.reg .pred p, q;\n\t"                                                                           \
+        "elect.sync _|q, 0xffffffff;\n\t"                                                                     \
+        "setp.ne.b32 p, %4, 0;\n\t"                                                                           \
+        "@q tcgen05.mma.cta_group::1.kind::f16" HINT " [%0], %1, %2, %3, p;\n\t}\n" ::"r"(d),                 \
+        "l"(a), "l"(b), "r"(OZ_IDESC), "r"(acc)                                                               \
+        : "memory")
+    if (H == 0) AFQ_OZ_MMA("");
+    else if (H == 1) AFQ_OZ_MMA(".collector::a::fill");
+    else if (H == 2) AFQ_OZ_MMA(".collector::a::use");
+    else AFQ_OZ_MMA(".collector::a::lastuse");
+#undef AFQ_OZ_MMA
+}
+__device__ __forceinline__ void oz_commit(uint32_t bar) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "elect.sync _|q, 0xffffffff;\n\t"
+        "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}\n" ::"r"(bar)
+        : "memory");
+}
+// accumulator slot of digit pairs s + t = d, `buf` the copy of d = 2, 3 in use
+__device__ __forceinline__ constexpr int oz_slot(int d, int buf) {
+    return d >= 5 ? OZ_D5 : d == 4 ? OZ_D4 : d == 1 ? OZ_D1 : d == 0 ? OZ_D0 : (d == 3 ? OZ_D3 : OZ_D2) + buf;
+}
+// products A_s B_0 .. A_s B_{min(6, 7-s)} of one k step; acc0 = 0: the row's new accumulator (d = s) begins
+template <int S>
+__device__ __forceinline__ void oz_row(uint32_t tmem, uint64_t ad, uint64_t bd, int buf, uint32_t acc0) {
+    constexpr int N = S == 0 ? OZ_S : OZ_S + 1 - S;
+#pragma unroll
+    for (int t = 0; t < N; ++t) {
+        const uint32_t d = tmem + oz_slot(S + t, buf) * OZ_TN;
+        const uint64_t b = bd + (uint64_t)((t * OZ_B_SL) >> 4);
+        const uint32_t acc = t == 0 ? acc0 : 1u;
+        if (t == 0) oz_mma<1>(d, ad, b, acc);
+        else if (t < N - 1) oz_mma<2>(d, ad, b, acc);
+        else oz_mma<3>(d, ad, b, acc);
+    }
+}
+
+// Wait of the MMA warp: expiry raises the CTA's abort flag and the error word,
+// and the warp carries on (its sums are lost, nothing is out of bounds), so
+// that the issue loop stays free of divergent exits and its descriptors in
+// uniform registers (recomputed ones cost 77 clocks an MMA).
+__device__ __noinline__ void oz_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err) {
+    if (!mbar_wait_inl(bar, parity, abort_flag)) {
+        atomicExch(err, 1);
+        *abort_flag = 1;
+    }
+}
+__device__ __forceinline__ void oz_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err) {
+    if (!mbar_try_wait(bar, parity)) oz_wait_slow(bar, parity, abort_flag, err);
+    __syncwarp();
+}
+
+// shared-memory offsets of the barriers (8 bytes each) after the tiles
+constexpr int OZ_BAR0 = OZ_STG * OZ_S * (OZ_A_SL + OZ_B_SL);
+enum {
+    OZB_FA = 0,                      // an A tile landed
+    OZB_FB = OZB_FA + OZ_STG * OZ_S, // a B tile landed
+    OZB_EA = OZB_FB + OZ_STG * OZ_S, // an A tile's row of MMAs finished
+    OZB_EB = OZB_EA + OZ_STG * OZ_S, // a stage's MMAs finished
+    OZB_TFS = OZB_EB + OZ_STG,       // the single accumulators hold their sums
+    OZB_TFD = OZB_TFS + 1,           // a copy of the double ones does
+    OZB_TE = OZB_TFD + 2,            // a slot has been drained
+    OZB_DRAIN = OZB_TE + OZ_SLOTS,
+    OZB_N = OZB_DRAIN + 1
+};
+static_assert(OZB_N * 8 + 8 <= 512, "barrier area");
+
+struct OzMmaState {
+    unsigned c, ns, nd;  // stages, drains of the single and of the double accumulators so far
+};
+// row S of the stage in buffer P
+template <int P, int S>
+__device__ __forceinline__ void oz_stage_row(uint32_t smem, uint32_t tmem, int k2, bool sd, bool ss, const OzMmaState& m,
+                                             int buf, volatile int* abort_flag, int* err) {
+    constexpr int J = OZ_S - 1 - S;
+    const uint32_t bars = smem + OZ_BAR0, par = (m.c >> 1) & 1;
+    // the row's last B tile: row 6 takes B_0 and B_1, every later one a further tile
+    if (S == 6) oz_wait(bars + 8 * (OZB_FB + P * OZ_S), par, abort_flag, err);
+    if (S > 0) oz_wait(bars + 8 * (OZB_FB + P * OZ_S + J + 1), par, abort_flag, err);
+    oz_wait(bars + 8 * (OZB_FA + P * OZ_S + J), par, abort_flag, err);
+    constexpr bool dbl = S == 2 || S == 3;
+    const bool st = S == 5 ? false : dbl ? sd : ss;
+    if (st) {
+        const uint32_t slot = dbl ? (S == 3 ? OZ_D3 : OZ_D2) + buf : oz_slot(S, 0);
+        oz_wait(bars + 8 * (OZB_TE + slot), ((dbl ? m.nd >> 1 : m.ns) & 1) ^ 1, abort_flag, err);
+    }
+    tc_fence_after();
+    const uint64_t ad = desc_k64(smem + (P * OZ_S + J) * OZ_A_SL);
+    const uint64_t bd = desc_k64(smem + OZ_STG * OZ_S * OZ_A_SL + P * OZ_S * OZ_B_SL);
+    oz_row<S>(tmem, ad, bd, buf, st ? 0u : 1u);
+    if (k2 > 1) oz_row<S>(tmem, ad + 2, bd + 2, buf, 1u);
+    oz_commit(bars + 8 * (OZB_EA + P * OZ_S + J));
+}
+template <int P>
+__device__ __forceinline__ void oz_stage(uint32_t smem, uint32_t tmem, int k2, bool sd, bool ss, const OzMmaState& m,
+                                         volatile int* abort_flag, int* err) {
+    const int buf = (int)(m.nd & 1);
+    oz_stage_row<P, 6>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<P, 5>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<P, 4>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<P, 3>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<P, 2>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<P, 1>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<P, 0>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_commit(smem + OZ_BAR0 + 8 * (OZB_EB + P));
+}
+
+__global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
+    extern __shared__ uint8_t smem_raw[];
+    const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
+    const uint32_t bars = smem + OZ_BAR0;
+    uint32_t* tmem_slot = (uint32_t*)(smem_raw + (bars + 8 * OZB_N - smem_u32(smem_raw)));
+    volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
+    const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
+    const int mt = (a.rows + OZ_ROWS - 1) / OZ_ROWS, nt = (a.cols + OZ_TN - 1) / OZ_TN;
+    const int ntiles = mt * nt * a.batch * a.splits, kst = (a.K + OZ_BK - 1) / OZ_BK;
+
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < OZB_N; ++i)  // one arrival an epilogue warp on a drained slot
+            mbar_init(bars + 8 * i, i >= OZB_TE && i < OZB_TE + OZ_SLOTS ? OZ_EW : 1);
+        *abort_flag = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+
+    if (warp == 0) {
+        if (lane == 0) {
+            unsigned c = 0;     // stages issued
+            bool ok = true;
+            for (int t = blockIdx.x; ok && t < ntiles; t += gridDim.x) {
+                int z, mb, nb;
+                oz_tile(a, t, mt, nt, z, mb, nb);
+                const int b = z / a.splits, sp = z - b * a.splits;
+                const int k0 = sp * a.cps * OZ_CHUNK, k1 = min(kst, k0 + a.cps * OZ_CHUNK);
+                const uint32_t ab = 64u * min(OZ_ROWS, a.r8a - mb * OZ_ROWS), bb = 64u * min(OZ_TN, a.r8b - nb * OZ_TN);
+                const long long pa = 64LL * a.r8a, pb = 64LL * a.r8b;  // plane bytes
+                const uint8_t* ga = a.da + ((long long)(a.adiv ? b / a.adiv : 0) * kst + k0) * OZ_S * pa + mb * OZ_ROWS * 64LL;
+                const uint8_t* gb = a.db + ((long long)(a.adiv ? b : 0) * kst + k0) * OZ_S * pb + nb * OZ_TN * 64LL;
+                for (int ks = k0; ks < k1; ++ks, ++c) {
+                    const uint32_t p = c & 1, par = ((c >> 1) & 1) ^ 1;
+                    // A_{6-j} as its row of two stages ago finishes, then the B tiles after that stage's end
+                    for (int j = 0; j < OZ_S; ++j) {
+                        const uint32_t i = p * OZ_S + j, fa = bars + 8 * (OZB_FA + i);
+                        if (!mbar_wait_inl(bars + 8 * (OZB_EA + i), par, abort_flag)) { ok = false; break; }
+                        mbar_expect_tx(fa, ab);
+                        oz_copy(smem + i * OZ_A_SL, ga + (OZ_S - 1 - j) * pa, ab, fa);
+                    }
+                    if (!ok || !mbar_wait_inl(bars + 8 * (OZB_EB + p), par, abort_flag)) { ok = false; break; }
+                    for (int j = 0; j < OZ_S; ++j) {
+                        const uint32_t i = p * OZ_S + j, fb = bars + 8 * (OZB_FB + i);
+                        mbar_expect_tx(fb, bb);
+                        oz_copy(smem + OZ_STG * OZ_S * OZ_A_SL + i * OZ_B_SL, gb + j * pb, bb, fb);
+                    }
+                    ga += OZ_S * pa;
+                    gb += OZ_S * pb;
+                }
+            }
+            if (!ok) {
+                atomicExch(a.err, 1);
+                *abort_flag = 1;
+            }
+            // every copy this thread issued lands before the CTA exits
+            if (ok) {
+                for (unsigned v = c > OZ_STG ? c - OZ_STG : 0; v < c; ++v)
+                    for (int j = 0; j < OZ_S; ++j) {
+                        mbar_wait(bars + 8 * (OZB_FA + (v & 1) * OZ_S + j), (v >> 1) & 1, nullptr);
+                        mbar_wait(bars + 8 * (OZB_FB + (v & 1) * OZ_S + j), (v >> 1) & 1, nullptr);
+                    }
+            } else {
+                const unsigned long long t0 = now_ns();  // copies in flight land within microseconds
+                while (now_ns() - t0 < 1000000ull) {}
+            }
+        }
+    } else if (warp == 1) {
+        OzMmaState m = {0, 0, 0};
+        for (int t = blockIdx.x; t < ntiles; t += gridDim.x) {
+            const int sp = (t / (mt * nt)) % a.splits;
+            const int k0 = sp * a.cps * OZ_CHUNK, n = min(kst, k0 + a.cps * OZ_CHUNK) - k0;
+            for (int i = 0; i < n; ++i, ++m.c) {
+                const bool sd = i % OZ_CHUNK == 0, ss = i % (2 * OZ_CHUNK) == 0;  // accumulators that begin here
+                const bool ed = i % OZ_CHUNK == OZ_CHUNK - 1 || i == n - 1;       // and that end
+                const bool es = i % (2 * OZ_CHUNK) == 2 * OZ_CHUNK - 1 || i == n - 1;
+                const int k2 = a.K - (k0 + i) * OZ_BK > 16 ? 2 : 1;
+                if (m.c & 1) oz_stage<1>(smem, tmem, k2, sd, ss, m, abort_flag, a.err);
+                else oz_stage<0>(smem, tmem, k2, sd, ss, m, abort_flag, a.err);
+                if (es) {
+                    oz_commit(bars + 8 * OZB_TFS);
+                    ++m.ns;
+                }
+                if (ed) {
+                    oz_commit(bars + 8 * (OZB_TFD + (m.nd & 1)));
+                    ++m.nd;
+                }
+            }
+        }
+        // every MMA issued finishes before the tensor memory is freed
+        oz_commit(bars + 8 * OZB_DRAIN);
+        mbar_wait(bars + 8 * OZB_DRAIN, 0, nullptr);
+    } else {
+        const int q = warp & 3, cb = ((warp - 2) >> 2) * OZ_CW;
+        unsigned ns = 0, nd = 0;
+        bool ok = true;
+        for (int t = blockIdx.x; ok && t < ntiles; t += gridDim.x) {
+            int z, mb, nb;
+            oz_tile(a, t, mt, nt, z, mb, nb);
+            const int b = z / a.splits, sp = z - b * a.splits;
+            const int k0 = sp * a.cps * OZ_CHUNK, ni = min(kst, k0 + a.cps * OZ_CHUNK) - k0;
+            const int row = mb * OZ_ROWS + 32 * q + lane, c0 = nb * OZ_TN + cb;
+            long long acc[OZ_CW];
+#pragma unroll
+            for (int j = 0; j < OZ_CW; ++j) acc[j] = 0;
+            float tail[OZ_CW];
+#pragma unroll
+            for (int j = 0; j < OZ_CW; ++j) tail[j] = 0.f;
+            // D_d 2^(-8 d), an integer multiple of 2^(-8 d) for d <= 4, into 2^-32 units; the last accumulator is summed
+            // in fp32 (its value is below 2^-22 of a sum's largest terms, its rounding below 2^-59 of the largest product)
+            auto take = [&](int d, int slot) {
+                const float sc = __int_as_float((127 + 8 * d) << 23);
+                uint32_t r[OZ_CW];
+                tmem_ld16(tmem + slot * OZ_TN + cb + ((uint32_t)(32 * q) << 16), r);
+#pragma unroll
+                for (int j = 0; j < OZ_CW; ++j) {
+                    const float x = __uint_as_float(r[j]);
+                    if (d == 5) tail[j] += x;
+                    else acc[j] += (long long)((unsigned long long)(long long)__float2int_rn(x * sc) << (32 - 8 * d));
+                }
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(bars + 8 * (OZB_TE + slot));
+            };
+            for (int i = OZ_CHUNK; ok; i += OZ_CHUNK) {
+                const bool end = i >= ni;
+                if (end || i % (2 * OZ_CHUNK) == 0) {
+                    if (!mbar_wait_inl(bars + 8 * OZB_TFS, ns & 1, abort_flag)) { ok = false; break; }
+                    tc_fence_after();
+                    take(5, OZ_D5);
+                    take(4, OZ_D4);
+                    take(1, OZ_D1);
+                    take(0, OZ_D0);
+                    ++ns;
+                }
+                if (!mbar_wait_inl(bars + 8 * (OZB_TFD + (nd & 1)), (nd >> 1) & 1, abort_flag)) { ok = false; break; }
+                tc_fence_after();
+                take(3, OZ_D3 + (int)(nd & 1));
+                take(2, OZ_D2 + (int)(nd & 1));
+                ++nd;
+                if (end) break;
+            }
+            if (!ok) {
+                atomicExch(a.err, 1);
+                *abort_flag = 1;
+                break;
+            }
+            if (row >= a.rows) continue;
+            if (a.splits > 1) {
+                const long long at = (long long)sp * a.cols * a.rows + row;
+#pragma unroll
+                for (int j = 0; j < OZ_CW; ++j)
+                    if (c0 + j < a.cols) {
+                        a.raw[at + (long long)(c0 + j) * a.rows] = acc[j];
+                        a.rawt[at + (long long)(c0 + j) * a.rows] = tail[j];
+                    }
+                continue;
+            }
+            const int* eb = a.eb + (a.adiv ? (long long)b * a.cols : 0) + c0;
+            const int ea = a.ea[(a.adiv ? b / a.adiv * a.rows : 0) + row];
+            const long long at = (long long)b * a.out.bs + (long long)row * a.out.rs;
+            const int ex = ea - 14 + a.out.aexp;
+#pragma unroll
+            for (int j = 0; j < OZ_CW; j += 2) {
+                if (c0 + j < a.cols) {
+                    const int e0 = eb[j], e1 = eb[j + 1], m = (c0 + j) >> 1;
+                    double2 v = make_double2(oz_to_double(acc[j], tail[j], ex + e0),
+                                             oz_to_double(acc[j + 1], tail[j + 1], ex + e1));
+                    if (ea == OZ_NAN || e0 == OZ_NAN) v.x = __longlong_as_double(0x7ff8000000000000ll);
+                    if (ea == OZ_NAN || e1 == OZ_NAN) v.y = __longlong_as_double(0x7ff8000000000000ll);
+                    const int mh = a.out.md == 1 ? m : m / a.out.md;
+                    const long long e = at + (long long)mh * a.out.ms1 + (long long)(m - mh * a.out.md) * a.out.ms0;
+                    if (a.out.add) v = cadd(v, a.out.add[e]);
+                    a.out.C[e] = v;
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        __syncwarp();
+        tc_fence_after();
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+    }
+}
+
+// The K splits' sums added (the integers exactly, the tails in order) and converted.
+__global__ void k_oz_finish(const OzArgs a) {
+    const long long total = (long long)a.rows * (a.cols >> 1);
+    for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
+         e += (long long)gridDim.x * blockDim.x) {
+        const int m = (int)(e / a.rows), row = (int)(e - (long long)m * a.rows);
+        long long re = 0, im = 0;
+        float tr = 0.f, ti = 0.f;
+        for (int z = 0; z < a.splits; ++z) {
+            const long long at = ((long long)z * a.cols + 2 * m) * a.rows + row;
+            re += a.raw[at];
+            im += a.raw[at + a.rows];
+            tr += a.rawt[at];
+            ti += a.rawt[at + a.rows];
+        }
+        const int ea = a.ea[row], e0 = a.eb[2 * m], e1 = a.eb[2 * m + 1], ex = ea - 14 + a.out.aexp;
+        double2 v = make_double2(oz_to_double(re, tr, ex + e0), oz_to_double(im, ti, ex + e1));
+        if (ea == OZ_NAN || e0 == OZ_NAN) v.x = __longlong_as_double(0x7ff8000000000000ll);
+        if (ea == OZ_NAN || e1 == OZ_NAN) v.y = __longlong_as_double(0x7ff8000000000000ll);
+        const int mh = m / a.out.md;
+        const long long at = (long long)row * a.out.rs + (long long)mh * a.out.ms1 + (long long)(m - mh * a.out.md) * a.out.ms0;
+        if (a.out.add) v = cadd(v, a.out.add[at]);
+        a.out.C[at] = v;
+    }
+}
+
+// ------------------------------------------------------------------ digits --
+__device__ __forceinline__ int oz_expo(double x) {  // biased binary64 exponent
+    return (int)(((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ffu);
+}
+// scale of a row whose largest biased exponent is eb: |x| < 2^E
+__device__ __forceinline__ int oz_scale(int eb) { return eb == 0x7ff ? OZ_NAN : eb - 1022; }
+
+// x 2^(55 - E) rounded to an integer, |.| <= 2^55, plus 0x808080808080, whose
+// low six bytes are then the lower digits plus 128 (zero for subnormal x and
+// in a row of scale OZ_NAN).
+__device__ __forceinline__ long long oz_fix(double x, int E) {
+    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
+    const int eb = (int)((u >> 52) & 0x7ffu);
+    long long y = 0;
+    if (eb != 0 && E != OZ_NAN) {
+        const unsigned long long m = (u & 0xfffffffffffffull) | (1ull << 52);
+        const int r = E + 1020 - eb;  // right shift, >= -2
+        if (r <= 0) y = (long long)(m << (-r));
+        else if (r < 60) y = (long long)((m + (1ull << (r - 1))) >> r);
+        if ((long long)u < 0) y = -y;
+    }
+    return y + 0x0000808080808080ll;
+}
+// digit s of y (from oz_fix) times 2^(-8 s), exact in fp32 and bf16
+template <int S>
+__device__ __forceinline__ float oz_dig(long long y) {
+    constexpr float sc = 1.0f / (float)(1ull << (8 * S));
+    if (S == 0) {  // the top digit, in [-128, 128]
+        const uint32_t t = (uint32_t)((int)(y >> 48) + 256);
+        return __uint_as_float(0x4B000000u | t) - 8388864.f;
+    }
+    const uint32_t t = (uint32_t)((unsigned long long)y >> (48 - 8 * S)) & 255u;
+    return fmaf(__uint_as_float(0x4B000000u | t), sc, -8388736.f * sc);
+}
+__device__ __forceinline__ uint32_t oz_pack(float lo, float hi) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *(const uint32_t*)&v;
+}
+template <int S>
+__device__ __forceinline__ uint4 oz_pack8(const long long (&y)[8]) {
+    return make_uint4(oz_pack(oz_dig<S>(y[0]), oz_dig<S>(y[1])), oz_pack(oz_dig<S>(y[2]), oz_dig<S>(y[3])),
+                      oz_pack(oz_dig<S>(y[4]), oz_dig<S>(y[5])), oz_pack(oz_dig<S>(y[6]), oz_dig<S>(y[7])));
+}
+// A digit array: [batch][32 k][digit] planes of r8 rows x 64 bytes.
+struct OzDst {
+    uint8_t* d;
+    int nks, r8;
+};
+// eight consecutive k (k a multiple of 8) of row r of batch b into the seven planes
+__device__ __forceinline__ void oz_store8(const OzDst& o, long long b, int r, int k, const long long (&y)[8]) {
+    const long long plane = 64LL * o.r8;
+    uint8_t* d = o.d + (b * o.nks + (k >> 5)) * OZ_S * plane + r * 64LL + ((((k >> 3) ^ (r >> 1)) & 3) << 4);
+    *(uint4*)(d) = oz_pack8<0>(y);
+    *(uint4*)(d + plane) = oz_pack8<1>(y);
+    *(uint4*)(d + 2 * plane) = oz_pack8<2>(y);
+    *(uint4*)(d + 3 * plane) = oz_pack8<3>(y);
+    *(uint4*)(d + 4 * plane) = oz_pack8<4>(y);
+    *(uint4*)(d + 5 * plane) = oz_pack8<5>(y);
+    *(uint4*)(d + 6 * plane) = oz_pack8<6>(y);
+}
+__device__ __forceinline__ int warp_max(int v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
+    return v;
+}
+
+// Real rows with K contiguous (row r at src + r ld), one warp a row; `per`
+// rows a batch; one: minus the identity.  Every split writes zeros from K up
+// to a multiple of 32.
+__global__ void __launch_bounds__(256) k_oz_rows(long long rows, int per, int K, const double* __restrict__ src,
+                                                 long long ld, int one, OzDst dst, int* __restrict__ ex) {
+    const int lane = threadIdx.x & 31;
+    for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * 8) {
+        const double* x = src + r * ld;
+        const long long rd = one ? r : -1;  // the diagonal entry to lower by one
+        int e = 0;
+        for (int k = lane; k < K; k += 32) e = max(e, oz_expo(k == rd ? x[k] - 1.0 : x[k]));
+        const int E = oz_scale(warp_max(e));
+        if (lane == 0) ex[r] = E;
+        const long long b = r / per;
+        for (int k = 8 * lane; k < 32 * dst.nks; k += 256) {
+            long long y[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] = oz_fix(k + i < K ? (k + i == rd ? x[k + i] - 1.0 : x[k + i]) : 0.0, E);
+            oz_store8(dst, b, (int)(r - b * per), k, y);
+        }
+    }
+}
+
+// Complex rows with K contiguous: digit rows 2 r (real parts) and 2 r + 1.
+__global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const double2* __restrict__ src, long long ld,
+                                                  OzDst dst, int* __restrict__ ex) {
+    const int lane = threadIdx.x & 31;
+    for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * 8) {
+        const double2* x = src + r * ld;
+        int e0 = 0, e1 = 0;
+        for (int k = lane; k < K; k += 32) {
+            const double2 v = x[k];
+            e0 = max(e0, oz_expo(v.x));
+            e1 = max(e1, oz_expo(v.y));
+        }
+        const int E0 = oz_scale(warp_max(e0)), E1 = oz_scale(warp_max(e1));
+        if (lane == 0) {
+            ex[2 * r] = E0;
+            ex[2 * r + 1] = E1;
+        }
+        for (int k = 8 * lane; k < 32 * dst.nks; k += 256) {
+            long long y[8], w[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const double2 v = k + i < K ? x[k + i] : make_double2(0.0, 0.0);
+                y[i] = oz_fix(v.x, E0);
+                w[i] = oz_fix(v.y, E1);
+            }
+            oz_store8(dst, 0, (int)(2 * r), k, y);
+            oz_store8(dst, 0, (int)(2 * r + 1), k, w);
+        }
+    }
+}
+
+// Real rows with K strided: row r's entry k at src[k ld + r]; 32 rows a CTA,
+// transposed through shared memory.
+__global__ void __launch_bounds__(256) k_oz_cols(int rows, int K, const double* __restrict__ src, long long ld,
+                                                 OzDst dst, int* __restrict__ ex) {
+    __shared__ double tile[32][65];
+    __shared__ int se[32];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, r0 = blockIdx.x * 32;
+    const bool in = r0 + tx < rows;
+    if (threadIdx.x < 32) se[threadIdx.x] = 0;
+    __syncthreads();
+    int e = 0;
+    if (in) {
+#pragma unroll 4
+        for (int k = ty; k < K; k += 8) e = max(e, oz_expo(src[(long long)k * ld + r0 + tx]));
+    }
+    atomicMax(&se[tx], e);
+    __syncthreads();
+    const int rr = threadIdx.x >> 3, kq = (threadIdx.x & 7) * 8, E = oz_scale(se[rr]);
+    if ((threadIdx.x & 7) == 0 && r0 + rr < rows) ex[r0 + rr] = E;
+    for (int k0 = 0; k0 < 32 * dst.nks; k0 += 64) {
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int k = k0 + ty + 8 * i;
+            tile[tx][ty + 8 * i] = in && k < K ? src[(long long)k * ld + r0 + tx] : 0.0;
+        }
+        __syncthreads();
+        if (r0 + rr < rows && k0 + kq < 32 * dst.nks) {
+            long long y[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) y[i] = oz_fix(tile[rr][kq + i], E);
+            oz_store8(dst, 0, r0 + rr, k0 + kq, y);
+        }
+    }
+}
+
+// Walker-shaped blocks (w, j, c), c fastest, eight columns c a CTA:
+//   WALK  digits of the block's columns over j, rows (w, c, part)
+//   INIT  T = W + Y; U = T; digits of T as the right operand of V T
+//   TERM  T = i s Y; U += T; digits of T as the right operand of V T
+//   LAST  T = i s Y; U += T; digits of U as WALK's
+// The right operand of V T (V's rows hold Re, Im interleaved): rows (c, Re)
+// [Tr, -Ti] and (c, Im) [Ti, Tr] over (j, part), a batch a walker.
+enum { OZ_WALK, OZ_INIT, OZ_TERM, OZ_LAST };
+constexpr int OZ_CB = 8;
+template <int MODE>
+__global__ void __launch_bounds__(256) k_oz_term(int n, int o, int ncg, double s, const double2* __restrict__ Y,
+                                                 const double2* __restrict__ W, double2* __restrict__ U, OzDst dst, int* __restrict__ ex) {
+    extern __shared__ double2 sh[];  // OZ_CB x (n + 1)
+    __shared__ int se[2 * OZ_CB];
+    const int w = blockIdx.x / ncg, c0 = (blockIdx.x - w * ncg) * OZ_CB, tid = threadIdx.x;
+    const int c = tid & (OZ_CB - 1), pitch = n + 1;
+    if (tid < 2 * OZ_CB) se[tid] = 0;
+    __syncthreads();
+    int e0 = 0, e1 = 0;
+    if (c0 + c < o) {
+        for (int j = tid / OZ_CB; j < n; j += 256 / OZ_CB) {
+            const long long at = ((long long)w * n + j) * o + c0 + c;
+            double2 t = Y[at];
+            if (MODE == OZ_TERM || MODE == OZ_LAST) {
+                t = make_double2(-s * t.y, s * t.x);
+                const double2 u = cadd(U[at], t);
+                U[at] = u;
+                if (MODE == OZ_LAST) t = u;
+            }
+            if (MODE == OZ_INIT) U[at] = t = cadd(W[at], t);
+            sh[c * pitch + j] = t;
+            e0 = max(e0, oz_expo(t.x));
+            e1 = max(e1, oz_expo(t.y));
+        }
+    }
+    atomicMax(&se[2 * c], e0);
+    atomicMax(&se[2 * c + 1], e1);
+    __syncthreads();
+    const int cn = min(OZ_CB, o - c0);
+    if (MODE == OZ_WALK || MODE == OZ_LAST) {
+        const int nq = 4 * dst.nks;
+        for (int it = tid; it < cn * nq; it += 256) {
+            const int cc = it / nq, j = (it - cc * nq) * 8;
+            const int E0 = oz_scale(se[2 * cc]), E1 = oz_scale(se[2 * cc + 1]);
+            long long y[8], x[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const double2 t = j + i < n ? sh[cc * pitch + j + i] : make_double2(0.0, 0.0);
+                y[i] = oz_fix(t.x, E0);
+                x[i] = oz_fix(t.y, E1);
+            }
+            const int row = 2 * (w * o + c0 + cc);
+            oz_store8(dst, 0, row, j, y);
+            oz_store8(dst, 0, row + 1, j, x);
+            if (j == 0) {
+                ex[row] = E0;
+                ex[row + 1] = E1;
+            }
+        }
+    } else {
+        const int nq = 4 * dst.nks;
+        for (int it = tid; it < cn * nq; it += 256) {
+            const int cc = it / nq, j = (it - cc * nq) * 4;
+            const int E = oz_scale(max(se[2 * cc], se[2 * cc + 1]));
+            long long y[8], x[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const double2 t = j + i < n ? sh[cc * pitch + j + i] : make_double2(0.0, 0.0);
+                y[2 * i] = oz_fix(t.x, E);
+                y[2 * i + 1] = oz_fix(-t.y, E);
+                x[2 * i] = oz_fix(t.y, E);
+                x[2 * i + 1] = y[2 * i];
+            }
+            const int row = 2 * (c0 + cc);
+            oz_store8(dst, w, row, 2 * j, y);
+            oz_store8(dst, w, row + 1, 2 * j, x);
+            if (j == 0) {
+                ex[(long long)w * 2 * o + row] = E;
+                ex[(long long)w * 2 * o + row + 1] = E;
+            }
+        }
+    }
+}
+
+// Coulomb and exchange partials of a chunk of ng Cholesky vectors from F
+// (rows (w, k), columns (g, i): f_g[i, k]), as launch_energy_partial's:
+// partial[w, chunk] = (sum_g (tr f_g)^2, sum_g sum_ik f_g[i, k] f_g[k, i]).
+__global__ void __launch_bounds__(256) k_oz_exchange(int o, int G, int NG, const double2* __restrict__ F,
+                                                     double2* __restrict__ partial) {
+    extern __shared__ double2 sh[];  // NG blocks of o x (o + 1)
+    const int nchunk = gridDim.x, w = blockIdx.y, g0 = blockIdx.x * NG, ng = min(NG, G - g0), tid = threadIdx.x;
+    const int pitch = o + 1, gi = ng * o;
+    const double2* Fw = F + (long long)w * o * G * o + (long long)g0 * o;
+    for (int e = tid; e < gi * o; e += 256) {
+        const int k = e / gi, x = e - k * gi, g = x / o, i = x - g * o;
+        sh[(g * o + k) * pitch + i] = Fw[(long long)k * G * o + x];
+    }
+    __syncthreads();
+    double cr = 0.0, ci = 0.0, xr = 0.0, xi = 0.0;
+    // f[i, k] f[k, i] once for i < k, doubled; the diagonal's squares
+    for (int e = tid; e < gi * o; e += 256) {
+        const int g = e / (o * o), rem = e - g * o * o, k = rem / o, i = rem - k * o;
+        if (i > k) continue;
+        const double2 p = cmul(sh[(g * o + k) * pitch + i], sh[(g * o + i) * pitch + k]);
+        const double f = i == k ? 1.0 : 2.0;
+        xr = fma(f, p.x, xr);
+        xi = fma(f, p.y, xi);
+    }
+    for (int g = tid; g < ng; g += 256) {
+        double2 c = make_double2(0.0, 0.0);
+        for (int i = 0; i < o; ++i) c = cadd(c, sh[(g * o + i) * pitch + i]);
+        const double2 c2 = cmul(c, c);
+        cr += c2.x;
+        ci += c2.y;
+    }
+    cr = warp_sum(cr); ci = warp_sum(ci); xr = warp_sum(xr); xi = warp_sum(xi);
+    __shared__ double red[8][4];
+    const int lane = tid & 31, wid = tid >> 5;
+    if (lane == 0) {
+        red[wid][0] = cr; red[wid][1] = ci; red[wid][2] = xr; red[wid][3] = xi;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        for (int i = 1; i < 8; ++i) {
+            cr += red[i][0]; ci += red[i][1]; xr += red[i][2]; xi += red[i][3];
+        }
+        partial[((size_t)w * nchunk + blockIdx.x) * 2] = make_double2(cr, ci);
+        partial[((size_t)w * nchunk + blockIdx.x) * 2 + 1] = make_double2(xr, xi);
+    }
+}
+
+constexpr int OZ_XSMEM = 96 * 1024;  // the exchange kernel's F blocks
+DeviceOnce g_oz, g_ozterm[4], g_ozx;
+
+int nks_of(int K) { return (K + OZ_BK - 1) / OZ_BK; }
+long long digit_row_bytes(int K) { return 64LL * OZ_S * nks_of(K); }
+
+// Digit arrays of one operand.
+struct OzDigits {
+    uint8_t* d;
+    int* ex;
+};
+
+// K splits (and 256-k chunks a split) so that few tiles still fill the GPU.
+void oz_splits(long long tiles, int K, int sms, int& splits, int& cps) {
+    const int nch = (K + OZ_BK * OZ_CHUNK - 1) / (OZ_BK * OZ_CHUNK);
+    int z = (int)(sms / (tiles > 0 ? tiles : 1));
+    if (z > nch) z = nch;
+    if (z < 1) z = 1;
+    cps = (nch + z - 1) / z;
+    splits = (nch + cps - 1) / cps;
+}
+
+int oz_launch(int rows, int cols, int K, int batch, int adiv, const OzDigits& A, const OzDigits& B, const OzOut& out,
+              int splits, int cps, long long* raw, int* err, cudaStream_t s) {
+    OzArgs a = {};
+    a.da = A.d; a.db = B.d;
+    a.r8a = (int)round_up(rows, 8); a.r8b = (int)round_up(cols, 8);
+    a.rows = rows; a.cols = cols; a.K = K; a.batch = batch; a.adiv = adiv;
+    a.splits = splits; a.cps = cps;
+    a.ea = A.ex; a.eb = B.ex; a.raw = raw; a.err = err; a.out = out;
+    a.rawt = (float*)(raw + (long long)splits * cols * rows);
+    const int mt = (rows + OZ_ROWS - 1) / OZ_ROWS, nt = (cols + OZ_TN - 1) / OZ_TN;
+    // column tiles fastest in groups whose digits take at most 40 MB of L2
+    const long long tb = OZ_TN * digit_row_bytes(K);
+    long long gn = (40LL << 20) / (tb > 0 ? tb : 1);
+    if (gn < 1) gn = 1;
+    if (gn > nt) gn = nt;
+    a.gn = (int)gn;
+    int sms = 0;
+    AFQ_TRY(device_sms(&sms));
+    const long long tiles = (long long)mt * nt * batch * splits;
+    if (tiles > 0x7fffffffLL) return fail(AFQ_E_UNSUPPORTED, "digit GEMM: %lld tiles", tiles);
+    const int grid = tiles < sms ? (int)tiles : sms;
+    AFQ_TRY(raise_smem_once(g_oz, k_ozgemm, OZ_GSMEM));
+    k_ozgemm<<<grid, OZ_GT, OZ_GSMEM, s>>>(a);
+    AFQ_LAUNCHED("k_ozgemm");
+    if (splits > 1) {
+        long long blocks = ((long long)rows * (cols >> 1) + 255) / 256;
+        if (blocks > 152 * 16) blocks = 152 * 16;
+        k_oz_finish<<<(unsigned)blocks, 256, 0, s>>>(a);
+        AFQ_LAUNCHED("k_oz_finish");
+    }
+    return AFQ_OK;
+}
+
+OzDst dst_of(const OzDigits& D, long long rows, int K) { return {D.d, nks_of(K), (int)round_up(rows, 8)}; }
+
+unsigned row_blocks(long long rows) {
+    const long long b = (rows + 7) / 8;
+    return (unsigned)(b > 152 * 64 ? 152 * 64 : b);
+}
+int split_rows(long long rows, int per, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s,
+               int one = 0) {
+    k_oz_rows<<<row_blocks(rows), 256, 0, s>>>(rows, per, K, src, ld, one, dst_of(D, per, K), D.ex);
+    AFQ_LAUNCHED("k_oz_rows");
+    return AFQ_OK;
+}
+int split_crows(long long rows, int K, const double2* src, long long ld, const OzDigits& D, cudaStream_t s) {
+    k_oz_crows<<<row_blocks(rows), 256, 0, s>>>(rows, K, src, ld, dst_of(D, 2 * rows, K), D.ex);
+    AFQ_LAUNCHED("k_oz_crows");
+    return AFQ_OK;
+}
+int split_cols(int rows, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s) {
+    k_oz_cols<<<(rows + 31) / 32, 256, 0, s>>>(rows, K, src, ld, dst_of(D, rows, K), D.ex);
+    AFQ_LAUNCHED("k_oz_cols");
+    return AFQ_OK;
+}
+OzDigits take_digits(Arena& a, size_t rows, int K, size_t batch = 1) {
+    OzDigits D;
+    D.d = a.take<uint8_t>(batch * round_up(rows, 8) * digit_row_bytes(K));
+    D.ex = a.take<int>(batch * rows);
+    return D;
+}
+
+// Digit scratch is bounded: operands whose digits take more than this are
+// processed in row chunks.
+constexpr long long OZ_CAP = 1LL << 30;
+int cap_rows(long long rows, long long bytes_per_row) {
+    long long c = OZ_CAP / (bytes_per_row > 0 ? bytes_per_row : 1) / OZ_ROWS * OZ_ROWS;
+    if (c < OZ_ROWS) c = OZ_ROWS;
+    return (int)(c < rows ? c : rows);
+}
+
+constexpr int OZ_TILE_SMS = 152;
+
+struct ZLayout {
+    int mc, nc;
+    OzDigits A, B;
+    long long* raw;
+};
+ZLayout z_layout(Arena& a, int M, int N, int K) {
+    ZLayout z;
+    const long long rb = digit_row_bytes(K);
+    z.mc = cap_rows(M, 2 * rb);
+    z.nc = cap_rows(N, rb);
+    z.A = take_digits(a, z.nc, K);
+    z.B = take_digits(a, 2 * (size_t)z.mc, K);
+    // K splits: at most one tile an SM, at most one split a 256-k chunk
+    const size_t nch = (K + 255) / 256, most = (size_t)OZ_TILE_SMS * OZ_ROWS * OZ_TN, all = nch * 2 * z.mc * z.nc;
+    z.raw = a.take<long long>((nch > 1 ? (all < most ? all : most) : 0) * 3 / 2);  // 64-bit sums, 32-bit tails
+    return z;
+}
+
+}  // namespace
+
+// Routes.  The binary64 kernels' own limits stay (a call past them is theirs
+// to refuse).  Measured in captured graphs, binary64 pipe -> digits:
+//   GEMM     wins from the smallest (M x N x K 5 x 7 x 1: 36 -> 21 us with launches; 64 x 144 x 48: 103 -> 28;
+//            1024 x 600 x 2400: 9.6 -> 0.32 ms; 1024 x 1000 x 6000: 24 -> 0.78 ms).
+//   Taylor   ~16 launches of 6-10 us at least: n = 45, o = 9: 191 -> 140 us at 8 walkers, 4797 -> 1159 at 2048;
+//            n = 30: o = 7 66 -> 123 at 8, 237 -> 262 at 512 walkers, o = 10 179 -> 170 at 200, 411 -> 311 at 512;
+//            the binary64 kernel takes 32 orbitals a pass and eight columns a CTA.
+//   energy   n = 8, o = 2, 40 vectors: 12 -> 24 us at 200 walkers, 64 -> 55 at 2048; n = 12, o = 6, 60 vectors: 27 ->
+//            29 at 8, 51 -> 34 at 200; n = 20, o = 5, 100 vectors: 41 -> 30 at 8, 547 -> 185 at 2048.
+bool zgemm_oz_pays(int M, int N, int K) { return M > 0 && N > 0 && K >= 1 && K <= 1 << 17 && M <= 65535 * 64; }
+bool trotter_oz_pays(int W, int n, int o, int n_terms) {
+    return W <= 65535 && n <= 512 && n_terms >= 1 && (n > 32 || (n >= 24 && o > 8 && W > 256));
+}
+bool energy_oz_pays(int W, int n, int o, int G) {
+    const int nchunk = energy_partial_chunks(o, G), ng = (G + nchunk - 1) / nchunk;
+    return W <= 65535 && energy_partial_fits(o, G, 1) && ng * o * (o + 1) * (int)sizeof(double2) <= OZ_XSMEM &&
+           (n >= 16 || (double)W * G * o * o * n >= 1 << 20);
+}
+
+size_t zgemm_oz_scratch(int M, int N, int K) {
+    Arena a;
+    z_layout(a, M, N, K);
+    return a.used + 256;
+}
+
+int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
+                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s) {
+    if (M <= 0 || N <= 0) return AFQ_OK;
+    int ae = 0;
+    if (frexp(alpha, &ae) != 0.5) return fail(AFQ_E_UNSUPPORTED, "digit GEMM: alpha=%g is no power of two", alpha);
+    Arena ar(scratch, (size_t)-1);
+    const ZLayout z = z_layout(ar, M, N, K);
+    int sms = 0;
+    AFQ_TRY(device_sms(&sms));
+    for (int m0 = 0; m0 < M; m0 += z.mc) {
+        const int mc = M - m0 < z.mc ? M - m0 : z.mc;
+        AFQ_TRY(split_crows(mc, K, A + (int64_t)m0 * lda, lda, z.B, s));
+        for (int n0 = 0; n0 < N; n0 += z.nc) {
+            const int nc = N - n0 < z.nc ? N - n0 : z.nc;
+            if (b_trans) AFQ_TRY(split_rows(nc, nc, K, B + (int64_t)n0 * ldb, ldb, z.A, s));
+            else AFQ_TRY(split_cols(nc, K, B + n0, ldb, z.A, s));
+            const OzOut out = {C + (int64_t)m0 * ldc + n0, 0, ldc, 0, 1, 1, ae - 1, nullptr};
+            const long long tiles = (long long)((nc + OZ_ROWS - 1) / OZ_ROWS) * ((2 * mc + OZ_TN - 1) / OZ_TN);
+            int splits, cps;
+            oz_splits(tiles, K, sms < OZ_TILE_SMS ? sms : OZ_TILE_SMS, splits, cps);
+            AFQ_TRY(oz_launch(nc, 2 * mc, K, 1, 0, z.A, z.B, out, splits, cps, z.raw, err, s));
+        }
+    }
+    return AFQ_OK;
+}
+
+// ---------------------------------------------------------------- Taylor --
+namespace {
+struct TrLayout {
+    int wc;
+    OzDigits E, V, T, X;  // E_half, V rows, right operands of V T, walker columns
+    double2 *Y, *U;
+};
+TrLayout tr_layout(Arena& a, int W, int n, int o, int vdiv) {
+    TrLayout t;
+    const long long per = round_up(n, 8) * digit_row_bytes(2 * n);  // digits of one V
+    long long wc = OZ_CAP / per / vdiv * vdiv * vdiv;               // walkers whose V digits fit
+    if (wc < vdiv) wc = vdiv;
+    if (wc > W) wc = W;
+    t.wc = (int)wc;
+    t.E = take_digits(a, n, n);
+    t.V = take_digits(a, n, 2 * n, (t.wc + vdiv - 1) / vdiv);
+    t.T = take_digits(a, 2 * o, 2 * n, t.wc);
+    t.X = take_digits(a, (size_t)t.wc * 2 * o, n);
+    t.Y = a.take<double2>((size_t)t.wc * n * o);
+    t.U = a.take<double2>((size_t)t.wc * n * o);
+    return t;
+}
+template <int MODE>
+int launch_term(int W, int n, int o, double s, const double2* Y, const double2* X, double2* U, const OzDigits& D,
+                cudaStream_t st) {
+    const int ncg = (o + OZ_CB - 1) / OZ_CB, smem = OZ_CB * (n + 1) * (int)sizeof(double2);
+    AFQ_TRY(raise_smem_once(g_ozterm[MODE], k_oz_term<MODE>, OZ_CB * 513 * (int)sizeof(double2)));
+    const OzDst dst = MODE == OZ_WALK || MODE == OZ_LAST ? dst_of(D, 2LL * W * o, n) : dst_of(D, 2 * o, 2 * n);
+    k_oz_term<MODE><<<(unsigned)W * ncg, 256, smem, st>>>(n, o, ncg, s, Y, X, U, dst, D.ex);
+    AFQ_LAUNCHED("k_oz_term");
+    return AFQ_OK;
+}
+}  // namespace
+
+size_t trotter_oz_scratch(int W, int n, int o, int vdiv) {
+    Arena a;
+    tr_layout(a, W, n, o, vdiv);
+    return a.used + 256;
+}
+
+// E_half . sum_{k <= K} (i sqrt_dt V)^k / k! . E_half . W, n_terms >= 1.
+// E_half X is formed as X + (E_half - I) X: E_half is close to the identity,
+// and a digit product's error scales with its operands' largest entries.
+int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
+                      const double2* win, double2* wout, int vdiv, void* scratch, int* err, cudaStream_t s) {
+    if (W <= 0) return AFQ_OK;
+    Arena ar(scratch, (size_t)-1);
+    const TrLayout t = tr_layout(ar, W, n, o, vdiv);
+    AFQ_TRY(split_rows(n, n, n, E, n, t.E, s, 1));
+    const size_t no = (size_t)n * o;
+    for (int w0 = 0; w0 < W; w0 += t.wc) {
+        const int wc = W - w0 < t.wc ? W - w0 : t.wc, nv = (wc + vdiv - 1) / vdiv;
+        AFQ_TRY(split_rows((long long)nv * n, n, 2 * n, (const double*)(V + (size_t)(w0 / vdiv) * n * n), 2 * n, t.V, s));
+        AFQ_TRY(launch_term<OZ_WALK>(wc, n, o, 0.0, win + w0 * no, nullptr, nullptr, t.X, s));
+        const OzOut xo = {t.Y, 0, (long long)no, 1, o, o, 0, nullptr};
+        AFQ_TRY(oz_launch(n, 2 * wc * o, n, 1, 0, t.E, t.X, xo, 1, (n + 255) / 256, nullptr, err, s));
+        AFQ_TRY(launch_term<OZ_INIT>(wc, n, o, 0.0, t.Y, win + w0 * no, t.U, t.T, s));
+        for (int k = 1; k <= n_terms; ++k) {
+            const OzOut to = {t.Y, (long long)no, 0, 1, o, 2 * o, 0, nullptr};
+            AFQ_TRY(oz_launch(n, 2 * o, 2 * n, wc, vdiv, t.V, t.T, to, 1, (2 * n + 255) / 256, nullptr, err, s));
+            if (k < n_terms) AFQ_TRY(launch_term<OZ_TERM>(wc, n, o, sqrt_dt / k, t.Y, nullptr, t.U, t.T, s));
+            else AFQ_TRY(launch_term<OZ_LAST>(wc, n, o, sqrt_dt / k, t.Y, nullptr, t.U, t.X, s));
+        }
+        const OzOut wo = {wout + w0 * no, 0, (long long)no, 1, o, o, 0, t.U};
+        AFQ_TRY(oz_launch(n, 2 * wc * o, n, 1, 0, t.E, t.X, wo, 1, (n + 255) / 256, nullptr, err, s));
+    }
+    return AFQ_OK;
+}
+
+// ---------------------------------------------------------------- energy --
+namespace {
+struct EnLayout {
+    int wc;
+    OzDigits L, X;
+    double2* F;
+};
+EnLayout en_layout(Arena& a, int W, int n, int o, int G) {
+    EnLayout e;
+    long long wc = OZ_CAP / ((long long)o * G * o * 16);
+    if (wc < 1) wc = 1;
+    if (wc > W) wc = W;
+    e.wc = (int)wc;
+    e.L = take_digits(a, (size_t)G * o, n);
+    e.X = take_digits(a, (size_t)e.wc * 2 * o, n);
+    e.F = a.take<double2>((size_t)e.wc * o * G * o);
+    return e;
+}
+}  // namespace
+
+size_t energy_oz_scratch(int W, int n, int o, int G) {
+    Arena a;
+    en_layout(a, W, n, o, G);
+    return a.used + 256;
+}
+
+int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, const double* rot_chol,
+                             double* partial_d, void* scratch, int* err, cudaStream_t s) {
+    if (W <= 0) return AFQ_OK;
+    Arena ar(scratch, (size_t)-1);
+    const EnLayout e = en_layout(ar, W, n, o, G);
+    const int nchunk = energy_partial_chunks(o, G), ng = (G + nchunk - 1) / nchunk;
+    const int smem = ng * o * (o + 1) * (int)sizeof(double2);
+    if (smem > OZ_XSMEM || W > 65535) return fail(AFQ_E_UNSUPPORTED, "digit energy: nocc=%d W=%d", o, W);
+    AFQ_TRY(raise_smem_once(g_ozx, k_oz_exchange, OZ_XSMEM));
+    AFQ_TRY(split_rows((long long)G * o, G * o, n, rot_chol, n, e.L, s));
+    for (int w0 = 0; w0 < W; w0 += e.wc) {
+        const int wc = W - w0 < e.wc ? W - w0 : e.wc;
+        AFQ_TRY(split_crows((long long)wc * o, n, green + (size_t)w0 * o * n, n, e.X, s));
+        const OzOut out = {e.F, 0, (long long)G * o, 0, 1, 1, 0, nullptr};
+        AFQ_TRY(oz_launch(G * o, 2 * wc * o, n, 1, 0, e.L, e.X, out, 1, (n + 255) / 256,
+                          nullptr, err, s));
+        k_oz_exchange<<<dim3(nchunk, wc), 256, smem, s>>>(o, G, ng, e.F, (double2*)partial_d + (size_t)w0 * nchunk * 2);
+        AFQ_LAUNCHED("k_oz_exchange");
+    }
+    return AFQ_OK;
+}
+
+// ---------------------------------------------------------------- routes --
+int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B, int64_t ldb,
+                      bool b_complex, bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s) {
+    if (!b_complex && zgemm_oz_pays(M, N, K))
+        return launch_zgemm_oz(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, ldc, oz.p, oz.err, s);
+    return launch_zgemm(M, N, K, alpha, A, lda, B, ldb, b_complex, b_trans, C, ldc, s);
+}
+
+int launch_trotter_auto(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
+                        const double2* win, double2* wout, int vdiv, const OzScratch& oz, cudaStream_t s) {
+    if (trotter_oz_pays(W, n, o, n_terms))
+        return launch_trotter_oz(W, n, o, n_terms, sqrt_dt, E, V, win, wout, vdiv, oz.p, oz.err, s);
+    return launch_trotter(W, n, o, n_terms, sqrt_dt, E, V, win, wout, s, vdiv);
+}
+
+int launch_energy_partial_auto(int W, int n, int o, int G, const double2* green, const void* rot_chol, int trial_real,
+                               double* partial, const OzScratch& oz, cudaStream_t s) {
+    if (trial_real && energy_oz_pays(W, n, o, G))
+        return launch_energy_partial_oz(W, n, o, G, green, (const double*)rot_chol, partial, oz.p, oz.err, s);
+    return launch_energy_partial(W, n, o, G, green, rot_chol, trial_real, partial, s);
+}
+
+}  // namespace afq

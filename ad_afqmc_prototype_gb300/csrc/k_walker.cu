@@ -613,10 +613,21 @@ int energy_partial_chunks(int o, int G) {
     return (G + ng - 1) / ng;
 }
 
+static size_t energy_smem(int o, int G, int trial_real) {
+    const int ng = energy_ng(o, G);
+    const size_t lsz = trial_real ? (size_t)(ng * o * EN_BJ + 1) / 2 : (size_t)ng * o * EN_BJ;
+    return ((size_t)o * EN_BJ + lsz + (size_t)ng * o * o) * sizeof(double2);
+}
+
+bool energy_partial_fits(int o, int G, int trial_real) {
+    return o * o <= EN_R * EN_THREADS && energy_smem(o, G, trial_real) <= 227 * 1024;
+}
+
 int launch_energy(int W, int n, int o, int G, double h0, const double2* green, const void* rot_chol,
-                  int trial_real, const double2* rot_h1, double* partial_d, double2* energy, cudaStream_t s) {
+                  int trial_real, const double2* rot_h1, double* partial_d, double2* energy, const OzScratch& oz,
+                  cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
-    AFQ_TRY(launch_energy_partial(W, n, o, G, green, rot_chol, trial_real, partial_d, s));
+    AFQ_TRY(launch_energy_partial_auto(W, n, o, G, green, rot_chol, trial_real, partial_d, oz, s));
     return launch_energy_finish(W, n, o, energy_partial_chunks(o, G), h0, green, rot_h1, (const double2*)partial_d,
                                 energy, s);
 }
@@ -628,8 +639,7 @@ int launch_energy_partial(int W, int n, int o, int G, const double2* green, cons
     const int ng = energy_ng(o, G);
     const int nchunk = (G + ng - 1) / ng;
     double2* partial = (double2*)partial_d;
-    size_t lsz = trial_real ? (size_t)(ng * o * EN_BJ + 1) / 2 : (size_t)ng * o * EN_BJ;
-    size_t smem = ((size_t)o * EN_BJ + lsz + (size_t)ng * o * o) * sizeof(double2);
+    const size_t smem = energy_smem(o, G, trial_real);
     dim3 grid(nchunk, W);
     if (W > 65535) return fail(AFQ_E_UNSUPPORTED, "energy: %d walkers > 65535 per call", W);
     if (trial_real) {

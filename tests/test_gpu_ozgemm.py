@@ -1,0 +1,70 @@
+"""Digit products of the binary64 form (csrc/k_ozgemm.cu) at the edges of their tiles, against the NumPy oracle.
+
+Sizes: orbitals around the 32 from which the Taylor series goes by digits and around the 128-row tile, columns
+around the 64-wide tile (2 nocc, 2 W), K around the 16-, 32-, 256- and 512-wide steps and drains, K splits.
+Tolerance: the oracle's own binary64 sums of K products carry about sqrt(K) 1.1e-16 of the result (7e-15 at
+the longest, K = 4225); 1e-13 allows it ten times that.
+"""
+import numpy as np
+import pytest
+import torch
+
+from ad_afqmc_prototype_gb300 import engine
+from oracle import afqmc_oracle as O
+
+pytestmark = pytest.mark.gpu
+
+RTOL = 1e-13
+SIZES = [(33, 7, 31, 5), (34, 8, 32, 33), (45, 9, 257, 31), (64, 8, 256, 32), (65, 65 - 1, 40, 2), (127, 7, 33, 3),
+         (128, 32, 48, 2), (129, 33, 49, 2), (65, 33, 513, 65), (200, 16, 16, 4), (130, 7, 1025, 2)]
+
+
+def _problem(n, o, G, W, seed=0):
+    rng = np.random.default_rng(seed)
+    h1 = np.diag(np.linspace(-2.0, 0.5, n)) + 0.05 * O_sym(rng.normal(size=(n, n)))
+    chol = O_sym(rng.normal(size=(G, n, n))) * (3.6 / n) * np.exp(-4.0 * np.arange(G) / G)[:, None, None]
+    mo = np.ascontiguousarray(np.linalg.eigh(h1)[1][:, :o])
+    w = mo + 0.2 / np.sqrt(n) * (rng.normal(size=(W, n, o)) + 1j * rng.normal(size=(W, n, o)))
+    xs = rng.normal(size=(W, G)) + 0.2j * rng.normal(size=(W, G))
+    return h1, chol, mo, w, xs
+
+
+def O_sym(b):
+    return 0.5 * (b + np.swapaxes(b, -1, -2))
+
+
+def _rel(got, want):
+    return np.linalg.norm(got.cpu().numpy() - want) / np.linalg.norm(want)
+
+
+def _dev(x, dtype=torch.float64):
+    return torch.as_tensor(x, dtype=dtype, device="cuda")
+
+
+@pytest.mark.parametrize("n,o,G,W", SIZES)
+def test_digit_products_match_oracle(n, o, G, W):
+    h1, chol, mo, w, xs = _problem(n, o, G, W)
+    ctx = O.build_meas_ctx(h1, chol, mo.astype(complex))
+    pctx = O.build_prop_ctx(0.0, h1, chol, O.get_rdm1(mo.astype(complex)), 0.005)
+    cm, wd = _dev(mo, torch.complex128), _dev(w, torch.complex128)
+    rot = _dev(np.ascontiguousarray(ctx.rot_chol.real))
+    fb = engine.force_bias(wd, cm, rot, True)
+    assert _rel(fb, O.force_bias_r(w, ctx, mo.astype(complex))) < RTOL
+    out = engine.apply_trotter(wd, _dev(xs, torch.complex128), _dev(chol), _dev(pctx.exp_h1_half), pctx.sqrt_dt, 6)
+    assert _rel(out, O.apply_trotter_r(w, xs, pctx, chol.reshape(G, -1), 6)) < RTOL
+    e = engine.energy(wd, 0.0, cm, _dev(ctx.rot_h1, torch.complex128), rot, True)
+    assert _rel(e, O.energy_r(w, 0.0, ctx, mo.astype(complex))) < RTOL
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_digit_products_keep_nonfinite_rows_apart(bad):
+    n, o, G, W = 45, 9, 100, 6
+    h1, chol, mo, w, xs = _problem(n, o, G, W)
+    pctx = O.build_prop_ctx(0.0, h1, chol, O.get_rdm1(mo.astype(complex)), 0.005)
+    want = O.apply_trotter_r(w, xs, pctx, chol.reshape(G, -1), 6)
+    xs[2, 17] = bad
+    out = engine.apply_trotter(_dev(w, torch.complex128), _dev(xs, torch.complex128), _dev(chol),
+                               _dev(pctx.exp_h1_half), pctx.sqrt_dt, 6).cpu()
+    assert not torch.isfinite(torch.view_as_real(out[2])).any()
+    keep = [i for i in range(W) if i != 2]
+    assert _rel(out[keep], want[keep]) < RTOL
