@@ -7,6 +7,8 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <algorithm>
+
 #include "afq_internal.cuh"
 
 namespace afq {
@@ -138,7 +140,6 @@ struct StepWS {
 // (7 norb 2^12 < 2^24).
 static bool oz_supported(const afq_dims* d) { return d->nocc <= 32 && d->norb <= 584; }
 
-static size_t max3(size_t a, size_t b, size_t c) { return a > b ? (a > c ? a : c) : (b > c ? b : c); }
 
 // Scratch of the binary64 form's digit products (one region, used by one at a time).
 static OzScratch take_oz(Arena& a, size_t bytes, int* status) {
@@ -148,15 +149,16 @@ static OzScratch take_oz(Arena& a, size_t bytes, int* status) {
     return z;
 }
 static size_t fb_oz_bytes(const afq_dims* d) {
-    return zgemm_oz_scratch(d->n_walkers, d->nchol, d->nocc * d->norb);
+    return std::max(zgemm_oz_scratch(d->n_walkers, d->nchol, d->nocc * d->norb),
+                    green_oz_scratch(d->n_walkers, d->norb, d->nocc));
 }
 static size_t trotter_oz_bytes(const afq_dims* d, int n_chunks) {
     const int n = d->norb, wc = chunk_size(d->n_walkers, n_chunks);
-    const size_t v = zgemm_oz_scratch(wc, n * n, d->nchol), t = trotter_oz_scratch(wc, n, d->nocc, 1);
-    return v > t ? v : t;
+    return std::max(zgemm_oz_scratch(wc, n * n, d->nchol), trotter_oz_scratch(wc, n, d->nocc, 1));
 }
 static size_t energy_oz_bytes(const afq_dims* d) {
-    return energy_oz_scratch(d->n_walkers, d->norb, d->nocc, d->nchol);
+    return std::max(energy_oz_scratch(d->n_walkers, d->norb, d->nocc, d->nchol),
+                    green_oz_scratch(d->n_walkers, d->norb, d->nocc));
 }
 
 static StepWS layout_step(Arena& a, const afq_dims* d, int n_chunks, size_t oz_bytes = 0) {
@@ -189,7 +191,7 @@ static StepWS layout_step(Arena& a, const afq_dims* d, int n_chunks, size_t oz_b
         s.fb = a.take<double2>(W * G);
         s.xs = a.take<double2>(W * G);
         s.V = a.take<double2>(Wc * n * n);
-        s.oz = take_oz(a, max3(oz_bytes, fb_oz_bytes(d), trotter_oz_bytes(d, n_chunks)), s.status);
+        s.oz = take_oz(a, std::max({oz_bytes, fb_oz_bytes(d), trotter_oz_bytes(d, n_chunks)}), s.status);
     }
     return s;
 }
@@ -408,8 +410,8 @@ static int energy_impl(const afq_problem* pb, const afq_state* st, const BlockWS
     const int W = d->n_walkers, n = d->norb, o = d->nocc, G = d->nchol;
     if (!green_ready) {
         AFQ_PHASE("green", s);
-        AFQ_TRY(launch_green(W, n, o, (const double2*)pb->mo_coeff, d->trial_is_real, (const double2*)st->walkers,
-                             nullptr, ws.green, s));
+        AFQ_TRY(launch_green_auto(W, n, o, (const double2*)pb->mo_coeff, d->trial_is_real,
+                                  (const double2*)st->walkers, nullptr, ws.green, 1, ws.step.oz, s));
     }
     AFQ_PHASE("energy", s);
     if (!is_mixed(d->precision))
@@ -454,6 +456,11 @@ static int check_state(const afq_state* st) {
     return AFQ_OK;
 }
 
+// whether a QR follows step i of a block (the one at the block's end not counted)
+static bool qr_after(const afq_params* p, int i) {
+    return p->qr_every > 0 && (i + 1) % p->qr_every == 0 && i + 1 < p->n_prop_steps;
+}
+
 static int check_params(const afq_params* p) {
     if (!p) return fail(AFQ_E_INVALID_ARGUMENT, "params is NULL");
     if (p->n_exp_terms < 0) return fail(AFQ_E_INVALID_ARGUMENT, "n_exp_terms=%d < 0", p->n_exp_terms);
@@ -462,9 +469,12 @@ static int check_params(const afq_params* p) {
     return AFQ_OK;
 }
 
+// green_ready: the Green's function of the walkers (mixed: its force-bias
+// operand) is in place; green_next (binary64): the pass that gives the new
+// overlaps leaves the new walkers' Green's function for the next step.
 static int step_impl(const afq_problem* pb, const afq_params* p, const afq_state* st, const double* fields,
                      uint64_t seed, uint64_t counter, const StepWS& ws, cudaStream_t s, bool green_ready = false,
-                     double2* green_out = nullptr) {
+                     double2* green_out = nullptr, bool green_next = false) {
     const afq_dims* d = &pb->dims;
     const int W = d->n_walkers, n = d->norb, o = d->nocc, G = d->nchol;
     const double2* mo = (const double2*)pb->mo_coeff;
@@ -476,7 +486,10 @@ static int step_impl(const afq_problem* pb, const afq_params* p, const afq_state
     }
     if (is_mixed(d->precision)) return step_mixed(pb, p, st, fields, ws, green_ready, s, green_out);
     // force bias (prop/afqmc.py:90-95)
-    { AFQ_PHASE("green", s); AFQ_TRY(launch_green(W, n, o, mo, d->trial_is_real, walk, nullptr, ws.green, s)); }
+    if (!green_ready) {
+        AFQ_PHASE("green", s);
+        AFQ_TRY(launch_green_auto(W, n, o, mo, d->trial_is_real, walk, nullptr, ws.green, 1, ws.oz, s));
+    }
     { AFQ_PHASE("fb_gemm", s); AFQ_TRY(force_bias_from_green(d, ws.green, pb->rot_chol, ws.fb, ws.oz, s)); }
     // shifts (prop/afqmc.py:97-101)
     { AFQ_PHASE("field_shift", s);
@@ -486,7 +499,9 @@ static int step_impl(const afq_problem* pb, const afq_params* p, const afq_state
     AFQ_TRY(trotter_chunked(d, p->n_exp_terms, pb->sqrt_dt, p->n_chunks, pb->chol, pb->exp_h1_half, walk, ws.xs,
                             walk, ws.V, ws.oz, s));
     // overlaps (prop/afqmc.py:112-114)
-    { AFQ_PHASE("overlap", s); AFQ_TRY(launch_green(W, n, o, mo, d->trial_is_real, walk, ws.ovl_new, nullptr, s)); }
+    { AFQ_PHASE("overlap", s); 
+      AFQ_TRY(launch_green_auto(W, n, o, mo, d->trial_is_real, walk, ws.ovl_new, green_next ? ws.green : nullptr, 1,
+                                ws.oz, s)); }
     AFQ_PHASE("weight_update", s);
     // weights (prop/afqmc.py:116-138)
     return launch_weight_update(W, p, pb->sqrt_dt, pb->dt, make_double2(pb->h0_prop_re, pb->h0_prop_im),
@@ -534,8 +549,8 @@ static int orthonormalize_refresh(const afq_problem* pb, const afq_state* st, cu
     if (green_out && d->precision == AFQ_PREC_MIXED_FAST)
         return launch_overlap_split(d->n_walkers, d->norb, d->nocc, (const double2*)pb->mo_coeff, walk,
                                     (double2*)st->overlaps, SplitOut{}, s, green_out, cs);
-    return launch_green(d->n_walkers, d->norb, d->nocc, (const double2*)pb->mo_coeff, d->trial_is_real, walk,
-                        (double2*)st->overlaps, green_out, s);
+    return launch_green_auto(d->n_walkers, d->norb, d->nocc, (const double2*)pb->mo_coeff, d->trial_is_real, walk,
+                             (double2*)st->overlaps, green_out, 1, green_ws ? green_ws->oz : ws ? ws->oz : OzScratch{}, s);
 }
 
 }  // namespace afq
@@ -721,8 +736,8 @@ int afq_force_bias(const afq_dims* d, const double* mo_coeff, const double* rot_
     const OzScratch oz = take_oz(a, fb_oz_bytes(d), status);
     AFQ_TRY(check_ws(a, workspace_bytes));
     cudaStream_t s = as_stream(stream);
-    AFQ_TRY(launch_green(d->n_walkers, d->norb, d->nocc, (const double2*)mo_coeff, d->trial_is_real,
-                         (const double2*)walkers, nullptr, green, s));
+    AFQ_TRY(launch_green_auto(d->n_walkers, d->norb, d->nocc, (const double2*)mo_coeff, d->trial_is_real,
+                              (const double2*)walkers, nullptr, green, 1, oz, s));
     return force_bias_from_green(d, green, rot_chol, (double2*)force_bias, oz, s);
 }
 
@@ -748,8 +763,8 @@ int afq_energy(const afq_dims* d, double h0, const double* mo_coeff, const doubl
     const OzScratch oz = take_oz(a, energy_oz_bytes(d), status);
     AFQ_TRY(check_ws(a, workspace_bytes));
     cudaStream_t s = as_stream(stream);
-    AFQ_TRY(launch_green(d->n_walkers, d->norb, d->nocc, (const double2*)mo_coeff, d->trial_is_real,
-                         (const double2*)walkers, nullptr, green, s));
+    AFQ_TRY(launch_green_auto(d->n_walkers, d->norb, d->nocc, (const double2*)mo_coeff, d->trial_is_real,
+                              (const double2*)walkers, nullptr, green, 1, oz, s));
     return launch_energy(d->n_walkers, d->norb, d->nocc, d->nchol, h0, green, rot_chol, d->trial_is_real,
                          (const double2*)rot_h1, partial, (double2*)energy, oz, s);
 }
@@ -966,12 +981,13 @@ int afq_block_cv(const afq_problem* pb, const afq_params* p, const afq_state* st
                             (cvmode != AFQ_CV_OFF || d->precision == AFQ_PREC_MIXED_FAST);
     // prop/blocks.py:38-51
     for (int st_i = 0; st_i < p->n_prop_steps; ++st_i) {
-        // from the second step on, the previous overlap kernel left the force-bias operand
-        const bool last = st_i + 1 == p->n_prop_steps;
+        // from the second step on, the previous overlap pass left the Green's function or force-bias operand
+        const bool last = st_i + 1 == p->n_prop_steps, qr = qr_after(p, st_i);
         AFQ_TRY(step_impl(pb, p, st, fields ? fields + st_i * fstride : nullptr, seed, counter + st_i, ws.step, s,
-                          st_i > 0, green_kept && last ? ws.green : nullptr));
-        if (p->qr_every > 0 && (st_i + 1) % p->qr_every == 0 && st_i + 1 < p->n_prop_steps)
-            AFQ_TRY(orthonormalize_refresh(pb, st, s, &ws.step, nullptr, nullptr, ws.step.ovl_new));
+                          st_i > 0, green_kept && last ? ws.green : nullptr, !last && !qr));
+        if (qr)
+            AFQ_TRY(orthonormalize_refresh(pb, st, s, &ws.step, is_mixed(d->precision) ? nullptr : ws.step.green,
+                                           nullptr, ws.step.ovl_new));
     }
     // prop/blocks.py:53-57, with the energy's Green's function from the same pass
     if (is_mixed(d->precision))
@@ -1105,17 +1121,18 @@ int run_block_taped(const afq_problem* pb, const afq_params* p, const afq_state*
     int op = 0;
     for (int st_i = 0; st_i < p->n_prop_steps; ++st_i) {
         AFQ_TRY(snap_state(d, st, snap, op++, s));
-        AFQ_TRY(step_impl(pb, p, st, nullptr, seed, counter + st_i, ws.step, s));
+        const bool last = st_i + 1 == p->n_prop_steps, qr = qr_after(p, st_i);
+        AFQ_TRY(step_impl(pb, p, st, nullptr, seed, counter + st_i, ws.step, s, st_i > 0, nullptr, !last && !qr));
         if (snap && snap->V && chunk_size(W, p->n_chunks) == W)
             AFQ_CUDA(cudaMemcpyAsync(snap->V + (size_t)st_i * W * n * n, ws.step.V, sizeof(double2) * (size_t)W * n * n,
                                      cudaMemcpyDeviceToDevice, s));
-        if (p->qr_every > 0 && (st_i + 1) % p->qr_every == 0 && st_i + 1 < p->n_prop_steps) {
+        if (qr) {
             AFQ_TRY(snap_state(d, st, snap, op++, s));
-            AFQ_TRY(orthonormalize_refresh(pb, st, s, &ws.step));
+            AFQ_TRY(orthonormalize_refresh(pb, st, s, &ws.step, ws.step.green));
         }
     }
     AFQ_TRY(snap_state(d, st, snap, op++, s));
-    AFQ_TRY(orthonormalize_refresh(pb, st, s, nullptr, ws.green, nullptr));
+    AFQ_TRY(orthonormalize_refresh(pb, st, s, nullptr, ws.green, nullptr, nullptr, false, &ws.step));
     AFQ_TRY(snap_state(d, st, snap, op++, s));
     AFQ_TRY(energy_impl(pb, st, ws, s, true));
     if (snap)

@@ -121,7 +121,8 @@ GradWS layout_grad(Arena& a, const afq_dims* d, const afq_params* p, int ck) {
         const int Wi = (int)W, Gi = (int)G, n2 = (int)(n * n), noi = (int)no, oi = (int)o, ni = (int)n, wo = (int)(wc * o);
         g.oz.p = a.take<char>(std::max({zgemm_oz_scratch(Wi, Gi, noi), zgemm_oz_scratch(Wi, n2, Gi),
                                         zgemm_oz_scratch(Wi, Gi, n2), zgemm_oz_scratch(Wi, noi, Gi),
-                                        zgemm_oz_scratch(wo, Gi * oi, ni), zgemm_oz_scratch(wo, ni, Gi * oi)}));
+                                        zgemm_oz_scratch(wo, Gi * oi, ni), zgemm_oz_scratch(wo, ni, Gi * oi),
+                                        green_oz_scratch(Wi, ni, oi)}));
         g.oz.err = g.status;
     }
     g.wk = a.take<double2>(W * no);
@@ -217,7 +218,7 @@ int step_adjoint(const Ctx& c, const BlockSnap& sn, int op, int st_i, uint64_t c
     {
         AFQ_PHASE("adj_recompute", s);
         AFQ_TRY(launch_philox((int64_t)W * G, c.seed, counter, 1, g.fields, s));
-        AFQ_TRY(launch_green(W, n, o, mo, 1, Wpre, nullptr, g.green, s));
+        AFQ_TRY(launch_green_auto(W, n, o, mo, 1, Wpre, nullptr, g.green, 1, g.oz, s));
         AFQ_TRY(launch_zgemm_auto(W, G, no, 2.0, g.green, no, pb->rot_chol, no, false, true, g.fb, G, g.oz, s));
         AFQ_TRY(launch_field_shift(W, G, pb->sqrt_dt, g.fields, g.fb, (const double2*)pb->mf_shifts, g.xs,
                                    g.shift_term, g.fb_term, s));
@@ -280,7 +281,7 @@ int block_adjoint(const Ctx& c, const BlockSnap& sn, const TapeLayout& t, int b,
     AFQ_TRY(launch_measure_adj(W, p->dt, p->shift_ema, wm, sn.energy, g.e_est, t.be + b, eb_bar + b, wb_bar + b,
                                g.pb, g.wb, g.ebar_w, s));
     // local energies -> G_half of the measured walkers
-    AFQ_TRY(launch_green(W, n, o, mo, 1, Wm, nullptr, g.green, s));
+    AFQ_TRY(launch_green_auto(W, n, o, mo, 1, Wm, nullptr, g.green, 1, g.oz, s));
     AFQ_TRY(launch_zgemm_auto(W, G, no, 1.0, g.green, no, pb->rot_chol, no, false, true, g.xtb, G, g.oz, s));   // c_g
     AFQ_TRY(launch_zgemm_auto(W, no, G, 1.0, g.xtb, G, pb->rot_chol, no, false, false, g.cl, no, g.oz, s));     // sum c_g L~_g
     const int wc = grad_energy_chunk(d);

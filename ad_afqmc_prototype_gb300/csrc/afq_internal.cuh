@@ -302,6 +302,10 @@ size_t zgemm_oz_scratch(int M, int N, int K);
 // launch_zgemm with a real right operand; alpha a power of two
 int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
                     bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s);
+bool green_oz_pays(int n, int o);
+size_t green_oz_scratch(int W, int n, int o);
+int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walkers, double2* ovlp_out,
+                    double2* green_out, int ov_square, void* scratch, int* err, cudaStream_t s);
 bool trotter_oz_pays(int W, int n, int o, int n_terms);
 size_t trotter_oz_scratch(int W, int n, int o, int vdiv);
 int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
@@ -318,9 +322,19 @@ int launch_trotter_auto(int W, int n, int o, int n_terms, double sqrt_dt, const 
 int launch_energy_partial_auto(int W, int n, int o, int G, const double2* green, const void* rot_chol, int trial_real,
                                double* partial, const OzScratch& oz, cudaStream_t s);
 
-// k_walker.cu
+// k_green.cu
 int launch_green(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
                  double2* ovlp_out, double2* green_out, cudaStream_t s);
+// det(C^H W) per walker (not squared: the unrestricted overlap's per-spin factor)
+int launch_green_det(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
+                     double2* det_out, double2* green_out, cudaStream_t s);
+// determinants (squared: ov_square) and, with inv_out, inverses of given m (W x o x o)
+int launch_lu(int W, int o, const double2* m, double2* ovlp_out, double2* inv_out, int ov_square, cudaStream_t s);
+// either of the above, m and G_half by digits where that pays (real trial, scratch given)
+int launch_green_auto(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
+                      double2* ovlp_out, double2* green_out, int ov_square, const OzScratch& oz, cudaStream_t s);
+
+// k_walker.cu
 // vdiv walkers share each V (2: the top and bottom halves of generalized walkers)
 int launch_trotter(int W, int n, int o, int n_terms, double sqrt_dt, const double* E,
                    const double2* V, const double2* win, double2* wout, cudaStream_t s, int vdiv = 1);
@@ -370,12 +384,6 @@ int launch_tc_gemm_tn_drain_split(int M, int N, int K, const void* A, long long 
                                   __nv_bfloat16* Ch, __nv_bfloat16* Cm, long long ldc, int* err, cudaStream_t s,
                                   int kd = 1);
 
-// k_walker.cu : Green's function with an optional split (bf16) output
-int launch_green_split(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
-                       double2* ovlp_out, double2* green_out, SplitOut split, cudaStream_t s, int ov_square = 1);
-// det(C^H W) per walker (not squared: the unrestricted overlap's per-spin factor)
-int launch_green_det(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
-                     double2* det_out, double2* green_out, cudaStream_t s);
 // the energy's per-chunk partials (sum c^2, sum exchange) without the finish
 int energy_partial_chunks(int o, int G);
 bool energy_partial_fits(int o, int G, int trial_real);

@@ -127,7 +127,8 @@ UWS layout_u(Arena& a, const afq_dims* d, int n_chunks) {
     u.ov_new = a.take<double2>(W);
     const int wc = chunk_of(d->n_walkers, n_chunks);
     u.V = a.take<double2>((size_t)wc * n * n);
-    u.oz.p = a.take<char>(oz_most({zgemm_oz_scratch(2 * d->n_walkers, d->nchol, (int)no),
+    u.oz.p = a.take<char>(oz_most({green_oz_scratch(2 * d->n_walkers, d->norb, d->nocc),
+                                   zgemm_oz_scratch(2 * d->n_walkers, d->nchol, (int)no),
                                    zgemm_oz_scratch(wc, (int)(n * n), d->nchol),
                                    trotter_oz_scratch(wc, d->norb, d->nocc, 1),
                                    energy_oz_scratch(2 * d->n_walkers, d->norb, d->nocc, d->nchol)}));
@@ -157,7 +158,7 @@ int check_u(const afq_dims* d) {
 // overlaps (and optionally both spins' G_half) of the pairs
 int overlap_u(const afq_dims* d, const double2* mo, const double2* walk, double2* ov, double2* green, const UWS& u,
               cudaStream_t s) {
-    AFQ_TRY(launch_green_det(2 * d->n_walkers, d->norb, d->nocc, mo, d->trial_is_real, walk, u.det, green, s));
+    AFQ_TRY(launch_green_auto(2 * d->n_walkers, d->norb, d->nocc, mo, d->trial_is_real, walk, u.det, green, 0, u.oz, s));
     return launch_spin_prod(d->n_walkers, u.det, ov, s);
 }
 
@@ -203,8 +204,9 @@ int energy_u(const afq_problem* pb, const UWS& u, cudaStream_t s) {
     return AFQ_OK;
 }
 
+// green_ready: u.green holds the walkers' G_half; green_next: the overlap pass leaves the new walkers' there
 int step_u(const afq_problem* pb, const afq_params* p, const afq_state* st, const double* fields, uint64_t seed,
-           uint64_t counter, const UWS& u, cudaStream_t s) {
+           uint64_t counter, const UWS& u, cudaStream_t s, bool green_ready = false, bool green_next = false) {
     const afq_dims* d = &pb->dims;
     const int W = d->n_walkers, G = d->nchol;
     const double2* mo = (const double2*)pb->mo_coeff;
@@ -214,15 +216,17 @@ int step_u(const afq_problem* pb, const afq_params* p, const afq_state* st, cons
         AFQ_TRY(launch_philox((int64_t)W * G, seed, counter, 1, u.fields, s));
         fields = u.fields;
     }
-    { AFQ_PHASE("green", s);
-      AFQ_TRY(launch_green(2 * W, d->norb, d->nocc, mo, d->trial_is_real, walk, nullptr, u.green, s)); }
+    if (!green_ready) {
+        AFQ_PHASE("green", s);
+        AFQ_TRY(launch_green_auto(2 * W, d->norb, d->nocc, mo, d->trial_is_real, walk, nullptr, u.green, 1, u.oz, s));
+    }
     { AFQ_PHASE("fb_gemm", s); AFQ_TRY(force_bias_u(d, pb->rot_chol, u, u.fb, s)); }
     { AFQ_PHASE("field_shift", s);
       AFQ_TRY(launch_field_shift(W, G, pb->sqrt_dt, fields, u.fb, (const double2*)pb->mf_shifts, u.xs, u.shift_term,
                                  u.fb_term, s)); }
     AFQ_TRY(trotter_u(d, p->n_exp_terms, pb->sqrt_dt, p->n_chunks, pb->chol, pb->exp_h1_half, walk, u.xs, walk, u.V,
                       u.oz, s));
-    { AFQ_PHASE("overlap", s); AFQ_TRY(overlap_u(d, mo, walk, u.ov_new, nullptr, u, s)); }
+    { AFQ_PHASE("overlap", s); AFQ_TRY(overlap_u(d, mo, walk, u.ov_new, green_next ? u.green : nullptr, u, s)); }
     AFQ_PHASE("weight_update", s);
     return launch_weight_update(W, p, pb->sqrt_dt, pb->dt, make_double2(pb->h0_prop_re, pb->h0_prop_im),
                                 u.shift_term, u.fb_term, u.ov_new, st->weights, (double2*)st->overlaps,
@@ -299,7 +303,8 @@ GWS layout_g(Arena& a, const afq_dims* d, int n_chunks) {
     g.gsum = a.take<double2>(W * o * n);
     const int wc = chunk_of(d->n_walkers, n_chunks);
     g.V = a.take<double2>((size_t)wc * n * n);
-    g.oz.p = a.take<char>(oz_most({zgemm_oz_scratch(d->n_walkers, d->nchol, (int)(n * o)),
+    g.oz.p = a.take<char>(oz_most({green_oz_scratch(d->n_walkers, 2 * d->norb, 2 * d->nocc),
+                                   zgemm_oz_scratch(d->n_walkers, d->nchol, (int)(n * o)),
                                    zgemm_oz_scratch(wc, (int)(n * n), d->nchol),
                                    trotter_oz_scratch(2 * wc, d->norb, 2 * d->nocc, 2)}));
     g.oz.err = g.status;
@@ -345,8 +350,8 @@ int afq_overlap_g(const afq_dims* d, const double* mo_coeff, const double* walke
     if (!a.ok()) return fail(AFQ_E_WORKSPACE, "workspace: %zu bytes < %zu", workspace_bytes, a.used);
     cudaStream_t s = as_stream(stream);
     AFQ_TRY(build_cg(d, (const double2*)mo_coeff, g, s));
-    return launch_green_det(d->n_walkers, 2 * d->norb, 2 * d->nocc, g.cg, d->trial_is_real, (const double2*)walkers,
-                            (double2*)overlaps, nullptr, s);
+    return launch_green_auto(d->n_walkers, 2 * d->norb, 2 * d->nocc, g.cg, d->trial_is_real, (const double2*)walkers,
+                             (double2*)overlaps, nullptr, 0, g.oz, s);
 }
 
 int afq_force_bias_g(const afq_dims* d, const double* mo_coeff, const double* rot_chol, const double* walkers,
@@ -360,7 +365,7 @@ int afq_force_bias_g(const afq_dims* d, const double* mo_coeff, const double* ro
     cudaStream_t s = as_stream(stream);
     const int W = d->n_walkers, n = d->norb, o = d->nocc, on = n * o;
     AFQ_TRY(build_cg(d, (const double2*)mo_coeff, g, s));
-    AFQ_TRY(launch_green(W, 2 * n, 2 * o, g.cg, d->trial_is_real, (const double2*)walkers, nullptr, g.green, s));
+    AFQ_TRY(launch_green_auto(W, 2 * n, 2 * o, g.cg, d->trial_is_real, (const double2*)walkers, nullptr, g.green, 1, g.oz, s));
     const long long total = (long long)W * on;
     long long blocks = (total + 255) / 256;
     if (blocks > 152 * 32) blocks = 152 * 32;
@@ -423,8 +428,8 @@ int afq_force_bias_u(const afq_dims* d, const double* mo_coeff, const double* ro
     const UWS u = layout_u(a, d, 1);
     if (!a.ok()) return fail(AFQ_E_WORKSPACE, "workspace: %zu bytes < %zu", workspace_bytes, a.used);
     cudaStream_t s = as_stream(stream);
-    AFQ_TRY(launch_green(2 * d->n_walkers, d->norb, d->nocc, (const double2*)mo_coeff, d->trial_is_real,
-                         (const double2*)walkers, nullptr, u.green, s));
+    AFQ_TRY(launch_green_auto(2 * d->n_walkers, d->norb, d->nocc, (const double2*)mo_coeff, d->trial_is_real,
+                              (const double2*)walkers, nullptr, u.green, 1, u.oz, s));
     return force_bias_u(d, rot_chol, u, (double2*)force_bias, s);
 }
 
@@ -443,8 +448,8 @@ int afq_energy_u(const afq_dims* d, double h0, const double* mo_coeff, const dou
     pb.mo_coeff = mo_coeff;
     pb.rot_h1 = rot_h1;
     pb.rot_chol = rot_chol;
-    AFQ_TRY(launch_green(2 * d->n_walkers, d->norb, d->nocc, (const double2*)mo_coeff, d->trial_is_real,
-                         (const double2*)walkers, nullptr, u.green, s));
+    AFQ_TRY(launch_green_auto(2 * d->n_walkers, d->norb, d->nocc, (const double2*)mo_coeff, d->trial_is_real,
+                              (const double2*)walkers, nullptr, u.green, 1, u.oz, s));
     u.energy = (double2*)energy;
     return energy_u(&pb, u, s);
 }
@@ -513,9 +518,10 @@ int afq_block_u(const afq_problem* pb, const afq_params* p, const afq_state* st,
     const size_t half = (size_t)W * d->norb * d->nocc;
     // prop/blocks.py:38-57
     for (int i = 0; i < p->n_prop_steps; ++i) {
-        AFQ_TRY(step_u(pb, p, st, fields ? fields + (size_t)i * W * G : nullptr, seed, counter + i, u, s));
-        if (p->qr_every > 0 && (i + 1) % p->qr_every == 0 && i + 1 < p->n_prop_steps)
-            AFQ_TRY(orthonormalize_u(pb, st, u, nullptr, s));
+        const bool last = i + 1 == p->n_prop_steps, qr = !last && p->qr_every > 0 && (i + 1) % p->qr_every == 0;
+        AFQ_TRY(step_u(pb, p, st, fields ? fields + (size_t)i * W * G : nullptr, seed, counter + i, u, s, i > 0,
+                       !last && !qr));
+        if (qr) AFQ_TRY(orthonormalize_u(pb, st, u, u.green, s));
     }
     AFQ_TRY(orthonormalize_u(pb, st, u, u.green, s));
     // prop/blocks.py:59-79

@@ -591,9 +591,9 @@ __global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const d
     }
 }
 
-// Real rows with K strided: row r's entry k at src[k ld + r]; 32 rows a CTA,
+// Real rows with K strided: row r's entry k at src[k ld + r es]; 32 rows a CTA,
 // transposed through shared memory.
-__global__ void __launch_bounds__(256) k_oz_cols(int rows, int K, const double* __restrict__ src, long long ld,
+__global__ void __launch_bounds__(256) k_oz_cols(int rows, int K, const double* __restrict__ src, long long ld, int es,
                                                  OzDst dst, int* __restrict__ ex) {
     __shared__ double tile[32][65];
     __shared__ int se[32];
@@ -604,7 +604,7 @@ __global__ void __launch_bounds__(256) k_oz_cols(int rows, int K, const double* 
     int e = 0;
     if (in) {
 #pragma unroll 4
-        for (int k = ty; k < K; k += 8) e = max(e, oz_expo(src[(long long)k * ld + r0 + tx]));
+        for (int k = ty; k < K; k += 8) e = max(e, oz_expo(src[(long long)k * ld + (r0 + tx) * es]));
     }
     atomicMax(&se[tx], e);
     __syncthreads();
@@ -615,7 +615,7 @@ __global__ void __launch_bounds__(256) k_oz_cols(int rows, int K, const double* 
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int k = k0 + ty + 8 * i;
-            tile[tx][ty + 8 * i] = in && k < K ? src[(long long)k * ld + r0 + tx] : 0.0;
+            tile[tx][ty + 8 * i] = in && k < K ? src[(long long)k * ld + (r0 + tx) * es] : 0.0;
         }
         __syncthreads();
         if (r0 + rr < rows && k0 + kq < 32 * dst.nks) {
@@ -629,12 +629,13 @@ __global__ void __launch_bounds__(256) k_oz_cols(int rows, int K, const double* 
 
 // Walker-shaped blocks (w, j, c), c fastest, eight columns c a CTA:
 //   WALK  digits of the block's columns over j, rows (w, c, part)
+//   PLAIN digits of T = Y as the right operand of V T
 //   INIT  T = W + Y; U = T; digits of T as the right operand of V T
 //   TERM  T = i s Y; U += T; digits of T as the right operand of V T
 //   LAST  T = i s Y; U += T; digits of U as WALK's
 // The right operand of V T (V's rows hold Re, Im interleaved): rows (c, Re)
 // [Tr, -Ti] and (c, Im) [Ti, Tr] over (j, part), a batch a walker.
-enum { OZ_WALK, OZ_INIT, OZ_TERM, OZ_LAST };
+enum { OZ_WALK, OZ_PLAIN, OZ_INIT, OZ_TERM, OZ_LAST };
 constexpr int OZ_CB = 8;
 template <int MODE>
 __global__ void __launch_bounds__(256) k_oz_term(int n, int o, int ncg, double s, const double2* __restrict__ Y,
@@ -759,7 +760,7 @@ __global__ void __launch_bounds__(256) k_oz_exchange(int o, int G, int NG, const
 }
 
 constexpr int OZ_XSMEM = 96 * 1024;  // the exchange kernel's F blocks
-DeviceOnce g_oz, g_ozterm[4], g_ozx;
+DeviceOnce g_oz, g_ozterm[5], g_ozx;
 
 int nks_of(int K) { return (K + OZ_BK - 1) / OZ_BK; }
 long long digit_row_bytes(int K) { return 64LL * OZ_S * nks_of(K); }
@@ -830,8 +831,8 @@ int split_crows(long long rows, int K, const double2* src, long long ld, const O
     AFQ_LAUNCHED("k_oz_crows");
     return AFQ_OK;
 }
-int split_cols(int rows, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s) {
-    k_oz_cols<<<(rows + 31) / 32, 256, 0, s>>>(rows, K, src, ld, dst_of(D, rows, K), D.ex);
+int split_cols(int rows, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s, int es = 1) {
+    k_oz_cols<<<(rows + 31) / 32, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex);
     AFQ_LAUNCHED("k_oz_cols");
     return AFQ_OK;
 }
@@ -880,9 +881,13 @@ ZLayout z_layout(Arena& a, int M, int N, int K) {
 //   Taylor   ~16 launches of 6-10 us at least: n = 45, o = 9: 191 -> 140 us at 8 walkers, 4797 -> 1159 at 2048;
 //            n = 30: o = 7 66 -> 123 at 8, 237 -> 262 at 512 walkers, o = 10 179 -> 170 at 200, 411 -> 311 at 512;
 //            the binary64 kernel takes 32 orbitals a pass and eight columns a CTA.
+//   green    m and G_half cost 6 n o^2 binary64 FMAs a walker against a 128 x 64 tile each, the factorisation is the
+//            same: n = 60, o = 10 (n o^2 = 6000): 230 -> 401 us at 2048 walkers; 60, 20 (24000): 107 -> 99 at 8, 790 ->
+//            724 at 2048; 120, 20 (48000): 154 -> 105 at 8, 1287 -> 891 at 2048; 200, 30: 467 -> 176 at 8, 4526 -> 1863.
 //   energy   n = 8, o = 2, 40 vectors: 12 -> 24 us at 200 walkers, 64 -> 55 at 2048; n = 12, o = 6, 60 vectors: 27 ->
 //            29 at 8, 51 -> 34 at 200; n = 20, o = 5, 100 vectors: 41 -> 30 at 8, 547 -> 185 at 2048.
 bool zgemm_oz_pays(int M, int N, int K) { return M > 0 && N > 0 && K >= 1 && K <= 1 << 17 && M <= 65535 * 64; }
+bool green_oz_pays(int n, int o) { return n <= 512 && n * o * o >= 24000; }
 bool trotter_oz_pays(int W, int n, int o, int n_terms) {
     return W <= 65535 && n <= 512 && n_terms >= 1 && (n > 32 || (n >= 24 && o > 8 && W > 256));
 }
@@ -989,6 +994,61 @@ int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const do
         }
         const OzOut wo = {wout + w0 * no, 0, (long long)no, 1, o, o, 0, t.U};
         AFQ_TRY(oz_launch(n, 2 * wc * o, n, 1, 0, t.E, t.X, wo, 1, (n + 255) / 256, nullptr, err, s));
+    }
+    return AFQ_OK;
+}
+
+// ----------------------------------------------------------------- green --
+namespace {
+struct GrLayout {
+    int wc;
+    OzDigits C, X, A, B;  // trial columns, walker columns, walker rows, right operands W^T m^-1
+    double2 *m, *inv;
+};
+GrLayout gr_layout(Arena& a, int W, int n, int o) {
+    GrLayout g;
+    const long long per = 2LL * o * digit_row_bytes(n) + round_up(n, 8) * digit_row_bytes(2 * o) +
+                          round_up(2 * o, 8) * digit_row_bytes(2 * o) + 32LL * o * o;
+    long long wc = OZ_CAP / per;
+    if (wc < 1) wc = 1;
+    if (wc > W) wc = W;
+    g.wc = (int)wc;
+    g.C = take_digits(a, o, n);
+    g.X = take_digits(a, (size_t)wc * 2 * o, n);
+    g.A = take_digits(a, n, 2 * o, wc);
+    g.B = take_digits(a, 2 * o, 2 * o, wc);
+    g.m = a.take<double2>((size_t)wc * o * o);
+    g.inv = a.take<double2>((size_t)wc * o * o);
+    return g;
+}
+}  // namespace
+
+size_t green_oz_scratch(int W, int n, int o) {
+    Arena a;
+    gr_layout(a, W, n, o);
+    return a.used + 256;
+}
+
+// m = C^T W of all walkers as one product, its factorisations, and G_half[b, i] = sum_a W[i, a] m^-1[a, b] a walker
+int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walkers, double2* ovlp_out,
+                    double2* green_out, int ov_square, void* scratch, int* err, cudaStream_t s) {
+    if (W <= 0) return AFQ_OK;
+    Arena ar(scratch, (size_t)-1);
+    const GrLayout g = gr_layout(ar, W, n, o);
+    const size_t no = (size_t)n * o;
+    AFQ_TRY(split_cols(o, n, (const double*)mo, 2LL * o, g.C, s, 2));
+    for (int w0 = 0; w0 < W; w0 += g.wc) {
+        const int wc = W - w0 < g.wc ? W - w0 : g.wc;
+        const double2* w = walkers + w0 * no;
+        AFQ_TRY(launch_term<OZ_WALK>(wc, n, o, 0.0, w, nullptr, nullptr, g.X, s));
+        const OzOut mout = {g.m, 0, (long long)o * o, 1, o, o, 0, nullptr};
+        AFQ_TRY(oz_launch(o, 2 * wc * o, n, 1, 0, g.C, g.X, mout, 1, (n + 255) / 256, nullptr, err, s));
+        AFQ_TRY(launch_lu(wc, o, g.m, ovlp_out ? ovlp_out + w0 : nullptr, green_out ? g.inv : nullptr, ov_square, s));
+        if (!green_out) continue;
+        AFQ_TRY(split_rows((long long)wc * n, n, 2 * o, (const double*)w, 2 * o, g.A, s));
+        AFQ_TRY(launch_term<OZ_PLAIN>(wc, o, o, 0.0, g.inv, nullptr, nullptr, g.B, s));
+        const OzOut gout = {green_out + w0 * no, (long long)no, 0, n, 1, 2 * o, 0, nullptr};
+        AFQ_TRY(oz_launch(n, 2 * o, 2 * o, wc, 1, g.A, g.B, gout, 1, (2 * o + 255) / 256, nullptr, err, s));
     }
     return AFQ_OK;
 }

@@ -16,227 +16,6 @@ static int set_smem(K kernel, size_t bytes) {
 }
 
 // =====================================================================
-// Overlap matrix, determinant and half-rotated Green's function.
-//   m = C^H W (o x o); Gauss-Jordan with partial pivoting gives det(m) and
-//   m^-1; overlap = det(m)^2 (meas/rhf.py:22-24); G_half^T = W m^-1, i.e.
-//   G_half = solve(m^T, W^T) (meas/rhf.py:15-19).  One CTA per walker.
-// =====================================================================
-template <bool CR, int MA>
-__global__ void __launch_bounds__(256) k_green(int n, int o, const double2* __restrict__ mo,
-                                               const double2* __restrict__ walkers,
-                                               double2* __restrict__ ovlp_out,
-                                               double2* __restrict__ green_out, SplitOut split, int ov_square) {
-    extern __shared__ double2 sm[];
-    double2* m = sm;          // o x o
-    double2* inv = sm + o * o;  // o x o
-    __shared__ int s_piv, s_zero;
-    __shared__ double2 s_det;
-    const int w = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const double2* Wp = walkers + (size_t)w * n * o;
-
-    // m[a, b] = sum_i conj(C[i, a]) W[i, b]: thread <-> column b and rows
-    // a = ag + AG k, so each thread streams its column of W once (coalesced
-    // across b) and takes C from L1.
-    {
-        // MA >= ceil(o / AG) rows per thread, a template argument so that the
-        // accumulators stay in registers without inflating smaller cases
-        const int AG = blockDim.x / o;
-        const int b = tid % o, ag = tid / o;
-        double2 acc[MA];
-#pragma unroll
-        for (int k = 0; k < MA; ++k) acc[k] = make_double2(0.0, 0.0);
-        if (ag < AG) {
-            for (int i = 0; i < n; ++i) {
-                const double2 x = Wp[(size_t)i * o + b];
-#pragma unroll
-                for (int k = 0; k < MA; ++k) {
-                    const int a = ag + AG * k;
-                    if (a < o) {
-                        const double2 c = mo[i * o + a];
-                        if (CR) {
-                            rfma(acc[k], c.x, x);
-                        } else {
-                            acc[k].x = fma(c.x, x.x, acc[k].x); acc[k].x = fma(c.y, x.y, acc[k].x);
-                            acc[k].y = fma(c.x, x.y, acc[k].y); acc[k].y = fma(-c.y, x.x, acc[k].y);
-                        }
-                    }
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < MA; ++k) {
-                const int a = ag + AG * k;
-                if (a < o) m[a * o + b] = acc[k];
-            }
-        }
-        for (int e = tid; e < o * o; e += blockDim.x)
-            inv[e] = make_double2((e / o) == (e % o) ? 1.0 : 0.0, 0.0);
-    }
-    if (tid == 0) {
-        s_det = make_double2(1.0, 0.0);
-        s_zero = 0;
-    }
-    __syncthreads();
-
-    for (int k = 0; k < o; ++k) {
-        if (wid == 0) {
-            double best = -1.0;
-            int bi = k;
-            for (int r = k + lane; r < o; r += 32) {
-                double v = cabs2(m[r * o + k]);
-                if (v > best) { best = v; bi = r; }
-            }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                double ob = __shfl_xor_sync(0xffffffffu, best, off);
-                int oi = __shfl_xor_sync(0xffffffffu, bi, off);
-                if (ob > best || (ob == best && oi < bi)) { best = ob; bi = oi; }
-            }
-            if (lane == 0) s_piv = bi;
-        }
-        __syncthreads();
-        const int p = s_piv;
-        if (p != k) {
-            for (int j = tid; j < 2 * o; j += blockDim.x) {
-                double2* X = j < o ? m : inv;
-                int jj = j < o ? j : j - o;
-                double2 t = X[k * o + jj];
-                X[k * o + jj] = X[p * o + jj];
-                X[p * o + jj] = t;
-            }
-        }
-        __syncthreads();
-        const double2 piv = m[k * o + k];
-        if (tid == 0) {
-            double2 d = cmul(s_det, piv);
-            s_det = (p != k) ? make_double2(-d.x, -d.y) : d;
-            if (piv.x == 0.0 && piv.y == 0.0) s_zero = 1;
-        }
-        const double2 rp = cdiv(make_double2(1.0, 0.0), piv);
-        __syncthreads();
-        // scale pivot row (columns > k of m, all of inv)
-        for (int j = tid; j < 2 * o; j += blockDim.x) {
-            if (j < o) { if (j > k) m[k * o + j] = cmul(m[k * o + j], rp); }
-            else inv[k * o + (j - o)] = cmul(inv[k * o + (j - o)], rp);
-        }
-        __syncthreads();
-        // eliminate column k from every other row (column k of m is left as is)
-        for (int e = tid; e < o * 2 * o; e += blockDim.x) {
-            int r = e / (2 * o), j = e % (2 * o);
-            if (r == k) continue;
-            double2 f = m[r * o + k];
-            if (j < o) {
-                if (j > k) m[r * o + j] = csub(m[r * o + j], cmul(f, m[k * o + j]));
-            } else {
-                inv[r * o + (j - o)] = csub(inv[r * o + (j - o)], cmul(f, inv[k * o + (j - o)]));
-            }
-        }
-        __syncthreads();
-    }
-    // An exactly zero pivot (the rest of its column is zero too: m is singular)
-    // makes det(m) exactly 0, as LAPACK's LU gives it (getrf leaves the zero
-    // on U's diagonal); the division by it has made the inverse, and so the
-    // Green's function, non-finite, as the reference's solve does.
-    if (ovlp_out && tid == 0)
-        ovlp_out[w] = s_zero ? make_double2(0.0, 0.0) : ov_square ? cmul(s_det, s_det) : s_det;
-    if (!green_out && !split.ptr) return;
-    // G_half[b, i] = sum_a W[i, a] inv[a, b]
-    if (green_out) {
-        double2* Gp = green_out + (size_t)w * o * n;
-        for (int e = tid; e < n * o; e += blockDim.x) {
-            int b = e / n, i = e % n;
-            double2 acc = make_double2(0.0, 0.0);
-            for (int a = 0; a < o; ++a) cfma(acc, Wp[i * o + a], inv[a * o + b]);
-            Gp[e] = acc;
-        }
-    }
-    if (!split.ptr) return;
-    // Force-bias operand: the same product in fp32 (the bf16 hi/lo split that
-    // consumes it resolves ~2^-17), written as the split left operand.
-    __nv_bfloat16* re_row = split.ptr + (size_t)w * split.ld;
-    __nv_bfloat16* im_row = split.ptr + (size_t)(split.W + w) * split.ld;
-    float2* invf = (float2*)(inv + o * o);
-    for (int e = tid; e < o * o; e += blockDim.x) invf[e] = make_float2((float)inv[e].x, (float)inv[e].y);
-    __syncthreads();
-    {
-        constexpr int BG = 8;
-        const int nbg = (o + BG - 1) / BG;
-        for (int t = tid; t < n * nbg; t += blockDim.x) {
-            const int i = t % n, bg = t / n;
-            float2 acc[BG];
-#pragma unroll
-            for (int j = 0; j < BG; ++j) acc[j] = make_float2(0.f, 0.f);
-            for (int a = 0; a < o; ++a) {
-                const double2 wv = Wp[(size_t)i * o + a];
-                const float2 x = make_float2((float)wv.x, (float)wv.y);
-#pragma unroll
-                for (int j = 0; j < BG; ++j) {
-                    const int b = bg * BG + j;
-                    if (b < o) {
-                        const float2 v = invf[a * o + b];
-                        acc[j].x = fmaf(x.x, v.x, acc[j].x); acc[j].x = fmaf(-x.y, v.y, acc[j].x);
-                        acc[j].y = fmaf(x.x, v.y, acc[j].y); acc[j].y = fmaf(x.y, v.x, acc[j].y);
-                    }
-                }
-            }
-#pragma unroll
-            for (int j = 0; j < BG; ++j) {
-                const int b = bg * BG + j;
-                if (b < o) {
-                    split_store(re_row, split.S, b * n + i, (double)acc[j].x, true, split.sec);
-                    split_store(im_row, split.S, b * n + i, (double)acc[j].y, true, split.sec);
-                }
-            }
-        }
-    }
-    {  // zero the section gaps and the tail of the row
-        for (int e = n * o + tid; e < split.S; e += blockDim.x) {
-            split_store(re_row, split.S, e, 0.0, true, split.sec);
-            split_store(im_row, split.S, e, 0.0, true, split.sec);
-        }
-        for (long long e = (long long)split.sec * split.S + tid; e < split.ld; e += blockDim.x) {
-            re_row[e] = __double2bfloat16(0.0);
-            im_row[e] = __double2bfloat16(0.0);
-        }
-    }
-}
-
-int launch_green_split(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
-                       double2* ovlp_out, double2* green_out, SplitOut split, cudaStream_t s, int ov_square) {
-    if (W <= 0) return AFQ_OK;
-    size_t smem = 2 * (size_t)o * o * sizeof(double2) + (split.ptr ? (size_t)o * o * sizeof(float2) : 0);
-    const int ag = 256 / o, ma = (o + ag - 1) / ag;  // rows of m per thread
-#define AFQ_GREEN(CRV, MAV)                                                                  \
-    do {                                                                                     \
-        AFQ_TRY(set_smem(k_green<CRV, MAV>, smem));                                          \
-        k_green<CRV, MAV><<<W, 256, smem, s>>>(n, o, mo, walkers, ovlp_out, green_out, split, ov_square); \
-    } while (0)
-#define AFQ_GREEN_MA(CRV)                \
-    do {                                 \
-        if (ma <= 1) AFQ_GREEN(CRV, 1);  \
-        else if (ma <= 2) AFQ_GREEN(CRV, 2); \
-        else if (ma <= 4) AFQ_GREEN(CRV, 4); \
-        else if (ma <= 8) AFQ_GREEN(CRV, 8); \
-        else AFQ_GREEN(CRV, 16);         \
-    } while (0)
-    if (trial_real) AFQ_GREEN_MA(true);
-    else AFQ_GREEN_MA(false);
-#undef AFQ_GREEN_MA
-#undef AFQ_GREEN
-    AFQ_LAUNCHED("k_green");
-    return AFQ_OK;
-}
-
-int launch_green(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
-                 double2* ovlp_out, double2* green_out, cudaStream_t s) {
-    return launch_green_split(W, n, o, mo, trial_real, walkers, ovlp_out, green_out, SplitOut{}, s, 1);
-}
-
-int launch_green_det(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
-                     double2* det_out, double2* green_out, cudaStream_t s) {
-    return launch_green_split(W, n, o, mo, trial_real, walkers, det_out, green_out, SplitOut{}, s, 0);
-}
-
-// =====================================================================
 // Trotter propagation  E_half . sum_{k<=K} (i sqrt_dt V)^k / k! . E_half . W
 // (prop/chol_afqmc_ops.py:173-183, prop/utils.py:20-31).  Walker columns are
 // independent, so a CTA owns (walker, OC columns): the current Taylor term
