@@ -307,9 +307,11 @@ size_t green_oz_scratch(int W, int n, int o);
 int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walkers, double2* ovlp_out,
                     double2* green_out, int ov_square, void* scratch, int* err, cudaStream_t s);
 bool trotter_oz_pays(int W, int n, int o, int n_terms);
-size_t trotter_oz_scratch(int W, int n, int o, int vdiv);
+size_t trotter_oz_scratch(int W, int n, int o, int ns);
+bool trotter_oz_whole(int W, int n);  // all walkers in one chunk of the scratch
 int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
-                      const double2* win, double2* wout, int vdiv, void* scratch, int* err, cudaStream_t s);
+                      const double2* win, double2* wout, int ns, long long ws, long long ss, void* scratch, int* err,
+                      cudaStream_t s);
 bool energy_oz_pays(int W, int n, int o, int G);
 size_t energy_oz_scratch(int W, int n, int o, int G);
 int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, const double* rot_chol,
@@ -319,6 +321,9 @@ int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64
                       bool b_complex, bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s);
 int launch_trotter_auto(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
                         const double2* win, double2* wout, int vdiv, const OzScratch& oz, cudaStream_t s);
+// both spins of W walkers with the walker's V, the second spin's blocks `half` entries after the first's
+int launch_trotter_spins(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
+                         const double2* win, double2* wout, size_t half, const OzScratch& oz, cudaStream_t s);
 int launch_energy_partial_auto(int W, int n, int o, int G, const double2* green, const void* rot_chol, int trial_real,
                                double* partial, const OzScratch& oz, cudaStream_t s);
 

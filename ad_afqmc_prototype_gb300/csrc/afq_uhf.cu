@@ -130,7 +130,7 @@ UWS layout_u(Arena& a, const afq_dims* d, int n_chunks) {
     u.oz.p = a.take<char>(oz_most({green_oz_scratch(2 * d->n_walkers, d->norb, d->nocc),
                                    zgemm_oz_scratch(2 * d->n_walkers, d->nchol, (int)no),
                                    zgemm_oz_scratch(wc, (int)(n * n), d->nchol),
-                                   trotter_oz_scratch(wc, d->norb, d->nocc, 1),
+                                   trotter_oz_scratch(wc, d->norb, d->nocc, 2),
                                    energy_oz_scratch(2 * d->n_walkers, d->norb, d->nocc, d->nchol)}));
     u.oz.err = u.status;
     u.partial = (double*)a.take<double2>(energy_partial_count(2 * d->n_walkers, d->nocc, d->nchol));
@@ -181,9 +181,8 @@ int trotter_u(const afq_dims* d, int n_terms, double sqrt_dt, int n_chunks, cons
           AFQ_TRY(launch_zgemm_auto(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, V,
                                     (int64_t)n * n, oz, s)); }
         AFQ_PHASE("trotter", s);
-        for (int spin = 0; spin < 2; ++spin)
-            AFQ_TRY(launch_trotter_auto(wc, n, o, n_terms, sqrt_dt, E, V, win + spin * half + (size_t)w0 * n * o,
-                                        wout + spin * half + (size_t)w0 * n * o, 1, oz, s));
+        AFQ_TRY(launch_trotter_spins(wc, n, o, n_terms, sqrt_dt, E, V, win + (size_t)w0 * n * o, wout + (size_t)w0 * n * o,
+                                     half, oz, s));
     }
     return AFQ_OK;
 }
@@ -306,7 +305,7 @@ GWS layout_g(Arena& a, const afq_dims* d, int n_chunks) {
     g.oz.p = a.take<char>(oz_most({green_oz_scratch(d->n_walkers, 2 * d->norb, 2 * d->nocc),
                                    zgemm_oz_scratch(d->n_walkers, d->nchol, (int)(n * o)),
                                    zgemm_oz_scratch(wc, (int)(n * n), d->nchol),
-                                   trotter_oz_scratch(2 * wc, d->norb, 2 * d->nocc, 2)}));
+                                   trotter_oz_scratch(wc, d->norb, 2 * d->nocc, 2)}));
     g.oz.err = g.status;
     return g;
 }

@@ -627,7 +627,9 @@ __global__ void __launch_bounds__(256) k_oz_cols(int rows, int K, const double* 
     }
 }
 
-// Walker-shaped blocks (w, j, c), c fastest, eight columns c a CTA:
+// Walker-shaped blocks (j, c), c fastest, `ws` entries apart, eight columns c
+// a CTA.  Two blocks `ss` apart may be taken as one of 2 `on` columns (the two
+// spins, or halves, that share a V: their products fill one tile's columns):
 //   WALK  digits of the block's columns over j, rows (w, c, part)
 //   PLAIN digits of T = Y as the right operand of V T
 //   INIT  T = W + Y; U = T; digits of T as the right operand of V T
@@ -638,7 +640,7 @@ __global__ void __launch_bounds__(256) k_oz_cols(int rows, int K, const double* 
 enum { OZ_WALK, OZ_PLAIN, OZ_INIT, OZ_TERM, OZ_LAST };
 constexpr int OZ_CB = 8;
 template <int MODE>
-__global__ void __launch_bounds__(256) k_oz_term(int n, int o, int ncg, double s, const double2* __restrict__ Y,
+__global__ void __launch_bounds__(256) k_oz_term(int n, int o, int on, long long ws, long long ss, int ncg, double s, const double2* __restrict__ Y,
                                                  const double2* __restrict__ W, double2* __restrict__ U, OzDst dst, int* __restrict__ ex) {
     extern __shared__ double2 sh[];  // OZ_CB x (n + 1)
     __shared__ int se[2 * OZ_CB];
@@ -648,8 +650,9 @@ __global__ void __launch_bounds__(256) k_oz_term(int n, int o, int ncg, double s
     __syncthreads();
     int e0 = 0, e1 = 0;
     if (c0 + c < o) {
+        const int spin = c0 + c >= on;
         for (int j = tid / OZ_CB; j < n; j += 256 / OZ_CB) {
-            const long long at = ((long long)w * n + j) * o + c0 + c;
+            const long long at = w * ws + (long long)j * on + (c0 + c - spin * on) + spin * ss;
             double2 t = Y[at];
             if (MODE == OZ_TERM || MODE == OZ_LAST) {
                 t = make_double2(-s * t.y, s * t.x);
@@ -712,40 +715,60 @@ __global__ void __launch_bounds__(256) k_oz_term(int n, int o, int ncg, double s
     }
 }
 
+__device__ __forceinline__ void cfma2(double& re, double& im, double2 a, double2 b) {
+    re = fma(a.x, b.x, re);
+    im = fma(a.x, b.y, im);
+    re = fma(-a.y, b.y, re);
+    im = fma(a.y, b.x, im);
+}
+
 // Coulomb and exchange partials of a chunk of ng Cholesky vectors from F
 // (rows (w, k), columns (g, i): f_g[i, k]), as launch_energy_partial's:
 // partial[w, chunk] = (sum_g (tr f_g)^2, sum_g sum_ik f_g[i, k] f_g[k, i]).
+// Its floor is the binary64 pipe: four FMAs a pair i < k.
 __global__ void __launch_bounds__(256) k_oz_exchange(int o, int G, int NG, const double2* __restrict__ F,
                                                      double2* __restrict__ partial) {
     extern __shared__ double2 sh[];  // NG blocks of o x (o + 1)
     const int nchunk = gridDim.x, w = blockIdx.y, g0 = blockIdx.x * NG, ng = min(NG, G - g0), tid = threadIdx.x;
+    const int lane = tid & 31, wid = tid >> 5;
     const int pitch = o + 1, gi = ng * o;
     const double2* Fw = F + (long long)w * o * G * o + (long long)g0 * o;
-    for (int e = tid; e < gi * o; e += 256) {
-        const int k = e / gi, x = e - k * gi, g = x / o, i = x - g * o;
-        sh[(g * o + k) * pitch + i] = Fw[(long long)k * G * o + x];
+    const float io = 1.0f / o;  // quotients of small integers below: (x + 0.5) / o is never within rounding of an integer
+    for (int x = tid; x < gi; x += 256) {
+        const int g = (int)((x + 0.5f) * io), i = x - g * o;
+        const double2* src = Fw + x;
+        double2* dst = sh + g * o * pitch + i;
+#pragma unroll 8
+        for (int k = 0; k < o; ++k) dst[k * pitch] = src[(long long)k * G * o];
     }
     __syncthreads();
     double cr = 0.0, ci = 0.0, xr = 0.0, xi = 0.0;
-    // f[i, k] f[k, i] once for i < k, doubled; the diagonal's squares
-    for (int e = tid; e < gi * o; e += 256) {
-        const int g = e / (o * o), rem = e - g * o * o, k = rem / o, i = rem - k * o;
-        if (i > k) continue;
-        const double2 p = cmul(sh[(g * o + k) * pitch + i], sh[(g * o + i) * pitch + k]);
-        const double f = i == k ? 1.0 : 2.0;
-        xr = fma(f, p.x, xr);
-        xi = fma(f, p.y, xi);
+    // sum over i < k of f[i, k] f[k, i], doubled below, a warp a vector: rows k = r and o - 1 - r hold o - 1 such pairs
+    // together (the middle row of an odd o half of that)
+    const int half = (o + 1) / 2, per = o > 1 ? o - 1 : 1, mid = o & 1 ? half - 1 : -1;
+    const float ip = 1.0f / per;
+    for (int g = wid; g < ng; g += 8) {
+        const double2* f = sh + g * o * pitch;
+        for (int e = lane; e < half * per; e += 32) {
+            const int r = (int)((e + 0.5f) * ip), c = e - r * per, hi = o - 1 - r;
+            const int k = c < hi ? hi : r, i = c < hi ? c : c - hi;
+            if (i >= k || (r == mid && c >= hi)) continue;
+            cfma2(xr, xi, f[k * pitch + i], f[i * pitch + k]);
+        }
+    }
+    xr *= 2.0;
+    xi *= 2.0;
+    for (int e = tid; e < gi; e += 256) {
+        const double2 f = sh[e * pitch + (e - (int)((e + 0.5f) * io) * o)];
+        cfma2(xr, xi, f, f);
     }
     for (int g = tid; g < ng; g += 256) {
         double2 c = make_double2(0.0, 0.0);
         for (int i = 0; i < o; ++i) c = cadd(c, sh[(g * o + i) * pitch + i]);
-        const double2 c2 = cmul(c, c);
-        cr += c2.x;
-        ci += c2.y;
+        cfma2(cr, ci, c, c);
     }
     cr = warp_sum(cr); ci = warp_sum(ci); xr = warp_sum(xr); xi = warp_sum(xi);
     __shared__ double red[8][4];
-    const int lane = tid & 31, wid = tid >> 5;
     if (lane == 0) {
         red[wid][0] = cr; red[wid][1] = ci; red[wid][2] = xr; red[wid][3] = xi;
     }
@@ -936,64 +959,77 @@ struct TrLayout {
     OzDigits E, V, T, X;  // E_half, V rows, right operands of V T, walker columns
     double2 *Y, *U;
 };
-TrLayout tr_layout(Arena& a, int W, int n, int o, int vdiv) {
+// W walkers of ns blocks (n x o) each
+TrLayout tr_layout(Arena& a, int W, int n, int o, int ns) {
     TrLayout t;
     const long long per = round_up(n, 8) * digit_row_bytes(2 * n);  // digits of one V
-    long long wc = OZ_CAP / per / vdiv * vdiv * vdiv;               // walkers whose V digits fit
-    if (wc < vdiv) wc = vdiv;
+    long long wc = OZ_CAP / per;                                    // walkers whose V digits fit
+    if (wc < 1) wc = 1;
     if (wc > W) wc = W;
     t.wc = (int)wc;
+    const size_t nb = (size_t)t.wc * ns;
     t.E = take_digits(a, n, n);
-    t.V = take_digits(a, n, 2 * n, (t.wc + vdiv - 1) / vdiv);
-    t.T = take_digits(a, 2 * o, 2 * n, t.wc);
-    t.X = take_digits(a, (size_t)t.wc * 2 * o, n);
-    t.Y = a.take<double2>((size_t)t.wc * n * o);
-    t.U = a.take<double2>((size_t)t.wc * n * o);
+    t.V = take_digits(a, n, 2 * n, t.wc);
+    t.T = take_digits(a, 2 * ns * o, 2 * n, t.wc);
+    t.X = take_digits(a, nb * 2 * o, n);
+    t.Y = a.take<double2>(nb * n * o);
+    t.U = a.take<double2>(nb * n * o);
     return t;
 }
+// W blocks of o columns, ns of them taken together (block strides ws, ss)
 template <int MODE>
 int launch_term(int W, int n, int o, double s, const double2* Y, const double2* X, double2* U, const OzDigits& D,
-                cudaStream_t st) {
-    const int ncg = (o + OZ_CB - 1) / OZ_CB, smem = OZ_CB * (n + 1) * (int)sizeof(double2);
+                cudaStream_t st, int ns = 1, long long ws = 0, long long ss = 0) {
+    const int oc = o * ns, ncg = (oc + OZ_CB - 1) / OZ_CB, smem = OZ_CB * (n + 1) * (int)sizeof(double2);
+    if (ns == 1) ws = (long long)n * o;
     AFQ_TRY(raise_smem_once(g_ozterm[MODE], k_oz_term<MODE>, OZ_CB * 513 * (int)sizeof(double2)));
-    const OzDst dst = MODE == OZ_WALK || MODE == OZ_LAST ? dst_of(D, 2LL * W * o, n) : dst_of(D, 2 * o, 2 * n);
-    k_oz_term<MODE><<<(unsigned)W * ncg, 256, smem, st>>>(n, o, ncg, s, Y, X, U, dst, D.ex);
+    const OzDst dst = MODE == OZ_WALK || MODE == OZ_LAST ? dst_of(D, 2LL * W * oc, n) : dst_of(D, 2 * oc, 2 * n);
+    k_oz_term<MODE><<<(unsigned)W * ncg, 256, smem, st>>>(n, oc, o, ws, ss, ncg, s, Y, X, U, dst, D.ex);
     AFQ_LAUNCHED("k_oz_term");
     return AFQ_OK;
 }
 }  // namespace
 
-size_t trotter_oz_scratch(int W, int n, int o, int vdiv) {
+size_t trotter_oz_scratch(int W, int n, int o, int ns) {
     Arena a;
-    tr_layout(a, W, n, o, vdiv);
+    tr_layout(a, W, n, o, ns);
     return a.used + 256;
 }
+bool trotter_oz_whole(int W, int n) {
+    Arena a;
+    return tr_layout(a, W, n, 1, 1).wc == W;
+}
 
-// E_half . sum_{k <= K} (i sqrt_dt V)^k / k! . E_half . W, n_terms >= 1.
+// E_half . sum_{k <= K} (i sqrt_dt V)^k / k! . E_half . X, n_terms >= 1, of the
+// ns blocks X of each walker, which share its V: block p of walker w is n x o at
+// w ws + p ss (ns = 2: ws = 2 n o, ss = n o, or ws = n o, ss = W n o where
+// trotter_oz_whole).
 // E_half X is formed as X + (E_half - I) X: E_half is close to the identity,
 // and a digit product's error scales with its operands' largest entries.
 int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
-                      const double2* win, double2* wout, int vdiv, void* scratch, int* err, cudaStream_t s) {
+                      const double2* win, double2* wout, int ns, long long ws, long long ss, void* scratch, int* err,
+                      cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
     Arena ar(scratch, (size_t)-1);
-    const TrLayout t = tr_layout(ar, W, n, o, vdiv);
+    const TrLayout t = tr_layout(ar, W, n, o, ns);
     AFQ_TRY(split_rows(n, n, n, E, n, t.E, s, 1));
     const size_t no = (size_t)n * o;
     for (int w0 = 0; w0 < W; w0 += t.wc) {
-        const int wc = W - w0 < t.wc ? W - w0 : t.wc, nv = (wc + vdiv - 1) / vdiv;
-        AFQ_TRY(split_rows((long long)nv * n, n, 2 * n, (const double*)(V + (size_t)(w0 / vdiv) * n * n), 2 * n, t.V, s));
-        AFQ_TRY(launch_term<OZ_WALK>(wc, n, o, 0.0, win + w0 * no, nullptr, nullptr, t.X, s));
+        const int wc = W - w0 < t.wc ? W - w0 : t.wc, nb = wc * ns;  // the chunk's blocks are contiguous
+        const double2* x = win + (size_t)w0 * ns * no;
+        AFQ_TRY(split_rows((long long)wc * n, n, 2 * n, (const double*)(V + (size_t)w0 * n * n), 2 * n, t.V, s));
+        AFQ_TRY(launch_term<OZ_WALK>(nb, n, o, 0.0, x, nullptr, nullptr, t.X, s));
         const OzOut xo = {t.Y, 0, (long long)no, 1, o, o, 0, nullptr};
-        AFQ_TRY(oz_launch(n, 2 * wc * o, n, 1, 0, t.E, t.X, xo, 1, (n + 255) / 256, nullptr, err, s));
-        AFQ_TRY(launch_term<OZ_INIT>(wc, n, o, 0.0, t.Y, win + w0 * no, t.U, t.T, s));
+        AFQ_TRY(oz_launch(n, 2 * nb * o, n, 1, 0, t.E, t.X, xo, 1, (n + 255) / 256, nullptr, err, s));
+        AFQ_TRY(launch_term<OZ_INIT>(wc, n, o, 0.0, t.Y, x, t.U, t.T, s, ns, ws, ss));
         for (int k = 1; k <= n_terms; ++k) {
-            const OzOut to = {t.Y, (long long)no, 0, 1, o, 2 * o, 0, nullptr};
-            AFQ_TRY(oz_launch(n, 2 * o, 2 * n, wc, vdiv, t.V, t.T, to, 1, (2 * n + 255) / 256, nullptr, err, s));
-            if (k < n_terms) AFQ_TRY(launch_term<OZ_TERM>(wc, n, o, sqrt_dt / k, t.Y, nullptr, t.U, t.T, s));
-            else AFQ_TRY(launch_term<OZ_LAST>(wc, n, o, sqrt_dt / k, t.Y, nullptr, t.U, t.X, s));
+            const OzOut to = {t.Y, ns == 1 ? (long long)no : ws, ss, 1, o, o, 0, nullptr};
+            AFQ_TRY(oz_launch(n, 2 * ns * o, 2 * n, wc, 1, t.V, t.T, to, 1, (2 * n + 255) / 256, nullptr, err, s));
+            if (k < n_terms) AFQ_TRY(launch_term<OZ_TERM>(wc, n, o, sqrt_dt / k, t.Y, nullptr, t.U, t.T, s, ns, ws, ss));
+            else AFQ_TRY(launch_term<OZ_LAST>(nb, n, o, sqrt_dt / k, t.Y, nullptr, t.U, t.X, s));
         }
-        const OzOut wo = {wout + w0 * no, 0, (long long)no, 1, o, o, 0, t.U};
-        AFQ_TRY(oz_launch(n, 2 * wc * o, n, 1, 0, t.E, t.X, wo, 1, (n + 255) / 256, nullptr, err, s));
+        const OzOut wo = {wout + (size_t)w0 * ns * no, 0, (long long)no, 1, o, o, 0, t.U};
+        AFQ_TRY(oz_launch(n, 2 * nb * o, n, 1, 0, t.E, t.X, wo, 1, (n + 255) / 256, nullptr, err, s));
     }
     return AFQ_OK;
 }
@@ -1111,9 +1147,20 @@ int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64
 
 int launch_trotter_auto(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
                         const double2* win, double2* wout, int vdiv, const OzScratch& oz, cudaStream_t s) {
+    const long long no = (long long)n * o;
     if (trotter_oz_pays(W, n, o, n_terms))
-        return launch_trotter_oz(W, n, o, n_terms, sqrt_dt, E, V, win, wout, vdiv, oz.p, oz.err, s);
+        return launch_trotter_oz(W / vdiv, n, o, n_terms, sqrt_dt, E, V, win, wout, vdiv, vdiv * no, no, oz.p, oz.err, s);
     return launch_trotter(W, n, o, n_terms, sqrt_dt, E, V, win, wout, s, vdiv);
+}
+
+int launch_trotter_spins(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
+                         const double2* win, double2* wout, size_t half, const OzScratch& oz, cudaStream_t s) {
+    const long long no = (long long)n * o;
+    if (trotter_oz_pays(W, n, o, n_terms) && (long long)half == W * no && trotter_oz_whole(W, n))
+        return launch_trotter_oz(W, n, o, n_terms, sqrt_dt, E, V, win, wout, 2, no, W * no, oz.p, oz.err, s);
+    for (int spin = 0; spin < 2; ++spin)
+        AFQ_TRY(launch_trotter_auto(W, n, o, n_terms, sqrt_dt, E, V, win + spin * half, wout + spin * half, 1, oz, s));
+    return AFQ_OK;
 }
 
 int launch_energy_partial_auto(int W, int n, int o, int G, const double2* green, const void* rot_chol, int trial_real,

@@ -68,3 +68,25 @@ def test_digit_products_keep_nonfinite_rows_apart(bad):
     assert not torch.isfinite(torch.view_as_real(out[2])).any()
     keep = [i for i in range(W) if i != 2]
     assert _rel(out[keep], want[keep]) < RTOL
+
+
+@pytest.mark.parametrize("n,o,W", [(33, 5, 3), (61, 9, 17), (64, 17, 4), (130, 33, 2)])
+def test_blocks_sharing_a_v_match_single_ones(n, o, W):
+    """Two spins (or halves) taken as one tile's columns give each column what it gets alone, bit for bit."""
+    G = 40
+    h1, chol, mo, w, xs = _problem(n, o, G, 2 * W)
+    pctx = O.build_prop_ctx(0.0, h1, chol, O.get_rdm1(mo.astype(complex)), 0.005)
+    x, L, e = _dev(xs[:W], torch.complex128), _dev(chol), _dev(pctx.exp_h1_half)
+    pair = _dev(w, torch.complex128).reshape(2, W, n, o)
+    both = engine.apply_trotter_u(pair, x, L, e, pctx.sqrt_dt, 6)
+    for spin in range(2):
+        one = engine.apply_trotter(pair[spin].contiguous(), x, L, e, pctx.sqrt_dt, 6)
+        assert torch.equal(both[spin], one)
+    if o % 2 == 0 or o > 32:
+        return
+    c = o - 1  # a generalized walker's halves are n x 2 nocc
+    halves = pair[:, :, :, :c].permute(1, 0, 2, 3).contiguous()
+    g = engine.apply_trotter_g(halves.reshape(W, 2 * n, c), x, L, e, pctx.sqrt_dt, 6).reshape(W, 2, n, c)
+    for p in range(2):
+        one = engine.apply_trotter(halves[:, p].contiguous(), x, L, e, pctx.sqrt_dt, 6)
+        assert torch.equal(g[:, p], one)
