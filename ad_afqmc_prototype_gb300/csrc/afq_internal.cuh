@@ -306,12 +306,15 @@ bool green_oz_pays(int n, int o);
 size_t green_oz_scratch(int W, int n, int o);
 int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walkers, double2* ovlp_out,
                     double2* green_out, int ov_square, void* scratch, int* err, cudaStream_t s);
-bool trotter_oz_pays(int W, int n, int o, int n_terms);
 size_t trotter_oz_scratch(int W, int n, int o, int ns);
 bool trotter_oz_whole(int W, int n);  // all walkers in one chunk of the scratch
 int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
                       const double2* win, double2* wout, int ns, long long ws, long long ss, void* scratch, int* err,
                       cudaStream_t s);
+// k_trotter_oz.cu : the same in one kernel a walker, n <= 64
+bool trotter_small_fits(int n, int oc, int n_terms);
+int launch_trotter_small(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
+                         const double2* win, double2* wout, int ns, long long ws, long long ss, cudaStream_t s);
 bool energy_oz_pays(int W, int n, int o, int G);
 size_t energy_oz_scratch(int W, int n, int o, int G);
 int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, const double* rot_chol,

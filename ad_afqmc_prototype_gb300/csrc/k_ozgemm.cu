@@ -42,6 +42,7 @@
 // core's collector buffer: 35 clocks an MMA of 128 x 64 x 16 against 48 (the
 // operands' shared-memory reads), as issued from resident operands.
 #include "afq_internal.cuh"
+#include "oz_digits.cuh"
 #include "tc_common.cuh"
 
 namespace afq {
@@ -50,7 +51,6 @@ namespace {
 
 using namespace tc;
 
-constexpr int OZ_S = 7;                   // digits
 constexpr int OZ_ROWS = 128;              // real-operand rows a tile (tensor-memory lanes)
 constexpr int OZ_BK = 32;                 // K a stage: one 64-byte swizzle row
 constexpr int OZ_TN = 64;                 // complex-operand digit rows a tile
@@ -66,7 +66,6 @@ enum { OZ_D5, OZ_D4, OZ_D1, OZ_D0, OZ_D3, OZ_D2 = 6, OZ_SLOTS = 8 };
 constexpr uint32_t OZ_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(OZ_TN >> 3) << 17) |
                               ((uint32_t)(OZ_ROWS >> 4) << 24);
 static_assert(OZ_GSMEM <= 227 * 1024, "digit GEMM shared memory");
-constexpr int OZ_NAN = 0x7fffffff;        // scale of a row holding inf or nan
 
 __device__ __forceinline__ void oz_copy(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
@@ -82,27 +81,6 @@ __device__ __forceinline__ uint64_t desc_k64(uint32_t saddr) {
     d |= (uint64_t)1 << 46;
     d |= (uint64_t)4 << 61;
     return d;
-}
-
-// (acc 2^-32 + tail) 2^ex in binary64, rounded to nearest even, by integer
-// operations (the binary64 pipe converts two a clock an SM): acc is shifted up
-// until it or the tail's last bits fill 62 bits, and the tail added there.
-__device__ __forceinline__ double oz_to_double(long long acc, float tail, int ex) {
-    const unsigned long long am = acc < 0 ? 0ull - (unsigned long long)acc : (unsigned long long)acc;
-    const int te = (int)((__float_as_uint(tail) >> 23) & 255u) - 127;  // |tail| < 2^(te + 1)
-    const int sh = min(am ? __clzll((long long)am) - 2 : 62, 29 - te);
-    const long long v = (long long)((unsigned long long)acc << sh) + __float2ll_rn(tail * __int_as_float((127 + 32 + sh) << 23));
-    const unsigned long long sign = (unsigned long long)v & 0x8000000000000000ull;
-    const unsigned long long mag = sign ? 0ull - (unsigned long long)v : (unsigned long long)v;
-    if (mag == 0) return 0.0;
-    const int lz = __clzll((long long)mag);
-    const unsigned long long nrm = mag << lz;
-    const unsigned long long m = (nrm >> 11) + (((nrm & 0x7ffull) + ((nrm >> 11) & 1ull)) > 0x400ull ? 1ull : 0ull);
-    const int e = 63 - lz + ex - 32 - sh + 1023;
-    if (e <= 0) return __longlong_as_double((long long)sign);
-    const unsigned long long bits = ((unsigned long long)(e - 1) << 52) + m;  // m carries its leading bit
-    if (e >= 2047) return __longlong_as_double((long long)(sign | 0x7ff0000000000000ull));
-    return __longlong_as_double((long long)(sign | bits));
 }
 
 // Where output (row r, complex column m) of batch b goes: C[b bs + (m / md)
@@ -472,48 +450,6 @@ __global__ void k_oz_finish(const OzArgs a) {
 }
 
 // ------------------------------------------------------------------ digits --
-__device__ __forceinline__ int oz_expo(double x) {  // biased binary64 exponent
-    return (int)(((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ffu);
-}
-// scale of a row whose largest biased exponent is eb: |x| < 2^E
-__device__ __forceinline__ int oz_scale(int eb) { return eb == 0x7ff ? OZ_NAN : eb - 1022; }
-
-// x 2^(55 - E) rounded to an integer, |.| <= 2^55, plus 0x808080808080, whose
-// low six bytes are then the lower digits plus 128 (zero for subnormal x and
-// in a row of scale OZ_NAN).
-__device__ __forceinline__ long long oz_fix(double x, int E) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(x);
-    const int eb = (int)((u >> 52) & 0x7ffu);
-    long long y = 0;
-    if (eb != 0 && E != OZ_NAN) {
-        const unsigned long long m = (u & 0xfffffffffffffull) | (1ull << 52);
-        const int r = E + 1020 - eb;  // right shift, >= -2
-        if (r <= 0) y = (long long)(m << (-r));
-        else if (r < 60) y = (long long)((m + (1ull << (r - 1))) >> r);
-        if ((long long)u < 0) y = -y;
-    }
-    return y + 0x0000808080808080ll;
-}
-// digit s of y (from oz_fix) times 2^(-8 s), exact in fp32 and bf16
-template <int S>
-__device__ __forceinline__ float oz_dig(long long y) {
-    constexpr float sc = 1.0f / (float)(1ull << (8 * S));
-    if (S == 0) {  // the top digit, in [-128, 128]
-        const uint32_t t = (uint32_t)((int)(y >> 48) + 256);
-        return __uint_as_float(0x4B000000u | t) - 8388864.f;
-    }
-    const uint32_t t = (uint32_t)((unsigned long long)y >> (48 - 8 * S)) & 255u;
-    return fmaf(__uint_as_float(0x4B000000u | t), sc, -8388736.f * sc);
-}
-__device__ __forceinline__ uint32_t oz_pack(float lo, float hi) {
-    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-    return *(const uint32_t*)&v;
-}
-template <int S>
-__device__ __forceinline__ uint4 oz_pack8(const long long (&y)[8]) {
-    return make_uint4(oz_pack(oz_dig<S>(y[0]), oz_dig<S>(y[1])), oz_pack(oz_dig<S>(y[2]), oz_dig<S>(y[3])),
-                      oz_pack(oz_dig<S>(y[4]), oz_dig<S>(y[5])), oz_pack(oz_dig<S>(y[6]), oz_dig<S>(y[7])));
-}
 // A digit array: [batch][32 k][digit] planes of r8 rows x 64 bytes.
 struct OzDst {
     uint8_t* d;
@@ -901,9 +837,11 @@ ZLayout z_layout(Arena& a, int M, int N, int K) {
 // to refuse).  Measured in captured graphs, binary64 pipe -> digits:
 //   GEMM     wins from the smallest (M x N x K 5 x 7 x 1: 36 -> 21 us with launches; 64 x 144 x 48: 103 -> 28;
 //            1024 x 600 x 2400: 9.6 -> 0.32 ms; 1024 x 1000 x 6000: 24 -> 0.78 ms).
-//   Taylor   ~16 launches of 6-10 us at least: n = 45, o = 9: 191 -> 140 us at 8 walkers, 4797 -> 1159 at 2048;
-//            n = 30: o = 7 66 -> 123 at 8, 237 -> 262 at 512 walkers, o = 10 179 -> 170 at 200, 411 -> 311 at 512;
-//            the binary64 kernel takes 32 orbitals a pass and eight columns a CTA.
+//   Taylor   one kernel a walker (k_trotter_oz.cu) against the binary64 kernel: n = 5, o = 2: 21 -> 24 us at 200
+//            walkers, 117 -> 33 at 2048; n = 8, o = 2: 26 -> 23 at 8; n = 30, o = 7: 66 -> 36 at 8, 120 -> 44 at 200,
+//            817 -> 191 at 2048.  Tiles of all walkers (16 launches at least) against one kernel a walker: n = 45, o =
+//            9: 218 / 94 at 200, 1177 / 649 at 2048; n = 60, o = 10: 168 / 92 at 8, 1317 / 1289 at 2048; n = 61, o =
+//            18: 170 / 136 at 8, 270 / 272 at 200, 1671 / 1935 at 2048 (mma.sync runs at a ninth of tcgen05's rate).
 //   green    m and G_half cost 6 n o^2 binary64 FMAs a walker against a 128 x 64 tile each, the factorisation is the
 //            same: n = 60, o = 10 (n o^2 = 6000): 230 -> 401 us at 2048 walkers; 60, 20 (24000): 107 -> 99 at 8, 790 ->
 //            724 at 2048; 120, 20 (48000): 154 -> 105 at 8, 1287 -> 891 at 2048; 200, 30: 467 -> 176 at 8, 4526 -> 1863.
@@ -911,8 +849,10 @@ ZLayout z_layout(Arena& a, int M, int N, int K) {
 //            29 at 8, 51 -> 34 at 200; n = 20, o = 5, 100 vectors: 41 -> 30 at 8, 547 -> 185 at 2048.
 bool zgemm_oz_pays(int M, int N, int K) { return M > 0 && N > 0 && K >= 1 && K <= 1 << 17 && M <= 65535 * 64; }
 bool green_oz_pays(int n, int o) { return n <= 512 && n * o * o >= 24000; }
-bool trotter_oz_pays(int W, int n, int o, int n_terms) {
-    return W <= 65535 && n <= 512 && n_terms >= 1 && (n > 32 || (n >= 24 && o > 8 && W > 256));
+bool trotter_oz_pays(int W, int n, int n_terms) { return W <= 65535 && n > 32 && n <= 512 && n_terms >= 1; }
+// W walkers, oc columns each
+bool trotter_small_pays(int W, int n, int oc, int n_terms) {
+    return W <= 65535 && trotter_small_fits(n, oc, n_terms) && (n <= 48 || oc <= 10 || W <= 152) && (n >= 8 || W > 256);
 }
 bool energy_oz_pays(int W, int n, int o, int G) {
     const int nchunk = energy_partial_chunks(o, G), ng = (G + nchunk - 1) / nchunk;
@@ -1148,15 +1088,20 @@ int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64
 int launch_trotter_auto(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
                         const double2* win, double2* wout, int vdiv, const OzScratch& oz, cudaStream_t s) {
     const long long no = (long long)n * o;
-    if (trotter_oz_pays(W, n, o, n_terms))
-        return launch_trotter_oz(W / vdiv, n, o, n_terms, sqrt_dt, E, V, win, wout, vdiv, vdiv * no, no, oz.p, oz.err, s);
+    const int wp = W / vdiv;  // walkers (blocks that share a V)
+    if (trotter_small_pays(wp, n, o * vdiv, n_terms))
+        return launch_trotter_small(wp, n, o, n_terms, sqrt_dt, E, V, win, wout, vdiv, vdiv * no, no, s);
+    if (trotter_oz_pays(W, n, n_terms))
+        return launch_trotter_oz(wp, n, o, n_terms, sqrt_dt, E, V, win, wout, vdiv, vdiv * no, no, oz.p, oz.err, s);
     return launch_trotter(W, n, o, n_terms, sqrt_dt, E, V, win, wout, s, vdiv);
 }
 
 int launch_trotter_spins(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
                          const double2* win, double2* wout, size_t half, const OzScratch& oz, cudaStream_t s) {
     const long long no = (long long)n * o;
-    if (trotter_oz_pays(W, n, o, n_terms) && (long long)half == W * no && trotter_oz_whole(W, n))
+    if (trotter_small_pays(W, n, 2 * o, n_terms))
+        return launch_trotter_small(W, n, o, n_terms, sqrt_dt, E, V, win, wout, 2, no, (long long)half, s);
+    if (trotter_oz_pays(W, n, n_terms) && (long long)half == W * no && trotter_oz_whole(W, n))
         return launch_trotter_oz(W, n, o, n_terms, sqrt_dt, E, V, win, wout, 2, no, W * no, oz.p, oz.err, s);
     for (int spin = 0; spin < 2; ++spin)
         AFQ_TRY(launch_trotter_auto(W, n, o, n_terms, sqrt_dt, E, V, win + spin * half, wout + spin * half, 1, oz, s));

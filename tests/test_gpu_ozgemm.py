@@ -56,6 +56,19 @@ def test_digit_products_match_oracle(n, o, G, W):
     assert _rel(e, O.energy_r(w, 0.0, ctx, mo.astype(complex))) < RTOL
 
 
+@pytest.mark.parametrize("n,o,W", [(1, 1, 300), (7, 7, 257), (8, 1, 3), (9, 4, 2), (16, 16, 3), (17, 5, 2), (31, 9, 2),
+                                   (32, 32, 2), (33, 12, 2), (48, 20, 2), (49, 10, 153), (64, 10, 2), (63, 23, 2)])
+@pytest.mark.parametrize("n_terms", [1, 6])
+def test_small_taylor_matches_oracle(n, o, W, n_terms):
+    """One kernel a walker (csrc/k_trotter_oz.cu): row tiles of 16, column tiles of 8, K steps of 16, its limits."""
+    G = 20
+    h1, chol, mo, w, xs = _problem(n, o, G, W)
+    pctx = O.build_prop_ctx(0.0, h1, chol, O.get_rdm1(mo.astype(complex)), 0.005)
+    out = engine.apply_trotter(_dev(w, torch.complex128), _dev(xs, torch.complex128), _dev(chol),
+                               _dev(pctx.exp_h1_half), pctx.sqrt_dt, n_terms)
+    assert _rel(out, O.apply_trotter_r(w, xs, pctx, chol.reshape(G, -1), n_terms)) < RTOL
+
+
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 def test_digit_products_keep_nonfinite_rows_apart(bad):
     n, o, G, W = 45, 9, 100, 6
@@ -72,7 +85,7 @@ def test_digit_products_keep_nonfinite_rows_apart(bad):
 
 @pytest.mark.parametrize("n,o,W", [(33, 5, 3), (61, 9, 17), (64, 17, 4), (130, 33, 2)])
 def test_blocks_sharing_a_v_match_single_ones(n, o, W):
-    """Two spins (or halves) taken as one tile's columns give each column what it gets alone, bit for bit."""
+    """Two spins (or halves) taken as one tile's columns give each column what it gets alone (either route's)."""
     G = 40
     h1, chol, mo, w, xs = _problem(n, o, G, 2 * W)
     pctx = O.build_prop_ctx(0.0, h1, chol, O.get_rdm1(mo.astype(complex)), 0.005)
@@ -81,7 +94,7 @@ def test_blocks_sharing_a_v_match_single_ones(n, o, W):
     both = engine.apply_trotter_u(pair, x, L, e, pctx.sqrt_dt, 6)
     for spin in range(2):
         one = engine.apply_trotter(pair[spin].contiguous(), x, L, e, pctx.sqrt_dt, 6)
-        assert torch.equal(both[spin], one)
+        assert _rel(both[spin], one.cpu().numpy()) < RTOL
     if o % 2 == 0 or o > 32:
         return
     c = o - 1  # a generalized walker's halves are n x 2 nocc
@@ -89,4 +102,4 @@ def test_blocks_sharing_a_v_match_single_ones(n, o, W):
     g = engine.apply_trotter_g(halves.reshape(W, 2 * n, c), x, L, e, pctx.sqrt_dt, 6).reshape(W, 2, n, c)
     for p in range(2):
         one = engine.apply_trotter(halves[:, p].contiguous(), x, L, e, pctx.sqrt_dt, 6)
-        assert torch.equal(g[:, p], one)
+        assert _rel(g[:, p], one.cpu().numpy()) < RTOL
