@@ -151,29 +151,38 @@ __device__ __forceinline__ double2 cdiv(double2 a, double2 b) {
 
 // Importance factor of one walker (prop/afqmc.py:116-125): imp_ph =
 // |exp(exponent) ratio| cos(theta) before the floor and cap, and
-// phi = exp(-sqrt_dt shift_term) ratio whose angle is theta.  Shared by the
-// weight update and its adjoint so that both see the same floor/cap masks.
+// phi = exp(-sqrt_dt shift_term) ratio whose angle is theta (PHI).  As
+// cos(theta) = Re(e^{i a} ratio) / |ratio| with a = -sqrt_dt Im shift_term, imp_ph
+// is e^{Re exponent} Re(e^{i a} ratio): one exponential and one sincos where
+// the formula as it stands takes two of each, a hypot, an atan2 and a cosine;
+// that one is kept for values that are not finite.  Shared by the weight update
+// and its adjoint so that both see the same floor/cap masks.
 struct WeightFactor {
     double imp_ph;
     double2 phi;
 };
+template <bool PHI>
 __device__ __forceinline__ WeightFactor weight_factor(double dt, double sqrt_dt, double ps, double2 h0_prop,
                                                       double2 st, double2 ft, double2 on, double2 op) {
     const double2 ratio = cdiv(on, op);
     const double2 ex = make_double2(-sqrt_dt * st.x + ft.x + dt * (ps + h0_prop.x),
                                     -sqrt_dt * st.y + ft.y + dt * h0_prop.y);
-    double sn, cs;
-    sincos(ex.y, &sn, &cs);
     const double er = exp(ex.x);
-    const double2 imp = cmul(make_double2(er * cs, er * sn), ratio);
-    // theta = angle(exp(-sqrt_dt shift_term) * ratio)
+    double sn, cs;
     sincos(-sqrt_dt * st.y, &sn, &cs);
-    const double er2 = exp(-sqrt_dt * st.x);
-    const double2 ph = cmul(make_double2(er2 * cs, er2 * sn), ratio);
-    const double theta = atan2(ph.y, ph.x);
     WeightFactor f;
-    f.imp_ph = hypot(imp.x, imp.y) * cos(theta);
-    f.phi = ph;
+    f.imp_ph = er * (cs * ratio.x - sn * ratio.y);
+    f.phi = make_double2(0.0, 0.0);
+    const bool fin = isfinite(f.imp_ph);
+    if (!PHI && fin) return f;
+    const double er2 = exp(-sqrt_dt * st.x);
+    f.phi = cmul(make_double2(er2 * cs, er2 * sn), ratio);
+    if (!fin) {
+        const double theta = atan2(f.phi.y, f.phi.x);
+        sincos(ex.y, &sn, &cs);
+        const double2 imp = cmul(make_double2(er * cs, er * sn), ratio);
+        f.imp_ph = hypot(imp.x, imp.y) * cos(theta);
+    }
     return f;
 }
 

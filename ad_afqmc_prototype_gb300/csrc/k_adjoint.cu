@@ -517,7 +517,7 @@ __global__ void __launch_bounds__(1024) k_weight_adj(
     double pacc = 0.0;
     for (int w = threadIdx.x; w < W; w += blockDim.x) {
         const double2 on = ov_post[w], op = ov_pre[w];
-        const WeightFactor f = weight_factor(dt, sqrt_dt, ps, h0_prop, shift_term[w], fb_term[w], on, op);
+        const WeightFactor f = weight_factor<true>(dt, sqrt_dt, ps, h0_prop, shift_term[w], fb_term[w], on, op);
         double imp_ph = f.imp_ph;
         bool alive = !(imp_ph < w_floor) && !(imp_ph > w_cap);
         if (!alive) imp_ph = 0.0;

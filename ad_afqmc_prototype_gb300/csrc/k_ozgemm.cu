@@ -192,8 +192,8 @@ struct OzMmaState {
     unsigned c, ns, nd;  // stages, drains of the single and of the double accumulators so far
 };
 // row S of the stage in buffer P
-template <int P, int S>
-__device__ __forceinline__ void oz_stage_row(uint32_t smem, uint32_t tmem, int k2, bool sd, bool ss, const OzMmaState& m,
+template <int S>
+__device__ __forceinline__ void oz_stage_row(int P, uint32_t smem, uint32_t tmem, int k2, bool sd, bool ss, const OzMmaState& m,
                                              int buf, volatile int* abort_flag, int* err) {
     constexpr int J = OZ_S - 1 - S;
     const uint32_t bars = smem + OZ_BAR0, par = (m.c >> 1) & 1;
@@ -214,17 +214,16 @@ __device__ __forceinline__ void oz_stage_row(uint32_t smem, uint32_t tmem, int k
     if (k2 > 1) oz_row<S>(tmem, ad + 2, bd + 2, buf, 1u);
     oz_commit(bars + 8 * (OZB_EA + P * OZ_S + J));
 }
-template <int P>
-__device__ __forceinline__ void oz_stage(uint32_t smem, uint32_t tmem, int k2, bool sd, bool ss, const OzMmaState& m,
+__device__ __forceinline__ void oz_stage(int P, uint32_t smem, uint32_t tmem, int k2, bool sd, bool ss, const OzMmaState& m,
                                          volatile int* abort_flag, int* err) {
     const int buf = (int)(m.nd & 1);
-    oz_stage_row<P, 6>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
-    oz_stage_row<P, 5>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
-    oz_stage_row<P, 4>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
-    oz_stage_row<P, 3>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
-    oz_stage_row<P, 2>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
-    oz_stage_row<P, 1>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
-    oz_stage_row<P, 0>(smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<6>(P, smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<5>(P, smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<4>(P, smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<3>(P, smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<2>(P, smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<1>(P, smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
+    oz_stage_row<0>(P, smem, tmem, k2, sd, ss, m, buf, abort_flag, err);
     oz_commit(smem + OZ_BAR0 + 8 * (OZB_EB + P));
 }
 
@@ -313,8 +312,7 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
                 const bool ed = i % OZ_CHUNK == OZ_CHUNK - 1 || i == n - 1;       // and that end
                 const bool es = i % (2 * OZ_CHUNK) == 2 * OZ_CHUNK - 1 || i == n - 1;
                 const int k2 = a.K - (k0 + i) * OZ_BK > 16 ? 2 : 1;
-                if (m.c & 1) oz_stage<1>(smem, tmem, k2, sd, ss, m, abort_flag, a.err);
-                else oz_stage<0>(smem, tmem, k2, sd, ss, m, abort_flag, a.err);
+                oz_stage((int)(m.c & 1), smem, tmem, k2, sd, ss, m, abort_flag, a.err);
                 if (es) {
                     oz_commit(bars + 8 * OZB_TFS);
                     ++m.ns;
@@ -811,6 +809,13 @@ int cap_rows(long long rows, long long bytes_per_row) {
     return (int)(c < rows ? c : rows);
 }
 
+// W walkers in equal chunks of at most `most`
+int even_chunk(int W, long long most) {
+    if (most < 1) most = 1;
+    const long long n = (W + most - 1) / most;
+    return (int)((W + n - 1) / n);
+}
+
 constexpr int OZ_TILE_SMS = 152;
 
 struct ZLayout {
@@ -904,9 +909,7 @@ TrLayout tr_layout(Arena& a, int W, int n, int o, int ns) {
     TrLayout t;
     const long long per = round_up(n, 8) * digit_row_bytes(2 * n);  // digits of one V
     long long wc = OZ_CAP / per;                                    // walkers whose V digits fit
-    if (wc < 1) wc = 1;
-    if (wc > W) wc = W;
-    t.wc = (int)wc;
+    t.wc = even_chunk(W, wc);
     const size_t nb = (size_t)t.wc * ns;
     t.E = take_digits(a, n, n);
     t.V = take_digits(a, n, 2 * n, t.wc);
@@ -986,15 +989,13 @@ GrLayout gr_layout(Arena& a, int W, int n, int o) {
     const long long per = 2LL * o * digit_row_bytes(n) + round_up(n, 8) * digit_row_bytes(2 * o) +
                           round_up(2 * o, 8) * digit_row_bytes(2 * o) + 32LL * o * o;
     long long wc = OZ_CAP / per;
-    if (wc < 1) wc = 1;
-    if (wc > W) wc = W;
-    g.wc = (int)wc;
+    g.wc = even_chunk(W, wc);
     g.C = take_digits(a, o, n);
-    g.X = take_digits(a, (size_t)wc * 2 * o, n);
-    g.A = take_digits(a, n, 2 * o, wc);
-    g.B = take_digits(a, 2 * o, 2 * o, wc);
-    g.m = a.take<double2>((size_t)wc * o * o);
-    g.inv = a.take<double2>((size_t)wc * o * o);
+    g.X = take_digits(a, (size_t)g.wc * 2 * o, n);
+    g.A = take_digits(a, n, 2 * o, g.wc);
+    g.B = take_digits(a, 2 * o, 2 * o, g.wc);
+    g.m = a.take<double2>((size_t)g.wc * o * o);
+    g.inv = a.take<double2>((size_t)g.wc * o * o);
     return g;
 }
 }  // namespace
@@ -1039,9 +1040,7 @@ struct EnLayout {
 EnLayout en_layout(Arena& a, int W, int n, int o, int G) {
     EnLayout e;
     long long wc = OZ_CAP / ((long long)o * G * o * 16);
-    if (wc < 1) wc = 1;
-    if (wc > W) wc = W;
-    e.wc = (int)wc;
+    e.wc = even_chunk(W, wc);
     e.L = take_digits(a, (size_t)G * o, n);
     e.X = take_digits(a, (size_t)e.wc * 2 * o, n);
     e.F = a.take<double2>((size_t)e.wc * o * G * o);

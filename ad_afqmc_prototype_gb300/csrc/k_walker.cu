@@ -134,6 +134,8 @@ int launch_trotter(int W, int n, int o, int n_terms, double sqrt_dt, const doubl
 // Field shifts (prop/afqmc.py:97-101), one warp per walker:
 //   fs = -sqrt_dt (i fb - mf);  x~ = x - fs;
 //   shift_term = sum_g x~ mf;   fb_term = sum_g (x fs - fs^2 / 2)
+// Bound by its 14 binary64 operations a field; few walkers go two warps a CTA
+// so that they reach every SM.
 // =====================================================================
 __global__ void k_field_shift(int W, int G, double sqrt_dt, const double* __restrict__ x,
                               const double2* __restrict__ fb, const double2* __restrict__ mf,
@@ -148,13 +150,17 @@ __global__ void k_field_shift(int W, int G, double sqrt_dt, const double* __rest
         const double2 f = fb[e], m = mf[g];
         const double xv = x[e];
         // i fb - mf = (-f.y - m.x, f.x - m.y)
-        const double2 fs = make_double2(-sqrt_dt * (-f.y - m.x), -sqrt_dt * (f.x - m.y));
+        const double2 fs = make_double2(sqrt_dt * (f.y + m.x), sqrt_dt * (m.y - f.x));
         const double2 xt = make_double2(xv - fs.x, -fs.y);
         xs[e] = xt;
-        sr += xt.x * m.x - xt.y * m.y;
-        si += xt.x * m.y + xt.y * m.x;
-        br += xv * fs.x - 0.5 * (fs.x * fs.x - fs.y * fs.y);
-        bi += xv * fs.y - 0.5 * (2.0 * fs.x * fs.y);
+        sr = fma(xt.x, m.x, sr);
+        sr = fma(-xt.y, m.y, sr);
+        si = fma(xt.x, m.y, si);
+        si = fma(xt.y, m.x, si);
+        // x fs - fs^2 / 2: real part fs.x (x - fs.x / 2) + fs.y^2 / 2, imaginary part fs.y (x - fs.x)
+        br = fma(fs.x, fma(-0.5, fs.x, xv), br);
+        br = fma(0.5 * fs.y, fs.y, br);
+        bi = fma(fs.y, xt.x, bi);
     }
     sr = warp_sum(sr); si = warp_sum(si); br = warp_sum(br); bi = warp_sum(bi);
     if (lane == 0) {
@@ -166,15 +172,17 @@ __global__ void k_field_shift(int W, int G, double sqrt_dt, const double* __rest
 int launch_field_shift(int W, int G, double sqrt_dt, const double* x, const double2* fb, const double2* mf,
                        double2* xs, double2* shift_term, double2* fb_term, cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
-    k_field_shift<<<(W + 7) / 8, 256, 0, s>>>(W, G, sqrt_dt, x, fb, mf, xs, shift_term, fb_term);
+    const int wpb = W < 8 * 152 ? 2 : 8;  // warps (walkers) a CTA
+    k_field_shift<<<(W + wpb - 1) / wpb, 32 * wpb, 0, s>>>(W, G, sqrt_dt, x, fb, mf, xs, shift_term, fb_term);
     AFQ_LAUNCHED("k_field_shift");
     return AFQ_OK;
 }
 
 // =====================================================================
 // Importance weights with the phaseless cut (prop/afqmc.py:116-138): one
-// thread a walker over W / 256 CTAs (the binary64 exp / sincos / atan2 of a
-// walker are a few hundred binary64 operations), then one CTA reduces the
+// thread a walker and one warp a CTA (a walker's exponential, sincos and
+// division are ~150 binary64 operations, of which a quarter of an SM starts one
+// warp's in 64 clocks, so warps go to different SMs: 200 walkers 16 -> 7 us), then one CTA reduces the
 // mean weight feeding the population-control shift in a fixed order
 // (thread t sums walkers t, t + 1024, ...; then the warps and the CTA).
 //
@@ -184,7 +192,7 @@ int launch_field_shift(int W, int G, double sqrt_dt, const double* x, const doub
 // NaN).  With a status word (status != nullptr) every such walker is counted
 // into status[1] and status[0] is set to AFQ_STATUS_NONFINITE if it was 0.
 // =====================================================================
-__global__ void __launch_bounds__(256) k_weight_update(
+__global__ void __launch_bounds__(32) k_weight_update(
     int W, double dt, double sqrt_dt, double w_floor, double w_cap, double2 h0_prop,
     const double2* __restrict__ shift_term, const double2* __restrict__ fb_term,
     const double2* __restrict__ ovlp_new, double* __restrict__ weights, double2* __restrict__ overlaps,
@@ -193,7 +201,7 @@ __global__ void __launch_bounds__(256) k_weight_update(
     if (w >= W) return;
     const double ps = pop_shift[0];
     const double2 on = ovlp_new[w];
-    double imp_ph = weight_factor(dt, sqrt_dt, ps, h0_prop, shift_term[w], fb_term[w], on, overlaps[w]).imp_ph;
+    double imp_ph = weight_factor<false>(dt, sqrt_dt, ps, h0_prop, shift_term[w], fb_term[w], on, overlaps[w]).imp_ph;
     if (imp_ph < w_floor) imp_ph = 0.0;
     if (imp_ph > w_cap) imp_ph = 0.0;
     double wn = weights[w] * imp_ph;
@@ -248,7 +256,7 @@ int launch_weight_update(int W, const afq_params* p, double sqrt_dt, double dt, 
                          double* weights, double2* overlaps, double* pop_shift, const double* e_est,
                          cudaStream_t s, int* status) {
     if (W <= 0) return AFQ_OK;
-    k_weight_update<<<(W + 255) / 256, 256, 0, s>>>(W, dt, sqrt_dt, p->weight_floor, p->weight_cap, h0_prop,
+    k_weight_update<<<(W + 31) / 32, 32, 0, s>>>(W, dt, sqrt_dt, p->weight_floor, p->weight_cap, h0_prop,
                                                     shift_term, fb_term, ovlp_new, weights, overlaps, pop_shift,
                                                     status);
     AFQ_LAUNCHED("k_weight_update");
