@@ -577,13 +577,13 @@ const char* afq_last_error(void) { return g_err; }
 
 // ------------------------------------------------------------------ set-up
 size_t afq_build_prop_ctx_workspace(int32_t norb, int32_t nchol) {
-    (void)nchol;
     Arena a;
     a.take<int>(64);  // status word: offset 0 of every workspace
     a.take<double2>((size_t)norb * norb);  // dm
     a.take<double>((size_t)norb * norb);   // h1_eff
     for (int k = 0; k < 3; ++k) a.take<double>((size_t)norb * norb);
     a.take<double>(1);
+    a.take<char>(h1_eff_scratch(norb, nchol));
     return a.used;
 }
 
@@ -604,6 +604,7 @@ int afq_build_prop_ctx(int32_t norb, int32_t nchol, double h0, double dt, const 
     double* t1 = a.take<double>((size_t)n * n);
     double* t2 = a.take<double>((size_t)n * n);
     double* nrm = a.take<double>(1);
+    void* h1s = a.take<char>(h1_eff_scratch(n, nchol));
     AFQ_TRY(check_ws(a, workspace_bytes));
     const double2* dmp = (const double2*)rdm1;
     if (rdm1_spin_blocks) {
@@ -612,7 +613,7 @@ int afq_build_prop_ctx(int32_t norb, int32_t nchol, double h0, double dt, const 
     }
     AFQ_TRY(launch_mf_shifts(n, nchol, chol, dmp, (double2*)mf_shifts, s));
     AFQ_TRY(launch_h0_prop(nchol, h0, (const double2*)mf_shifts, (double2*)h0_prop, s));
-    AFQ_TRY(launch_h1_eff(n, nchol, h1, chol, (const double2*)mf_shifts, h1e, s));
+    AFQ_TRY(launch_h1_eff(n, nchol, h1, chol, (const double2*)mf_shifts, h1e, h1s, s));
     AFQ_TRY(launch_expm(n, -0.5 * dt, h1e, exp_h1_half, t0, t1, t2, nrm, s));
     return AFQ_OK;
 }

@@ -79,7 +79,7 @@ struct GradWS {
     double2* cl; double2* y; double2* F; double2* Ft; double* ebar_w;
     // accumulators
     double* ebar_part; double2* sg_part; double* ebar; double2* sg;
-    double* h1e; double* ftmp;
+    double* h1e; double* ftmp; void* h1s;
 };
 
 // The forward uses the first two regions only (status word and a block's workspace).
@@ -122,7 +122,7 @@ GradWS layout_grad(Arena& a, const afq_dims* d, const afq_params* p, int ck) {
         g.oz.p = a.take<char>(std::max({zgemm_oz_scratch(Wi, Gi, noi), zgemm_oz_scratch(Wi, n2, Gi),
                                         zgemm_oz_scratch(Wi, Gi, n2), zgemm_oz_scratch(Wi, noi, Gi),
                                         zgemm_oz_scratch(wo, Gi * oi, ni), zgemm_oz_scratch(wo, ni, Gi * oi),
-                                        green_oz_scratch(Wi, ni, oi)}));
+                                        green_oz_scratch(Wi, ni, oi), vbar_oz_scratch(Wi, ni, oi, (int)K)}));
         g.oz.err = g.status;
     }
     g.wk = a.take<double2>(W * no);
@@ -159,6 +159,7 @@ GradWS layout_grad(Arena& a, const afq_dims* d, const afq_params* p, int ck) {
     g.sg = a.take<double2>(no);
     g.h1e = a.take<double>(n * n);
     g.ftmp = a.take<double>(5 * 4 * n * n + 2);
+    g.h1s = a.take<char>(h1_eff_scratch((int)n, (int)G));
     return g;
 }
 
@@ -247,7 +248,8 @@ int step_adjoint(const Ctx& c, const BlockSnap& sn, int op, int st_i, uint64_t c
     { AFQ_PHASE("adj_ebar", s);
       AFQ_TRY(launch_ebar(W, n, o, g.tbar, (long long)(K + 1) * no, Wpre, no, g.ebar_part, s)); }
     // V = sum_g x~_g L_g: x~b = Vb . L^T
-    { AFQ_PHASE("adj_vbar", s); AFQ_TRY(launch_vbar(W, n, o, K, pb->sqrt_dt, g.tbar, g.terms, g.V, s)); }
+    { AFQ_PHASE("adj_vbar", s);
+      AFQ_TRY(launch_vbar_oz(W, n, o, K, pb->sqrt_dt, g.tbar, g.terms, g.V, g.oz.p, g.oz.err, s)); }
     { AFQ_PHASE("adj_xbar_gemm", s);
       AFQ_TRY(zgemm_adj(g, W, G, n * n, 1.0, g.V, (int64_t)n * n, pb->chol, (int64_t)n * n, true, g.xtb, s)); }
     // field shifts, then the force bias fb = 2 L~ vec(G_half)
@@ -441,6 +443,6 @@ int afq_grad_backward(const afq_problem* pb, const afq_params* p, const double* 
     }
     AFQ_TRY(launch_sum_partials(n * n, ns, g.ebar_part, g.ebar, s));
     AFQ_TRY(launch_sum_partials(2 * no, ns, (const double*)g.sg_part, (double*)g.sg, s));
-    AFQ_TRY(launch_h1_eff(n, d->nchol, h1, pb->chol, (const double2*)pb->mf_shifts, g.h1e, s));
+    AFQ_TRY(launch_h1_eff(n, d->nchol, h1, pb->chol, (const double2*)pb->mf_shifts, g.h1e, g.h1s, s));
     return launch_h1bar(n, o, pb->dt, g.h1e, g.ebar, (const double2*)pb->mo_coeff, g.sg, h1_bar, g.ftmp, s);
 }

@@ -277,8 +277,9 @@ inline cudaStream_t as_stream(void* s) { return (cudaStream_t)s; }
 // k_setup.cu
 int launch_mf_shifts(int n, int G, const double* chol, const double2* dm, double2* mf,
                      cudaStream_t s);
-int launch_h1_eff(int n, int G, const double* h1, const double* chol, const double2* mf,
-                  double* h1_eff, cudaStream_t s);
+size_t h1_eff_scratch(int n, int G);  // bytes
+int launch_h1_eff(int n, int G, const double* h1, const double* chol, const double2* mf, double* h1_eff, void* scratch,
+                  cudaStream_t s);
 int launch_expm(int n, double scale, const double* a, double* out, double* tmp0, double* tmp1,
                 double* tmp2, double* norm_dev, cudaStream_t s);
 int launch_trial_rdm1(int n, int o, const double2* mo, double2* rdm1, cudaStream_t s);
@@ -324,6 +325,11 @@ int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const do
 bool trotter_small_fits(int n, int oc, int n_terms);
 int launch_trotter_small(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
                          const double2* win, double2* wout, int ns, long long ws, long long ss, cudaStream_t s);
+// its terms kept, and its reverse (k_adjoint.cu's kernels where it does not fit)
+int launch_taylor_tape_small(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                             const double2* win, double2* terms, double2* w2, cudaStream_t s);
+int launch_taylor_adj_small(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                            const double2* wbar_post, double2* tbar, double2* wbar_pre, cudaStream_t s);
 bool energy_oz_pays(int W, int n, int o, int G);
 size_t energy_oz_scratch(int W, int n, int o, int G);
 int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, const double* rot_chol,
@@ -484,8 +490,10 @@ int launch_taylor_tape(int W, int n, int o, int K, double sqrt_dt, const double*
                        const double2* win, double2* terms, double2* w2, cudaStream_t s);
 int launch_taylor_adj(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
                       const double2* wbar_post, double2* tbar, double2* wbar_pre, cudaStream_t s);
-int launch_vbar(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms, double2* vbar,
-                cudaStream_t s);
+// Vb_w = sum_{k = 1 .. K} conj(i sqrt_dt / k) tb_k t_{k-1}^H by digits on the tensor cores (k_ozgemm.cu)
+size_t vbar_oz_scratch(int W, int n, int o, int K);
+int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms,
+                   double2* vbar, void* scratch, int* err, cudaStream_t s);
 int ebar_splits(int W);
 int launch_ebar(int W, int n, int o, const double2* X, long long xs, const double2* Y, long long ys, double* partial,
                 cudaStream_t s);

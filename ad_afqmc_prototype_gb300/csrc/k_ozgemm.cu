@@ -525,31 +525,33 @@ __global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const d
     }
 }
 
-// Real rows with K strided: row r's entry k at src[k ld + r es]; 32 rows a CTA,
-// transposed through shared memory.
+// Real rows with K strided: row r's entry k at src[k ld + r es]; RB rows a CTA
+// (32, or 8 where few rows would leave SMs idle), transposed through shared memory.
+template <int RB>
 __global__ void __launch_bounds__(256) k_oz_cols(int rows, int K, const double* __restrict__ src, long long ld, int es,
                                                  OzDst dst, int* __restrict__ ex) {
-    __shared__ double tile[32][65];
-    __shared__ int se[32];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, r0 = blockIdx.x * 32;
+    constexpr int TY = 256 / RB, KT = 8 * TY;  // threads a row; k at a time
+    __shared__ double tile[RB][KT + 1];
+    __shared__ int se[RB];
+    const int tx = threadIdx.x % RB, ty = threadIdx.x / RB, r0 = blockIdx.x * RB;
     const bool in = r0 + tx < rows;
-    if (threadIdx.x < 32) se[threadIdx.x] = 0;
+    if (threadIdx.x < RB) se[threadIdx.x] = 0;
     __syncthreads();
     int e = 0;
     if (in) {
-#pragma unroll 4
-        for (int k = ty; k < K; k += 8) e = max(e, oz_expo(src[(long long)k * ld + (r0 + tx) * es]));
+#pragma unroll 8
+        for (int k = ty; k < K; k += TY) e = max(e, oz_expo(src[(long long)k * ld + (r0 + tx) * es]));
     }
     atomicMax(&se[tx], e);
     __syncthreads();
-    const int rr = threadIdx.x >> 3, kq = (threadIdx.x & 7) * 8, E = oz_scale(se[rr]);
-    if ((threadIdx.x & 7) == 0 && r0 + rr < rows) ex[r0 + rr] = E;
-    for (int k0 = 0; k0 < 32 * dst.nks; k0 += 64) {
+    const int rr = threadIdx.x / TY, kq = (threadIdx.x % TY) * 8, E = oz_scale(se[rr]);
+    if (threadIdx.x % TY == 0 && r0 + rr < rows) ex[r0 + rr] = E;
+    for (int k0 = 0; k0 < 32 * dst.nks; k0 += KT) {
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int k = k0 + ty + 8 * i;
-            tile[tx][ty + 8 * i] = in && k < K ? src[(long long)k * ld + (r0 + tx) * es] : 0.0;
+            const int k = k0 + ty + TY * i;
+            tile[tx][ty + TY * i] = in && k < K ? src[(long long)k * ld + (r0 + tx) * es] : 0.0;
         }
         __syncthreads();
         if (r0 + rr < rows && k0 + kq < 32 * dst.nks) {
@@ -654,6 +656,62 @@ __device__ __forceinline__ void cfma2(double& re, double& im, double2 a, double2
     im = fma(a.x, b.y, im);
     re = fma(-a.y, b.y, re);
     im = fma(a.y, b.x, im);
+}
+
+// The adjoint's outer products: row i of walker w over (k, c, part) is
+// conj(i sqrt_dt / k) tb_k[i, c] = (sqrt_dt / k) (tb.y, -tb.x), k = 1 .. K (A); the right
+// operand's rows (j, Re) [Re, Im] and (j, Im) [-Im, Re] of t_{k-1}[j, c] give
+// sum a conj(t).  One warp a row.
+__global__ void __launch_bounds__(256) k_oz_vbar(int W, int n, int o, int K, double sqrt_dt,
+                                                 const double2* __restrict__ tbar, const double2* __restrict__ terms,
+                                                 OzDst A, int* __restrict__ ea, OzDst B, int* __restrict__ eb) {
+    const int lane = threadIdx.x & 31, no = n * o, L = K * o;
+    const long long rows = (long long)W * n;
+    for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < 2 * rows; r += (long long)gridDim.x * 8) {
+        const bool right = r >= rows;
+        const long long x = right ? r - rows : r;
+        const int w = (int)(x / n), i = (int)(x - (long long)w * n);
+        // entry l = (k - 1) o + c of the row
+        const double2* src = right ? terms + (long long)w * K * no + (long long)i * o
+                                   : tbar + ((long long)w * (K + 1) + 1) * no + (long long)i * o;
+        auto at = [&](int l) {
+            const int k = l / o;
+            double2 v = src[(long long)k * no + (l - k * o)];
+            if (!right) {
+                const double c = sqrt_dt / (k + 1);
+                v = make_double2(c * v.y, -c * v.x);
+            }
+            return v;
+        };
+        int e = 0;
+        for (int l = lane; l < L; l += 32) {
+            const double2 v = at(l);
+            e = max(e, max(oz_expo(v.x), oz_expo(v.y)));
+        }
+        const int E = oz_scale(warp_max(e));
+        if (lane == 0) {
+            if (right) eb[2 * x] = eb[2 * x + 1] = E;
+            else ea[x] = E;
+        }
+        for (int k = 8 * lane; k < 32 * A.nks; k += 256) {
+            long long y[8], z[8];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int l = k / 2 + q;
+                const double2 v = l < L ? at(l) : make_double2(0.0, 0.0);
+                y[2 * q] = oz_fix(v.x, E);
+                y[2 * q + 1] = oz_fix(v.y, E);
+                z[2 * q] = oz_fix(-v.y, E);
+                z[2 * q + 1] = y[2 * q];
+            }
+            if (right) {
+                oz_store8(B, w, 2 * i, k, y);
+                oz_store8(B, w, 2 * i + 1, k, z);
+            } else {
+                oz_store8(A, w, i, k, y);
+            }
+        }
+    }
 }
 
 // Coulomb and exchange partials of a chunk of ng Cholesky vectors from F
@@ -789,7 +847,8 @@ int split_crows(long long rows, int K, const double2* src, long long ld, const O
     return AFQ_OK;
 }
 int split_cols(int rows, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s, int es = 1) {
-    k_oz_cols<<<(rows + 31) / 32, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex);
+    if (rows <= 32 * 152) k_oz_cols<8><<<(rows + 7) / 8, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex);
+    else k_oz_cols<32><<<(rows + 31) / 32, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex);
     AFQ_LAUNCHED("k_oz_cols");
     return AFQ_OK;
 }
@@ -1026,6 +1085,52 @@ int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walke
         AFQ_TRY(launch_term<OZ_PLAIN>(wc, o, o, 0.0, g.inv, nullptr, nullptr, g.B, s));
         const OzOut gout = {green_out + w0 * no, (long long)no, 0, n, 1, 2 * o, 0, nullptr};
         AFQ_TRY(oz_launch(n, 2 * o, 2 * o, wc, 1, g.A, g.B, gout, 1, (2 * o + 255) / 256, nullptr, err, s));
+    }
+    return AFQ_OK;
+}
+
+// ------------------------------------------------- adjoint outer products --
+namespace {
+struct VbLayout {
+    int wc;
+    OzDigits A, B;
+};
+VbLayout vb_layout(Arena& a, int W, int n, int o, int K) {
+    VbLayout v;
+    const int k2 = 2 * K * o;
+    v.wc = even_chunk(W, OZ_CAP / (3 * round_up(n, 8) * digit_row_bytes(k2)));
+    v.A = take_digits(a, n, k2, v.wc);
+    v.B = take_digits(a, 2 * n, k2, v.wc);
+    return v;
+}
+}  // namespace
+
+size_t vbar_oz_scratch(int W, int n, int o, int K) {
+    Arena a;
+    vb_layout(a, W, n, o, K > 0 ? K : 1);
+    return a.used + 256;
+}
+
+// Vb_w = sum_{k = 1 .. K} conj(i sqrt_dt / k) tb_k t_{k-1}^H
+int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms,
+                   double2* vbar, void* scratch, int* err, cudaStream_t s) {
+    if (W <= 0) return AFQ_OK;
+    if (K == 0) {
+        AFQ_CUDA(cudaMemsetAsync(vbar, 0, sizeof(double2) * (size_t)W * n * n, s));
+        return AFQ_OK;
+    }
+    Arena ar(scratch, (size_t)-1);
+    const VbLayout v = vb_layout(ar, W, n, o, K);
+    const int k2 = 2 * K * o;
+    const long long no = (long long)n * o, n2 = (long long)n * n;
+    for (int w0 = 0; w0 < W; w0 += v.wc) {
+        const int wc = W - w0 < v.wc ? W - w0 : v.wc;
+        k_oz_vbar<<<row_blocks(2LL * wc * n), 256, 0, s>>>(wc, n, o, K, sqrt_dt, tbar + (long long)w0 * (K + 1) * no,
+                                                          terms + (long long)w0 * K * no, dst_of(v.A, n, k2), v.A.ex,
+                                                          dst_of(v.B, 2 * n, k2), v.B.ex);
+        AFQ_LAUNCHED("k_oz_vbar");
+        const OzOut out = {vbar + w0 * n2, n2, 0, 1, n, n, 0, nullptr};
+        AFQ_TRY(oz_launch(n, 2 * n, k2, wc, 1, v.A, v.B, out, 1, (k2 + 255) / 256, nullptr, err, s));
     }
     return AFQ_OK;
 }

@@ -77,30 +77,86 @@ int launch_mf_shifts(int n, int G, const double* chol, const double2* dm, double
 
 // h1_eff = h1 - 0.5 sum_g L_g L_g - sum_g Re(i mf_g) L_g
 // (prop/chol_afqmc_ops.py:86-94)
-__global__ void __launch_bounds__(256) k_h1_eff(int n, int G, const double* __restrict__ h1,
-                                                const double* __restrict__ chol,
-                                                const double2* __restrict__ mf,
-                                                double* __restrict__ h1_eff) {
-    int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= n * n) return;
-    int i = e / n, j = e % n;
-    double v0 = 0.0, v1 = 0.0;
-    for (int g = 0; g < G; ++g) {
-        const double* L = chol + (size_t)g * n * n;
-        double acc = 0.0;
-        for (int k = 0; k < n; ++k) acc = fma(L[i * n + k], L[k * n + j], acc);
-        v0 += acc;
-        double mf_r = -mf[g].y;  // Re(i * mf_g)
-        v1 = fma(mf_r, L[e], v1);
+//
+// Two passes over chunks of Cholesky vectors: all products L_g L_g of a chunk
+// (32 x 32 tiles, two by two outputs a thread, each one chain of FMAs in order of
+// k), then their sum in order of g, carried from chunk to chunk.  60 orbitals
+// and 300 vectors: 2.9 ms with one thread an output running over g and k.
+constexpr int H1_T = 32, H1_K = 16;
+__global__ void __launch_bounds__(256) k_chol_square(int n, const double* __restrict__ chol, double* __restrict__ out) {
+    __shared__ double A[H1_K][H1_T + 1], B[H1_K][H1_T + 1];
+    const double* L = chol + (size_t)blockIdx.z * n * n;
+    const int i0 = blockIdx.y * H1_T, j0 = blockIdx.x * H1_T, tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    double acc[2][2] = {};
+    for (int k0 = 0; k0 < n; k0 += H1_K) {
+        const int kn = min(H1_K, n - k0);
+        __syncthreads();
+        for (int e = threadIdx.x; e < H1_K * H1_T; e += 256) {
+            const int r = e / H1_K, k = e % H1_K, kb = e / H1_T, c = e % H1_T;
+            A[k][r] = i0 + r < n && k < kn ? L[(size_t)(i0 + r) * n + k0 + k] : 0.0;
+            B[kb][c] = j0 + c < n && kb < kn ? L[(size_t)(k0 + kb) * n + j0 + c] : 0.0;
+        }
+        __syncthreads();
+        for (int k = 0; k < kn; ++k) {
+            const double a0 = A[k][ty], a1 = A[k][ty + 16], b0 = B[k][tx], b1 = B[k][tx + 16];
+            acc[0][0] = fma(a0, b0, acc[0][0]);
+            acc[0][1] = fma(a0, b1, acc[0][1]);
+            acc[1][0] = fma(a1, b0, acc[1][0]);
+            acc[1][1] = fma(a1, b1, acc[1][1]);
+        }
     }
-    h1_eff[e] = h1[e] - 0.5 * v0 - v1;
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const int i = i0 + ty + 16 * r, j = j0 + tx + 16 * c;
+            if (i < n && j < n) out[((size_t)blockIdx.z * n + i) * n + j] = acc[r][c];
+        }
 }
 
-int launch_h1_eff(int n, int G, const double* h1, const double* chol, const double2* mf,
-                  double* h1_eff, cudaStream_t s) {
-    int nn = n * n;
-    k_h1_eff<<<(nn + 255) / 256, 256, 0, s>>>(n, G, h1, chol, mf, h1_eff);
-    AFQ_LAUNCHED("k_h1_eff");
+// v0, v1: the sums so far (vectors before g0); the last chunk writes h1_eff.
+__global__ void __launch_bounds__(64) k_h1_eff(int nn, int gc, int g0, int last, const double* __restrict__ h1,
+                                               const double* __restrict__ chol, const double2* __restrict__ mf,
+                                               const double* __restrict__ sq, double* __restrict__ v01,
+                                               double* __restrict__ h1_eff) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= nn) return;
+    double v0 = g0 ? v01[e] : 0.0, v1 = g0 ? v01[nn + e] : 0.0;
+#pragma unroll 8
+    for (int g = 0; g < gc; ++g) {
+        v0 += sq[(size_t)g * nn + e];
+        const double mf_r = -mf[g0 + g].y;  // Re(i * mf_g)
+        v1 = fma(mf_r, chol[(size_t)(g0 + g) * nn + e], v1);
+    }
+    if (last) {
+        h1_eff[e] = h1[e] - 0.5 * v0 - v1;
+    } else {
+        v01[e] = v0;
+        v01[nn + e] = v1;
+    }
+}
+
+static int h1_chunk(int n, int G) {
+    const long long c = (32LL << 20) / (8LL * n * n);
+    return (int)(c < 1 ? 1 : c < G ? c : G);
+}
+
+size_t h1_eff_scratch(int n, int G) { return ((size_t)h1_chunk(n, G) + 2) * n * n * sizeof(double); }
+
+int launch_h1_eff(int n, int G, const double* h1, const double* chol, const double2* mf, double* h1_eff, void* scratch,
+                  cudaStream_t s) {
+    const int nn = n * n, gc = h1_chunk(n, G), t = (n + H1_T - 1) / H1_T;
+    double* v01 = (double*)scratch;
+    double* sq = v01 + 2 * (size_t)nn;
+    for (int g0 = 0; g0 < G; g0 += gc) {
+        for (int z = 0; z < min(gc, G - g0); z += 65535) {
+            const int m = min(65535, min(gc, G - g0) - z);
+            k_chol_square<<<dim3(t, t, m), 256, 0, s>>>(n, chol + (size_t)(g0 + z) * nn, sq + (size_t)z * nn);
+            AFQ_LAUNCHED("k_chol_square");
+        }
+        k_h1_eff<<<(nn + 63) / 64, 64, 0, s>>>(nn, min(gc, G - g0), g0, g0 + gc >= G, h1, chol, mf, sq, v01, h1_eff);
+        AFQ_LAUNCHED("k_h1_eff");
+    }
     return AFQ_OK;
 }
 

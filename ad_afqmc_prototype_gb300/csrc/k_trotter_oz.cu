@@ -24,7 +24,7 @@ namespace afq {
 
 namespace {
 
-constexpr int TS_NMAX = 64;
+constexpr int TS_NMAX = 64;  // orbitals
 
 __device__ __forceinline__ uint32_t sm_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 __device__ __forceinline__ void ldm_x4(uint32_t (&r)[4], uint32_t addr) {
@@ -54,8 +54,9 @@ struct TsGeo {
 };
 
 // Digits of A's rows: eight k a lane, GL lanes a row, the scale from a max over
-// the row's lanes.  ONE: A = E - I with E real (its Im parts zero).
-template <bool ONE>
+// the row's lanes.  ONE: A = E - I with E real (its Im parts zero).  ADJ: of
+// the conjugate transpose.
+template <bool ONE, bool ADJ>
 __device__ void ts_load_a(const TsGeo& g, int n, const void* __restrict__ src, __nv_bfloat16* As, int* s_ea) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int l8 = g.kp / 8, gl = l8 <= 2 ? 2 : l8 <= 4 ? 4 : l8 <= 8 ? 8 : 16;  // lanes a row
@@ -68,8 +69,10 @@ __device__ void ts_load_a(const TsGeo& g, int n, const void* __restrict__ src, _
             const int j = k / 2 + i;
             double2 v = make_double2(0.0, 0.0);
             if (r < n && j < n) {
-                if (ONE) v.x = ((const double*)src)[r * n + j] - (r == j ? 1.0 : 0.0);
-                else v = ((const double2*)src)[(size_t)r * n + j];
+                const int at = ADJ ? j * n + r : r * n + j;
+                if (ONE) v.x = ((const double*)src)[at] - (r == j ? 1.0 : 0.0);
+                else v = ((const double2*)src)[at];
+                if (ADJ) v.y = -v.y;
             }
             x[2 * i] = v.x;
             x[2 * i + 1] = v.y;
@@ -106,11 +109,17 @@ __device__ __forceinline__ void ts_put(uint32_t* d, size_t plane, int pw, long l
 
 // NT: 8-column tiles a warp; warps = mt x (column groups).  Block p of walker w
 // (ns of them, o columns each) is at w ws + p ss; V of the walker at w n^2.
-template <int NT>
+// MODE:
+//   TS_STEP  wout = E sum_k t_k, t_0 = E W, t_k = (i sqrt_dt / k) V t_{k-1}
+//   TS_TAPE  the terms t_0 .. t_{K-1} to `terms` (W, K, n, o), wout = sum_k t_k
+//   TS_ADJ   the reverse: b = E^T W, t_K = b, t_k = b + conj(i sqrt_dt / (k + 1)) V^H
+//            t_{k+1} to `terms` (W, K + 1, n, o), wout = E^T t_0
+enum { TS_STEP, TS_TAPE, TS_ADJ };
+template <int NT, int MODE>
 __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long long ws, long long ss, int n_terms,
                                                     double sqrt_dt, const double* __restrict__ E,
-                                                    const double2* __restrict__ V, const double2* __restrict__ win,
-                                                    double2* __restrict__ wout) {
+                                                    const double2* __restrict__ V, const double2* win, double2* wout,
+                                                    double2* __restrict__ terms) {
     extern __shared__ __align__(16) uint8_t smem_raw[];
     const int oc = o * ns;
     const TsGeo g(n, oc);
@@ -125,7 +134,7 @@ __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long l
 
     for (int e = tid; e < 2 * TS_NMAX; e += blockDim.x) s_eb[0][e] = 0;
     for (int e = tid; e < (int)(g.b_bytes / 16); e += blockDim.x) ((uint4*)Bs)[e] = make_uint4(0, 0, 0, 0);
-    ts_load_a<true>(g, n, E, As, s_ea);
+    ts_load_a<true, MODE == TS_ADJ>(g, n, E, As, s_ea);
 
     // entry (t, h): row r0 + 8 h, column c = 4 (n0 + t) + q
     double2 U[NT][2], T[NT][2];
@@ -139,6 +148,16 @@ __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long l
         }
     __syncthreads();
 
+    const size_t no = (size_t)n * o;
+    auto keep = [&](size_t slot) {  // T to terms[slot]
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = r0 + 8 * h, c = 4 * (n0 + t) + q;
+                if (r < n && c < oc) terms[slot * no + (size_t)r * o + c] = T[t][h];
+            }
+    };
     int buf = 0;
     // T's digits into Bs (after every warp has read the last ones)
     auto put = [&]() {
@@ -234,34 +253,49 @@ __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long l
 #pragma unroll
         for (int h = 0; h < 2; ++h) U[t][h] = T[t][h] = cadd(U[t][h], T[t][h]);
     __syncthreads();
-    ts_load_a<false>(g, n, V + (size_t)w * n * n, As, s_ea);
+    ts_load_a<false, MODE == TS_ADJ>(g, n, V + (size_t)w * n * n, As, s_ea);
+    if (MODE == TS_TAPE) keep((size_t)w * n_terms);
+    if (MODE == TS_ADJ) keep((size_t)w * (n_terms + 1) + n_terms);
     for (int k = 1; k <= n_terms; ++k) {
         put();
         mul();
-        const double s = sqrt_dt / k;  // (i sqrt_dt / k) * z = s * (-z.y, z.x)
+        // (i sqrt_dt / k) z = s (-z.y, z.x); the adjoint's coefficient is conj(i sqrt_dt / (K + 1 - k))
+        const double s = sqrt_dt / (MODE == TS_ADJ ? n_terms + 1 - k : k);
 #pragma unroll
         for (int t = 0; t < NT; ++t)
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                T[t][h] = make_double2(-s * T[t][h].y, s * T[t][h].x);
-                U[t][h] = cadd(U[t][h], T[t][h]);
+                if (MODE == TS_ADJ) {
+                    T[t][h] = make_double2(fma(s, T[t][h].y, U[t][h].x), fma(-s, T[t][h].x, U[t][h].y));
+                } else {
+                    T[t][h] = make_double2(-s * T[t][h].y, s * T[t][h].x);
+                    U[t][h] = cadd(U[t][h], T[t][h]);
+                }
             }
+        if (MODE == TS_TAPE && k < n_terms) keep((size_t)w * n_terms + k);
+        if (MODE == TS_ADJ) keep((size_t)w * (n_terms + 1) + n_terms - k);
     }
-    __syncthreads();
-    ts_load_a<true>(g, n, E, As, s_ea);
+    if (MODE != TS_TAPE) {
+        __syncthreads();
+        ts_load_a<true, MODE == TS_ADJ>(g, n, E, As, s_ea);
 #pragma unroll
-    for (int t = 0; t < NT; ++t)
+        for (int t = 0; t < NT; ++t)
 #pragma unroll
-        for (int h = 0; h < 2; ++h) T[t][h] = U[t][h];
-    put();
-    mul();
+            for (int h = 0; h < 2; ++h) {
+                if (MODE == TS_ADJ) U[t][h] = T[t][h];
+                else T[t][h] = U[t][h];
+            }
+        put();
+        mul();
+    }
 #pragma unroll
     for (int t = 0; t < NT; ++t)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int r = r0 + 8 * h, c = 4 * (n0 + t) + q, p = c >= o;
             if (r < n && c < oc)
-                wout[w * ws + (long long)r * o + (c - p * o) + p * ss] = cadd(U[t][h], T[t][h]);
+                wout[w * ws + (long long)r * o + (c - p * o) + p * ss] =
+                    MODE == TS_TAPE ? U[t][h] : cadd(U[t][h], T[t][h]);
         }
 }
 
@@ -274,14 +308,35 @@ void ts_split(const TsGeo& g, int& groups, int& per) {
     groups = (g.nt + per - 1) / per;
 }
 
-template <int NT>
+template <int NT, int MODE>
 int ts_run(int W, int n, int o, int ns, long long ws, long long ss, int n_terms, double sqrt_dt, const double* E,
-           const double2* V, const double2* win, double2* wout, int warps, size_t smem, cudaStream_t s) {
+           const double2* V, const double2* win, double2* wout, double2* terms, int warps, size_t smem, cudaStream_t s) {
     static DeviceOnce once;
-    AFQ_TRY(raise_smem_once(once, k_trotter_oz<NT>, (int)TS_SMEM));
-    k_trotter_oz<NT><<<W, 32 * warps, smem, s>>>(n, o, ns, ws, ss, n_terms, sqrt_dt, E, V, win, wout);
+    AFQ_TRY(raise_smem_once(once, k_trotter_oz<NT, MODE>, (int)TS_SMEM));
+    k_trotter_oz<NT, MODE><<<W, 32 * warps, smem, s>>>(n, o, ns, ws, ss, n_terms, sqrt_dt, E, V, win, wout, terms);
     AFQ_LAUNCHED("k_trotter_oz");
     return AFQ_OK;
+}
+
+template <int MODE>
+int ts_launch(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V, const double2* win,
+              double2* wout, double2* terms, int ns, long long ws, long long ss, cudaStream_t s) {
+    if (W <= 0) return AFQ_OK;
+    if (!trotter_small_fits(n, o * ns, n_terms)) return fail(AFQ_E_UNSUPPORTED, "small trotter: norb=%d nocc=%d", n, o * ns);
+    const TsGeo g(n, o * ns);
+    int groups, per;
+    ts_split(g, groups, per);
+#define AFQ_TS(NT)                                                                                                       \
+    if (per <= NT)                                                                                                       \
+    return ts_run<NT, MODE>(W, n, o, ns, ws, ss, n_terms, sqrt_dt, E, V, win, wout, terms, g.mt * groups,                \
+                            g.a_bytes + g.b_bytes, s)
+    AFQ_TS(1);
+    AFQ_TS(2);
+    AFQ_TS(3);
+    AFQ_TS(4);
+    AFQ_TS(6);
+#undef AFQ_TS
+    return fail(AFQ_E_UNSUPPORTED, "small trotter: %d column tiles a warp", per);
 }
 
 }  // namespace
@@ -296,20 +351,17 @@ bool trotter_small_fits(int n, int oc, int n_terms) {
 
 int launch_trotter_small(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
                          const double2* win, double2* wout, int ns, long long ws, long long ss, cudaStream_t s) {
-    if (W <= 0) return AFQ_OK;
-    if (!trotter_small_fits(n, o * ns, n_terms)) return fail(AFQ_E_UNSUPPORTED, "small trotter: norb=%d nocc=%d", n, o * ns);
-    const TsGeo g(n, o * ns);
-    int groups, per;
-    ts_split(g, groups, per);
-#define AFQ_TS(NT) \
-    if (per <= NT) return ts_run<NT>(W, n, o, ns, ws, ss, n_terms, sqrt_dt, E, V, win, wout, g.mt * groups, g.a_bytes + g.b_bytes, s)
-    AFQ_TS(1);
-    AFQ_TS(2);
-    AFQ_TS(3);
-    AFQ_TS(4);
-    AFQ_TS(6);
-#undef AFQ_TS
-    return fail(AFQ_E_UNSUPPORTED, "small trotter: %d column tiles a warp", per);
+    return ts_launch<TS_STEP>(W, n, o, n_terms, sqrt_dt, E, V, win, wout, nullptr, ns, ws, ss, s);
+}
+
+int launch_taylor_tape_small(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                             const double2* win, double2* terms, double2* w2, cudaStream_t s) {
+    return ts_launch<TS_TAPE>(W, n, o, K, sqrt_dt, E, V, win, w2, terms, 1, (long long)n * o, 0, s);
+}
+
+int launch_taylor_adj_small(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                            const double2* wbar_post, double2* tbar, double2* wbar_pre, cudaStream_t s) {
+    return ts_launch<TS_ADJ>(W, n, o, K, sqrt_dt, E, V, wbar_post, wbar_pre, tbar, 1, (long long)n * o, 0, s);
 }
 
 }  // namespace afq
