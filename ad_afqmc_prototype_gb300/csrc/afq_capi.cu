@@ -233,6 +233,7 @@ static BlockWS layout_block(Arena& a, const afq_dims* d, int n_chunks) {
     BlockWS b = {};
     b.step = layout_step(a, d, n_chunks, is_mixed(d->precision) ? 0 : energy_oz_bytes(d));
     const size_t W = d->n_walkers;
+    if (!is_mixed(d->precision)) take_oz_block(a, d, b.step.oz);
     b.green = is_mixed(d->precision) ? a.take<double2>(W * d->nocc * d->norb) : b.step.green;
     b.energy = a.take<double2>(W);
     if (is_mixed(d->precision)) {
@@ -268,7 +269,7 @@ static int force_bias_from_green(const afq_dims* d, const double2* green, const 
                                  double2* fb, const OzScratch& oz, cudaStream_t s) {
     const int on = d->nocc * d->norb;
     return launch_zgemm_auto(d->n_walkers, d->nchol, on, 2.0, green, on, rot_chol, on, !d->trial_is_real, true, fb,
-                             d->nchol, oz, s);
+                             d->nchol, oz, s, oz.rot);
 }
 
 static int trotter_chunked(const afq_dims* d, int n_terms, double sqrt_dt, int n_chunks, const double* chol,
@@ -281,7 +282,7 @@ static int trotter_chunked(const afq_dims* d, int n_terms, double sqrt_dt, int n
         // V (wc x n^2) = x~ (wc x G) . chol (G x n^2)   (prop/chol_afqmc_ops.py:70-74)
         { AFQ_PHASE("vbuild_gemm", s);
         AFQ_TRY(launch_zgemm_auto(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, V,
-                                  (int64_t)n * n, oz, s)); }
+                                  (int64_t)n * n, oz, s, oz.chol)); }
         { AFQ_PHASE("trotter", s);
         AFQ_TRY(launch_trotter_auto(wc, n, o, n_terms, sqrt_dt, E, V, win + (size_t)w0 * n * o,
                                     wout + (size_t)w0 * n * o, 1, oz, s)); }
@@ -975,6 +976,8 @@ int afq_block_cv(const afq_problem* pb, const afq_params* p, const afq_state* st
     cudaStream_t s = as_stream(stream);
     const int W = d->n_walkers, n = d->norb, o = d->nocc, G = d->nchol;
     const size_t fstride = (size_t)W * G;
+    if (!is_mixed(d->precision) && p->n_prop_steps > 0)
+        AFQ_TRY(split_oz_block(d, pb->chol, pb->rot_chol, ws.step.oz, s));
     // the block-end measurement reads the fp32 Green's function that the last
     // step's overlap pass writes (the QR leaves it unchanged): the three-section
     // form's energy, and either mixed form's control-variate measurement
@@ -1119,6 +1122,7 @@ int run_block_taped(const afq_problem* pb, const afq_params* p, const afq_state*
     BlockWS ws = layout_block(a, d, p->n_chunks);
     AFQ_TRY(check_ws(a, workspace_bytes));
     const int W = d->n_walkers, n = d->norb, o = d->nocc;
+    if (p->n_prop_steps > 0) AFQ_TRY(split_oz_block(d, pb->chol, pb->rot_chol, ws.step.oz, s));
     int op = 0;
     for (int st_i = 0; st_i < p->n_prop_steps; ++st_i) {
         AFQ_TRY(snap_state(d, st, snap, op++, s));

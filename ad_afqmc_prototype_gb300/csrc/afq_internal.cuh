@@ -306,12 +306,22 @@ int launch_zgemm_splitk(int M, int N, int K, double alpha, const double2* A, int
 struct OzScratch {
     void* p = nullptr;
     int* err = nullptr;
+    // a block's steps: digits of chol (n^2 rows over the vectors) and of rot_chol (vectors over nocc norb), or null
+    void* chol = nullptr;
+    void* rot = nullptr;
 };
+// room for a block's kept digits, and their split (once a block)
+void take_oz_block(Arena& a, const afq_dims* d, OzScratch& oz);
+int split_oz_block(const afq_dims* d, const double* chol, const double* rot_chol, const OzScratch& oz, cudaStream_t s);
 bool zgemm_oz_pays(int M, int N, int K);
 size_t zgemm_oz_scratch(int M, int N, int K);
 // launch_zgemm with a real right operand; alpha a power of two
 int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
-                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s);
+                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s,
+                    const void* real = nullptr);
+// digits of the real operand kept over several products (`real` above and below): bytes (0: not kept), and the split
+size_t oz_real_bytes(int N, int K);
+int oz_real_split(int N, int K, const double* B, int64_t ldb, bool b_trans, void* real, cudaStream_t s);
 bool green_oz_pays(int n, int o);
 size_t green_oz_scratch(int W, int n, int o);
 int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walkers, double2* ovlp_out,
@@ -336,7 +346,8 @@ int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, c
                              double* partial, void* scratch, int* err, cudaStream_t s);
 // the product by digits where that pays, else on the binary64 pipe
 int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B, int64_t ldb,
-                      bool b_complex, bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s);
+                      bool b_complex, bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s,
+                      const void* real = nullptr);
 int launch_trotter_auto(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
                         const double2* win, double2* wout, int vdiv, const OzScratch& oz, cudaStream_t s);
 // both spins of W walkers with the walker's V, the second spin's blocks `half` entries after the first's

@@ -111,7 +111,8 @@ struct UWS {
     double2* ocopy;      // W
 };
 
-UWS layout_u(Arena& a, const afq_dims* d, int n_chunks) {
+// block: with room for the digits that a block's steps share
+UWS layout_u(Arena& a, const afq_dims* d, int n_chunks, bool block = false) {
     const size_t W = d->n_walkers, n = d->norb, o = d->nocc, G = d->nchol, no = n * o;
     UWS u = {};
     u.status = a.take<int>(64);  // status word: offset 0 of every workspace
@@ -141,6 +142,7 @@ UWS layout_u(Arena& a, const afq_dims* d, int n_chunks) {
     u.zeta = a.take<double>(1);
     u.wcopy = a.take<double2>(2 * W * no);
     u.ocopy = a.take<double2>(W);
+    if (block) take_oz_block(a, d, u.oz);
     return u;
 }
 
@@ -167,7 +169,7 @@ int force_bias_u(const afq_dims* d, const double* rot_chol, const UWS& u, double
     const int W = d->n_walkers, on = d->norb * d->nocc;
     AFQ_TRY(launch_spin_sum((long long)W * on, u.green, u.gsum, s));
     return launch_zgemm_auto(W, d->nchol, on, 1.0, u.gsum, on, rot_chol, on, !d->trial_is_real, true, fb, d->nchol,
-                             u.oz, s);
+                             u.oz, s, u.oz.rot);
 }
 
 int trotter_u(const afq_dims* d, int n_terms, double sqrt_dt, int n_chunks, const double* chol, const double* E,
@@ -179,7 +181,7 @@ int trotter_u(const afq_dims* d, int n_terms, double sqrt_dt, int n_chunks, cons
         const int wc = W - w0 < Wc ? W - w0 : Wc;
         { AFQ_PHASE("vbuild_gemm", s);
           AFQ_TRY(launch_zgemm_auto(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, V,
-                                    (int64_t)n * n, oz, s)); }
+                                    (int64_t)n * n, oz, s, oz.chol)); }
         AFQ_PHASE("trotter", s);
         AFQ_TRY(launch_trotter_spins(wc, n, o, n_terms, sqrt_dt, E, V, win + (size_t)w0 * n * o, wout + (size_t)w0 * n * o,
                                      half, oz, s));
@@ -403,7 +405,7 @@ int afq_apply_trotter_g(const afq_dims* d, int32_t n_terms, double sqrt_dt, int3
 size_t afq_u_workspace(const afq_dims* d, int32_t n_chunks) {
     if (check_u(d) != AFQ_OK) return 0;
     Arena a;
-    layout_u(a, d, n_chunks);
+    layout_u(a, d, n_chunks, true);
     return a.used;
 }
 
@@ -509,12 +511,13 @@ int afq_block_u(const afq_problem* pb, const afq_params* p, const afq_state* st,
     if (!p || !workspace || !block_energy || !block_weight)
         return fail(AFQ_E_INVALID_ARGUMENT, "NULL params, outputs or workspace");
     Arena a(workspace, workspace_bytes);
-    const UWS u = layout_u(a, &pb->dims, p->n_chunks);
+    const UWS u = layout_u(a, &pb->dims, p->n_chunks, true);
     if (!a.ok()) return fail(AFQ_E_WORKSPACE, "workspace: %zu bytes < %zu", workspace_bytes, a.used);
     cudaStream_t s = as_stream(stream);
     const afq_dims* d = &pb->dims;
     const int W = d->n_walkers, G = d->nchol;
     const size_t half = (size_t)W * d->norb * d->nocc;
+    if (p->n_prop_steps > 0) AFQ_TRY(split_oz_block(d, pb->chol, pb->rot_chol, u.oz, s));
     // prop/blocks.py:38-57
     for (int i = 0; i < p->n_prop_steps; ++i) {
         const bool last = i + 1 == p->n_prop_steps, qr = !last && p->qr_every > 0 && (i + 1) % p->qr_every == 0;

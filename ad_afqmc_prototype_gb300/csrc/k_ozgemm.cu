@@ -471,21 +471,38 @@ __device__ __forceinline__ int warp_max(int v) {
     return v;
 }
 
-// Real rows with K contiguous (row r at src + r ld), one warp a row; `per`
-// rows a batch; one: minus the identity.  Every split writes zeros from K up
-// to a multiple of 32.
+// The largest of the WR warps' values that share a row (WR = 1 or 8: the CTA).
+template <int WR>
+__device__ __forceinline__ int row_max(int e, int* s_max) {
+    e = warp_max(e);
+    if (WR == 1) return e;
+    __syncthreads();  // the last row's values have been read
+    if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = e;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) e = max(e, s_max[i]);
+    return e;
+}
+
+// Real rows with K contiguous (row r at src + r ld), a warp a row, or a CTA
+// (WR = 8) where rows are few; `per` rows a batch; one: minus the identity.
+// Every split writes zeros from K up to a multiple of 32.
+template <int WR>
 __global__ void __launch_bounds__(256) k_oz_rows(long long rows, int per, int K, const double* __restrict__ src,
                                                  long long ld, int one, OzDst dst, int* __restrict__ ex) {
-    const int lane = threadIdx.x & 31;
-    for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * 8) {
+    __shared__ int s_max[8];
+    const int t = WR == 1 ? threadIdx.x & 31 : threadIdx.x;  // place in the row's threads
+    for (long long r = (long long)blockIdx.x * (8 / WR) + (WR == 1 ? threadIdx.x >> 5 : 0); r < rows;
+         r += (long long)gridDim.x * (8 / WR)) {
         const double* x = src + r * ld;
         const long long rd = one ? r : -1;  // the diagonal entry to lower by one
         int e = 0;
-        for (int k = lane; k < K; k += 32) e = max(e, oz_expo(k == rd ? x[k] - 1.0 : x[k]));
-        const int E = oz_scale(warp_max(e));
-        if (lane == 0) ex[r] = E;
+#pragma unroll 4
+        for (int k = t; k < K; k += 32 * WR) e = max(e, oz_expo(k == rd ? x[k] - 1.0 : x[k]));
+        const int E = oz_scale(row_max<WR>(e, s_max));
+        if (t == 0) ex[r] = E;
         const long long b = r / per;
-        for (int k = 8 * lane; k < 32 * dst.nks; k += 256) {
+        for (int k = 8 * t; k < 32 * dst.nks; k += 256 * WR) {
             long long y[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) y[i] = oz_fix(k + i < K ? (k + i == rd ? x[k + i] - 1.0 : x[k + i]) : 0.0, E);
@@ -495,23 +512,27 @@ __global__ void __launch_bounds__(256) k_oz_rows(long long rows, int per, int K,
 }
 
 // Complex rows with K contiguous: digit rows 2 r (real parts) and 2 r + 1.
+template <int WR>
 __global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const double2* __restrict__ src, long long ld,
                                                   OzDst dst, int* __restrict__ ex) {
-    const int lane = threadIdx.x & 31;
-    for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < rows; r += (long long)gridDim.x * 8) {
+    __shared__ int s_max[2][8];
+    const int t = WR == 1 ? threadIdx.x & 31 : threadIdx.x;
+    for (long long r = (long long)blockIdx.x * (8 / WR) + (WR == 1 ? threadIdx.x >> 5 : 0); r < rows;
+         r += (long long)gridDim.x * (8 / WR)) {
         const double2* x = src + r * ld;
         int e0 = 0, e1 = 0;
-        for (int k = lane; k < K; k += 32) {
+#pragma unroll 4
+        for (int k = t; k < K; k += 32 * WR) {
             const double2 v = x[k];
             e0 = max(e0, oz_expo(v.x));
             e1 = max(e1, oz_expo(v.y));
         }
-        const int E0 = oz_scale(warp_max(e0)), E1 = oz_scale(warp_max(e1));
-        if (lane == 0) {
+        const int E0 = oz_scale(row_max<WR>(e0, s_max[0])), E1 = oz_scale(row_max<WR>(e1, s_max[1]));
+        if (t == 0) {
             ex[2 * r] = E0;
             ex[2 * r + 1] = E1;
         }
-        for (int k = 8 * lane; k < 32 * dst.nks; k += 256) {
+        for (int k = 8 * t; k < 32 * dst.nks; k += 256 * WR) {
             long long y[8], w[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -831,18 +852,24 @@ int oz_launch(int rows, int cols, int K, int batch, int adiv, const OzDigits& A,
 
 OzDst dst_of(const OzDigits& D, long long rows, int K) { return {D.d, nks_of(K), (int)round_up(rows, 8)}; }
 
-unsigned row_blocks(long long rows) {
-    const long long b = (rows + 7) / 8;
+unsigned row_blocks(long long rows, int per_cta = 8) {
+    const long long b = (rows + per_cta - 1) / per_cta;
     return (unsigned)(b > 152 * 64 ? 152 * 64 : b);
 }
+// A warp a row leaves SMs idle below some 16 warps an SM; a row of a few hundred k is short for a CTA.
+bool row_cta(long long rows, int K) { return rows < 16 * 152 && K >= 512; }
 int split_rows(long long rows, int per, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s,
                int one = 0) {
-    k_oz_rows<<<row_blocks(rows), 256, 0, s>>>(rows, per, K, src, ld, one, dst_of(D, per, K), D.ex);
+    const OzDst dst = dst_of(D, per, K);
+    if (row_cta(rows, K)) k_oz_rows<8><<<row_blocks(rows, 1), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
+    else k_oz_rows<1><<<row_blocks(rows), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
     AFQ_LAUNCHED("k_oz_rows");
     return AFQ_OK;
 }
 int split_crows(long long rows, int K, const double2* src, long long ld, const OzDigits& D, cudaStream_t s) {
-    k_oz_crows<<<row_blocks(rows), 256, 0, s>>>(rows, K, src, ld, dst_of(D, 2 * rows, K), D.ex);
+    const OzDst dst = dst_of(D, 2 * rows, K);
+    if (row_cta(rows, K)) k_oz_crows<8><<<row_blocks(rows, 1), 256, 0, s>>>(rows, K, src, ld, dst, D.ex);
+    else k_oz_crows<1><<<row_blocks(rows), 256, 0, s>>>(rows, K, src, ld, dst, D.ex);
     AFQ_LAUNCHED("k_oz_crows");
     return AFQ_OK;
 }
@@ -930,13 +957,34 @@ size_t zgemm_oz_scratch(int M, int N, int K) {
     return a.used + 256;
 }
 
+// Digits of a real operand kept by the caller (a block's steps share theirs): bytes, 0 where they would take more
+// than OZ_KEEP.
+constexpr long long OZ_KEEP = 640LL << 20;
+size_t oz_real_bytes(int N, int K) {
+    if (!zgemm_oz_pays(1, N, K) || round_up(N, 8) * digit_row_bytes(K) > OZ_KEEP) return 0;
+    Arena a;
+    take_digits(a, N, K);
+    return a.used + 256;
+}
+
+int oz_real_split(int N, int K, const double* B, int64_t ldb, bool b_trans, void* real, cudaStream_t s) {
+    Arena a(real, (size_t)-1);
+    const OzDigits D = take_digits(a, N, K);
+    return b_trans ? split_rows(N, N, K, B, ldb, D, s) : split_cols(N, K, B, ldb, D, s);
+}
+
 int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
-                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s) {
+                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s, const void* real) {
     if (M <= 0 || N <= 0) return AFQ_OK;
     int ae = 0;
     if (frexp(alpha, &ae) != 0.5) return fail(AFQ_E_UNSUPPORTED, "digit GEMM: alpha=%g is no power of two", alpha);
     Arena ar(scratch, (size_t)-1);
-    const ZLayout z = z_layout(ar, M, N, K);
+    ZLayout z = z_layout(ar, M, N, K);
+    if (real) {
+        Arena a((void*)real, (size_t)-1);
+        z.A = take_digits(a, N, K);
+        z.nc = N;
+    }
     int sms = 0;
     AFQ_TRY(device_sms(&sms));
     for (int m0 = 0; m0 < M; m0 += z.mc) {
@@ -944,7 +992,8 @@ int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t
         AFQ_TRY(split_crows(mc, K, A + (int64_t)m0 * lda, lda, z.B, s));
         for (int n0 = 0; n0 < N; n0 += z.nc) {
             const int nc = N - n0 < z.nc ? N - n0 : z.nc;
-            if (b_trans) AFQ_TRY(split_rows(nc, nc, K, B + (int64_t)n0 * ldb, ldb, z.A, s));
+            if (real) {}
+            else if (b_trans) AFQ_TRY(split_rows(nc, nc, K, B + (int64_t)n0 * ldb, ldb, z.A, s));
             else AFQ_TRY(split_cols(nc, K, B + n0, ldb, z.A, s));
             const OzOut out = {C + (int64_t)m0 * ldc + n0, 0, ldc, 0, 1, 1, ae - 1, nullptr};
             const long long tiles = (long long)((nc + OZ_ROWS - 1) / OZ_ROWS) * ((2 * mc + OZ_TN - 1) / OZ_TN);
@@ -1181,11 +1230,26 @@ int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, c
     return AFQ_OK;
 }
 
+void take_oz_block(Arena& a, const afq_dims* d, OzScratch& oz) {
+    const int n2 = d->norb * d->norb, on = d->nocc * d->norb;
+    const size_t c = oz_real_bytes(n2, d->nchol), r = d->trial_is_real ? oz_real_bytes(d->nchol, on) : 0;
+    oz.chol = c ? a.take<char>(c) : nullptr;
+    oz.rot = r ? a.take<char>(r) : nullptr;
+}
+
+int split_oz_block(const afq_dims* d, const double* chol, const double* rot_chol, const OzScratch& oz, cudaStream_t s) {
+    const int n2 = d->norb * d->norb, on = d->nocc * d->norb;
+    if (oz.chol) AFQ_TRY(oz_real_split(n2, d->nchol, chol, n2, false, oz.chol, s));
+    if (oz.rot) AFQ_TRY(oz_real_split(d->nchol, on, rot_chol, on, true, oz.rot, s));
+    return AFQ_OK;
+}
+
 // ---------------------------------------------------------------- routes --
 int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B, int64_t ldb,
-                      bool b_complex, bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s) {
+                      bool b_complex, bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s,
+                      const void* real) {
     if (!b_complex && zgemm_oz_pays(M, N, K))
-        return launch_zgemm_oz(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, ldc, oz.p, oz.err, s);
+        return launch_zgemm_oz(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, ldc, oz.p, oz.err, s, real);
     return launch_zgemm(M, N, K, alpha, A, lda, B, ldb, b_complex, b_trans, C, ldc, s);
 }
 
