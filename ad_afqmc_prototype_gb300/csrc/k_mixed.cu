@@ -185,19 +185,22 @@ int launch_field_shift_mixed(int W, int G, int Wc, double sqrt_dt, const double*
 }
 
 // ------------------------------------------------------- Taylor propagation
-// One CTA per (walker, 32 columns).  The current Taylor term T (fp32, all n
-// rows x 32 columns) stays in shared memory; the operand (V of this walker,
-// or E_half - I) streams through a two-stage cp.async ring, TR_BJ columns per
-// stage, so the next columns are in flight while the current ones are
-// multiplied.  Thread (rg, cg) owns rows rg + RG q (q < NR) and the complex
-// columns 2cg, 2cg+1, 16+2cg, 16+2cg+1 (so a warp's T reads are contiguous
-// 128-byte rows).  Each thread touches only its own entries of the output
+// One CTA per (walker, OC columns), OC = 4 CG <= 32.  The current Taylor term T
+// (fp32, all n rows x OC columns) stays in shared memory; the operand (V of
+// this walker, or E_half - I) streams through a two-stage cp.async ring, TR_BJ
+// columns per stage, so the next columns are in flight while the current ones
+// are multiplied.  Thread (rg, cg) owns rows rg + RG q (q < NR) and the complex
+// columns 2cg, 2cg+1, OC/2+2cg, OC/2+2cg+1 (so a warp's T reads are contiguous
+// rows).  The fp32 pipe bounds it, so the split wastes few rows and columns:
+// CG covers nocc in steps of four, and (RG, NR) is chosen for the fewest warps x
+// rows (launch_trotter_mixed).  With 32 columns and 32 row groups always, 75
+// orbitals x 13 took 2.4 times the multiplies they take now.  Each thread touches only its own entries of the output
 // walker (walkers_out may alias walkers_in) and of the fp32 scratch Ts that
 // sums the series terms, so the binary64 pipe sees three additions per
 // entry, not one per term:
 //   W1 = W + (E-I) W;  Ts = sum_k (i sqrt_dt V)^k / k! W1 (fp32);
 //   out = W1 + Ts;  W' = out + (E-I) out.
-constexpr int TR_CG = 8, TR_OC = 32, TR_BJ = 8;
+constexpr int TR_OC = 32, TR_BJ = 8;  // most columns a CTA; operand columns a stage
 // Row stride (floats) of a staged operand plane: 16-byte rows for cp.async,
 // and rows 0..3 of a warp start in different banks.
 constexpr int TR_VS = TR_BJ + 4;
@@ -241,10 +244,11 @@ __device__ __forceinline__ void tr_stage(int n, int j0, const float* __restrict_
 // acc = M T for the n x n operand M (real when im == nullptr).  stg holds two
 // stages of two planes, rows padded to RG*NR and zero beyond n.  Ends with a
 // barrier, so the caller may overwrite T and the stages.
-template <int NR, bool CPLX>
+template <int NR, bool CPLX, int CGT>
 __device__ __forceinline__ void tr_matmul(int n, const float* __restrict__ re, const float* __restrict__ im,
                                           const float4* __restrict__ T4, float* stg, int rows, float2 (&acc)[NR][4],
-                                          int cg, int rg, int RG, bool v16) {
+                                          int cg, int CGr, int rg, int RG, bool v16) {
+    const int CG = CGT ? CGT : CGr;
 #pragma unroll
     for (int q = 0; q < NR; ++q)
 #pragma unroll
@@ -261,7 +265,7 @@ __device__ __forceinline__ void tr_matmul(int n, const float* __restrict__ re, c
             float* nr_ = stg + ((b + 1) & 1) * 2 * plane;
             tr_stage(n, (b + 1) * TR_BJ, re, im, nr_, nr_ + plane, v16);
         }
-        const float4* tb = T4 + (size_t)b * TR_BJ * (TR_OC / 2);
+        const float4* tb = T4 + (size_t)b * TR_BJ * (2 * CG) + cg;
 #pragma unroll 1
         for (int jj = 0; jj < TR_BJ; jj += 2) {
             float2 mr[NR], mi[NR];
@@ -273,7 +277,8 @@ __device__ __forceinline__ void tr_matmul(int n, const float* __restrict__ re, c
             }
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const float4 ta = tb[(jj + h) * (TR_OC / 2) + cg], tc = tb[(jj + h) * (TR_OC / 2) + TR_CG + cg];
+                const float4 ta = tb[0], tc = tb[CG];
+                tb += 2 * CG;
                 const float2 t[4] = {make_float2(ta.x, ta.y), make_float2(ta.z, ta.w), make_float2(tc.x, tc.y),
                                      make_float2(tc.z, tc.w)};
                 float2 tn[4];  // i t
@@ -296,21 +301,25 @@ __device__ __forceinline__ void tr_matmul(int n, const float* __restrict__ re, c
     __syncthreads();
 }
 
-__device__ __forceinline__ int tr_col(int cg, int j) { return j < 2 ? 2 * cg + j : TR_OC / 2 + 2 * cg + (j - 2); }
+__device__ __forceinline__ int tr_col(int cg, int CG, int j) { return j < 2 ? 2 * cg + j : 2 * CG + 2 * cg + (j - 2); }
 
-template <int NR>
+// CGT: the column groups where that is a constant (8, for nocc a little below a multiple of 32), else 0.
+template <int NR, int CGT>
 __global__ void __launch_bounds__(512) k_trotter_mixed(int n, int o, int n_terms, float sqrt_dt,
                                                           const float* __restrict__ emi, const float* __restrict__ vm,
                                                           long long ldv, int wc, const double2* win, double2* wout,
-                                                          float2* __restrict__ tsum, int v16) {
+                                                          float2* __restrict__ tsum, int v16, int CGr, int RG) {
     extern __shared__ float4 smf4[];
-    const int RG = blockDim.x / TR_CG, rows = RG * NR;
+    const int CG = CGT ? CGT : CGr;
+    const int rows = RG * NR, OC = 4 * CG;
     const int nT = (n + TR_BJ - 1) / TR_BJ * TR_BJ;
-    float4* T4 = smf4;                              // nT x 32 complex, as float4 pairs
+    float4* T4 = smf4;                              // nT x OC complex, as float4 pairs
     float2* T = (float2*)smf4;
-    float* stg = (float*)(smf4 + (size_t)nT * (TR_OC / 2));  // 2 stages x 2 planes x rows x TR_VS
-    const int w = blockIdx.y, c0 = blockIdx.x * TR_OC;
-    const int cg = threadIdx.x % TR_CG, rg = threadIdx.x / TR_CG;
+    float* stg = (float*)(smf4 + (size_t)nT * (OC / 2));  // 2 stages x 2 planes x rows x TR_VS
+    const int w = blockIdx.y, c0 = blockIdx.x * OC;
+    // threads past RG x CG (the last warp's rest) repeat row group 0 and write nothing
+    const bool act = threadIdx.x < RG * CG;
+    const int cg = threadIdx.x % CG, rg = act ? threadIdx.x / CG : 0;
     const double2* Wp = win + (size_t)w * n * o;
     double2* Wo = wout + (size_t)w * n * o;
     const float* Vr = vm + (long long)w * ldv;
@@ -318,8 +327,8 @@ __global__ void __launch_bounds__(512) k_trotter_mixed(int n, int o, int n_terms
     float2* Ts = tsum + (size_t)w * n * o;
 
     for (int e = threadIdx.x; e < 4 * rows * TR_VS; e += blockDim.x) stg[e] = 0.f;
-    for (int e = threadIdx.x; e < nT * TR_OC; e += blockDim.x) {
-        const int i = e / TR_OC, cc = e % TR_OC;
+    for (int e = threadIdx.x; e < nT * OC; e += blockDim.x) {
+        const int i = e / OC, cc = e - i * OC;
         float2 t = make_float2(0.f, 0.f);
         if (i < n && c0 + cc < o) {
             const double2 v = Wp[(size_t)i * o + c0 + cc];
@@ -331,7 +340,7 @@ __global__ void __launch_bounds__(512) k_trotter_mixed(int n, int o, int n_terms
     float2 acc[NR][4];
     int rgl;  // rg, opaque to the compiler: entry addresses are recomputed per epilogue, not held in registers
     // W1 = W + (E - I) W
-    tr_matmul<NR, false>(n, emi, nullptr, T4, stg, rows, acc, cg, rg, RG, v16);
+    tr_matmul<NR, false, CGT>(n, emi, nullptr, T4, stg, rows, acc, cg, CG, rg, RG, v16);
     rgl = rg;
     asm volatile("" : "+r"(rgl));
 #pragma unroll
@@ -339,18 +348,18 @@ __global__ void __launch_bounds__(512) k_trotter_mixed(int n, int o, int n_terms
         const int i = rgl + RG * q;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int cl = tr_col(cg, j), c = c0 + cl;
-            if (i < n && c < o) {
+            const int cl = tr_col(cg, CG, j), c = c0 + cl;
+            if (act && i < n && c < o) {
                 const double2 v = Wp[(size_t)i * o + c];
                 const double2 w1 = make_double2(v.x + (double)acc[q][j].x, v.y + (double)acc[q][j].y);
                 Wo[(size_t)i * o + c] = w1;
-                T[i * TR_OC + cl] = make_float2((float)w1.x, (float)w1.y);
+                T[i * OC + cl] = make_float2((float)w1.x, (float)w1.y);
             }
         }
     }
     __syncthreads();
     for (int k = 1; k <= n_terms; ++k) {
-        tr_matmul<NR, true>(n, Vr, Vi, T4, stg, rows, acc, cg, rg, RG, v16);
+        tr_matmul<NR, true, CGT>(n, Vr, Vi, T4, stg, rows, acc, cg, CG, rg, RG, v16);
         const float sk = sqrt_dt / (float)k;  // (i sqrt_dt / k) z = sk (-z.y, z.x)
         rgl = rg;
         asm volatile("" : "+r"(rgl));
@@ -359,10 +368,10 @@ __global__ void __launch_bounds__(512) k_trotter_mixed(int n, int o, int n_terms
             const int i = rgl + RG * q;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const int cl = tr_col(cg, j), c = c0 + cl;
+                const int cl = tr_col(cg, CG, j), c = c0 + cl;
                 const float2 t = make_float2(-sk * acc[q][j].y, sk * acc[q][j].x);
-                if (i < n) T[i * TR_OC + cl] = (c < o) ? t : make_float2(0.f, 0.f);
-                if (i < n && c < o) {
+                if (act && i < n) T[i * OC + cl] = (c < o) ? t : make_float2(0.f, 0.f);
+                if (act && i < n && c < o) {
                     float2* ts = Ts + (size_t)i * o + c;
                     if (k == 1) {
                         *ts = t;
@@ -383,8 +392,8 @@ __global__ void __launch_bounds__(512) k_trotter_mixed(int n, int o, int n_terms
         const int i = rgl + RG * q;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int cl = tr_col(cg, j), c = c0 + cl;
-            if (i < n && c < o) {
+            const int cl = tr_col(cg, CG, j), c = c0 + cl;
+            if (act && i < n && c < o) {
                 double2 v = Wo[(size_t)i * o + c];
                 if (n_terms > 0) {
                     const float2 u = Ts[(size_t)i * o + c];
@@ -392,12 +401,12 @@ __global__ void __launch_bounds__(512) k_trotter_mixed(int n, int o, int n_terms
                     v.y += (double)u.y;
                     Wo[(size_t)i * o + c] = v;
                 }
-                T[i * TR_OC + cl] = make_float2((float)v.x, (float)v.y);
+                T[i * OC + cl] = make_float2((float)v.x, (float)v.y);
             }
         }
     }
     __syncthreads();
-    tr_matmul<NR, false>(n, emi, nullptr, T4, stg, rows, acc, cg, rg, RG, v16);
+    tr_matmul<NR, false, CGT>(n, emi, nullptr, T4, stg, rows, acc, cg, CG, rg, RG, v16);
     rgl = rg;
     asm volatile("" : "+r"(rgl));
 #pragma unroll
@@ -405,8 +414,8 @@ __global__ void __launch_bounds__(512) k_trotter_mixed(int n, int o, int n_terms
         const int i = rgl + RG * q;
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-            const int c = c0 + tr_col(cg, j);
-            if (i < n && c < o) {
+            const int c = c0 + tr_col(cg, CG, j);
+            if (act && i < n && c < o) {
                 double2 v = Wo[(size_t)i * o + c];
                 v.x += (double)acc[q][j].x;
                 v.y += (double)acc[q][j].y;
@@ -428,24 +437,60 @@ int launch_trotter_mixed(int wc, int n, int o, int n_terms, double sqrt_dt, cons
                          long long ldv, const double2* win, double2* wout, float2* tsum, cudaStream_t s) {
     if (wc <= 0) return AFQ_OK;
     if (wc > 65535) return fail(AFQ_E_UNSUPPORTED, "mixed trotter: chunk of %d walkers > 65535", wc);
-    // 256 threads (32 row groups) up to 7 rows each, else 512 threads
-    const int threads = n <= 32 * 7 ? 256 : 512, RG = threads / TR_CG;
-    const int nr = (n + RG - 1) / RG;
-    if (nr > 8) return fail(AFQ_E_UNSUPPORTED, "mixed trotter: norb=%d too large", n);
+    // Columns in as many groups of four as nocc needs.  Rows a thread: for two operand columns a warp issues 16 r
+    // paired FMAs (two clocks each) behind ~100 clocks of shared-memory latency, and an SM's CTAs share four
+    // schedulers: few walkers take few rows a thread (75 orbitals, 8 walkers: more warps), many the fewest multiplies,
+    // as long as the registers leave 16 warps an SM (180 x 32: nine warps of five rows, one CTA an SM, took 1.5 times
+    // as long as eight of six, two an SM).
+    static const int regs[9] = {0, 48, 64, 80, 104, 120, 128, 128, 128};  // by rows a thread
+    const int nb = (o + TR_OC - 1) / TR_OC;
+    int CG = ((o + nb - 1) / nb + 3) / 4;
+    const long long q = ((long long)nb * wc + 151) / 152;
+    int nr = 0, RG = 0;
+    long long best = 0;
+    for (int r = 8; r >= 1; --r) {
+        const int g = (n + r - 1) / r, warps = (g * CG + 31) / 32;
+        if (warps > 16) continue;
+        const long long ctas = 65536 / (32 * warps * regs[r]), res = warps * (ctas < q ? ctas : q);  // warps an SM holds
+        // eight rows spill
+        const long long lat = 100 + 32 * r, thr = (r == 8 ? 10 : 8) * q * warps * r * 16 / (res > 0 && res < 16 ? res : 16);
+        const long long cost = (lat > thr ? lat : thr) * 16 + warps;
+        if (res == 0 || (nr && cost >= best)) continue;
+        nr = r;
+        RG = g;
+        best = cost;
+    }
+    if (!nr) return fail(AFQ_E_UNSUPPORTED, "mixed trotter: norb=%d too large", n);
+    if (q == 1) {  // an SM has one CTA: all 32 columns over 256 or 512 threads unless that is much more work (250 x 27,
+                   // 8 walkers: 863 us, 887 with seven column groups)
+        const int g = n <= 32 * 7 ? 32 : 64, r = (n + g - 1) / g;
+        if (r <= 8 && (RG * CG + 31) / 32 * nr * 100 > 85 * (g / 4) * r) {
+            CG = 8;
+            RG = g;
+            nr = r;
+        }
+    }
+    const int threads = (RG * CG + 31) / 32 * 32;
     const int nT = (n + TR_BJ - 1) / TR_BJ * TR_BJ;
-    const size_t smem = (size_t)nT * TR_OC * sizeof(float2) + (size_t)4 * RG * nr * TR_VS * sizeof(float);
+    const size_t smem = (size_t)nT * 4 * CG * sizeof(float2) + (size_t)4 * RG * nr * TR_VS * sizeof(float);
     const int v16 = (n % 4 == 0) && (ldv % 4 == 0) && ((((uintptr_t)vm) | ((uintptr_t)emi)) & 15) == 0;
-    dim3 grid((o + TR_OC - 1) / TR_OC, wc);
-#define AFQ_TM(NRV)                                                                                      \
-    case NRV:                                                                                            \
-        AFQ_TRY(smem_attr(k_trotter_mixed<NRV>, smem));                                                  \
-        k_trotter_mixed<NRV><<<grid, threads, smem, s>>>(n, o, n_terms, (float)sqrt_dt, emi, vm, ldv, wc, win, \
-                                                         wout, tsum, v16);                               \
+    dim3 grid(nb, wc);
+#define AFQ_TM2(NRV, CGV)                                                                                       \
+    do {                                                                                                        \
+        AFQ_TRY(smem_attr(k_trotter_mixed<NRV, CGV>, smem));                                                    \
+        k_trotter_mixed<NRV, CGV><<<grid, threads, smem, s>>>(n, o, n_terms, (float)sqrt_dt, emi, vm, ldv, wc, win, \
+                                                              wout, tsum, v16, CG, RG);                         \
+    } while (0)
+#define AFQ_TM(NRV)                      \
+    case NRV:                            \
+        if (CG == 8) AFQ_TM2(NRV, 8);    \
+        else AFQ_TM2(NRV, 0);            \
         break;
     switch (nr) {
         AFQ_TM(1) AFQ_TM(2) AFQ_TM(3) AFQ_TM(4) AFQ_TM(5) AFQ_TM(6) AFQ_TM(7) AFQ_TM(8)
     }
 #undef AFQ_TM
+#undef AFQ_TM2
     AFQ_LAUNCHED("k_trotter_mixed");
     return AFQ_OK;
 }
