@@ -194,7 +194,11 @@ int launch_field_shift_mixed(int W, int G, int Wc, double sqrt_dt, const double*
 // rows).  The fp32 pipe bounds it, so the split wastes few rows and columns:
 // CG covers nocc in steps of four, and (RG, NR) is chosen for the fewest warps x
 // rows (launch_trotter_mixed).  With 32 columns and 32 row groups always, 75
-// orbitals x 13 took 2.4 times the multiplies they take now.  Each thread touches only its own entries of the output
+// orbitals x 13 took 2.4 times the multiplies they take now.  Next to the FMAs
+// the copies' index arithmetic counts, so the operand's planes are a constant
+// of the copy loop.  Six terms, against 32 x 32 groups: 75 x 13, 777 walkers
+// 542 -> 236 us; 120 x 20, 2048 walkers 1.96 -> 1.16 ms; 200 x 30, 2048
+// walkers 4.82 -> 4.41 ms.  Each thread touches only its own entries of the output
 // walker (walkers_out may alias walkers_in) and of the fp32 scratch Ts that
 // sums the series terms, so the binary64 pipe sees three additions per
 // entry, not one per term:
@@ -218,23 +222,27 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 
 // Columns [j0, j0 + TR_BJ) of rows 0..n-1 of the operand planes (row stride
 // n floats) into a stage; columns past n are zero.
+template <bool CPLX>
 __device__ __forceinline__ void tr_stage(int n, int j0, const float* __restrict__ re, const float* __restrict__ im,
                                          float* sr, float* si, bool v16) {
     const int jn = min(TR_BJ, n - j0);
-    const int planes = im ? 2 : 1;
     if (v16) {  // n % 4 == 0 and 16-byte aligned planes: jn is a multiple of 4
-        constexpr int CH = TR_BJ / 4;
-        for (int e = threadIdx.x; e < n * CH * planes; e += blockDim.x) {
-            const int i = e / (CH * planes), r = e % (CH * planes), pl = r / CH, h = r % CH;
+        constexpr int CH = TR_BJ / 4, G = CPLX ? 2 * CH : CH;
+        for (int e = threadIdx.x; e < n * G; e += blockDim.x) {
+            const int i = e / G, r = e % G, pl = r / CH, h = r % CH;
             float* dst = (pl ? si : sr) + i * TR_VS + 4 * h;
             if (4 * h < jn) cp_async16(dst, (pl ? im : re) + (size_t)i * n + j0 + 4 * h);
             else *(float4*)dst = make_float4(0.f, 0.f, 0.f, 0.f);
         }
     } else {
-        for (int e = threadIdx.x; e < n * TR_BJ * planes; e += blockDim.x) {
-            const int i = e / (TR_BJ * planes), r = e % (TR_BJ * planes), pl = r / TR_BJ, jj = r % TR_BJ;
-            float* dst = (pl ? si : sr) + i * TR_VS + jj;
-            if (jj < jn) cp_async4(dst, (pl ? im : re) + (size_t)i * n + j0 + jj);
+        // four times the copies: a thread keeps its plane and column (blockDim.x
+        // is a multiple of 32, so of G) and walks the rows by two additions
+        constexpr int G = CPLX ? 2 * TR_BJ : TR_BJ;
+        const int step = blockDim.x / G, i0 = threadIdx.x / G, r = threadIdx.x % G, pl = r / TR_BJ, jj = r % TR_BJ;
+        float* dst = (pl ? si : sr) + i0 * TR_VS + jj;
+        const float* src = (pl ? im : re) + (size_t)i0 * n + j0 + jj;
+        for (int i = i0; i < n; i += step, dst += step * TR_VS, src += (size_t)step * n) {
+            if (jj < jn) cp_async4(dst, src);
             else *dst = 0.f;
         }
     }
@@ -255,7 +263,7 @@ __device__ __forceinline__ void tr_matmul(int n, const float* __restrict__ re, c
         for (int j = 0; j < 4; ++j) acc[q][j] = make_float2(0.f, 0.f);
     const int plane = rows * TR_VS;
     const int nb = (n + TR_BJ - 1) / TR_BJ;
-    tr_stage(n, 0, re, im, stg, stg + plane, v16);
+    tr_stage<CPLX>(n, 0, re, im, stg, stg + plane, v16);
     for (int b = 0; b < nb; ++b) {
         cp_async_wait_all();
         __syncthreads();
@@ -263,7 +271,7 @@ __device__ __forceinline__ void tr_matmul(int n, const float* __restrict__ re, c
         const float* si = sr + plane;
         if (b + 1 < nb) {
             float* nr_ = stg + ((b + 1) & 1) * 2 * plane;
-            tr_stage(n, (b + 1) * TR_BJ, re, im, nr_, nr_ + plane, v16);
+            tr_stage<CPLX>(n, (b + 1) * TR_BJ, re, im, nr_, nr_ + plane, v16);
         }
         const float4* tb = T4 + (size_t)b * TR_BJ * (2 * CG) + cg;
 #pragma unroll 1
