@@ -281,8 +281,7 @@ static int trotter_chunked(const afq_dims* d, int n_terms, double sqrt_dt, int n
         const int wc = W - w0 < Wc ? W - w0 : Wc;
         // V (wc x n^2) = x~ (wc x G) . chol (G x n^2)   (prop/chol_afqmc_ops.py:70-74)
         { AFQ_PHASE("vbuild_gemm", s);
-        AFQ_TRY(launch_zgemm_auto(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, V,
-                                  (int64_t)n * n, oz, s, oz.chol)); }
+        AFQ_TRY(launch_vbuild(wc, n, G, xs + (size_t)w0 * G, chol, V, oz, s)); }
         { AFQ_PHASE("trotter", s);
         AFQ_TRY(launch_trotter_auto(wc, n, o, n_terms, sqrt_dt, E, V, win + (size_t)w0 * n * o,
                                     wout + (size_t)w0 * n * o, 1, oz, s)); }

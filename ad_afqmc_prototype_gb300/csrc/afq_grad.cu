@@ -227,8 +227,7 @@ int step_adjoint(const Ctx& c, const BlockSnap& sn, int op, int st_i, uint64_t c
     const double2* V = sn.V ? sn.V + (size_t)st_i * W * n * n : g.V;
     if (!sn.V) {
         AFQ_PHASE("adj_vbuild_gemm", s);
-        AFQ_TRY(launch_zgemm_auto(W, n * n, G, 1.0, g.xs, G, pb->chol, (int64_t)n * n, false, false, g.V,
-                             (int64_t)n * n, g.oz, s));
+        AFQ_TRY(launch_vbuild(W, n, G, g.xs, pb->chol, g.V, g.oz, s));
     }
     { AFQ_PHASE("adj_taylor_tape", s);
       AFQ_TRY(launch_taylor_tape(W, n, o, K, pb->sqrt_dt, pb->exp_h1_half, V, Wpre, g.terms, g.w2, s)); }

@@ -309,6 +309,7 @@ struct OzScratch {
     // a block's steps: digits of chol (n^2 rows over the vectors) and of rot_chol (vectors over nocc norb), or null
     void* chol = nullptr;
     void* rot = nullptr;
+    int* asym = nullptr;  // with chol: its rows are in the order of symmetric vectors unless *asym
 };
 // room for a block's kept digits, and their split (once a block)
 void take_oz_block(Arena& a, const afq_dims* d, OzScratch& oz);
@@ -319,9 +320,8 @@ size_t zgemm_oz_scratch(int M, int N, int K);
 int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
                     bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s,
                     const void* real = nullptr);
-// digits of the real operand kept over several products (`real` above and below): bytes (0: not kept), and the split
+// room for digits of the real operand kept over several products (`real` above and below); 0: not kept
 size_t oz_real_bytes(int N, int K);
-int oz_real_split(int N, int K, const double* B, int64_t ldb, bool b_trans, void* real, cudaStream_t s);
 bool green_oz_pays(int n, int o);
 size_t green_oz_scratch(int W, int n, int o);
 int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walkers, double2* ovlp_out,
@@ -348,6 +348,9 @@ int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, c
 int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B, int64_t ldb,
                       bool b_complex, bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s,
                       const void* real = nullptr);
+// V (W x n^2) = xs (W x G) . chol (G x n^2), half of it where chol is symmetric and that pays
+int launch_vbuild(int W, int n, int G, const double2* xs, const double* chol, double2* V, const OzScratch& oz,
+                  cudaStream_t s);
 int launch_trotter_auto(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
                         const double2* win, double2* wout, int vdiv, const OzScratch& oz, cudaStream_t s);
 // both spins of W walkers with the walker's V, the second spin's blocks `half` entries after the first's

@@ -180,8 +180,7 @@ int trotter_u(const afq_dims* d, int n_terms, double sqrt_dt, int n_chunks, cons
     for (int w0 = 0; w0 < W; w0 += Wc) {
         const int wc = W - w0 < Wc ? W - w0 : Wc;
         { AFQ_PHASE("vbuild_gemm", s);
-          AFQ_TRY(launch_zgemm_auto(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, V,
-                                    (int64_t)n * n, oz, s, oz.chol)); }
+          AFQ_TRY(launch_vbuild(wc, n, G, xs + (size_t)w0 * G, chol, V, oz, s)); }
         AFQ_PHASE("trotter", s);
         AFQ_TRY(launch_trotter_spins(wc, n, o, n_terms, sqrt_dt, E, V, win + (size_t)w0 * n * o, wout + (size_t)w0 * n * o,
                                      half, oz, s));
@@ -392,8 +391,7 @@ int afq_apply_trotter_g(const afq_dims* d, int32_t n_terms, double sqrt_dt, int3
     const double2* xs = (const double2*)shifted_fields;
     for (int w0 = 0; w0 < W; w0 += Wc) {
         const int wc = W - w0 < Wc ? W - w0 : Wc;
-        AFQ_TRY(launch_zgemm_auto(wc, n * n, G, 1.0, xs + (size_t)w0 * G, G, chol, (int64_t)n * n, false, false, g.V,
-                                  (int64_t)n * n, g.oz, s));
+        AFQ_TRY(launch_vbuild(wc, n, G, xs + (size_t)w0 * G, chol, g.V, g.oz, s));
         // the top and bottom n x 2o halves of each walker, both with the walker's V
         AFQ_TRY(launch_trotter_auto(2 * wc, n, 2 * o, n_terms, sqrt_dt, exp_h1_half, g.V,
                                     (const double2*)walkers + (size_t)w0 * 4 * n * o,

@@ -83,6 +83,35 @@ __device__ __forceinline__ uint64_t desc_k64(uint32_t saddr) {
     return d;
 }
 
+// Symmetric Cholesky vectors: V-build rows (i, j) and (j, i) are the same
+// sums, so only the 8 x 8 blocks (I <= J) of the n x n rows are cut and
+// multiplied, in the order J (J + 1) / 2 + I, and a result is written to both
+// places (an entry of its own would have the same bits).  Whether the vectors
+// are symmetric is seen on the device (*asym == 0); otherwise the rows are the
+// n^2 of L as they come.  Blocks of 8 keep the mirrored writes at whole 32-byte
+// sectors and cost n = 61 2304 rows of 3721, n = 200 20800 of 40000.
+struct OzSym {
+    const int* asym;  // null: rows as they come
+    int n, r0;        // orbitals; first row of this chunk (rows as they come: added to their place)
+};
+__host__ __device__ __forceinline__ int oz_sym_total(int n) { return ((n + 7) / 8) * ((n + 7) / 8 + 1) * 32; }
+__device__ __forceinline__ bool oz_sym_on(const OzSym& y) { return y.asym && *y.asym == 0; }
+// rows of the chunk, of `rows` as they come
+__device__ __forceinline__ int oz_sym_rows(const OzSym& y, bool on, int rows) {
+    return on ? max(0, min(rows, oz_sym_total(y.n) - y.r0)) : rows;
+}
+// entry (i, j) of row r; false: a block's part past n
+__device__ __forceinline__ bool oz_sym_at(const OzSym& y, int r, int& i, int& j) {
+    r += y.r0;
+    const int b = r >> 6;
+    int J = (int)((sqrtf(8.f * b + 1.f) - 1.f) * 0.5f);
+    if (J * (J + 1) / 2 > b) --J;
+    if ((J + 1) * (J + 2) / 2 <= b) ++J;
+    i = 8 * (b - J * (J + 1) / 2) + ((r >> 3) & 7);
+    j = 8 * J + (r & 7);
+    return i < y.n && j < y.n;
+}
+
 // Where output (row r, complex column m) of batch b goes: C[b bs + (m / md)
 // ms1 + (m % md) ms0 + r rs], times 2^aexp, plus the same entry of add.
 struct OzOut {
@@ -104,6 +133,7 @@ struct OzArgs {
     float* rawt;
     int* err;
     OzOut out;
+    OzSym sym;
 };
 
 __device__ __forceinline__ void oz_tile(const OzArgs& a, int t, int mt, int nt, int& z, int& mb, int& nb) {
@@ -234,8 +264,11 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
     uint32_t* tmem_slot = (uint32_t*)(smem_raw + (bars + 8 * OZB_N - smem_u32(smem_raw)));
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const int mt = (a.rows + OZ_ROWS - 1) / OZ_ROWS, nt = (a.cols + OZ_TN - 1) / OZ_TN;
+    const bool sym = oz_sym_on(a.sym);
+    const int rows = oz_sym_rows(a.sym, sym, a.rows);
+    const int mt = (rows + OZ_ROWS - 1) / OZ_ROWS, nt = (a.cols + OZ_TN - 1) / OZ_TN;
     const int ntiles = mt * nt * a.batch * a.splits, kst = (a.K + OZ_BK - 1) / OZ_BK;
+    if ((int)blockIdx.x >= ntiles) return;  // the symmetric rows take fewer CTAs
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < OZB_N; ++i)  // one arrival an epilogue warp on a drained slot
@@ -381,7 +414,7 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
                 *abort_flag = 1;
                 break;
             }
-            if (row >= a.rows) continue;
+            if (row >= rows) continue;
             if (a.splits > 1) {
                 const long long at = (long long)sp * a.cols * a.rows + row;
 #pragma unroll
@@ -394,7 +427,15 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
             }
             const int* eb = a.eb + (a.adiv ? (long long)b * a.cols : 0) + c0;
             const int ea = a.ea[(a.adiv ? b / a.adiv * a.rows : 0) + row];
-            const long long at = (long long)b * a.out.bs + (long long)row * a.out.rs;
+            long long at = (long long)b * a.out.bs + (long long)row * a.out.rs, mirror = 0;
+            if (sym) {
+                int i, j;
+                if (!oz_sym_at(a.sym, row, i, j)) continue;
+                at = (long long)i * a.sym.n + j;
+                if (i >> 3 != j >> 3) mirror = (long long)j * a.sym.n + i - at;
+            } else {
+                at += a.sym.r0;
+            }
             const int ex = ea - 14 + a.out.aexp;
 #pragma unroll
             for (int j = 0; j < OZ_CW; j += 2) {
@@ -408,6 +449,7 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
                     const long long e = at + (long long)mh * a.out.ms1 + (long long)(m - mh * a.out.md) * a.out.ms0;
                     if (a.out.add) v = cadd(v, a.out.add[e]);
                     a.out.C[e] = v;
+                    if (mirror) a.out.C[e + mirror] = v;
                 }
             }
         }
@@ -423,10 +465,14 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
 
 // The K splits' sums added (the integers exactly, the tails in order) and converted.
 __global__ void k_oz_finish(const OzArgs a) {
-    const long long total = (long long)a.rows * (a.cols >> 1);
+    const bool sym = oz_sym_on(a.sym);
+    const int rows = oz_sym_rows(a.sym, sym, a.rows);
+    const long long total = (long long)rows * (a.cols >> 1);
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (long long)gridDim.x * blockDim.x) {
-        const int m = (int)(e / a.rows), row = (int)(e - (long long)m * a.rows);
+        const int m = (int)(e / rows), row = (int)(e - (long long)m * rows);
+        int i = 0, j = 0;
+        if (sym && !oz_sym_at(a.sym, row, i, j)) continue;
         long long re = 0, im = 0;
         float tr = 0.f, ti = 0.f;
         for (int z = 0; z < a.splits; ++z) {
@@ -441,10 +487,38 @@ __global__ void k_oz_finish(const OzArgs a) {
         if (ea == OZ_NAN || e0 == OZ_NAN) v.x = __longlong_as_double(0x7ff8000000000000ll);
         if (ea == OZ_NAN || e1 == OZ_NAN) v.y = __longlong_as_double(0x7ff8000000000000ll);
         const int mh = m / a.out.md;
-        const long long at = (long long)row * a.out.rs + (long long)mh * a.out.ms1 + (long long)(m - mh * a.out.md) * a.out.ms0;
+        const long long am = (long long)mh * a.out.ms1 + (long long)(m - mh * a.out.md) * a.out.ms0;
+        const long long at = am + (sym ? (long long)i * a.sym.n + j : (long long)row * a.out.rs + a.sym.r0);
         if (a.out.add) v = cadd(v, a.out.add[at]);
         a.out.C[at] = v;
+        if (sym && i >> 3 != j >> 3) a.out.C[am + (long long)j * a.sym.n + i] = v;
     }
+}
+
+// *asym |= the G matrices (n x n) are not all symmetric, bit for bit: 32 x 32 blocks I <= J against their mirrors.
+__global__ void __launch_bounds__(256) k_oz_asym(int n, int G, const double* __restrict__ L, int* asym) {
+    __shared__ unsigned long long tile[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+    int J = 0, I = blockIdx.x;
+    while (I > J) I -= ++J;
+    bool bad = false;
+    for (int g = blockIdx.y; g < G; g += gridDim.y) {
+        const unsigned long long* x = (const unsigned long long*)L + (size_t)g * n * n;
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int i = 32 * I + ty + 8 * q, j = 32 * J + tx;
+            tile[ty + 8 * q][tx] = i < n && j < n ? x[(size_t)i * n + j] : 0ull;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int j = 32 * J + ty + 8 * q, i = 32 * I + tx;
+            if (i < n && j < n && x[(size_t)j * n + i] != tile[tx][ty + 8 * q]) bad = true;
+        }
+        if (__syncthreads_or(bad || *(volatile int*)asym)) break;
+    }
+    if (bad) *asym = 1;
 }
 
 // ------------------------------------------------------------------ digits --
@@ -546,22 +620,34 @@ __global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const d
     }
 }
 
-// Real rows with K strided: row r's entry k at src[k ld + r es]; RB rows a CTA
-// (32, or 8 where few rows would leave SMs idle), transposed through shared memory.
+// Real rows with K strided: row r's entry k at src[k ld + r es] (or at the
+// place of symmetric vectors' row r); RB rows a CTA (32, or 8 where few rows
+// would leave SMs idle), transposed through shared memory.
 template <int RB>
-__global__ void __launch_bounds__(256) k_oz_cols(int rows, int K, const double* __restrict__ src, long long ld, int es,
-                                                 OzDst dst, int* __restrict__ ex) {
+__global__ void __launch_bounds__(256) k_oz_cols(int nrows, int K, const double* __restrict__ src, long long ld, int es,
+                                                 OzDst dst, int* __restrict__ ex, OzSym sym) {
     constexpr int TY = 256 / RB, KT = 8 * TY;  // threads a row; k at a time
     __shared__ double tile[RB][KT + 1];
     __shared__ int se[RB];
     const int tx = threadIdx.x % RB, ty = threadIdx.x / RB, r0 = blockIdx.x * RB;
-    const bool in = r0 + tx < rows;
+    const bool sy = oz_sym_on(sym);
+    const int rows = oz_sym_rows(sym, sy, nrows);
+    if (r0 >= rows) return;
+    bool in = r0 + tx < rows;
+    long long at = (long long)(r0 + tx) * es;
+    if (sy) {
+        int i, j;
+        in = oz_sym_at(sym, r0 + tx, i, j) && in;
+        at = (long long)i * sym.n + j;
+    } else {
+        at += sym.r0;
+    }
     if (threadIdx.x < RB) se[threadIdx.x] = 0;
     __syncthreads();
     int e = 0;
     if (in) {
 #pragma unroll 8
-        for (int k = ty; k < K; k += TY) e = max(e, oz_expo(src[(long long)k * ld + (r0 + tx) * es]));
+        for (int k = ty; k < K; k += TY) e = max(e, oz_expo(src[(long long)k * ld + at]));
     }
     atomicMax(&se[tx], e);
     __syncthreads();
@@ -572,7 +658,7 @@ __global__ void __launch_bounds__(256) k_oz_cols(int rows, int K, const double* 
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
             const int k = k0 + ty + TY * i;
-            tile[tx][ty + TY * i] = in && k < K ? src[(long long)k * ld + (r0 + tx) * es] : 0.0;
+            tile[tx][ty + TY * i] = in && k < K ? src[(long long)k * ld + at] : 0.0;
         }
         __syncthreads();
         if (r0 + rr < rows && k0 + kq < 32 * dst.nks) {
@@ -818,8 +904,9 @@ void oz_splits(long long tiles, int K, int sms, int& splits, int& cps) {
 }
 
 int oz_launch(int rows, int cols, int K, int batch, int adiv, const OzDigits& A, const OzDigits& B, const OzOut& out,
-              int splits, int cps, long long* raw, int* err, cudaStream_t s) {
+              int splits, int cps, long long* raw, int* err, cudaStream_t s, const OzSym& sym = {}) {
     OzArgs a = {};
+    a.sym = sym;
     a.da = A.d; a.db = B.d;
     a.r8a = (int)round_up(rows, 8); a.r8b = (int)round_up(cols, 8);
     a.rows = rows; a.cols = cols; a.K = K; a.batch = batch; a.adiv = adiv;
@@ -873,10 +960,18 @@ int split_crows(long long rows, int K, const double2* src, long long ld, const O
     AFQ_LAUNCHED("k_oz_crows");
     return AFQ_OK;
 }
-int split_cols(int rows, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s, int es = 1) {
-    if (rows <= 32 * 152) k_oz_cols<8><<<(rows + 7) / 8, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex);
-    else k_oz_cols<32><<<(rows + 31) / 32, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex);
+int split_cols(int rows, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s, int es = 1,
+               const OzSym& sym = {}) {
+    if (rows <= 32 * 152) k_oz_cols<8><<<(rows + 7) / 8, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex, sym);
+    else k_oz_cols<32><<<(rows + 31) / 32, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex, sym);
     AFQ_LAUNCHED("k_oz_cols");
+    return AFQ_OK;
+}
+int launch_asym(int n, int G, const double* chol, int* asym, cudaStream_t s) {
+    AFQ_CUDA(cudaMemsetAsync(asym, 0, sizeof(int), s));
+    const int nt = (n + 31) / 32, pairs = nt * (nt + 1) / 2, gy = (152 * 8 + pairs - 1) / pairs;
+    k_oz_asym<<<dim3(pairs, gy < G ? gy : G), 256, 0, s>>>(n, G, chol, asym);
+    AFQ_LAUNCHED("k_oz_asym");
     return AFQ_OK;
 }
 OzDigits take_digits(Arena& a, size_t rows, int K, size_t batch = 1) {
@@ -908,6 +1003,7 @@ struct ZLayout {
     int mc, nc;
     OzDigits A, B;
     long long* raw;
+    int* asym;
 };
 ZLayout z_layout(Arena& a, int M, int N, int K) {
     ZLayout z;
@@ -919,6 +1015,7 @@ ZLayout z_layout(Arena& a, int M, int N, int K) {
     // K splits: at most one tile an SM, at most one split a 256-k chunk
     const size_t nch = (K + 255) / 256, most = (size_t)OZ_TILE_SMS * OZ_ROWS * OZ_TN, all = nch * 2 * z.mc * z.nc;
     z.raw = a.take<long long>((nch > 1 ? (all < most ? all : most) : 0) * 3 / 2);  // 64-bit sums, 32-bit tails
+    z.asym = a.take<int>(64);
     return z;
 }
 
@@ -939,6 +1036,14 @@ ZLayout z_layout(Arena& a, int M, int N, int K) {
 //   energy   n = 8, o = 2, 40 vectors: 12 -> 24 us at 200 walkers, 64 -> 55 at 2048; n = 12, o = 6, 60 vectors: 27 ->
 //            29 at 8, 51 -> 34 at 200; n = 20, o = 5, 100 vectors: 41 -> 30 at 8, 547 -> 185 at 2048.
 bool zgemm_oz_pays(int M, int N, int K) { return M > 0 && N > 0 && K >= 1 && K <= 1 << 17 && M <= 65535 * 64; }
+// Symmetric vectors' half V-build: where the whole one is more than a wave of tiles (a smaller one takes the same time)
+// and the 8 x 8 blocks cover at most four fifths of n^2 (from n = 29 on).  n = 120, 600 vectors, 2048 walkers: 1.46 ->
+// 0.87 ms with the cut; 200, 1000, 1024: 3.34 -> 1.95; 400, 2000, 128: 5.01 -> 3.59 (0.4 of it the vectors' check, which
+// a block makes once and which stops at the first pair that differs).
+static bool vbuild_sym_pays(int W, int n) {
+    const long long n2 = (long long)n * n;
+    return 5LL * oz_sym_total(n) <= 4 * n2 && ((n2 + OZ_ROWS - 1) / OZ_ROWS) * ((2LL * W + OZ_TN - 1) / OZ_TN) > 152;
+}
 bool green_oz_pays(int n, int o) { return n <= 512 && n * o * o >= 24000; }
 bool trotter_oz_pays(int W, int n, int n_terms) { return W <= 65535 && n > 32 && n <= 512 && n_terms >= 1; }
 // W walkers, oc columns each
@@ -967,14 +1072,17 @@ size_t oz_real_bytes(int N, int K) {
     return a.used + 256;
 }
 
-int oz_real_split(int N, int K, const double* B, int64_t ldb, bool b_trans, void* real, cudaStream_t s) {
+static int oz_real_split(int N, int K, const double* B, int64_t ldb, bool b_trans, void* real, cudaStream_t s,
+                         const OzSym& sym = {}) {
     Arena a(real, (size_t)-1);
     const OzDigits D = take_digits(a, N, K);
-    return b_trans ? split_rows(N, N, K, B, ldb, D, s) : split_cols(N, K, B, ldb, D, s);
+    return b_trans ? split_rows(N, N, K, B, ldb, D, s) : split_cols(N, K, B, ldb, D, s, 1, sym);
 }
 
-int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
-                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s, const void* real) {
+// sn > 0: the V-build over sn orbitals, whose symmetric vectors' rows are in OzSym's order (asym: the flag of `real`)
+static int zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
+                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s, const void* real,
+                    int sn, const int* asym) {
     if (M <= 0 || N <= 0) return AFQ_OK;
     int ae = 0;
     if (frexp(alpha, &ae) != 0.5) return fail(AFQ_E_UNSUPPORTED, "digit GEMM: alpha=%g is no power of two", alpha);
@@ -984,6 +1092,9 @@ int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t
         Arena a((void*)real, (size_t)-1);
         z.A = take_digits(a, N, K);
         z.nc = N;
+    } else if (sn) {
+        AFQ_TRY(launch_asym(sn, K, B, z.asym, s));
+        asym = z.asym;
     }
     int sms = 0;
     AFQ_TRY(device_sms(&sms));
@@ -992,17 +1103,23 @@ int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t
         AFQ_TRY(split_crows(mc, K, A + (int64_t)m0 * lda, lda, z.B, s));
         for (int n0 = 0; n0 < N; n0 += z.nc) {
             const int nc = N - n0 < z.nc ? N - n0 : z.nc;
+            const OzSym sym = {sn ? asym : nullptr, sn, n0};  // the chunk's first row
             if (real) {}
             else if (b_trans) AFQ_TRY(split_rows(nc, nc, K, B + (int64_t)n0 * ldb, ldb, z.A, s));
-            else AFQ_TRY(split_cols(nc, K, B + n0, ldb, z.A, s));
-            const OzOut out = {C + (int64_t)m0 * ldc + n0, 0, ldc, 0, 1, 1, ae - 1, nullptr};
+            else AFQ_TRY(split_cols(nc, K, B, ldb, z.A, s, 1, sym));
+            const OzOut out = {C + (int64_t)m0 * ldc, 0, ldc, 0, 1, 1, ae - 1, nullptr};
             const long long tiles = (long long)((nc + OZ_ROWS - 1) / OZ_ROWS) * ((2 * mc + OZ_TN - 1) / OZ_TN);
             int splits, cps;
             oz_splits(tiles, K, sms < OZ_TILE_SMS ? sms : OZ_TILE_SMS, splits, cps);
-            AFQ_TRY(oz_launch(nc, 2 * mc, K, 1, 0, z.A, z.B, out, splits, cps, z.raw, err, s));
+            AFQ_TRY(oz_launch(nc, 2 * mc, K, 1, 0, z.A, z.B, out, splits, cps, z.raw, err, s, sym));
         }
     }
     return AFQ_OK;
+}
+
+int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
+                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s, const void* real) {
+    return zgemm_oz(M, N, K, alpha, A, lda, B, ldb, b_trans, C, ldc, scratch, err, s, real, 0, nullptr);
 }
 
 // ---------------------------------------------------------------- Taylor --
@@ -1234,12 +1351,14 @@ void take_oz_block(Arena& a, const afq_dims* d, OzScratch& oz) {
     const int n2 = d->norb * d->norb, on = d->nocc * d->norb;
     const size_t c = oz_real_bytes(n2, d->nchol), r = d->trial_is_real ? oz_real_bytes(d->nchol, on) : 0;
     oz.chol = c ? a.take<char>(c) : nullptr;
+    oz.asym = c && vbuild_sym_pays(d->n_walkers, d->norb) ? a.take<int>(64) : nullptr;
     oz.rot = r ? a.take<char>(r) : nullptr;
 }
 
 int split_oz_block(const afq_dims* d, const double* chol, const double* rot_chol, const OzScratch& oz, cudaStream_t s) {
     const int n2 = d->norb * d->norb, on = d->nocc * d->norb;
-    if (oz.chol) AFQ_TRY(oz_real_split(n2, d->nchol, chol, n2, false, oz.chol, s));
+    if (oz.asym) AFQ_TRY(launch_asym(d->norb, d->nchol, chol, oz.asym, s));
+    if (oz.chol) AFQ_TRY(oz_real_split(n2, d->nchol, chol, n2, false, oz.chol, s, {oz.asym, d->norb, 0}));
     if (oz.rot) AFQ_TRY(oz_real_split(d->nchol, on, rot_chol, on, true, oz.rot, s));
     return AFQ_OK;
 }
@@ -1251,6 +1370,14 @@ int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64
     if (!b_complex && zgemm_oz_pays(M, N, K))
         return launch_zgemm_oz(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, ldc, oz.p, oz.err, s, real);
     return launch_zgemm(M, N, K, alpha, A, lda, B, ldb, b_complex, b_trans, C, ldc, s);
+}
+
+int launch_vbuild(int W, int n, int G, const double2* xs, const double* chol, double2* V, const OzScratch& oz,
+                  cudaStream_t s) {
+    const int n2 = n * n, sn = (oz.chol ? oz.asym != nullptr : vbuild_sym_pays(W, n)) ? n : 0;
+    if (zgemm_oz_pays(W, n2, G))
+        return zgemm_oz(W, n2, G, 1.0, xs, G, chol, n2, false, V, n2, oz.p, oz.err, s, oz.chol, sn, oz.asym);
+    return launch_zgemm(W, n2, G, 1.0, xs, G, chol, n2, false, false, V, n2, s);
 }
 
 int launch_trotter_auto(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,

@@ -10,6 +10,14 @@ import pytest
 import torch
 
 from ad_afqmc_prototype_gb300 import engine
+from ad_afqmc_prototype_gb300.core.system import system
+from ad_afqmc_prototype_gb300.ham.chol import ham_chol
+from ad_afqmc_prototype_gb300.meas.rhf import make_rhf_meas_ops
+from ad_afqmc_prototype_gb300.prop.afqmc import afqmc_step, init_prop_state
+from ad_afqmc_prototype_gb300.prop.blocks import afqmc_block
+from ad_afqmc_prototype_gb300.prop.chol_afqmc_ops import make_chol_afqmc_ops
+from ad_afqmc_prototype_gb300.prop.types import afqmc_params
+from ad_afqmc_prototype_gb300.trial.rhf import get_rdm1, make_rhf_trial_ops, rhf_trial
 from oracle import afqmc_oracle as O
 
 pytestmark = pytest.mark.gpu
@@ -103,3 +111,51 @@ def test_blocks_sharing_a_v_match_single_ones(n, o, W):
     for p in range(2):
         one = engine.apply_trotter(halves[:, p].contiguous(), x, L, e, pctx.sqrt_dt, 6)
         assert _rel(g[:, p], one.cpu().numpy()) < RTOL
+
+
+# more than a wave of 128 x 64 tiles, n^2 well above its 8 x 8 blocks I <= J: the rule of the half V-build
+@pytest.mark.parametrize("n,o,W", [(29, 4, 705), (40, 9, 400), (65, 10, 161), (130, 7, 33), (200, 16, 20)])
+def test_symmetric_vectors_halve_the_v_build(n, o, W):
+    """Symmetric vectors' V from half its rows is the whole V's, bit for bit: a further vector that is not symmetric,
+    with fields of zero, takes the whole product and adds zeros."""
+    G = 40
+    h1, chol, mo, w, xs = _problem(n, o, G, W)
+    pctx = O.build_prop_ctx(0.0, h1, chol, O.get_rdm1(mo.astype(complex)), 0.005)
+    odd = np.concatenate([chol, 0.01 * chol[:1]])
+    odd[G, n - 1, 0] *= 1.5
+    wd, e = _dev(w, torch.complex128), _dev(pctx.exp_h1_half)
+    half = engine.apply_trotter(wd, _dev(xs, torch.complex128), _dev(chol), e, pctx.sqrt_dt, 6)
+    x0 = np.concatenate([xs, np.zeros((W, 1))], axis=1)
+    whole = engine.apply_trotter(wd, _dev(x0, torch.complex128), _dev(odd), e, pctx.sqrt_dt, 6)
+    assert torch.equal(half, whole)
+    few = slice(0, W, max(1, W // 8))
+    assert _rel(half[few], O.apply_trotter_r(w[few], xs[few], pctx, chol.reshape(G, -1), 6)) < RTOL
+    odd[G, n - 1, 0] *= 100.0
+    x0[:, G] = xs[:, 0]
+    got = engine.apply_trotter(wd, _dev(x0, torch.complex128), _dev(odd), e, pctx.sqrt_dt, 6)
+    assert _rel(got[few], O.apply_trotter_r(w[few], x0[few], pctx, odd.reshape(G + 1, -1), 6)) < RTOL
+
+
+@pytest.mark.parametrize("symmetric", [True, False])
+def test_kept_vector_digits_match_the_step_s(symmetric):
+    """A block cuts the vectors once, in either order of rows: its weights are those of single steps."""
+    n, o, G, W, steps = 65, 10, 40, 161, 2
+    h1, chol, mo, w, xs = _problem(n, o, G, W)
+    if not symmetric:
+        chol[G // 2, 3, 50] *= 1.5
+    h1, chol, mo, w = _dev(h1), _dev(chol), _dev(mo), _dev(mo + 0.05 * (w - mo), torch.complex128)
+    sys_ = system(norb=n, nelec=(o, o), walker_kind="restricted")
+    ham, trial = ham_chol(h0=0.0, h1=h1, chol=chol), rhf_trial(mo)
+    params = afqmc_params(n_walkers=W, n_prop_steps=steps, qr_every=0, precision="fp64")
+    m_ops, p_ops = make_rhf_meas_ops(sys_), make_chol_afqmc_ops(ham, "restricted")
+    kw = dict(params=params, ham_data=ham, trial_data=trial, meas_ops=m_ops, prop_ops=p_ops,
+              prop_ctx=p_ops.build_prop_ctx(get_rdm1(trial), params.dt), meas_ctx=m_ops.build_meas_ctx(ham, trial))
+    st = init_prop_state(sys=sys_, n_walkers=W, seed=1, ham_data=ham, trial_ops_=make_rhf_trial_ops(sys_),
+                         trial_data=trial, meas_ops=m_ops, initial_walkers=w)
+    fields = torch.randn((steps, W, G), generator=torch.Generator("cuda").manual_seed(3), device="cuda",
+                         dtype=torch.float64)
+    _, obs = afqmc_block(st, sys=sys_, fields=fields, zeta=0.5, **kw)
+    for i in range(steps):
+        st = afqmc_step(st, fields=fields[i], **kw)
+    # phases and magnitudes of overlaps through two steps of ~40 products each: 1e-13 a walker, ten times that
+    assert abs(float(obs.scalars["weight"]) / float(st.weights.sum()) - 1.0) < 1e-12
