@@ -10,6 +10,7 @@
 #include <algorithm>
 
 #include "afq_internal.cuh"
+#include "sym_blocks.cuh"
 
 namespace afq {
 
@@ -94,11 +95,29 @@ static LowpDims lowp_dims(const afq_dims* d) {
 // Exchange partials per walker of the mixed energy (one with the fused GEMM).
 static int exch_chunks(const afq_dims* d) { return lowp_dims(d).xf ? 1 : exchange_chunks(d->nchol); }
 
+// the three-section form's Taylor products on the tensor cores, from a split V
+static bool tc_taylor_form(const afq_dims* d, const LowpDims& L) {
+    return d->precision == AFQ_PREC_MIXED_FAST && trotter_tc_supported(d->norb, d->nocc) &&
+           L.ldv == (long long)d->norb * d->norb;
+}
+
 struct LowpBufs {
     __nv_bfloat16* Bv;  // n^2 x Kt_V   right operand [hi lo hi] of chol^T
     __nv_bfloat16* Bf;  // G x Kt_F     right operand of rot_chol_flat
     __nv_bfloat16* Le;  // G o x Kt_E   left operand [hi hi lo] of rot_chol
+    int* asym;          // Bv's rows are in the order of symmetric vectors unless *asym (null: n^2 rows)
 };
+
+// Half a V-build over symmetric vectors, where the mirrored writes are whole 16-byte vectors and the 8 x 8 blocks
+// cover at most four fifths of n^2 (n >= 32; not a function of the walkers, the operand is laid out once).  The split
+// form's blocks cost a second kernel, so its V needs tiles enough that few walkers, one row tile, gain as well.  V-build of
+// 120 orbitals, 600 vectors, 2048 walkers, six sections: 0.58 -> 0.39 ms; 200, 1000, 4096, three sections: 1.79 -> 1.30.
+// Blocks of ten steps, three sections, 120 orbitals: 2.61 -> 2.73 ms at 8 walkers and 9.88 -> 9.83 at 1024 with it; at
+// 160 and 200 orbitals no size was slower.
+static bool lowp_sym(const afq_dims* d) {
+    const int n = d->norb;
+    return n % 4 == 0 && 5 * sym_total(n) <= 4 * n * n && (n >= 160 || !tc_taylor_form(d, lowp_dims(d)));
+}
 
 static LowpBufs layout_lowp(Arena& a, const afq_dims* d) {
     const LowpDims L = lowp_dims(d);
@@ -107,6 +126,7 @@ static LowpBufs layout_lowp(Arena& a, const afq_dims* d) {
     b.Bv = a.take<__nv_bfloat16>(n * n * L.Kt_V);
     b.Bf = a.take<__nv_bfloat16>(G * L.Kt_F);
     b.Le = a.take<__nv_bfloat16>(G * L.Pe * L.Kt_E);
+    b.asym = lowp_sym(d) ? a.take<int>(64) : nullptr;
     (void)o;
     return b;
 }
@@ -126,6 +146,7 @@ struct StepWS {
     float* fbm;         // 2W x G
     __nv_bfloat16* Av;  // 2W x Kt_V
     float* Vm;          // 2Wc x ldv
+    __nv_bfloat16* Vp;  // 2 x 2Wc x sym_total(n): a split V's blocks (tensor-core Taylor, half V-build)
     float* emi;         // n*n
     float2* tsum;       // Wc*n*o: fp32 sum of the Taylor terms of a chunk
     __nv_bfloat16* esplit;  // 2 n*n: E - I as bf16 hi, mid (tensor-core Taylor products)
@@ -176,6 +197,7 @@ static StepWS layout_step(Arena& a, const afq_dims* d, int n_chunks, size_t oz_b
         s.fbm = a.take<float>(2 * W * G);
         s.Av = a.take<__nv_bfloat16>(2 * W * L.Kt_V);
         s.Vm = a.take<float>(2 * Wc * L.ldv);
+        s.Vp = tc_taylor_form(d, L) && lowp_sym(d) ? a.take<__nv_bfloat16>(4 * Wc * sym_total((int)n)) : nullptr;
         s.emi = a.take<float>(n * n);
         s.tsum = a.take<float2>(Wc * n * o);
         s.esplit = a.take<__nv_bfloat16>(2 * n * n);
@@ -367,16 +389,15 @@ static int step_mixed(const afq_problem* pb, const afq_params* p, const afq_stat
                                        L.S_V, L.Kt_V, L.sec, ws.shift_term, ws.fb_term, s)); }
     // three-section form: V-build writes V as bf16 hi/mid pieces and the
     // Taylor products run on the tensor cores
-    const bool tc_taylor = d->precision == AFQ_PREC_MIXED_FAST && trotter_tc_supported(n, o) && L.ldv == (long long)n * n;
-    if (tc_taylor) {
+    if (tc_taylor_form(d, L)) {
         AFQ_TRY(launch_e_minus_i_split(n, pb->exp_h1_half, ws.esplit, ws.esplit + (size_t)n * n, s));
         for (int w0 = 0; w0 < W; w0 += Wc) {
             const int wc = W - w0 < Wc ? W - w0 : Wc;
             __nv_bfloat16* vh = (__nv_bfloat16*)ws.Vm;
             __nv_bfloat16* vmid = vh + (size_t)2 * wc * L.ldv;
             { AFQ_PHASE("vbuild_gemm", s);
-              AFQ_TRY(launch_tc_gemm_tn_drain_split(2 * wc, n * n, L.Kt_V, ws.Av + (size_t)2 * w0 * L.Kt_V, L.Kt_V,
-                                                    lb.Bv, L.Kt_V, vh, vmid, L.ldv, ws.status, s, L.kd)); }
+              AFQ_TRY(launch_tc_vbuild(2 * wc, n, L.Kt_V, ws.Av + (size_t)2 * w0 * L.Kt_V, L.Kt_V, lb.Bv, L.Kt_V,
+                                       lb.asym, nullptr, vh, vmid, ws.Vp, L.ldv, ws.status, s, L.kd)); }
             { AFQ_PHASE("trotter", s);
               AFQ_TRY(launch_trotter_tc(wc, n, o, p->n_exp_terms, pb->sqrt_dt, ws.esplit, ws.esplit + (size_t)n * n, vh,
                                         vmid, walk + (size_t)w0 * n * o, walk + (size_t)w0 * n * o, ws.status, s)); }
@@ -386,8 +407,8 @@ static int step_mixed(const afq_problem* pb, const afq_params* p, const afq_stat
     for (int w0 = 0; w0 < W; w0 += Wc) {
         const int wc = W - w0 < Wc ? W - w0 : Wc;
         { AFQ_PHASE("vbuild_gemm", s);
-          AFQ_TRY(launch_tc_gemm_tn_drain(2 * wc, n * n, L.Kt_V, ws.Av + (size_t)2 * w0 * L.Kt_V, L.Kt_V, lb.Bv, L.Kt_V,
-                                    ws.Vm, L.ldv, ws.status, s)); }
+          AFQ_TRY(launch_tc_vbuild(2 * wc, n, L.Kt_V, ws.Av + (size_t)2 * w0 * L.Kt_V, L.Kt_V, lb.Bv, L.Kt_V, lb.asym,
+                                   ws.Vm, nullptr, nullptr, nullptr, L.ldv, ws.status, s)); }
         { AFQ_PHASE("trotter", s);
           AFQ_TRY(launch_trotter_mixed(wc, n, o, p->n_exp_terms, pb->sqrt_dt, ws.emi, ws.Vm, L.ldv,
                                        walk + (size_t)w0 * n * o, walk + (size_t)w0 * n * o, ws.tsum, s)); }
@@ -687,7 +708,8 @@ int afq_prepare_lowp(const afq_dims* d, const double* chol, const double* rot_ch
     const long long n = d->norb, o = d->nocc, G = d->nchol;
     cudaStream_t s = as_stream(stream);
     // chol^T: row j = (i, k) of L_g[i, k] over g   (right operand of the V-build)
-    AFQ_TRY(launch_split_rows(n * n, (int)G, L.S_V, L.Kt_V, chol, 1, n * n, b.Bv, 0, L.sec, s));
+    if (b.asym) AFQ_TRY(launch_asym((int)n, (int)G, chol, b.asym, s));
+    AFQ_TRY(launch_split_rows(n * n, (int)G, L.S_V, L.Kt_V, chol, 1, n * n, b.Bv, 0, L.sec, s, 0, 0, b.asym, (int)n));
     // rot_chol_flat: row g over (p, j)              (right operand of the force bias)
     AFQ_TRY(launch_split_rows(G, (int)(o * n), L.S_F, L.Kt_F, rot_chol, o * n, 1, b.Bf, 0, L.sec, s));
     // rot_chol rows (g, p) over j                   (left operand of the energy);

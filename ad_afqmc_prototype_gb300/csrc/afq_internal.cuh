@@ -348,6 +348,8 @@ int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, c
 int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B, int64_t ldb,
                       bool b_complex, bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s,
                       const void* real = nullptr);
+// *asym = the G matrices n x n are not all symmetric, bit for bit (sym_blocks.cuh)
+int launch_asym(int n, int G, const double* chol, int* asym, cudaStream_t s);
 // V (W x n^2) = xs (W x G) . chol (G x n^2), half of it where chol is symmetric and that pays
 int launch_vbuild(int W, int n, int G, const double2* xs, const double* chol, double2* V, const OzScratch& oz,
                   cudaStream_t s);
@@ -416,10 +418,12 @@ int launch_tc_gemm_tn(int M, int N, int K, const void* A, long long lda, const v
 // (round-to-nearest) instead of in the tensor cores' truncating accumulator.
 int launch_tc_gemm_tn_drain(int M, int N, int K, const void* A, long long lda, const void* B, long long ldb, float* C,
                             long long ldc, int* err, cudaStream_t s, int kd = 1);
-// Same product, written as the two-piece bf16 split (hi, mid) of each sum.
-int launch_tc_gemm_tn_drain_split(int M, int N, int K, const void* A, long long lda, const void* B, long long ldb,
-                                  __nv_bfloat16* Ch, __nv_bfloat16* Cm, long long ldc, int* err, cudaStream_t s,
-                                  int kd = 1);
+// The V-build: N = n^2, C in fp32 or, with Ch and Cm, the two-piece bf16 split (hi, mid) of each sum.  With asym (set
+// by launch_asym) B's rows are in the order of symmetric vectors unless *asym; rows of C are then whole vectors, n % 4
+// == 0 (split: 8), and the split form takes scratch P of 2 M sym_total(n).
+int launch_tc_vbuild(int M, int n, int K, const void* A, long long lda, const void* B, long long ldb, const int* asym,
+                     float* C, __nv_bfloat16* Ch, __nv_bfloat16* Cm, __nv_bfloat16* P, long long ldc, int* err,
+                     cudaStream_t s, int kd = 1);
 
 // the energy's per-chunk partials (sum c^2, sum exchange) without the finish
 int energy_partial_chunks(int o, int G);
@@ -432,7 +436,8 @@ int launch_energy_finish(int W, int n, int o, int nchunk, double h0, const doubl
 
 // k_mixed.cu
 int launch_split_rows(long long rows, int K, int S, int Kt, const double* src, long long rs, long long ks,
-                      __nv_bfloat16* dst, int left, int sec, cudaStream_t s, int grp = 0, int grp_pad = 0);
+                      __nv_bfloat16* dst, int left, int sec, cudaStream_t s, int grp = 0, int grp_pad = 0,
+                      const int* asym = nullptr, int sn = 0);
 int launch_e_minus_i(int n, const double* E, float* out, cudaStream_t s);
 int launch_field_shift_mixed(int W, int G, int Wc, double sqrt_dt, const double* x, const float* fbm, long long ldf,
                              const double2* mf, __nv_bfloat16* av, int S, int Kt, int sec, double2* shift_term,

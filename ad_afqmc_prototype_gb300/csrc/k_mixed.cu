@@ -10,6 +10,7 @@
 // double-float (fp32 pairs) on the fp32 pipe; the determinant's LU, the
 // phaseless cut, the weights and every energy accumulator stay binary64.
 #include "afq_internal.cuh"
+#include "sym_blocks.cuh"
 
 namespace afq {
 
@@ -18,9 +19,13 @@ namespace afq {
 // entries [3S, Kt) and [K, S) of each section are zero.
 // src(r, k) = src[r * rs + k * ks].  With grp > 0 source row r goes to dst
 // row (r / grp) grp_pad + r % grp (groups padded to grp_pad rows; the pad
-// rows are not written).
-__global__ void k_split_rows(long long rows, int K, int S, int Kt, const double* __restrict__ src, long long rs,
-                             long long ks, __nv_bfloat16* __restrict__ dst, int left, int sec, int grp, int grp_pad) {
+// rows are not written).  sym: rows in the order of symmetric vectors where
+// the device says so.
+__global__ void k_split_rows(long long nrows, int K, int S, int Kt, const double* __restrict__ src, long long rs,
+                             long long ks, __nv_bfloat16* __restrict__ dst, int left, int sec, int grp, int grp_pad,
+                             SymRows sym) {
+    const bool sy = sym_on(sym);
+    const long long rows = sym.asym ? sym_rows(sym, sy, (int)nrows) : nrows;
     const long long total = rows * (long long)Kt;
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (long long)gridDim.x * blockDim.x) {
@@ -29,7 +34,14 @@ __global__ void k_split_rows(long long rows, int K, int S, int Kt, const double*
         const long long dr = grp > 0 ? (r / grp) * grp_pad + r % grp : r;
         __nv_bfloat16* row = dst + dr * Kt;
         if (kk < S) {
-            const double x = kk < K ? src[r * rs + (long long)kk * ks] : 0.0;
+            long long at = r;
+            bool in = kk < K;
+            if (sy) {
+                int i, j;
+                in = sym_at(sym, (int)r, i, j) && in;
+                at = (long long)i * sym.n + j;
+            }
+            const double x = in ? src[at * rs + (long long)kk * ks] : 0.0;
             split_store(row, S, kk, x, left != 0, sec);
         } else if (kk >= sec * S) {
             row[kk] = __double2bfloat16(0.0);
@@ -38,11 +50,12 @@ __global__ void k_split_rows(long long rows, int K, int S, int Kt, const double*
 }
 
 int launch_split_rows(long long rows, int K, int S, int Kt, const double* src, long long rs, long long ks,
-                      __nv_bfloat16* dst, int left, int sec, cudaStream_t s, int grp, int grp_pad) {
+                      __nv_bfloat16* dst, int left, int sec, cudaStream_t s, int grp, int grp_pad, const int* asym,
+                      int sn) {
     const long long total = rows * (long long)Kt;
     long long blocks = (total + 255) / 256;
     if (blocks > 152 * 64) blocks = 152 * 64;
-    k_split_rows<<<(unsigned)blocks, 256, 0, s>>>(rows, K, S, Kt, src, rs, ks, dst, left, sec, grp, grp_pad);
+    k_split_rows<<<(unsigned)blocks, 256, 0, s>>>(rows, K, S, Kt, src, rs, ks, dst, left, sec, grp, grp_pad, {asym, sn, 0});
     AFQ_LAUNCHED("k_split_rows");
     return AFQ_OK;
 }

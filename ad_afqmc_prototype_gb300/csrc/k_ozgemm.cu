@@ -43,6 +43,7 @@
 // operands' shared-memory reads), as issued from resident operands.
 #include "afq_internal.cuh"
 #include "oz_digits.cuh"
+#include "sym_blocks.cuh"
 #include "tc_common.cuh"
 
 namespace afq {
@@ -83,35 +84,6 @@ __device__ __forceinline__ uint64_t desc_k64(uint32_t saddr) {
     return d;
 }
 
-// Symmetric Cholesky vectors: V-build rows (i, j) and (j, i) are the same
-// sums, so only the 8 x 8 blocks (I <= J) of the n x n rows are cut and
-// multiplied, in the order J (J + 1) / 2 + I, and a result is written to both
-// places (an entry of its own would have the same bits).  Whether the vectors
-// are symmetric is seen on the device (*asym == 0); otherwise the rows are the
-// n^2 of L as they come.  Blocks of 8 keep the mirrored writes at whole 32-byte
-// sectors and cost n = 61 2304 rows of 3721, n = 200 20800 of 40000.
-struct OzSym {
-    const int* asym;  // null: rows as they come
-    int n, r0;        // orbitals; first row of this chunk (rows as they come: added to their place)
-};
-__host__ __device__ __forceinline__ int oz_sym_total(int n) { return ((n + 7) / 8) * ((n + 7) / 8 + 1) * 32; }
-__device__ __forceinline__ bool oz_sym_on(const OzSym& y) { return y.asym && *y.asym == 0; }
-// rows of the chunk, of `rows` as they come
-__device__ __forceinline__ int oz_sym_rows(const OzSym& y, bool on, int rows) {
-    return on ? max(0, min(rows, oz_sym_total(y.n) - y.r0)) : rows;
-}
-// entry (i, j) of row r; false: a block's part past n
-__device__ __forceinline__ bool oz_sym_at(const OzSym& y, int r, int& i, int& j) {
-    r += y.r0;
-    const int b = r >> 6;
-    int J = (int)((sqrtf(8.f * b + 1.f) - 1.f) * 0.5f);
-    if (J * (J + 1) / 2 > b) --J;
-    if ((J + 1) * (J + 2) / 2 <= b) ++J;
-    i = 8 * (b - J * (J + 1) / 2) + ((r >> 3) & 7);
-    j = 8 * J + (r & 7);
-    return i < y.n && j < y.n;
-}
-
 // Where output (row r, complex column m) of batch b goes: C[b bs + (m / md)
 // ms1 + (m % md) ms0 + r rs], times 2^aexp, plus the same entry of add.
 struct OzOut {
@@ -133,7 +105,7 @@ struct OzArgs {
     float* rawt;
     int* err;
     OzOut out;
-    OzSym sym;
+    SymRows sym;
 };
 
 __device__ __forceinline__ void oz_tile(const OzArgs& a, int t, int mt, int nt, int& z, int& mb, int& nb) {
@@ -264,8 +236,8 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
     uint32_t* tmem_slot = (uint32_t*)(smem_raw + (bars + 8 * OZB_N - smem_u32(smem_raw)));
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const bool sym = oz_sym_on(a.sym);
-    const int rows = oz_sym_rows(a.sym, sym, a.rows);
+    const bool sym = sym_on(a.sym);
+    const int rows = sym_rows(a.sym, sym, a.rows);
     const int mt = (rows + OZ_ROWS - 1) / OZ_ROWS, nt = (a.cols + OZ_TN - 1) / OZ_TN;
     const int ntiles = mt * nt * a.batch * a.splits, kst = (a.K + OZ_BK - 1) / OZ_BK;
     if ((int)blockIdx.x >= ntiles) return;  // the symmetric rows take fewer CTAs
@@ -430,7 +402,7 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
             long long at = (long long)b * a.out.bs + (long long)row * a.out.rs, mirror = 0;
             if (sym) {
                 int i, j;
-                if (!oz_sym_at(a.sym, row, i, j)) continue;
+                if (!sym_at(a.sym, row, i, j)) continue;
                 at = (long long)i * a.sym.n + j;
                 if (i >> 3 != j >> 3) mirror = (long long)j * a.sym.n + i - at;
             } else {
@@ -465,14 +437,14 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
 
 // The K splits' sums added (the integers exactly, the tails in order) and converted.
 __global__ void k_oz_finish(const OzArgs a) {
-    const bool sym = oz_sym_on(a.sym);
-    const int rows = oz_sym_rows(a.sym, sym, a.rows);
+    const bool sym = sym_on(a.sym);
+    const int rows = sym_rows(a.sym, sym, a.rows);
     const long long total = (long long)rows * (a.cols >> 1);
     for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < total;
          e += (long long)gridDim.x * blockDim.x) {
         const int m = (int)(e / rows), row = (int)(e - (long long)m * rows);
         int i = 0, j = 0;
-        if (sym && !oz_sym_at(a.sym, row, i, j)) continue;
+        if (sym && !sym_at(a.sym, row, i, j)) continue;
         long long re = 0, im = 0;
         float tr = 0.f, ti = 0.f;
         for (int z = 0; z < a.splits; ++z) {
@@ -625,19 +597,19 @@ __global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const d
 // would leave SMs idle), transposed through shared memory.
 template <int RB>
 __global__ void __launch_bounds__(256) k_oz_cols(int nrows, int K, const double* __restrict__ src, long long ld, int es,
-                                                 OzDst dst, int* __restrict__ ex, OzSym sym) {
+                                                 OzDst dst, int* __restrict__ ex, SymRows sym) {
     constexpr int TY = 256 / RB, KT = 8 * TY;  // threads a row; k at a time
     __shared__ double tile[RB][KT + 1];
     __shared__ int se[RB];
     const int tx = threadIdx.x % RB, ty = threadIdx.x / RB, r0 = blockIdx.x * RB;
-    const bool sy = oz_sym_on(sym);
-    const int rows = oz_sym_rows(sym, sy, nrows);
+    const bool sy = sym_on(sym);
+    const int rows = sym_rows(sym, sy, nrows);
     if (r0 >= rows) return;
     bool in = r0 + tx < rows;
     long long at = (long long)(r0 + tx) * es;
     if (sy) {
         int i, j;
-        in = oz_sym_at(sym, r0 + tx, i, j) && in;
+        in = sym_at(sym, r0 + tx, i, j) && in;
         at = (long long)i * sym.n + j;
     } else {
         at += sym.r0;
@@ -904,7 +876,7 @@ void oz_splits(long long tiles, int K, int sms, int& splits, int& cps) {
 }
 
 int oz_launch(int rows, int cols, int K, int batch, int adiv, const OzDigits& A, const OzDigits& B, const OzOut& out,
-              int splits, int cps, long long* raw, int* err, cudaStream_t s, const OzSym& sym = {}) {
+              int splits, int cps, long long* raw, int* err, cudaStream_t s, const SymRows& sym = {}) {
     OzArgs a = {};
     a.sym = sym;
     a.da = A.d; a.db = B.d;
@@ -961,17 +933,10 @@ int split_crows(long long rows, int K, const double2* src, long long ld, const O
     return AFQ_OK;
 }
 int split_cols(int rows, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s, int es = 1,
-               const OzSym& sym = {}) {
+               const SymRows& sym = {}) {
     if (rows <= 32 * 152) k_oz_cols<8><<<(rows + 7) / 8, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex, sym);
     else k_oz_cols<32><<<(rows + 31) / 32, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex, sym);
     AFQ_LAUNCHED("k_oz_cols");
-    return AFQ_OK;
-}
-int launch_asym(int n, int G, const double* chol, int* asym, cudaStream_t s) {
-    AFQ_CUDA(cudaMemsetAsync(asym, 0, sizeof(int), s));
-    const int nt = (n + 31) / 32, pairs = nt * (nt + 1) / 2, gy = (152 * 8 + pairs - 1) / pairs;
-    k_oz_asym<<<dim3(pairs, gy < G ? gy : G), 256, 0, s>>>(n, G, chol, asym);
-    AFQ_LAUNCHED("k_oz_asym");
     return AFQ_OK;
 }
 OzDigits take_digits(Arena& a, size_t rows, int K, size_t batch = 1) {
@@ -1036,13 +1001,21 @@ ZLayout z_layout(Arena& a, int M, int N, int K) {
 //   energy   n = 8, o = 2, 40 vectors: 12 -> 24 us at 200 walkers, 64 -> 55 at 2048; n = 12, o = 6, 60 vectors: 27 ->
 //            29 at 8, 51 -> 34 at 200; n = 20, o = 5, 100 vectors: 41 -> 30 at 8, 547 -> 185 at 2048.
 bool zgemm_oz_pays(int M, int N, int K) { return M > 0 && N > 0 && K >= 1 && K <= 1 << 17 && M <= 65535 * 64; }
+int launch_asym(int n, int G, const double* chol, int* asym, cudaStream_t s) {
+    AFQ_CUDA(cudaMemsetAsync(asym, 0, sizeof(int), s));
+    const int nt = (n + 31) / 32, pairs = nt * (nt + 1) / 2, gy = (152 * 8 + pairs - 1) / pairs;
+    k_oz_asym<<<dim3(pairs, gy < G ? gy : G), 256, 0, s>>>(n, G, chol, asym);
+    AFQ_LAUNCHED("k_oz_asym");
+    return AFQ_OK;
+}
+
 // Symmetric vectors' half V-build: where the whole one is more than a wave of tiles (a smaller one takes the same time)
 // and the 8 x 8 blocks cover at most four fifths of n^2 (from n = 29 on).  n = 120, 600 vectors, 2048 walkers: 1.46 ->
 // 0.87 ms with the cut; 200, 1000, 1024: 3.34 -> 1.95; 400, 2000, 128: 5.01 -> 3.59 (0.4 of it the vectors' check, which
 // a block makes once and which stops at the first pair that differs).
 static bool vbuild_sym_pays(int W, int n) {
     const long long n2 = (long long)n * n;
-    return 5LL * oz_sym_total(n) <= 4 * n2 && ((n2 + OZ_ROWS - 1) / OZ_ROWS) * ((2LL * W + OZ_TN - 1) / OZ_TN) > 152;
+    return 5LL * sym_total(n) <= 4 * n2 && ((n2 + OZ_ROWS - 1) / OZ_ROWS) * ((2LL * W + OZ_TN - 1) / OZ_TN) > 152;
 }
 bool green_oz_pays(int n, int o) { return n <= 512 && n * o * o >= 24000; }
 bool trotter_oz_pays(int W, int n, int n_terms) { return W <= 65535 && n > 32 && n <= 512 && n_terms >= 1; }
@@ -1073,13 +1046,13 @@ size_t oz_real_bytes(int N, int K) {
 }
 
 static int oz_real_split(int N, int K, const double* B, int64_t ldb, bool b_trans, void* real, cudaStream_t s,
-                         const OzSym& sym = {}) {
+                         const SymRows& sym = {}) {
     Arena a(real, (size_t)-1);
     const OzDigits D = take_digits(a, N, K);
     return b_trans ? split_rows(N, N, K, B, ldb, D, s) : split_cols(N, K, B, ldb, D, s, 1, sym);
 }
 
-// sn > 0: the V-build over sn orbitals, whose symmetric vectors' rows are in OzSym's order (asym: the flag of `real`)
+// sn > 0: the V-build over sn orbitals, whose symmetric vectors' rows are in SymRows's order (asym: the flag of `real`)
 static int zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
                     bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s, const void* real,
                     int sn, const int* asym) {
@@ -1103,7 +1076,7 @@ static int zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t
         AFQ_TRY(split_crows(mc, K, A + (int64_t)m0 * lda, lda, z.B, s));
         for (int n0 = 0; n0 < N; n0 += z.nc) {
             const int nc = N - n0 < z.nc ? N - n0 : z.nc;
-            const OzSym sym = {sn ? asym : nullptr, sn, n0};  // the chunk's first row
+            const SymRows sym = {sn ? asym : nullptr, sn, n0};  // the chunk's first row
             if (real) {}
             else if (b_trans) AFQ_TRY(split_rows(nc, nc, K, B + (int64_t)n0 * ldb, ldb, z.A, s));
             else AFQ_TRY(split_cols(nc, K, B, ldb, z.A, s, 1, sym));

@@ -21,6 +21,7 @@
 #include <cudaTypedefs.h>
 
 #include "afq_internal.cuh"
+#include "sym_blocks.cuh"
 #include "tc_common.cuh"
 
 namespace afq {
@@ -271,6 +272,31 @@ __device__ __forceinline__ void halfwarp_transpose16(uint32_t (&v)[16], int lane
     }
 }
 
+// The 8 x 8 block (I, J) of one row's symmetric n x n matrix, entry (r, c) in
+// a[(8 r + c) / 2], and its mirror image.  fp32: n % 4 == 0.
+__device__ __forceinline__ float sym_get(const float2* a, int r, int c) {
+    return (c & 1) ? a[4 * r + (c >> 1)].y : a[4 * r + (c >> 1)].x;
+}
+__device__ __forceinline__ void sym_store(const float2 (&a)[32], int I, int J, int n, float* v) {
+    float* d = v + (size_t)(8 * I) * n + 8 * J;
+    const int ni = n - 8 * I, nj = n - 8 * J;
+#pragma unroll
+    for (int r = 0; r < 8; ++r)
+#pragma unroll
+        for (int c = 0; c < 8; c += 4)
+            if (r < ni && c < nj)
+                *(float4*)(d + (size_t)r * n + c) = make_float4(sym_get(a, r, c), sym_get(a, r, c + 1),
+                                                                sym_get(a, r, c + 2), sym_get(a, r, c + 3));
+    if (I == J) return;
+    d = v + (size_t)(8 * J) * n + 8 * I;
+#pragma unroll
+    for (int c = 0; c < 8; ++c)
+#pragma unroll
+        for (int r = 0; r < 8; r += 4)
+            if (r < ni && c < nj)
+                *(float4*)(d + (size_t)c * n + r) = make_float4(sym_get(a, r, c), sym_get(a, r + 1, c),
+                                                                sym_get(a, r + 2, c), sym_get(a, r + 3, c));
+}
 // MODE 0: fp32 C.  MODE 1 (split): the two-piece bf16 split of each sum to
 // Ch (hi) and Cm (mid = bf16(c - hi)), same row stride ldc.  MODE 2: the
 // exchange contraction of each 32 x 32 block (ExchOut) instead of C.
@@ -296,14 +322,29 @@ __device__ __forceinline__ void drain_tile(int t, int mt, int nt, int order, int
 // N tile; the launcher picks N tiles fastest when A is the large operand and
 // B fits in L2, and groups the M tiles when neither fits (each group's A then
 // stays in L2 beside the output stream, B is read once per group).
-template <int BNT, int MODE, int EWN>
+//
+// SYM: B's rows are in the order of symmetric vectors (sym_blocks.cuh) where
+// the device says so, an epilogue thread's 64 columns are then one 8 x 8 block
+// of V: written to both places in fp32, whose block rows are whole sectors; as
+// they come to P (rows of N entries, the hi and the mid parts M rows apart) in
+// the split form (k_sym_expand).
+template <int BNT, int MODE, int EWN, bool SYM>
 __global__ void __launch_bounds__(Drain<BNT, EWN>::THREADS, 1)
     k_gemm_tn_drain(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                     float* __restrict__ C, __nv_bfloat16* __restrict__ Ch, __nv_bfloat16* __restrict__ Cm, int M,
-                    int N, int K, long long ldc, int kd, int* __restrict__ err, ExchOut xo, int order) {
+                    int N_, int K, long long ldc, int kd, int* __restrict__ err, ExchOut xo, int order, SymRows sy,
+                    __nv_bfloat16* __restrict__ P) {
     using D = Drain<BNT, EWN>;
-    static_assert(MODE != 2 || EWN == 8, "the exchange epilogue's transpose buffers are sized for eight warps");
+    static_assert(!SYM || D::CW == 64, "an epilogue thread writes whole 8 x 8 blocks");
     constexpr bool SPLIT = MODE == 1;
+    const bool sym = SYM && sym_on(sy);
+    const int N = SYM ? sym_rows(sy, sym, N_) : N_;
+    if (SYM && SPLIT && sym) {
+        ldc = N;
+        Ch = P;
+        Cm = P + (size_t)M * N;
+    }
+    static_assert(MODE != 2 || EWN == 8, "the exchange epilogue's transpose buffers are sized for eight warps");
     static_assert(MODE != 2 || BNT % 64 == 0, "the exchange epilogue takes whole 32 x 32 blocks per warp");
     constexpr int STG = D::STG, SLOTS = D::SLOTS, CW = D::CW;
     extern __shared__ uint8_t smem_raw[];
@@ -500,6 +541,16 @@ __global__ void __launch_bounds__(Drain<BNT, EWN>::THREADS, 1)
             }
             const int row = mb * BM + q * 32 + lane;
             const int col0 = nb * BNT + cb;
+            if constexpr (SYM && !SPLIT) {
+                if (sym) {
+                    if (row < M && col0 < N) {
+                        int I, J;
+                        sym_block(col0 >> 6, I, J);
+                        sym_store(acc, I, J, sy.n, C + (long long)row * ldc);
+                    }
+                    continue;
+                }
+            }
             if constexpr (SPLIT && CW == 64) {
                 // the warp's 32 rows x 64 columns of bf16 pairs (hi, mid) in 16-word halves, each
                 // transposed within the half-warps so that one store writes 64 contiguous bytes
@@ -587,6 +638,48 @@ __global__ void __launch_bounds__(Drain<BNT, EWN>::THREADS, 1)
     }
 }
 
+// The symmetric V of one row (walker, part) from its 8 x 8 blocks I <= J, hi
+// (blockIdx.y 0) or mid parts: the blocks are staged in shared memory and V's
+// rows written as they lie, 16 bytes a thread.  Memory-bound (1.5 V's bytes).
+// Writing both places from the GEMM's epilogue instead scatters 16-byte pieces
+// (200 orbitals, 1000 vectors, 4096 walkers: 2.0-2.7 ms against 1.8 for all of
+// V and 1.3 for the half and this, 0.33 of it here).  n % 8 == 0.
+__global__ void __launch_bounds__(256) k_sym_expand(int M, const __nv_bfloat16* __restrict__ P,
+                                                    __nv_bfloat16* __restrict__ Ch, __nv_bfloat16* __restrict__ Cm,
+                                                    long long ldc, SymRows sy) {
+    extern __shared__ uint32_t sew[];  // a block's 32 words, 33 apart: neither access meets a bank twice
+    if (!sym_on(sy)) return;
+    const int total = sym_total(sy.n), nb = sy.n / 8;
+    const uint4* src = (const uint4*)(P + ((size_t)blockIdx.y * M + blockIdx.x) * total);
+    for (int e = threadIdx.x; e < total / 8; e += 256) {
+        const uint4 v = __ldcs(src + e);
+        uint32_t* w = sew + (e >> 3) * 33 + (e & 7) * 4;
+        w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+    }
+    __syncthreads();
+    __nv_bfloat16* dst = (blockIdx.y ? Cm : Ch) + (long long)blockIdx.x * ldc;
+    for (int e = threadIdx.x; e < sy.n / 2 * nb; e += 256) {  // rows i, i + 1 of block (I, J)
+        const int i = e / nb * 2, J = e - i / 2 * nb, I = i >> 3, r = i & 7;
+        uint32_t a[4], b[4];
+        if (I <= J) {
+            const uint32_t* w = sew + (J * (J + 1) / 2 + I) * 33 + r * 4;
+#pragma unroll
+            for (int k = 0; k < 4; ++k) { a[k] = w[k]; b[k] = w[k + 4]; }
+        } else {  // columns r, r + 1 of the block stored as (J, I)
+            const uint32_t* w = sew + (I * (I + 1) / 2 + J) * 33 + (r >> 1);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const uint32_t x = w[8 * k], y = w[8 * k + 4];
+                a[k] = __byte_perm(x, y, 0x5410);
+                b[k] = __byte_perm(x, y, 0x7632);
+            }
+        }
+        uint4* o = (uint4*)(dst + (size_t)i * sy.n + 8 * J);
+        __stcs(o, make_uint4(a[0], a[1], a[2], a[3]));
+        __stcs(o + nb, make_uint4(b[0], b[1], b[2], b[3]));
+    }
+}
+
 }  // namespace tc
 
 static DeviceOnce g_tn_smem;
@@ -612,14 +705,15 @@ int launch_tc_gemm_tn(int M, int N, int K, const void* A, long long lda, const v
 
 // Persistent launch: one CTA per SM (the shared-memory ring admits one), or
 // one per tile when there are fewer tiles.
-template <int BNT, int MODE, int EWN>
+template <int BNT, int MODE, int EWN, bool SYM = false>
 static int launch_drain(int M, int N, int K, const void* A, long long lda, const void* B, long long ldb, float* C,
                         __nv_bfloat16* Ch, __nv_bfloat16* Cm, long long ldc, int kd, int* err, cudaStream_t s,
-                        tc::ExchOut xo = tc::ExchOut{}, int mgroup = 0) {
+                        tc::ExchOut xo = tc::ExchOut{}, int mgroup = 0, SymRows sy = {},
+                        __nv_bfloat16* P = nullptr) {
     using namespace tc;
     static DeviceOnce smem_once;
     constexpr int SMEM = Drain<BNT, EWN>::SMEM + (MODE == 2 ? XT_BYTES : 0);
-    auto kern = k_gemm_tn_drain<BNT, MODE, EWN>;
+    auto kern = k_gemm_tn_drain<BNT, MODE, EWN, SYM>;
     CUtensorMap ma, mb;
     AFQ_TRY(make_map(&ma, A, M, K, lda, BM));
     AFQ_TRY(make_map(&mb, B, N, K, ldb, BNT));
@@ -644,7 +738,7 @@ static int launch_drain(int M, int N, int K, const void* A, long long lda, const
         const int ng = (int)(((long long)mt * tile_a + kAGroup - 1) / kAGroup);
         order = mgroup > 0 ? mgroup : (mt + ng - 1) / ng;
     }
-    kern<<<grid, Drain<BNT, EWN>::THREADS, SMEM, s>>>(ma, mb, C, Ch, Cm, M, N, K, ldc, kd, err, xo, order);
+    kern<<<grid, Drain<BNT, EWN>::THREADS, SMEM, s>>>(ma, mb, C, Ch, Cm, M, N, K, ldc, kd, err, xo, order, sy, P);
     AFQ_LAUNCHED(MODE == 2 ? "k_gemm_tn_drain(exchange)" : "k_gemm_tn_drain");
     return AFQ_OK;
 }
@@ -663,12 +757,24 @@ int launch_tc_gemm_tn_drain(int M, int N, int K, const void* A, long long lda, c
     return launch_drain<256, 0, 16>(M, N, K, A, lda, B, ldb, C, nullptr, nullptr, ldc, kd, err, s);
 }
 
-int launch_tc_gemm_tn_drain_split(int M, int N, int K, const void* A, long long lda, const void* B, long long ldb,
-                                  __nv_bfloat16* Ch, __nv_bfloat16* Cm, long long ldc, int* err, cudaStream_t s,
-                                  int kd) {
-    if (M <= 0 || N <= 0) return AFQ_OK;
+int launch_tc_vbuild(int M, int n, int K, const void* A, long long lda, const void* B, long long ldb, const int* asym,
+                     float* C, __nv_bfloat16* Ch, __nv_bfloat16* Cm, __nv_bfloat16* P, long long ldc, int* err,
+                     cudaStream_t s, int kd) {
+    if (M <= 0 || n <= 0) return AFQ_OK;
     AFQ_TRY(drain_prologue(K, kd));
-    return launch_drain<256, 1, 16>(M, N, K, A, lda, B, ldb, nullptr, Ch, Cm, ldc, kd, err, s);
+    const SymRows sy = {asym, n, 0};
+    if (!Ch) {  // groups of eight M tiles: both places of a block's sectors are written while they are in L2
+        return asym ? launch_drain<256, 0, 16, true>(M, n * n, K, A, lda, B, ldb, C, Ch, Cm, ldc, kd, err, s, {}, 8, sy)
+                    : launch_drain<256, 0, 16>(M, n * n, K, A, lda, B, ldb, C, Ch, Cm, ldc, kd, err, s);
+    }
+    if (!asym) return launch_drain<256, 1, 16>(M, n * n, K, A, lda, B, ldb, C, Ch, Cm, ldc, kd, err, s);
+    AFQ_TRY((launch_drain<256, 1, 16, true>(M, n * n, K, A, lda, B, ldb, C, Ch, Cm, ldc, kd, err, s, {}, 0, sy, P)));
+    static DeviceOnce expand_once;
+    const size_t smem = (size_t)sym_total(n) / 64 * 33 * 4;
+    AFQ_TRY(raise_smem_once(expand_once, tc::k_sym_expand, 227 * 1024));
+    tc::k_sym_expand<<<dim3(M, 2), 256, smem, s>>>(M, P, Ch, Cm, ldc, sy);
+    AFQ_LAUNCHED("k_sym_expand");
+    return AFQ_OK;
 }
 
 int launch_tc_gemm_exchange(int nw, int G, int K, const void* A, long long lda, const void* B, long long ldb,

@@ -136,6 +136,18 @@ def test_symmetric_vectors_halve_the_v_build(n, o, W):
     assert _rel(got[few], O.apply_trotter_r(w[few], x0[few], pctx, odd.reshape(G + 1, -1), 6)) < RTOL
 
 
+def _run_objects(h1, chol, mo, w, **params):
+    n, o = mo.shape
+    sys_ = system(norb=n, nelec=(o, o), walker_kind="restricted")
+    ham, trial, params = ham_chol(h0=0.0, h1=_dev(h1), chol=_dev(chol)), rhf_trial(_dev(mo)), afqmc_params(**params)
+    m_ops, p_ops = make_rhf_meas_ops(sys_), make_chol_afqmc_ops(ham, "restricted")
+    kw = dict(params=params, ham_data=ham, trial_data=trial, meas_ops=m_ops, prop_ops=p_ops,
+              prop_ctx=p_ops.build_prop_ctx(get_rdm1(trial), params.dt), meas_ctx=m_ops.build_meas_ctx(ham, trial))
+    st = init_prop_state(sys=sys_, n_walkers=params.n_walkers, seed=1, ham_data=ham, trial_ops_=make_rhf_trial_ops(sys_),
+                         trial_data=trial, meas_ops=m_ops, initial_walkers=_dev(w, torch.complex128))
+    return st, kw, sys_
+
+
 @pytest.mark.parametrize("symmetric", [True, False])
 def test_kept_vector_digits_match_the_step_s(symmetric):
     """A block cuts the vectors once, in either order of rows: its weights are those of single steps."""
@@ -143,15 +155,8 @@ def test_kept_vector_digits_match_the_step_s(symmetric):
     h1, chol, mo, w, xs = _problem(n, o, G, W)
     if not symmetric:
         chol[G // 2, 3, 50] *= 1.5
-    h1, chol, mo, w = _dev(h1), _dev(chol), _dev(mo), _dev(mo + 0.05 * (w - mo), torch.complex128)
-    sys_ = system(norb=n, nelec=(o, o), walker_kind="restricted")
-    ham, trial = ham_chol(h0=0.0, h1=h1, chol=chol), rhf_trial(mo)
-    params = afqmc_params(n_walkers=W, n_prop_steps=steps, qr_every=0, precision="fp64")
-    m_ops, p_ops = make_rhf_meas_ops(sys_), make_chol_afqmc_ops(ham, "restricted")
-    kw = dict(params=params, ham_data=ham, trial_data=trial, meas_ops=m_ops, prop_ops=p_ops,
-              prop_ctx=p_ops.build_prop_ctx(get_rdm1(trial), params.dt), meas_ctx=m_ops.build_meas_ctx(ham, trial))
-    st = init_prop_state(sys=sys_, n_walkers=W, seed=1, ham_data=ham, trial_ops_=make_rhf_trial_ops(sys_),
-                         trial_data=trial, meas_ops=m_ops, initial_walkers=w)
+    st, kw, sys_ = _run_objects(h1, chol, mo, mo + 0.05 * (w - mo), n_walkers=W, n_prop_steps=steps, qr_every=0,
+                                precision="fp64")
     fields = torch.randn((steps, W, G), generator=torch.Generator("cuda").manual_seed(3), device="cuda",
                          dtype=torch.float64)
     _, obs = afqmc_block(st, sys=sys_, fields=fields, zeta=0.5, **kw)
@@ -159,3 +164,22 @@ def test_kept_vector_digits_match_the_step_s(symmetric):
         st = afqmc_step(st, fields=fields[i], **kw)
     # phases and magnitudes of overlaps through two steps of ~40 products each: 1e-13 a walker, ten times that
     assert abs(float(obs.scalars["weight"]) / float(st.weights.sum()) - 1.0) < 1e-12
+
+
+@pytest.mark.parametrize("precision,n,o,G,W", [
+    ("mixed", 36, 5, 40, 70), ("mixed", 40, 7, 33, 3), ("mixed", 132, 9, 40, 65), ("mixed_fast", 132, 9, 40, 7), ("mixed_fast", 160, 12, 40, 70),
+    ("mixed_fast", 200, 30, 50, 129), ("mixed_fast", 264, 8, 40, 33)])
+def test_mixed_symmetric_vectors_halve_the_v_build(precision, n, o, G, W):
+    """One zero of a vector with a minus sign makes it unsymmetric in bits and changes no value: a step through the
+    whole V-build gives the bits of one through half of it."""
+    h1, chol, mo, w, _ = _problem(n, o, G, W)
+    chol[0, n - 1, 2] = chol[0, 2, n - 1] = 0.0
+    out = []
+    for sign in (1.0, -1.0):
+        chol[0, n - 1, 2] = sign * 0.0
+        st, kw, _ = _run_objects(h1, chol, mo, mo + 0.05 * (w - mo), n_walkers=W, precision=precision)
+        fields = torch.randn((W, G), generator=torch.Generator("cuda").manual_seed(3), device="cuda", dtype=torch.float64)
+        out.append(afqmc_step(st, fields=fields, **kw))
+    assert torch.equal(out[0].walkers, out[1].walkers)
+    assert torch.equal(out[0].weights, out[1].weights)
+    assert bool(torch.isfinite(out[0].weights).all())
