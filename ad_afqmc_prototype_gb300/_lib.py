@@ -90,6 +90,8 @@ _SIGS = {
     "afq_apply_trotter": (c_int32, [POINTER(afq_dims), c_int32, c_double, c_int32, P, P, P, P, P, P,
                                     c_size_t, P]),
     "afq_orthogonalize": (c_int32, [POINTER(afq_dims), P, P, P, P]),
+    "afq_orthogonalize_workspace": (c_size_t, [POINTER(afq_dims)]),
+    "afq_orthogonalize_ws": (c_int32, [POINTER(afq_dims), P, P, P, P, c_size_t, P]),
     "afq_sr_workspace": (c_size_t, [c_int32]),
     "afq_sr_indices": (c_int32, [c_int32, P, c_double, P, P, P, c_size_t, P]),
     "afq_sr_indices_static": (c_int32, [c_int32, P, c_double, P, P, P]),

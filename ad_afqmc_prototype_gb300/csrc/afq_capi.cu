@@ -253,7 +253,7 @@ struct BlockWS {
 
 static BlockWS layout_block(Arena& a, const afq_dims* d, int n_chunks) {
     BlockWS b = {};
-    b.step = layout_step(a, d, n_chunks, is_mixed(d->precision) ? 0 : energy_oz_bytes(d));
+    b.step = layout_step(a, d, n_chunks, is_mixed(d->precision) ? 0 : std::max(energy_oz_bytes(d), qr_oz_scratch(d->n_walkers, d->norb, d->nocc)));
     const size_t W = d->n_walkers;
     if (!is_mixed(d->precision)) take_oz_block(a, d, b.step.oz);
     b.green = is_mixed(d->precision) ? a.take<double2>(W * d->nocc * d->norb) : b.step.green;
@@ -550,11 +550,13 @@ static int orthonormalize_refresh(const afq_problem* pb, const afq_state* st, cu
     const afq_dims* d = &pb->dims;
     double2* walk = (double2*)st->walkers;
     const bool keep = is_mixed(d->precision) && det_buf && (ws || green_kept);
+    const StepWS* sw = ws ? ws : green_ws;
+    void* qr_scratch = sw ? sw->oz.p : nullptr;
     {
         AFQ_PHASE("qr", s);
         if (is_mixed(d->precision))
             AFQ_TRY(launch_cholqr2(d->n_walkers, d->norb, d->nocc, walk, walk, keep ? det_buf : nullptr, s));
-        else AFQ_TRY(launch_qr(d->n_walkers, d->norb, d->nocc, walk, walk, nullptr, s));
+        else AFQ_TRY(launch_qr_auto(d->n_walkers, d->norb, d->nocc, walk, walk, nullptr, qr_scratch, s));
     }
     if (keep) {
         AFQ_PHASE("overlap_rescale", s);
@@ -825,6 +827,22 @@ int afq_orthogonalize(const afq_dims* d, const double* walkers, double* walkers_
                               (double2*)det_r, as_stream(stream));
     return launch_qr(d->n_walkers, d->norb, d->nocc, (const double2*)walkers, (double2*)walkers_out,
                      (double2*)det_r, as_stream(stream));
+}
+
+size_t afq_orthogonalize_workspace(const afq_dims* d) {
+    if (check_dims(d, false) != AFQ_OK || is_mixed(d->precision)) return 0;
+    return qr_oz_scratch(d->n_walkers, d->norb, d->nocc);
+}
+
+int afq_orthogonalize_ws(const afq_dims* d, const double* walkers, double* walkers_out, double* det_r, void* workspace,
+                         size_t workspace_bytes, void* stream) {
+    const size_t need = afq_orthogonalize_workspace(d);
+    if (need == 0) return afq_orthogonalize(d, walkers, walkers_out, det_r, stream);
+    AFQ_NOTNULL(walkers); AFQ_NOTNULL(walkers_out); AFQ_NOTNULL(workspace);
+    if (workspace_bytes < need) return fail(AFQ_E_WORKSPACE, "workspace of %zu bytes < %zu needed", workspace_bytes, need);
+    if (((uintptr_t)workspace) & 255) return fail(AFQ_E_INVALID_ARGUMENT, "workspace must be 256-byte aligned");
+    return launch_qr_auto(d->n_walkers, d->norb, d->nocc, (const double2*)walkers, (double2*)walkers_out,
+                          (double2*)det_r, workspace, as_stream(stream));
 }
 
 size_t afq_sr_workspace(int32_t n_walkers) {

@@ -361,6 +361,16 @@ int launch_trotter_spins(int W, int n, int o, int n_terms, double sqrt_dt, const
 int launch_energy_partial_auto(int W, int n, int o, int G, const double2* green, const void* rot_chol, int trial_real,
                                double* partial, const OzScratch& oz, cudaStream_t s);
 
+// binary64 QR by digits with the Householder form for the walkers it does not suit; scratch bytes (0: not taken)
+bool qr_oz_pays(int W, int n, int o);
+size_t qr_oz_scratch(int W, int n, int o);
+int launch_qr_oz(int W, int n, int o, const double2* win, double2* wout, double2* det_r, void* scratch, cudaStream_t s);
+int launch_qr_auto(int W, int n, int o, const double2* win, double2* wout, double2* det_r, void* scratch, cudaStream_t s);
+// k_qr_oz.cu : its small kernels
+int launch_qr_factor(int W, int o, const double2* gram, double2* tinv, double* det, int* flag, cudaStream_t s);
+int launch_qr_finish(int W, int n, int o, const double2* q1, const double2* gram, const double* det, const int* err,
+                     double2* out, double2* det_out, int* flag, cudaStream_t s);
+
 // k_green.cu
 int launch_green(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
                  double2* ovlp_out, double2* green_out, cudaStream_t s);
@@ -390,8 +400,9 @@ int launch_weight_update(int W, const afq_params* p, double sqrt_dt, double dt,
 int launch_energy(int W, int n, int o, int G, double h0, const double2* green,
                   const void* rot_chol, int trial_real, const double2* rot_h1,
                   double* partial, double2* energy, const OzScratch& oz, cudaStream_t s);
-int launch_qr(int W, int n, int o, const double2* win, double2* wout, double2* det_r,
-              cudaStream_t s);
+// flag (optional): only the walkers it marks
+int launch_qr(int W, int n, int o, const double2* win, double2* wout, double2* det_r, cudaStream_t s,
+              const int* flag = nullptr);
 int launch_sr_scan(int W, const double* weights, double zeta, double* levels, int32_t* idx,
                    double* cumsum_out, double* avg_out, cudaStream_t s);
 int launch_gather(int W, int64_t row, const int32_t* idx, const double2* src, double2* dst,

@@ -132,6 +132,7 @@ UWS layout_u(Arena& a, const afq_dims* d, int n_chunks, bool block = false) {
                                    zgemm_oz_scratch(2 * d->n_walkers, d->nchol, (int)no),
                                    zgemm_oz_scratch(wc, (int)(n * n), d->nchol),
                                    trotter_oz_scratch(wc, d->norb, d->nocc, 2),
+                                   qr_oz_scratch(2 * d->n_walkers, d->norb, d->nocc),
                                    energy_oz_scratch(2 * d->n_walkers, d->norb, d->nocc, d->nchol)}));
     u.oz.err = u.status;
     u.partial = (double*)a.take<double2>(energy_partial_count(2 * d->n_walkers, d->nocc, d->nchol));
@@ -237,7 +238,7 @@ int step_u(const afq_problem* pb, const afq_params* p, const afq_state* st, cons
 int orthonormalize_u(const afq_problem* pb, const afq_state* st, const UWS& u, double2* green, cudaStream_t s) {
     const afq_dims* d = &pb->dims;
     double2* walk = (double2*)st->walkers;
-    { AFQ_PHASE("qr", s); AFQ_TRY(launch_qr(2 * d->n_walkers, d->norb, d->nocc, walk, walk, nullptr, s)); }
+    { AFQ_PHASE("qr", s); AFQ_TRY(launch_qr_auto(2 * d->n_walkers, d->norb, d->nocc, walk, walk, nullptr, u.oz.p, s)); }
     AFQ_PHASE(green ? "green" : "overlap", s);
     return overlap_u(d, (const double2*)pb->mo_coeff, walk, (double2*)st->overlaps, green, u, s);
 }

@@ -517,11 +517,12 @@ __device__ __forceinline__ int warp_max(int v) {
     return v;
 }
 
-// The largest of the WR warps' values that share a row (WR = 1 or 8: the CTA).
-template <int WR>
+// The largest of the values of the LN threads that share a row (LN <= 32 lanes of a warp, or the CTA's 256).
+template <int LN>
 __device__ __forceinline__ int row_max(int e, int* s_max) {
-    e = warp_max(e);
-    if (WR == 1) return e;
+#pragma unroll
+    for (int o = (LN < 32 ? LN : 32) / 2; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
+    if (LN <= 32) return e;
     __syncthreads();  // the last row's values have been read
     if ((threadIdx.x & 31) == 0) s_max[threadIdx.x >> 5] = e;
     __syncthreads();
@@ -530,25 +531,32 @@ __device__ __forceinline__ int row_max(int e, int* s_max) {
     return e;
 }
 
-// Real rows with K contiguous (row r at src + r ld), a warp a row, or a CTA
-// (WR = 8) where rows are few; `per` rows a batch; one: minus the identity.
-// Every split writes zeros from K up to a multiple of 32.
-template <int WR>
+// Real rows with K contiguous (row r at src + r ld), LN threads a row: a lane
+// cuts eight entries, so a warp takes four rows of up to 64 entries, and a CTA
+// takes one where rows are few and long.  `per` rows a batch; one: minus the
+// identity.  Every split writes zeros from K up to a multiple of 32.
+template <int LN>
 __global__ void __launch_bounds__(256) k_oz_rows(long long rows, int per, int K, const double* __restrict__ src,
                                                  long long ld, int one, OzDst dst, int* __restrict__ ex) {
     __shared__ int s_max[8];
-    const int t = WR == 1 ? threadIdx.x & 31 : threadIdx.x;  // place in the row's threads
-    for (long long r = (long long)blockIdx.x * (8 / WR) + (WR == 1 ? threadIdx.x >> 5 : 0); r < rows;
-         r += (long long)gridDim.x * (8 / WR)) {
-        const double* x = src + r * ld;
+    const int t = threadIdx.x % LN;  // place in the row's threads
+    constexpr int RC = 256 / LN;     // rows a CTA
+    // every thread of a warp stays for the shuffles
+    for (long long r0 = (long long)blockIdx.x * RC; r0 < rows; r0 += (long long)gridDim.x * RC) {
+        const long long r = r0 + threadIdx.x / LN;
+        const bool in = r < rows;
+        const double* x = src + (in ? r : 0) * ld;
         const long long rd = one ? r : -1;  // the diagonal entry to lower by one
         int e = 0;
+        if (in) {
 #pragma unroll 4
-        for (int k = t; k < K; k += 32 * WR) e = max(e, oz_expo(k == rd ? x[k] - 1.0 : x[k]));
-        const int E = oz_scale(row_max<WR>(e, s_max));
+            for (int k = t; k < K; k += LN) e = max(e, oz_expo(k == rd ? x[k] - 1.0 : x[k]));
+        }
+        const int E = oz_scale(row_max<LN>(e, s_max));
+        if (!in) continue;
         if (t == 0) ex[r] = E;
         const long long b = r / per;
-        for (int k = 8 * t; k < 32 * dst.nks; k += 256 * WR) {
+        for (int k = 8 * t; k < 32 * dst.nks; k += 8 * LN) {
             long long y[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) y[i] = oz_fix(k + i < K ? (k + i == rd ? x[k + i] - 1.0 : x[k + i]) : 0.0, E);
@@ -558,27 +566,27 @@ __global__ void __launch_bounds__(256) k_oz_rows(long long rows, int per, int K,
 }
 
 // Complex rows with K contiguous: digit rows 2 r (real parts) and 2 r + 1.
-template <int WR>
+template <int LN>
 __global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const double2* __restrict__ src, long long ld,
                                                   OzDst dst, int* __restrict__ ex) {
     __shared__ int s_max[2][8];
-    const int t = WR == 1 ? threadIdx.x & 31 : threadIdx.x;
-    for (long long r = (long long)blockIdx.x * (8 / WR) + (WR == 1 ? threadIdx.x >> 5 : 0); r < rows;
-         r += (long long)gridDim.x * (8 / WR)) {
+    const int t = threadIdx.x % LN;
+    for (long long r = (long long)blockIdx.x * (256 / LN) + threadIdx.x / LN; r < rows;
+         r += (long long)gridDim.x * (256 / LN)) {
         const double2* x = src + r * ld;
         int e0 = 0, e1 = 0;
 #pragma unroll 4
-        for (int k = t; k < K; k += 32 * WR) {
+        for (int k = t; k < K; k += LN) {
             const double2 v = x[k];
             e0 = max(e0, oz_expo(v.x));
             e1 = max(e1, oz_expo(v.y));
         }
-        const int E0 = oz_scale(row_max<WR>(e0, s_max[0])), E1 = oz_scale(row_max<WR>(e1, s_max[1]));
+        const int E0 = oz_scale(row_max<LN>(e0, s_max[0])), E1 = oz_scale(row_max<LN>(e1, s_max[1]));
         if (t == 0) {
             ex[2 * r] = E0;
             ex[2 * r + 1] = E1;
         }
-        for (int k = 8 * t; k < 32 * dst.nks; k += 256 * WR) {
+        for (int k = 8 * t; k < 32 * dst.nks; k += 8 * LN) {
             long long y[8], w[8];
 #pragma unroll
             for (int i = 0; i < 8; ++i) {
@@ -652,7 +660,8 @@ __global__ void __launch_bounds__(256) k_oz_cols(int nrows, int K, const double*
 //   LAST  T = i s Y; U += T; digits of U as WALK's
 // The right operand of V T (V's rows hold Re, Im interleaved): rows (c, Re)
 // [Tr, -Ti] and (c, Im) [Ti, Tr] over (j, part), a batch a walker.
-enum { OZ_WALK, OZ_PLAIN, OZ_INIT, OZ_TERM, OZ_LAST };
+//   COLS  as WALK, a batch a walker (both operands of its Gram matrix)
+enum { OZ_WALK, OZ_PLAIN, OZ_INIT, OZ_TERM, OZ_LAST, OZ_COLS };
 constexpr int OZ_CB = 8;
 template <int MODE>
 __global__ void __launch_bounds__(256) k_oz_term(int n, int o, int on, long long ws, long long ss, int ncg, double s, const double2* __restrict__ Y,
@@ -685,7 +694,7 @@ __global__ void __launch_bounds__(256) k_oz_term(int n, int o, int on, long long
     atomicMax(&se[2 * c + 1], e1);
     __syncthreads();
     const int cn = min(OZ_CB, o - c0);
-    if (MODE == OZ_WALK || MODE == OZ_LAST) {
+    if (MODE == OZ_WALK || MODE == OZ_LAST || MODE == OZ_COLS) {
         const int nq = 4 * dst.nks;
         for (int it = tid; it < cn * nq; it += 256) {
             const int cc = it / nq, j = (it - cc * nq) * 8;
@@ -697,12 +706,12 @@ __global__ void __launch_bounds__(256) k_oz_term(int n, int o, int on, long long
                 y[i] = oz_fix(t.x, E0);
                 x[i] = oz_fix(t.y, E1);
             }
-            const int row = 2 * (w * o + c0 + cc);
-            oz_store8(dst, 0, row, j, y);
-            oz_store8(dst, 0, row + 1, j, x);
+            const int b = MODE == OZ_COLS ? w : 0, row = 2 * ((w - b) * o + c0 + cc);
+            oz_store8(dst, b, row, j, y);
+            oz_store8(dst, b, row + 1, j, x);
             if (j == 0) {
-                ex[row] = E0;
-                ex[row + 1] = E1;
+                ex[(long long)b * 2 * o + row] = E0;
+                ex[(long long)b * 2 * o + row + 1] = E1;
             }
         }
     } else {
@@ -854,7 +863,7 @@ __global__ void __launch_bounds__(256) k_oz_exchange(int o, int G, int NG, const
 }
 
 constexpr int OZ_XSMEM = 96 * 1024;  // the exchange kernel's F blocks
-DeviceOnce g_oz, g_ozterm[5], g_ozx;
+DeviceOnce g_oz, g_ozterm[6], g_ozx;
 
 int nks_of(int K) { return (K + OZ_BK - 1) / OZ_BK; }
 long long digit_row_bytes(int K) { return 64LL * OZ_S * nks_of(K); }
@@ -920,15 +929,17 @@ bool row_cta(long long rows, int K) { return rows < 16 * 152 && K >= 512; }
 int split_rows(long long rows, int per, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s,
                int one = 0) {
     const OzDst dst = dst_of(D, per, K);
-    if (row_cta(rows, K)) k_oz_rows<8><<<row_blocks(rows, 1), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
-    else k_oz_rows<1><<<row_blocks(rows), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
+    if (row_cta(rows, K)) k_oz_rows<256><<<row_blocks(rows, 1), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
+    else if (K <= 64) k_oz_rows<8><<<row_blocks(rows, 32), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
+    else if (K <= 128) k_oz_rows<16><<<row_blocks(rows, 16), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
+    else k_oz_rows<32><<<row_blocks(rows), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
     AFQ_LAUNCHED("k_oz_rows");
     return AFQ_OK;
 }
 int split_crows(long long rows, int K, const double2* src, long long ld, const OzDigits& D, cudaStream_t s) {
     const OzDst dst = dst_of(D, 2 * rows, K);
-    if (row_cta(rows, K)) k_oz_crows<8><<<row_blocks(rows, 1), 256, 0, s>>>(rows, K, src, ld, dst, D.ex);
-    else k_oz_crows<1><<<row_blocks(rows), 256, 0, s>>>(rows, K, src, ld, dst, D.ex);
+    if (row_cta(rows, K)) k_oz_crows<256><<<row_blocks(rows, 1), 256, 0, s>>>(rows, K, src, ld, dst, D.ex);
+    else k_oz_crows<32><<<row_blocks(rows), 256, 0, s>>>(rows, K, src, ld, dst, D.ex);
     AFQ_LAUNCHED("k_oz_crows");
     return AFQ_OK;
 }
@@ -998,6 +1009,11 @@ ZLayout z_layout(Arena& a, int M, int N, int K) {
 //   green    m and G_half cost 6 n o^2 binary64 FMAs a walker against a 128 x 64 tile each, the factorisation is the
 //            same: n = 60, o = 10 (n o^2 = 6000): 230 -> 401 us at 2048 walkers; 60, 20 (24000): 107 -> 99 at 8, 790 ->
 //            724 at 2048; 120, 20 (48000): 154 -> 105 at 8, 1287 -> 891 at 2048; 200, 30: 467 -> 176 at 8, 4526 -> 1863.
+//   QR       nine launches against one kernel a walker, whose work goes as n o^2 where the digits' goes as n o: 24 x 24
+//            138 -> 114 us at 8 walkers, 2097 -> 1503 at 4096; 64 x 17 113 -> 109 at 64, 1806 -> 1537 at 4096; 61 x 18
+//            125 -> 102 at 8, 2028 -> 1327 at 4096; 120 x 20 224 -> 121, 4379 -> 1757; 200 x 30 535 -> 165, 12.4 -> 3.3
+//            ms; 400 x 50 3178 -> 407 us, 114 -> 13.5 ms.  But 20 x 16 80 -> 93 at 8; 75 x 13 121 -> 139 at 200; 200 x
+//            10 140 -> 193 at 200, 1595 -> 2469 at 4096.
 //   energy   n = 8, o = 2, 40 vectors: 12 -> 24 us at 200 walkers, 64 -> 55 at 2048; n = 12, o = 6, 60 vectors: 27 ->
 //            29 at 8, 51 -> 34 at 200; n = 20, o = 5, 100 vectors: 41 -> 30 at 8, 547 -> 185 at 2048.
 bool zgemm_oz_pays(int M, int N, int K) { return M > 0 && N > 0 && K >= 1 && K <= 1 << 17 && M <= 65535 * 64; }
@@ -1017,6 +1033,7 @@ static bool vbuild_sym_pays(int W, int n) {
     const long long n2 = (long long)n * n;
     return 5LL * sym_total(n) <= 4 * n2 && ((n2 + OZ_ROWS - 1) / OZ_ROWS) * ((2LL * W + OZ_TN - 1) / OZ_TN) > 152;
 }
+bool qr_oz_pays(int W, int n, int o) { return W > 0 && n <= 512 && n >= o && o <= 64 && o >= 17 && n * o * o >= 13000; }
 bool green_oz_pays(int n, int o) { return n <= 512 && n * o * o >= 24000; }
 bool trotter_oz_pays(int W, int n, int n_terms) { return W <= 65535 && n > 32 && n <= 512 && n_terms >= 1; }
 // W walkers, oc columns each
@@ -1124,7 +1141,9 @@ int launch_term(int W, int n, int o, double s, const double2* Y, const double2* 
     const int oc = o * ns, ncg = (oc + OZ_CB - 1) / OZ_CB, smem = OZ_CB * (n + 1) * (int)sizeof(double2);
     if (ns == 1) ws = (long long)n * o;
     AFQ_TRY(raise_smem_once(g_ozterm[MODE], k_oz_term<MODE>, OZ_CB * 513 * (int)sizeof(double2)));
-    const OzDst dst = MODE == OZ_WALK || MODE == OZ_LAST ? dst_of(D, 2LL * W * oc, n) : dst_of(D, 2 * oc, 2 * n);
+    const OzDst dst = MODE == OZ_WALK || MODE == OZ_LAST ? dst_of(D, 2LL * W * oc, n)
+                      : MODE == OZ_COLS                  ? dst_of(D, 2 * oc, n)
+                                                         : dst_of(D, 2 * oc, 2 * n);
     k_oz_term<MODE><<<(unsigned)W * ncg, 256, smem, st>>>(n, oc, o, ws, ss, ncg, s, Y, X, U, dst, D.ex);
     AFQ_LAUNCHED("k_oz_term");
     return AFQ_OK;
@@ -1226,6 +1245,72 @@ int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walke
         AFQ_TRY(oz_launch(n, 2 * o, 2 * o, wc, 1, g.A, g.B, gout, 1, (2 * o + 255) / 256, nullptr, err, s));
     }
     return AFQ_OK;
+}
+
+// -------------------------------------------------------------------- QR --
+// What bounds it is the factorisation's chain of steps and the tiles' fill (2 nocc of 128 rows), so a chunk holds as
+// many walkers as the scratch allows: 4096 walkers of 200 x 30 took 3.7 ms in chunks of 256 MiB, 3.3 in 1 GiB.
+namespace {
+struct QrLayout {
+    int wc;
+    OzDigits X, A, B;  // walker columns, walker rows, right operands R1^-1
+    double2 *q1, *gram, *tinv;
+    double* det;
+    int *flag, *err;
+};
+QrLayout qr_layout(Arena& a, int W, int n, int o) {
+    QrLayout g;
+    const long long per = round_up(2 * o, 8) * (digit_row_bytes(n) + digit_row_bytes(2 * o)) +
+                          round_up(n, 8) * digit_row_bytes(2 * o) + 16LL * n * o + 48LL * o * o;
+    g.wc = even_chunk(W, OZ_CAP / per);
+    g.X = take_digits(a, 2 * o, n, g.wc);
+    g.A = take_digits(a, n, 2 * o, g.wc);
+    g.B = take_digits(a, 2 * o, 2 * o, g.wc);
+    g.q1 = a.take<double2>((size_t)g.wc * n * o);
+    g.gram = a.take<double2>((size_t)g.wc * 2 * o * o);
+    g.tinv = a.take<double2>((size_t)g.wc * o * o);
+    g.det = a.take<double>(g.wc);
+    g.flag = a.take<int>(W);
+    g.err = a.take<int>(64);
+    return g;
+}
+}  // namespace
+
+size_t qr_oz_scratch(int W, int n, int o) {
+    if (!qr_oz_pays(W, n, o)) return 0;
+    Arena a;
+    qr_layout(a, W, n, o);
+    return a.used + 256;
+}
+
+int launch_qr_oz(int W, int n, int o, const double2* win, double2* wout, double2* det_r, void* scratch, cudaStream_t s) {
+    if (W <= 0) return AFQ_OK;
+    Arena ar(scratch, (size_t)-1);
+    const QrLayout g = qr_layout(ar, W, n, o);
+    const size_t no = (size_t)n * o;
+    const OzOut gout = {g.gram, 2LL * o * o, 2 * o, 0, 1, 1, 0, nullptr};      // gram[b][2 a + part]
+    const OzOut qout = {g.q1, (long long)no, 1, 0, o, 1, 0, nullptr};          // q1[i][c]
+    AFQ_CUDA(cudaMemsetAsync(g.err, 0, sizeof(int), s));
+    for (int w0 = 0; w0 < W; w0 += g.wc) {
+        const int wc = W - w0 < g.wc ? W - w0 : g.wc;
+        const double2* w = win + w0 * no;
+        AFQ_TRY(launch_term<OZ_COLS>(wc, n, o, 0.0, w, nullptr, nullptr, g.X, s));
+        AFQ_TRY(oz_launch(2 * o, 2 * o, n, wc, 1, g.X, g.X, gout, 1, (n + 255) / 256, nullptr, g.err, s));
+        AFQ_TRY(launch_qr_factor(wc, o, g.gram, g.tinv, g.det, g.flag + w0, s));
+        AFQ_TRY(split_rows((long long)wc * n, n, 2 * o, (const double*)w, 2 * o, g.A, s));
+        AFQ_TRY(launch_term<OZ_PLAIN>(wc, o, o, 0.0, g.tinv, nullptr, nullptr, g.B, s));
+        AFQ_TRY(oz_launch(n, 2 * o, 2 * o, wc, 1, g.A, g.B, qout, 1, (2 * o + 255) / 256, nullptr, g.err, s));
+        AFQ_TRY(launch_term<OZ_COLS>(wc, n, o, 0.0, g.q1, nullptr, nullptr, g.X, s));
+        AFQ_TRY(oz_launch(2 * o, 2 * o, n, wc, 1, g.X, g.X, gout, 1, (n + 255) / 256, nullptr, g.err, s));
+        AFQ_TRY(launch_qr_finish(wc, n, o, g.q1, g.gram, g.det, g.err, wout + w0 * no, det_r ? det_r + w0 : nullptr,
+                                 g.flag + w0, s));
+    }
+    return launch_qr(W, n, o, win, wout, det_r, s, g.flag);
+}
+
+int launch_qr_auto(int W, int n, int o, const double2* win, double2* wout, double2* det_r, void* scratch, cudaStream_t s) {
+    if (scratch && qr_oz_pays(W, n, o)) return launch_qr_oz(W, n, o, win, wout, det_r, scratch, s);
+    return launch_qr(W, n, o, win, wout, det_r, s);
 }
 
 // ------------------------------------------------- adjoint outer products --

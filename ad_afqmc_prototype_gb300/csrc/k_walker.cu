@@ -535,7 +535,9 @@ __device__ __forceinline__ void qr_apply_all(double2* A, int ld, int rs, int k, 
 // shared memory; otherwise A[j ld + i] in shared memory.
 template <bool GLOBAL>
 __global__ void __launch_bounds__(256) k_qr(int n, int o, const double2* __restrict__ win,
-                                            double2* __restrict__ wout, double2* __restrict__ det_out) {
+                                            double2* __restrict__ wout, double2* __restrict__ det_out,
+                                            const int* __restrict__ flag) {
+    if (flag && !flag[blockIdx.x]) return;
     extern __shared__ double2 Asm[];
     __shared__ double2 s_ph[64];             // alpha / |alpha|, the phase that makes diag(R) >= 0
     __shared__ double s_tau[64], s_nx[64];   // reflector scales and |R_kk|
@@ -549,6 +551,8 @@ __global__ void __launch_bounds__(256) k_qr(int n, int o, const double2* __restr
             int i = e / o, j = e % o;
             A[j * ld + i] = Wp[e];
         }
+    } else if (flag && win != wout) {
+        for (int e = tid; e < n * o; e += blockDim.x) A[e] = win[(size_t)w * n * o + e];
     }
     __syncthreads();
     for (int k = 0; k < o; ++k) {
@@ -608,20 +612,21 @@ __global__ void __launch_bounds__(256) k_qr(int n, int o, const double2* __restr
     }
 }
 
-int launch_qr(int W, int n, int o, const double2* win, double2* wout, double2* det_r, cudaStream_t s) {
+int launch_qr(int W, int n, int o, const double2* win, double2* wout, double2* det_r, cudaStream_t s,
+              const int* flag) {
     if (W <= 0) return AFQ_OK;
     if (o > 64) return fail(AFQ_E_UNSUPPORTED, "qr: nocc=%d > 64", o);
     size_t smem = (size_t)(n | 1) * o * sizeof(double2);
     if (smem <= 200 * 1024) {
         AFQ_TRY(set_smem(k_qr<false>, smem));
-        k_qr<false><<<W, 256, smem, s>>>(n, o, win, wout, det_r);
+        k_qr<false><<<W, 256, smem, s>>>(n, o, win, wout, det_r, flag);
         AFQ_LAUNCHED("k_qr");
         return AFQ_OK;
     }
     // too large for shared memory: in place in wout
-    if (wout != win)
+    if (wout != win && !flag)
         AFQ_CUDA(cudaMemcpyAsync(wout, win, sizeof(double2) * (size_t)W * n * o, cudaMemcpyDeviceToDevice, s));
-    k_qr<true><<<W, 256, 0, s>>>(n, o, wout, wout, det_r);
+    k_qr<true><<<W, 256, 0, s>>>(n, o, flag ? win : wout, wout, det_r, flag);
     AFQ_LAUNCHED("k_qr(global)");
     return AFQ_OK;
 }

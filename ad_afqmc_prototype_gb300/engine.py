@@ -205,8 +205,10 @@ def apply_trotter(walkers, shifted_fields, chol, exp_h1_half, sqrt_dt: float, n_
 
 
 def orthogonalize(walkers, out: Optional[torch.Tensor] = None, precision: int = _lib.AFQ_PREC_FP64):
-    """Returns (Q, det_r) with diag(R) >= 0 (walkers.py:169-203); Householder
-    for the FP64 precision, CholeskyQR2 for the mixed ones."""
+    """Returns (Q, det_r) with diag(R) >= 0 (walkers.py:169-203); for the FP64
+    precision by digit products (scratch of the call's own, so that calls on
+    several streams stay apart; without room for it by Householder),
+    CholeskyQR2 for the mixed ones."""
     w = as_device(walkers, C128)
     if w.dim() != 3:
         raise ValueError("walkers must be (n_walkers, norb, nocc)")
@@ -215,7 +217,15 @@ def orthogonalize(walkers, out: Optional[torch.Tensor] = None, precision: int = 
         out = torch.empty_like(w)
     det = torch.empty((W,), dtype=C128, device=w.device)
     d = make_dims(W, n, o, 1, True, precision)
-    _lib.call("afq_orthogonalize", ctypes.byref(d), ptr(w), ptr(out), ptr(det), stream_ptr())
+    need = int(_lib.load().afq_orthogonalize_workspace(ctypes.byref(d)))
+    try:
+        scratch = torch.empty(need, dtype=torch.uint8, device=w.device) if need else None
+    except torch.cuda.OutOfMemoryError:
+        scratch = None
+    if scratch is None:
+        _lib.call("afq_orthogonalize", ctypes.byref(d), ptr(w), ptr(out), ptr(det), stream_ptr())
+    else:
+        _lib.call("afq_orthogonalize_ws", ctypes.byref(d), ptr(w), ptr(out), ptr(det), ptr(scratch), need, stream_ptr())
     return out, det
 
 

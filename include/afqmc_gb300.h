@@ -215,6 +215,14 @@ int afq_apply_trotter(const afq_dims* d, int32_t n_terms, double sqrt_dt, int32_
  * same Q and R to ~cond(W) * 1e-16; the mixed block uses it). */
 int afq_orthogonalize(const afq_dims* d, const double* walkers, double* walkers_out,
                       double* det_r, void* stream);
+/* The same with scratch (256-byte aligned; afq_orthogonalize_workspace bytes, 0:
+ * none is used): FP64 QR by Gram matrices and triangular inverses formed as
+ * integer-digit products on the tensor cores, Householder for walkers whose
+ * columns are far from orthogonal or of very different norms (and non-finite
+ * ones).  Same Q and R to ~cond(W) * 1e-16; the FP64 blocks use it. */
+size_t afq_orthogonalize_workspace(const afq_dims* d);
+int afq_orthogonalize_ws(const afq_dims* d, const double* walkers, double* walkers_out, double* det_r,
+                         void* workspace, size_t workspace_bytes, void* stream);
 
 /* _sr_indices (walkers.py:233-240): comb indices (int32) and the inclusive
  * prefix sum of |w| (optional, may be NULL).  The prefix sum adds in the
