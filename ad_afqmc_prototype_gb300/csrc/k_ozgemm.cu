@@ -229,6 +229,8 @@ __device__ __forceinline__ void oz_stage(int P, uint32_t smem, uint32_t tmem, in
     oz_commit(smem + OZ_BAR0 + 8 * (OZB_EB + P));
 }
 
+// SYM: the real operand's rows may be those of symmetric vectors (sym_blocks.cuh).
+template <bool SYM>
 __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -236,11 +238,11 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
     uint32_t* tmem_slot = (uint32_t*)(smem_raw + (bars + 8 * OZB_N - smem_u32(smem_raw)));
     volatile int* abort_flag = (volatile int*)(tmem_slot + 1);
     const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-    const bool sym = sym_on(a.sym);
-    const int rows = sym_rows(a.sym, sym, a.rows);
+    const bool sym = SYM && sym_on(a.sym);
+    const int rows = SYM ? sym_rows(a.sym, sym, a.rows) : a.rows;
     const int mt = (rows + OZ_ROWS - 1) / OZ_ROWS, nt = (a.cols + OZ_TN - 1) / OZ_TN;
     const int ntiles = mt * nt * a.batch * a.splits, kst = (a.K + OZ_BK - 1) / OZ_BK;
-    if ((int)blockIdx.x >= ntiles) return;  // the symmetric rows take fewer CTAs
+    if (SYM && (int)blockIdx.x >= ntiles) return;  // the symmetric rows take fewer CTAs
 
     if (threadIdx.x == 0) {
         for (int i = 0; i < OZB_N; ++i)  // one arrival an epilogue warp on a drained slot
@@ -405,7 +407,7 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
                 if (!sym_at(a.sym, row, i, j)) continue;
                 at = (long long)i * a.sym.n + j;
                 if (i >> 3 != j >> 3) mirror = (long long)j * a.sym.n + i - at;
-            } else {
+            } else if (SYM) {
                 at += a.sym.r0;
             }
             const int ex = ea - 14 + a.out.aexp;
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
                     const long long e = at + (long long)mh * a.out.ms1 + (long long)(m - mh * a.out.md) * a.out.ms0;
                     if (a.out.add) v = cadd(v, a.out.add[e]);
                     a.out.C[e] = v;
-                    if (mirror) a.out.C[e + mirror] = v;
+                    if (SYM && mirror) a.out.C[e + mirror] = v;
                 }
             }
         }
@@ -469,25 +471,33 @@ __global__ void k_oz_finish(const OzArgs a) {
 
 // *asym |= the G matrices (n x n) are not all symmetric, bit for bit: 32 x 32 blocks I <= J against their mirrors.
 __global__ void __launch_bounds__(256) k_oz_asym(int n, int G, const double* __restrict__ L, int* asym) {
-    __shared__ unsigned long long tile[32][33];
+    __shared__ unsigned long long tile[2][32][33];
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
     int J = 0, I = blockIdx.x;
     while (I > J) I -= ++J;
+    const int i = 32 * I, j = 32 * J;
     bool bad = false;
-    for (int g = blockIdx.y; g < G; g += gridDim.y) {
-        const unsigned long long* x = (const unsigned long long*)L + (size_t)g * n * n;
+    for (int g = 2 * blockIdx.y; g < G; g += 2 * gridDim.y) {  // two matrices at a time: bytes in flight
+        unsigned long long a[2][4], b[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const unsigned long long* x = (const unsigned long long*)L + (size_t)(g + h) * n * n;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int r = ty + 8 * q;
+                a[h][q] = g + h < G && i + r < n && j + tx < n ? x[(size_t)(i + r) * n + j + tx] : 0ull;
+                b[h][q] = g + h < G && j + r < n && i + tx < n ? x[(size_t)(j + r) * n + i + tx] : 0ull;
+            }
+        }
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tile[h][ty + 8 * q][tx] = a[h][q];
         __syncthreads();
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int i = 32 * I + ty + 8 * q, j = 32 * J + tx;
-            tile[ty + 8 * q][tx] = i < n && j < n ? x[(size_t)i * n + j] : 0ull;
-        }
-        __syncthreads();
+        for (int h = 0; h < 2; ++h)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int j = 32 * J + ty + 8 * q, i = 32 * I + tx;
-            if (i < n && j < n && x[(size_t)j * n + i] != tile[tx][ty + 8 * q]) bad = true;
-        }
+            for (int q = 0; q < 4; ++q) bad |= b[h][q] != tile[h][tx][ty + 8 * q];
         if (__syncthreads_or(bad || *(volatile int*)asym)) break;
     }
     if (bad) *asym = 1;
@@ -863,7 +873,7 @@ __global__ void __launch_bounds__(256) k_oz_exchange(int o, int G, int NG, const
 }
 
 constexpr int OZ_XSMEM = 96 * 1024;  // the exchange kernel's F blocks
-DeviceOnce g_oz, g_ozterm[6], g_ozx;
+DeviceOnce g_oz, g_ozsym, g_ozterm[6], g_ozx;
 
 int nks_of(int K) { return (K + OZ_BK - 1) / OZ_BK; }
 long long digit_row_bytes(int K) { return 64LL * OZ_S * nks_of(K); }
@@ -906,8 +916,13 @@ int oz_launch(int rows, int cols, int K, int batch, int adiv, const OzDigits& A,
     const long long tiles = (long long)mt * nt * batch * splits;
     if (tiles > 0x7fffffffLL) return fail(AFQ_E_UNSUPPORTED, "digit GEMM: %lld tiles", tiles);
     const int grid = tiles < sms ? (int)tiles : sms;
-    AFQ_TRY(raise_smem_once(g_oz, k_ozgemm, OZ_GSMEM));
-    k_ozgemm<<<grid, OZ_GT, OZ_GSMEM, s>>>(a);
+    if (sym.asym) {
+        AFQ_TRY(raise_smem_once(g_ozsym, k_ozgemm<true>, OZ_GSMEM));
+        k_ozgemm<true><<<grid, OZ_GT, OZ_GSMEM, s>>>(a);
+    } else {
+        AFQ_TRY(raise_smem_once(g_oz, k_ozgemm<false>, OZ_GSMEM));
+        k_ozgemm<false><<<grid, OZ_GT, OZ_GSMEM, s>>>(a);
+    }
     AFQ_LAUNCHED("k_ozgemm");
     if (splits > 1) {
         long long blocks = ((long long)rows * (cols >> 1) + 255) / 256;
@@ -1027,7 +1042,7 @@ int launch_asym(int n, int G, const double* chol, int* asym, cudaStream_t s) {
 
 // Symmetric vectors' half V-build: where the whole one is more than a wave of tiles (a smaller one takes the same time)
 // and the 8 x 8 blocks cover at most four fifths of n^2 (from n = 29 on).  n = 120, 600 vectors, 2048 walkers: 1.46 ->
-// 0.87 ms with the cut; 200, 1000, 1024: 3.34 -> 1.95; 400, 2000, 128: 5.01 -> 3.59 (0.4 of it the vectors' check, which
+// 0.87 ms with the cut; 200, 1000, 1024: 3.34 -> 1.95; 400, 2000, 128: 5.01 -> 3.22 (0.4 of it the vectors' check, which
 // a block makes once and which stops at the first pair that differs).
 static bool vbuild_sym_pays(int W, int n) {
     const long long n2 = (long long)n * n;
@@ -1097,11 +1112,11 @@ static int zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t
             if (real) {}
             else if (b_trans) AFQ_TRY(split_rows(nc, nc, K, B + (int64_t)n0 * ldb, ldb, z.A, s));
             else AFQ_TRY(split_cols(nc, K, B, ldb, z.A, s, 1, sym));
-            const OzOut out = {C + (int64_t)m0 * ldc, 0, ldc, 0, 1, 1, ae - 1, nullptr};
+            const OzOut out = {C + (int64_t)m0 * ldc + (sn ? 0 : n0), 0, ldc, 0, 1, 1, ae - 1, nullptr};
             const long long tiles = (long long)((nc + OZ_ROWS - 1) / OZ_ROWS) * ((2 * mc + OZ_TN - 1) / OZ_TN);
             int splits, cps;
             oz_splits(tiles, K, sms < OZ_TILE_SMS ? sms : OZ_TILE_SMS, splits, cps);
-            AFQ_TRY(oz_launch(nc, 2 * mc, K, 1, 0, z.A, z.B, out, splits, cps, z.raw, err, s, sym));
+            AFQ_TRY(oz_launch(nc, 2 * mc, K, 1, 0, z.A, z.B, out, splits, cps, z.raw, err, s, sn ? sym : SymRows{}));
         }
     }
     return AFQ_OK;
