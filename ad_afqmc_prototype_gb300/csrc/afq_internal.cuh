@@ -293,6 +293,10 @@ int launch_sum_spin_blocks(int n, const double2* rdm1, double2* dm, cudaStream_t
 int launch_zgemm(int M, int N, int K, double alpha, const double2* A, int64_t lda,
                  const void* B, int64_t ldb, bool b_complex, bool b_trans, double2* C,
                  int64_t ldc, cudaStream_t s);
+// a real B; pays: where the digits' launches would take longer
+bool zgemm_small_pays(int M, int N, int K);
+int launch_zgemm_small(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
+                       bool b_trans, double2* C, int64_t ldc, cudaStream_t s);
 // Same product with K split over CTA layers when the M x N tiles alone would
 // not fill the GPU; C dense (ldc = N); part: zgemm_splits(M, N, K) x M x N
 // scratch; the layers are added in a fixed order (deterministic).

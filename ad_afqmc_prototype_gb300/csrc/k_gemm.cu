@@ -164,4 +164,107 @@ int launch_zgemm_splitk(int M, int N, int K, double alpha, const double2* A, int
     return AFQ_OK;
 }
 
+// ------------------------------------------------------------ few products --
+// Products of a few million multiplies, real right operand: a CTA of 128
+// threads takes TM x 16 outputs, TM / 8 a thread, so that the binary64 pipe of
+// every SM has the same share; the next 32 k are loaded while these are
+// multiplied (one warp a quarter: nothing else hides the loads).
+template <int TM, bool BT>
+__global__ void __launch_bounds__(128) k_zgemm_small(int M, int N, int K, double alpha, const double2* __restrict__ A,
+                                                     int64_t lda, const double* __restrict__ B, int64_t ldb,
+                                                     double2* __restrict__ C, int64_t ldc) {
+    constexpr int KS = 32, TN = 16, R = TM / 8;
+    __shared__ double2 As[TM][KS + 1];
+    __shared__ double Bs[KS][TN + 1];
+    const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4, m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
+    double2 acc[R], pa[2 * R];
+    double pb[4];
+#pragma unroll
+    for (int r = 0; r < R; ++r) acc[r] = make_double2(0.0, 0.0);
+    auto load = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < 2 * R; ++q) {
+            const int m = m0 + (tid >> 5) + 4 * q, k = k0 + (tid & 31);
+            pa[q] = m < M && k < K ? A[m * lda + k] : make_double2(0.0, 0.0);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int k = k0 + (BT ? tid & 31 : (tid >> 4) + 8 * q), n = n0 + (BT ? (tid >> 5) + 4 * q : tid & 15);
+            pb[q] = k < K && n < N ? (BT ? B[n * ldb + k] : B[k * ldb + n]) : 0.0;
+        }
+    };
+    load(0);
+    for (int k0 = 0; k0 < K; k0 += KS) {
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 2 * R; ++q) As[(tid >> 5) + 4 * q][tid & 31] = pa[q];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (BT) Bs[tid & 31][(tid >> 5) + 4 * q] = pb[q];
+            else Bs[(tid >> 4) + 8 * q][tid & 15] = pb[q];
+        }
+        __syncthreads();
+        if (k0 + KS < K) load(k0 + KS);
+        const int kn = min(KS, K - k0);
+#pragma unroll 4
+        for (int k = 0; k < kn; ++k) {
+            const double b = Bs[k][tx];
+#pragma unroll
+            for (int r = 0; r < R; ++r) {
+                const double2 a = As[ty + 8 * r][k];
+                acc[r].x = fma(a.x, b, acc[r].x);
+                acc[r].y = fma(a.y, b, acc[r].y);
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int m = m0 + ty + 8 * r;
+        if (m < M && n0 + tx < N) C[m * ldc + n0 + tx] = make_double2(alpha * acc[r].x, alpha * acc[r].y);
+    }
+}
+
+// rows a CTA: the least work on the fullest SM, the larger tile at a tie; work: products a thread there and k
+static int small_rows(int M, int N, long long* work) {
+    int tm = 0;
+    for (int t = 32; t >= 8; t /= 2) {
+        const long long ctas = (long long)((M + t - 1) / t) * ((N + 15) / 16), w = (ctas + 151) / 152 * (t / 8);
+        if (tm && w >= *work) continue;
+        tm = t;
+        *work = w;
+    }
+    return tm;
+}
+
+// A product and k costs a thread 128 clocks (two operations of a warp on the binary64 pipe), the digits 20-30 us of
+// launches and a tile's chain whatever the size.  In captured graphs, small -> digits: M x N x K 256 x 144 x 48 9.0 ->
+// 21.9 us, 256 x 48 x 72 7.5 -> 23.4, 8 x 150 x 210 18.5 -> 28.7, 400 x 100 x 100 (work 300) 21.3 -> 26.3; 500 x 500 x
+// 20 (280) 20.8 -> 21.2; 200 x 150 x 210 (420) 34.0 -> 31.1, 8 x 301 x 549 (549) 45.9 -> 28.7.
+bool zgemm_small_pays(int M, int N, int K) {
+    if (M <= 0 || N <= 0) return false;
+    long long work = 0;
+    small_rows(M, N, &work);
+    return work * K <= 300;
+}
+
+int launch_zgemm_small(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
+                       bool b_trans, double2* C, int64_t ldc, cudaStream_t s) {
+    if (M <= 0 || N <= 0) return AFQ_OK;
+    long long work = 0;
+    const int tm = small_rows(M, N, &work);
+    const dim3 grid((N + 15) / 16, (M + tm - 1) / tm);
+    if (grid.y > 65535) return fail(AFQ_E_UNSUPPORTED, "small gemm: M=%d", M);
+#define AFQ_ZS(TM)                                                                                          \
+    do {                                                                                                    \
+        if (b_trans) k_zgemm_small<TM, true><<<grid, 128, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, C, ldc);  \
+        else k_zgemm_small<TM, false><<<grid, 128, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, C, ldc);         \
+    } while (0)
+    if (tm == 32) AFQ_ZS(32);
+    else if (tm == 16) AFQ_ZS(16);
+    else AFQ_ZS(8);
+#undef AFQ_ZS
+    AFQ_LAUNCHED("k_zgemm_small");
+    return AFQ_OK;
+}
+
 }  // namespace afq

@@ -1014,8 +1014,9 @@ ZLayout z_layout(Arena& a, int M, int N, int K) {
 
 // Routes.  The binary64 kernels' own limits stay (a call past them is theirs
 // to refuse).  Measured in captured graphs, binary64 pipe -> digits:
-//   GEMM     wins from the smallest (M x N x K 5 x 7 x 1: 36 -> 21 us with launches; 64 x 144 x 48: 103 -> 28;
-//            1024 x 600 x 2400: 9.6 -> 0.32 ms; 1024 x 1000 x 6000: 24 -> 0.78 ms).
+//   GEMM     wins over k_zgemm from the smallest (M x N x K 5 x 7 x 1: 36 -> 21 us with launches; 64 x 144 x 48: 103 ->
+//            28; 1024 x 600 x 2400: 9.6 -> 0.32 ms; 1024 x 1000 x 6000: 24 -> 0.78 ms); below that k_zgemm_small
+//            (zgemm_small_pays).
 //   Taylor   one kernel a walker (k_trotter_oz.cu) against the binary64 kernel: n = 5, o = 2: 21 -> 24 us at 200
 //            walkers, 117 -> 33 at 2048; n = 8, o = 2: 26 -> 23 at 8; n = 30, o = 7: 66 -> 36 at 8, 120 -> 44 at 200,
 //            817 -> 191 at 2048.  Tiles of all walkers (16 launches at least) against one kernel a walker: n = 45, o =
@@ -1422,7 +1423,9 @@ int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, c
 
 void take_oz_block(Arena& a, const afq_dims* d, OzScratch& oz) {
     const int n2 = d->norb * d->norb, on = d->nocc * d->norb;
-    const size_t c = oz_real_bytes(n2, d->nchol), r = d->trial_is_real ? oz_real_bytes(d->nchol, on) : 0;
+    const int W = d->n_walkers;  // (parts of the walkers take the small product where all of them do)
+    const size_t c = zgemm_small_pays(W, n2, d->nchol) ? 0 : oz_real_bytes(n2, d->nchol);
+    const size_t r = !d->trial_is_real || zgemm_small_pays(W, d->nchol, on) ? 0 : oz_real_bytes(d->nchol, on);
     oz.chol = c ? a.take<char>(c) : nullptr;
     oz.asym = c && vbuild_sym_pays(d->n_walkers, d->norb) ? a.take<int>(64) : nullptr;
     oz.rot = r ? a.take<char>(r) : nullptr;
@@ -1440,6 +1443,8 @@ int split_oz_block(const afq_dims* d, const double* chol, const double* rot_chol
 int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B, int64_t ldb,
                       bool b_complex, bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s,
                       const void* real) {
+    if (!b_complex && zgemm_small_pays(M, N, K))
+        return launch_zgemm_small(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, ldc, s);
     if (!b_complex && zgemm_oz_pays(M, N, K))
         return launch_zgemm_oz(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, ldc, oz.p, oz.err, s, real);
     return launch_zgemm(M, N, K, alpha, A, lda, B, ldb, b_complex, b_trans, C, ldc, s);
@@ -1448,6 +1453,7 @@ int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64
 int launch_vbuild(int W, int n, int G, const double2* xs, const double* chol, double2* V, const OzScratch& oz,
                   cudaStream_t s) {
     const int n2 = n * n, sn = (oz.chol ? oz.asym != nullptr : vbuild_sym_pays(W, n)) ? n : 0;
+    if (zgemm_small_pays(W, n2, G)) return launch_zgemm_small(W, n2, G, 1.0, xs, G, chol, n2, false, V, n2, s);
     if (zgemm_oz_pays(W, n2, G))
         return zgemm_oz(W, n2, G, 1.0, xs, G, chol, n2, false, V, n2, oz.p, oz.err, s, oz.chol, sn, oz.asym);
     return launch_zgemm(W, n2, G, 1.0, xs, G, chol, n2, false, false, V, n2, s);
