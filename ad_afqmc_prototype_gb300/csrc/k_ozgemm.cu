@@ -15,8 +15,8 @@
 // seven signed base-256 digits X = sum_s a_s 2^(-8 s), |a_s| <= 128, stored as
 // bf16 (a_s 2^(-8 s), exact).  A digit array is stored as the MMAs read it: for
 // each 32 k and digit a (rows x 64 bytes) plane with the 64-byte swizzle, so
-// that a tile is one contiguous bulk copy (tensor-map copies of 64-byte rows
-// moved 18-25 bytes a clock an SM) and rows past the end are never copied.  The product of two rows is
+// that a tile is one contiguous bulk copy and rows past the end are never
+// copied.  The product of two rows is
 // sum_{s,t} 2^(-8 (s + t)) sum_k a_s b_t; the pairs s + t <= 7 are kept.  What
 // is dropped is below the rounding to 55 bits (with s + t <= 6 it is eight
 // times that, and the error of a force bias passes the binary64 chain's).
@@ -35,12 +35,17 @@
 // stay in tensor memory and each digit tile is read once for its 34 products.
 // The digit tiles of a 32-k stage arrive as seven units (A_{6-j}, B_j) in the
 // order in which the rows of products A_s B_0 .. A_s B_{6-s}, s = 6 .. 0,
-// need them (s + t = 7 included); an A tile is released after its row, the B tiles after the
-// stage, so that copies run more than two stages ahead (two whole stages in
-// flight, released at once, waited on the copies: 120 clocks an MMA at a
-// V-build of 1000 x 40000 x 1024 walkers).  A row's MMAs keep A_s in the tensor
-// core's collector buffer: 35 clocks an MMA of 128 x 64 x 16 against 48 (the
-// operands' shared-memory reads), as issued from resident operands.
+// need them (s + t = 7 included); an A tile is released after its row, the B
+// tiles after the stage, so that one stage is refilled while the other is
+// multiplied (three stages of B gained nothing).  A row's MMAs keep A_s in the
+// tensor core's collector buffer: 35 clocks an MMA of 128 x 64 x 16 against 48
+// (the operands' shared-memory reads), as issued from resident operands.  The
+// whole MMA warp runs the issue loop and elects a lane in each instruction:
+// descriptors then stay in uniform registers (recomputed ones cost 77 clocks an
+// MMA).  In long products the MMAs bound it (V-build of 200 orbitals, 1000
+// vectors, 1024 walkers: 3.0 ms for 2.4 of MMAs), in short ones the drains and
+// the conversion of six accumulators a tile, in single tiles the chain of both
+// (18-25 us).
 #include "afq_internal.cuh"
 #include "oz_digits.cuh"
 #include "sym_blocks.cuh"

@@ -36,8 +36,7 @@ SPLIT_SECTIONS = {"mixed": 6, "mixed_fast": 3}
 # DRAM bytes (read + write) per launch of a kernel, from one ncu capture of this bench's own command
 # (profiles/launches_block_c4_n200_o30_g1000_w4096_mixed_fast.md), keyed by (workload, precision,
 # walkers, phase); the roofline reports them beside the algorithmic bytes
-MEASURED_TRAFFIC = {("c4_n200_o30_g1000_w4096", "mixed_fast", 4096, "vbuild_gemm"): 564473600 + 1283924736,
-                    ("c4_n200_o30_g1000_w4096", "mixed_fast", 4096, "trotter"): 1741291520 + 368705536,
+MEASURED_TRAFFIC = {("c4_n200_o30_g1000_w4096", "mixed_fast", 4096, "trotter"): 1741291520 + 368705536,
                     ("c4_n200_o30_g1000_w4096", "mixed_fast", 4096, "fb_gemm"): 368115712 + 19635200}
 
 
@@ -128,9 +127,19 @@ def _r64(x):
     return (x + 63) // 64 * 64
 
 
+def vbuild_columns(n, o, precision):
+    """Columns of V the mixed V-build multiplies for symmetric Cholesky vectors (synth.py's are): the 8 x 8 blocks on
+    and above the diagonal, or all n^2 where that form is not taken (lowp_sym in csrc/afq_capi.cu)."""
+    nb = (n + 7) // 8
+    packed = nb * (nb + 1) * 32
+    tc_taylor = precision == "mixed_fast" and n % 8 == 0 and n <= 256 and o <= 32
+    return packed if n % 4 == 0 and 5 * packed <= 4 * n * n and (n >= 160 or not tc_taylor) else n * n
+
+
 def phase_work(n, o, G, W, trial_real=True, precision="fp64", n_terms=6):
     """(work per launch, pipe) of each timed phase.  FP64 form: algorithmic
-    real flops.  Mixed forms: the tensor-core phases count the flops of the
+    real flops, against the FP64 pipe (its products run as integer digits on
+    the tensor cores, so a fraction may pass one).  Mixed forms: the tensor-core phases count the flops of the
     bf16 split operands (2 M N K with K the split row length; the energy GEMM
     without the padding of its exchange-fused layout; the Taylor kernel's
     128 x N x 16 MMAs, N = norb rounded up to 16, two a K step (V's hi and mid
@@ -152,7 +161,7 @@ def phase_work(n, o, G, W, trial_real=True, precision="fp64", n_terms=6):
     }
     if precision in SPLIT_SECTIONS:
         ks = SPLIT_SECTIONS[precision]
-        work["vbuild_gemm"] = (2.0 * (2 * W) * n * n * _r64(ks * G), "tensor")
+        work["vbuild_gemm"] = (2.0 * (2 * W) * vbuild_columns(n, o, precision) * _r64(ks * G), "tensor")
         work["fb_gemm"] = (2.0 * (2 * W) * G * _r64(ks * o * n), "tensor")
         del work["energy"]  # composite phase: e_green_rows + e_gemm + e_exchange
         work["e_gemm"] = (2.0 * (G * o) * (2 * o * W) * _r64(ks * n), "tensor")
@@ -355,11 +364,6 @@ def run_ours(args, rank, world):
         if t is not None:
             roof["traffic"] = t
             roof["traffic_source"] = "ncu dram__bytes_read.sum + dram__bytes_write.sum, one full-size launch"
-            if roof["kernel"] == "vbuild_gemm" and args.precision in SPLIT_SECTIONS:
-                ks = SPLIT_SECTIONS[args.precision]
-                # split x~ and chol^T rows (bf16) read, V written (bf16 hi + mid, or fp32): 8 W n^2 bytes
-                roof["traffic_algorithmic"] = int(2 * (2 * W) * _r64(ks * G) + 2 * n * n * _r64(ks * G)
-                                                  + 8 * W * n * n)
             if roof["kernel"] == "trotter":
                 # V hi + mid of every walker read once (2 planes x n^2 x 2 pieces x 2 bytes), walkers read
                 # and written in binary64 (16 n o bytes each way)
