@@ -145,7 +145,7 @@ int launch_zgemm_splitk(int M, int N, int K, double alpha, const double2* A, int
     if (M <= 0 || N <= 0) return AFQ_OK;
     const int z = zgemm_splits(M, N, K);
     if (z == 1) return launch_zgemm(M, N, K, alpha, A, lda, B, ldb, b_complex, b_trans, C, N, s);
-    const int kc = (K / z + BK - 1) / BK * BK;
+    const int kc = ((K + z - 1) / z + BK - 1) / BK * BK;  // z layers of kc cover K
     dim3 grid((N + BN - 1) / BN, (M + BM - 1) / BM, z);
     if (grid.y > 65535u) return fail(AFQ_E_UNSUPPORTED, "zgemm: M=%d too large", M);
     const int64_t cs = (int64_t)M * N;
