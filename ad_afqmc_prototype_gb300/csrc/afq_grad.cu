@@ -122,7 +122,7 @@ GradWS layout_grad(Arena& a, const afq_dims* d, const afq_params* p, int ck) {
         g.oz.p = a.take<char>(std::max({zgemm_oz_scratch(Wi, Gi, noi), zgemm_oz_scratch(Wi, n2, Gi),
                                         zgemm_oz_scratch(Wi, Gi, n2), zgemm_oz_scratch(Wi, noi, Gi),
                                         zgemm_oz_scratch(wo, Gi * oi, ni), zgemm_oz_scratch(wo, ni, Gi * oi),
-                                        green_oz_scratch(Wi, ni, oi), vbar_oz_scratch(Wi, ni, oi, (int)K)}));
+                                        green_oz_scratch(Wi, ni, oi), taylor_grad_oz_scratch(Wi, ni, oi), vbar_oz_scratch(Wi, ni, oi, (int)K)}));
         g.oz.err = g.status;
     }
     g.wk = a.take<double2>(W * no);
@@ -230,7 +230,7 @@ int step_adjoint(const Ctx& c, const BlockSnap& sn, int op, int st_i, uint64_t c
         AFQ_TRY(launch_vbuild(W, n, G, g.xs, pb->chol, g.V, g.oz, s));
     }
     { AFQ_PHASE("adj_taylor_tape", s);
-      AFQ_TRY(launch_taylor_tape(W, n, o, K, pb->sqrt_dt, pb->exp_h1_half, V, Wpre, g.terms, g.w2, s)); }
+      AFQ_TRY(launch_taylor_tape(W, n, o, K, pb->sqrt_dt, pb->exp_h1_half, V, Wpre, g.terms, g.w2, g.oz, s)); }
     AFQ_PHASE("adj_step_rest", s);
     // weights, population shift and overlap ratio
     AFQ_TRY(launch_weight_adj(W, c.p, pb->sqrt_dt, pb->dt, make_double2(pb->h0_prop_re, pb->h0_prop_im),
@@ -243,7 +243,7 @@ int step_adjoint(const Ctx& c, const BlockSnap& sn, int op, int st_i, uint64_t c
     // W' = E W2: dL/dE += Re W'b W2^H; Taylor reverse; W1 = E W: dL/dE += Re W1b W^H
     { AFQ_PHASE("adj_ebar", s); AFQ_TRY(launch_ebar(W, n, o, g.wk, no, g.w2, no, g.ebar_part, s)); }
     { AFQ_PHASE("adj_taylor", s);
-      AFQ_TRY(launch_taylor_adj(W, n, o, K, pb->sqrt_dt, pb->exp_h1_half, V, g.wk, g.tbar, g.wk, s)); }
+      AFQ_TRY(launch_taylor_adj(W, n, o, K, pb->sqrt_dt, pb->exp_h1_half, V, g.wk, g.tbar, g.wk, g.oz, s)); }
     { AFQ_PHASE("adj_ebar", s);
       AFQ_TRY(launch_ebar(W, n, o, g.tbar, (long long)(K + 1) * no, Wpre, no, g.ebar_part, s)); }
     // V = sum_g x~_g L_g: x~b = Vb . L^T

@@ -326,6 +326,7 @@ int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t
                     const void* real = nullptr);
 // room for digits of the real operand kept over several products (`real` above and below); 0: not kept
 size_t oz_real_bytes(int N, int K);
+bool trotter_oz_pays(int W, int n, int n_terms);
 bool green_oz_pays(int n, int o);
 size_t green_oz_scratch(int W, int n, int o);
 int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walkers, double2* ovlp_out,
@@ -344,6 +345,12 @@ int launch_taylor_tape_small(int W, int n, int o, int K, double sqrt_dt, const d
                              const double2* win, double2* terms, double2* w2, cudaStream_t s);
 int launch_taylor_adj_small(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
                             const double2* wbar_post, double2* tbar, double2* wbar_pre, cudaStream_t s);
+size_t taylor_grad_oz_scratch(int W, int n, int o);
+int launch_taylor_tape_oz(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                          const double2* win, double2* terms, double2* w2, void* scratch, int* err, cudaStream_t s);
+int launch_taylor_adj_oz(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                         const double2* wbar_post, double2* tbar, double2* wbar_pre, void* scratch, int* err,
+                         cudaStream_t s);
 bool energy_oz_pays(int W, int n, int o, int G);
 size_t energy_oz_scratch(int W, int n, int o, int G);
 int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, const double* rot_chol,
@@ -521,9 +528,9 @@ int launch_exchange_finish(int nw, int G, const float* x, const float* c, double
 
 // k_adjoint.cu : reverse-mode kernels of the binary64 step and block
 int launch_taylor_tape(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
-                       const double2* win, double2* terms, double2* w2, cudaStream_t s);
+                       const double2* win, double2* terms, double2* w2, const OzScratch& oz, cudaStream_t s);
 int launch_taylor_adj(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
-                      const double2* wbar_post, double2* tbar, double2* wbar_pre, cudaStream_t s);
+                      const double2* wbar_post, double2* tbar, double2* wbar_pre, const OzScratch& oz, cudaStream_t s);
 // Vb_w = sum_{k = 1 .. K} conj(i sqrt_dt / k) tb_k t_{k-1}^H by digits on the tensor cores (k_ozgemm.cu)
 size_t vbar_oz_scratch(int W, int n, int o, int K);
 int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms,

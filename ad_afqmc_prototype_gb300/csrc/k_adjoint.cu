@@ -72,12 +72,13 @@ __global__ void __launch_bounds__(256) k_taylor_tape(int n, int o, int K, double
 }
 
 int launch_taylor_tape(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
-                       const double2* win, double2* terms, double2* w2, cudaStream_t s) {
+                       const double2* win, double2* terms, double2* w2, const OzScratch& oz, cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
     if (trotter_small_fits(n, o, K)) return launch_taylor_tape_small(W, n, o, K, sqrt_dt, E, V, win, terms, w2, s);
     const size_t smem = 2 * sizeof(double2) * (size_t)n * o;
     if (smem > 227 * 1024)
         return fail(AFQ_E_UNSUPPORTED, "Taylor adjoint: norb %d x nocc %d needs %zu bytes of shared memory", n, o, smem);
+    if (trotter_oz_pays(W, n, K)) return launch_taylor_tape_oz(W, n, o, K, sqrt_dt, E, V, win, terms, w2, oz.p, oz.err, s);
     AFQ_TRY(allow_smem(k_taylor_tape, smem));
     k_taylor_tape<<<W, 256, smem, s>>>(n, o, K, sqrt_dt, E, V, win, terms, w2);
     AFQ_LAUNCHED("k_taylor_tape");
@@ -138,13 +139,15 @@ __global__ void __launch_bounds__(256) k_taylor_adj(int n, int o, int K, double 
 }
 
 int launch_taylor_adj(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
-                      const double2* wbar_post, double2* tbar, double2* wbar_pre, cudaStream_t s) {
+                      const double2* wbar_post, double2* tbar, double2* wbar_pre, const OzScratch& oz, cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
     if (trotter_small_fits(n, o, K))
         return launch_taylor_adj_small(W, n, o, K, sqrt_dt, E, V, wbar_post, tbar, wbar_pre, s);
     const size_t smem = 2 * sizeof(double2) * (size_t)n * o;
     if (smem > 227 * 1024)
         return fail(AFQ_E_UNSUPPORTED, "Taylor adjoint: norb %d x nocc %d needs %zu bytes of shared memory", n, o, smem);
+    if (trotter_oz_pays(W, n, K))
+        return launch_taylor_adj_oz(W, n, o, K, sqrt_dt, E, V, wbar_post, tbar, wbar_pre, oz.p, oz.err, s);
     AFQ_TRY(allow_smem(k_taylor_adj, smem));
     k_taylor_adj<<<W, 256, smem, s>>>(n, o, K, sqrt_dt, E, V, wbar_post, tbar, wbar_pre);
     AFQ_LAUNCHED("k_taylor_adj");

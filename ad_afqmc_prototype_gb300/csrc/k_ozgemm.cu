@@ -676,11 +676,16 @@ __global__ void __launch_bounds__(256) k_oz_cols(int nrows, int K, const double*
 // The right operand of V T (V's rows hold Re, Im interleaved): rows (c, Re)
 // [Tr, -Ti] and (c, Im) [Ti, Tr] over (j, part), a batch a walker.
 //   COLS  as WALK, a batch a walker (both operands of its Gram matrix)
-enum { OZ_WALK, OZ_PLAIN, OZ_INIT, OZ_TERM, OZ_LAST, OZ_COLS };
+//   BACK  T = U - i s Y; digits of T as the right operand of V T
+//   BACKL T = U = U - i s Y; digits of U as WALK's
+// tp (optional): T also there, tw entries a walker apart.
+enum { OZ_WALK, OZ_PLAIN, OZ_INIT, OZ_TERM, OZ_LAST, OZ_COLS, OZ_BACK, OZ_BACKL };
 constexpr int OZ_CB = 8;
 template <int MODE>
 __global__ void __launch_bounds__(256) k_oz_term(int n, int o, int on, long long ws, long long ss, int ncg, double s, const double2* __restrict__ Y,
-                                                 const double2* __restrict__ W, double2* __restrict__ U, OzDst dst, int* __restrict__ ex) {
+                                                 const double2* __restrict__ W, double2* __restrict__ U, OzDst dst, int* __restrict__ ex,
+                                                 double2* __restrict__ tp, long long tw) {
+    constexpr bool SERIES = MODE == OZ_INIT || MODE == OZ_TERM || MODE == OZ_LAST || MODE == OZ_BACK || MODE == OZ_BACKL;
     extern __shared__ double2 sh[];  // OZ_CB x (n + 1)
     __shared__ int se[2 * OZ_CB];
     const int w = blockIdx.x / ncg, c0 = (blockIdx.x - w * ncg) * OZ_CB, tid = threadIdx.x;
@@ -700,6 +705,12 @@ __global__ void __launch_bounds__(256) k_oz_term(int n, int o, int on, long long
                 if (MODE == OZ_LAST) t = u;
             }
             if (MODE == OZ_INIT) U[at] = t = cadd(W[at], t);
+            if (MODE == OZ_BACK || MODE == OZ_BACKL) {
+                const double2 u = U[at];
+                t = make_double2(fma(s, t.y, u.x), fma(-s, t.x, u.y));
+                if (MODE == OZ_BACKL) U[at] = t;
+            }
+            if (SERIES && MODE != OZ_LAST && tp) tp[w * tw + (long long)j * on + c0 + c] = t;
             sh[c * pitch + j] = t;
             e0 = max(e0, oz_expo(t.x));
             e1 = max(e1, oz_expo(t.y));
@@ -709,7 +720,7 @@ __global__ void __launch_bounds__(256) k_oz_term(int n, int o, int on, long long
     atomicMax(&se[2 * c + 1], e1);
     __syncthreads();
     const int cn = min(OZ_CB, o - c0);
-    if (MODE == OZ_WALK || MODE == OZ_LAST || MODE == OZ_COLS) {
+    if (MODE == OZ_WALK || MODE == OZ_LAST || MODE == OZ_COLS || MODE == OZ_BACKL) {
         const int nq = 4 * dst.nks;
         for (int it = tid; it < cn * nq; it += 256) {
             const int cc = it / nq, j = (it - cc * nq) * 8;
@@ -878,7 +889,7 @@ __global__ void __launch_bounds__(256) k_oz_exchange(int o, int G, int NG, const
 }
 
 constexpr int OZ_XSMEM = 96 * 1024;  // the exchange kernel's F blocks
-DeviceOnce g_oz, g_ozsym, g_ozterm[6], g_ozx;
+DeviceOnce g_oz, g_ozsym, g_ozterm[8], g_ozx;
 
 int nks_of(int K) { return (K + OZ_BK - 1) / OZ_BK; }
 long long digit_row_bytes(int K) { return 64LL * OZ_S * nks_of(K); }
@@ -1158,14 +1169,14 @@ TrLayout tr_layout(Arena& a, int W, int n, int o, int ns) {
 // W blocks of o columns, ns of them taken together (block strides ws, ss)
 template <int MODE>
 int launch_term(int W, int n, int o, double s, const double2* Y, const double2* X, double2* U, const OzDigits& D,
-                cudaStream_t st, int ns = 1, long long ws = 0, long long ss = 0) {
+                cudaStream_t st, int ns = 1, long long ws = 0, long long ss = 0, double2* tp = nullptr, long long tw = 0) {
     const int oc = o * ns, ncg = (oc + OZ_CB - 1) / OZ_CB, smem = OZ_CB * (n + 1) * (int)sizeof(double2);
     if (ns == 1) ws = (long long)n * o;
     AFQ_TRY(raise_smem_once(g_ozterm[MODE], k_oz_term<MODE>, OZ_CB * 513 * (int)sizeof(double2)));
-    const OzDst dst = MODE == OZ_WALK || MODE == OZ_LAST ? dst_of(D, 2LL * W * oc, n)
-                      : MODE == OZ_COLS                  ? dst_of(D, 2 * oc, n)
-                                                         : dst_of(D, 2 * oc, 2 * n);
-    k_oz_term<MODE><<<(unsigned)W * ncg, 256, smem, st>>>(n, oc, o, ws, ss, ncg, s, Y, X, U, dst, D.ex);
+    const OzDst dst = MODE == OZ_WALK || MODE == OZ_LAST || MODE == OZ_BACKL ? dst_of(D, 2LL * W * oc, n)
+                      : MODE == OZ_COLS                                      ? dst_of(D, 2 * oc, n)
+                                                                             : dst_of(D, 2 * oc, 2 * n);
+    k_oz_term<MODE><<<(unsigned)W * ncg, 256, smem, st>>>(n, oc, o, ws, ss, ncg, s, Y, X, U, dst, D.ex, tp, tw);
     AFQ_LAUNCHED("k_oz_term");
     return AFQ_OK;
 }
@@ -1211,6 +1222,112 @@ int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const do
         }
         const OzOut wo = {wout + (size_t)w0 * ns * no, 0, (long long)no, 1, o, o, 0, t.U};
         AFQ_TRY(oz_launch(n, 2 * nb * o, n, 1, 0, t.E, t.X, wo, 1, (n + 255) / 256, nullptr, err, s));
+    }
+    return AFQ_OK;
+}
+
+// ------------------------------------------ Taylor series with its terms --
+// The differentiated step's series (k_adjoint.cu has the formulas) where a walker does not fit k_trotter_oz.cu's kernel:
+// launch_trotter_oz's products with every term kept, and its reverse with V^H and E^T.  Five steps forward and back, the
+// two by k_adjoint.cu's binary64 kernels -> by digits: 66 x 8, 8 walkers 10.9 -> 9.9 ms; 80 x 16, 64 walkers 19.0 ->
+// 14.2; 100 x 20, 200 walkers 56.6 -> 33.8; 120 x 32, 100 walkers 67.3 -> 38.9.
+namespace {
+// out[w][i][j] = conj(in[w][j][i]) (double2), or the transpose (double)
+__device__ __forceinline__ double oz_conj(double x) { return x; }
+__device__ __forceinline__ double2 oz_conj(double2 x) { return make_double2(x.x, -x.y); }
+template <typename T>
+__global__ void __launch_bounds__(256) k_oz_adjoint(int n, const T* __restrict__ in, T* __restrict__ out) {
+    __shared__ T tile[32][33];
+    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, i0 = 32 * blockIdx.x, j0 = 32 * blockIdx.y;
+    const size_t b = (size_t)blockIdx.z * n * n;
+    for (int r = ty; r < 32; r += 8)
+        if (j0 + r < n && i0 + tx < n) tile[r][tx] = in[b + (size_t)(j0 + r) * n + i0 + tx];
+    __syncthreads();
+    for (int r = ty; r < 32; r += 8)
+        if (i0 + r < n && j0 + tx < n) out[b + (size_t)(i0 + r) * n + j0 + tx] = oz_conj(tile[tx][r]);
+}
+struct TgLayout {
+    int wc;
+    OzDigits E, V, T, X;
+    double2 *Y, *U, *vh;
+    double* et;
+};
+TgLayout tg_layout(Arena& a, int W, int n, int o) {
+    TgLayout t;
+    const long long n2 = (long long)n * n, per = round_up(n, 8) * digit_row_bytes(2 * n) + 16 * n2;
+    const long long most = OZ_CAP / per;
+    t.wc = even_chunk(W, most < 65535 ? most : 65535);
+    t.E = take_digits(a, n, n);
+    t.V = take_digits(a, n, 2 * n, t.wc);
+    t.T = take_digits(a, 2 * o, 2 * n, t.wc);
+    t.X = take_digits(a, (size_t)t.wc * 2 * o, n);
+    t.Y = a.take<double2>((size_t)t.wc * n * o);
+    t.U = a.take<double2>((size_t)t.wc * n * o);
+    t.vh = a.take<double2>(t.wc * n2);
+    t.et = a.take<double>(n2);
+    return t;
+}
+}  // namespace
+
+size_t taylor_grad_oz_scratch(int W, int n, int o) {
+    Arena a;
+    tg_layout(a, W, n, o);
+    return a.used + 256;
+}
+
+int launch_taylor_tape_oz(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                          const double2* win, double2* terms, double2* w2, void* scratch, int* err, cudaStream_t s) {
+    Arena ar(scratch, (size_t)-1);
+    const TgLayout t = tg_layout(ar, W, n, o);
+    const size_t no = (size_t)n * o;
+    AFQ_TRY(split_rows(n, n, n, E, n, t.E, s, 1));
+    const OzOut xo = {t.Y, 0, (long long)no, 1, o, o, 0, nullptr}, to = {t.Y, (long long)no, 0, 1, o, o, 0, nullptr};
+    for (int w0 = 0; w0 < W; w0 += t.wc) {
+        const int wc = W - w0 < t.wc ? W - w0 : t.wc;
+        const double2* x = win + w0 * no;
+        double2 *u = w2 + w0 * no, *tp = terms + w0 * K * no;
+        AFQ_TRY(split_rows((long long)wc * n, n, 2 * n, (const double*)(V + (size_t)w0 * n * n), 2 * n, t.V, s));
+        AFQ_TRY(launch_term<OZ_WALK>(wc, n, o, 0.0, x, nullptr, nullptr, t.X, s));
+        AFQ_TRY(oz_launch(n, 2 * wc * o, n, 1, 0, t.E, t.X, xo, 1, (n + 255) / 256, nullptr, err, s));
+        AFQ_TRY(launch_term<OZ_INIT>(wc, n, o, 0.0, t.Y, x, u, t.T, s, 1, 0, 0, tp, K * no));
+        for (int k = 1; k <= K; ++k) {
+            AFQ_TRY(oz_launch(n, 2 * o, 2 * n, wc, 1, t.V, t.T, to, 1, (2 * n + 255) / 256, nullptr, err, s));
+            if (k < K) AFQ_TRY(launch_term<OZ_TERM>(wc, n, o, sqrt_dt / k, t.Y, nullptr, u, t.T, s, 1, 0, 0, tp + k * no, K * no));
+            else AFQ_TRY(launch_term<OZ_LAST>(wc, n, o, sqrt_dt / k, t.Y, nullptr, u, t.X, s));
+        }
+    }
+    return AFQ_OK;
+}
+
+int launch_taylor_adj_oz(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                         const double2* wbar_post, double2* tbar, double2* wbar_pre, void* scratch, int* err,
+                         cudaStream_t s) {
+    Arena ar(scratch, (size_t)-1);
+    const TgLayout t = tg_layout(ar, W, n, o);
+    const size_t no = (size_t)n * o;
+    const unsigned nt = (n + 31) / 32;
+    k_oz_adjoint<double><<<dim3(nt, nt, 1), 256, 0, s>>>(n, E, t.et);
+    AFQ_LAUNCHED("k_oz_adjoint");
+    AFQ_TRY(split_rows(n, n, n, t.et, n, t.E, s, 1));
+    const OzOut xo = {t.Y, 0, (long long)no, 1, o, o, 0, nullptr}, to = {t.Y, (long long)no, 0, 1, o, o, 0, nullptr};
+    for (int w0 = 0; w0 < W; w0 += t.wc) {
+        const int wc = W - w0 < t.wc ? W - w0 : t.wc;
+        const double2* x = wbar_post + w0 * no;
+        double2* tp = tbar + w0 * (K + 1) * no;
+        k_oz_adjoint<double2><<<dim3(nt, nt, wc), 256, 0, s>>>(n, V + (size_t)w0 * n * n, t.vh);
+        AFQ_LAUNCHED("k_oz_adjoint");
+        AFQ_TRY(split_rows((long long)wc * n, n, 2 * n, (const double*)t.vh, 2 * n, t.V, s));
+        AFQ_TRY(launch_term<OZ_WALK>(wc, n, o, 0.0, x, nullptr, nullptr, t.X, s));
+        AFQ_TRY(oz_launch(n, 2 * wc * o, n, 1, 0, t.E, t.X, xo, 1, (n + 255) / 256, nullptr, err, s));
+        AFQ_TRY(launch_term<OZ_INIT>(wc, n, o, 0.0, t.Y, x, t.U, t.T, s, 1, 0, 0, tp + K * no, (K + 1) * no));
+        for (int k = K - 1; k >= 0; --k) {
+            AFQ_TRY(oz_launch(n, 2 * o, 2 * n, wc, 1, t.V, t.T, to, 1, (2 * n + 255) / 256, nullptr, err, s));
+            const double c = sqrt_dt / (k + 1);
+            if (k > 0) AFQ_TRY(launch_term<OZ_BACK>(wc, n, o, c, t.Y, nullptr, t.U, t.T, s, 1, 0, 0, tp + k * no, (K + 1) * no));
+            else AFQ_TRY(launch_term<OZ_BACKL>(wc, n, o, c, t.Y, nullptr, t.U, t.X, s, 1, 0, 0, tp, (K + 1) * no));
+        }
+        const OzOut wo = {wbar_pre + w0 * no, 0, (long long)no, 1, o, o, 0, t.U};
+        AFQ_TRY(oz_launch(n, 2 * wc * o, n, 1, 0, t.E, t.X, wo, 1, (n + 255) / 256, nullptr, err, s));
     }
     return AFQ_OK;
 }
