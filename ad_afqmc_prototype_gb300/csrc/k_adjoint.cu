@@ -236,7 +236,9 @@ int launch_sum_partials(int count, int ns, const double* partial, double* out, c
 // =====================================================================
 // Gauss-Jordan inverse with partial pivoting of the o x o matrix in aug
 // (row stride 2o, left half), result in the right half.  Returns false if a
-// pivot is zero.
+// pivot is zero.  The binary64 pipe (two lanes a clock an SM) bounds it: one
+// warp looks for the pivot and forms its reciprocal (all eight did, and one
+// thread looked), and columns that are unit vectors already are left out.
 __device__ bool gj_inverse(int o, double2* aug) {
     const int ld = 2 * o;
     for (int e = threadIdx.x; e < o * o; e += blockDim.x) {
@@ -244,39 +246,47 @@ __device__ bool gj_inverse(int o, double2* aug) {
         aug[r * ld + o + c] = make_double2(r == c ? 1.0 : 0.0, 0.0);
     }
     __shared__ int piv;
-    __shared__ bool bad;
-    if (threadIdx.x == 0) bad = false;
+    __shared__ double2 s_inv;
     __syncthreads();
     for (int k = 0; k < o; ++k) {
-        if (threadIdx.x == 0) {
-            int best = k;
-            double bv = cabs2(aug[k * ld + k]);
-            for (int r = k + 1; r < o; ++r) {
-                const double v = cabs2(aug[r * ld + k]);
-                if (v > bv) { bv = v; best = r; }
+        if (threadIdx.x < 32) {  // one warp: every other one's binary64 instructions would take the same pipe
+            unsigned long long best = 0;
+            int at = k;
+            bool nan = false;
+            for (int r = k + (int)threadIdx.x; r < o; r += 32) {
+                const unsigned long long v = (unsigned long long)__double_as_longlong(cabs2(aug[r * ld + k]));
+                if (v <= 0x7ff0000000000000ull && v > best) { best = v; at = r; }  // nan is never chosen over a number
+                if (r == k) nan = v > 0x7ff0000000000000ull;                       // on the diagonal: no inverse
             }
-            piv = best;
-            if (!(bv > 0.0)) bad = true;
+            nan = __any_sync(0xffffffffu, nan);
+#pragma unroll
+            for (int d = 16; d > 0; d >>= 1) {
+                const unsigned long long v = __shfl_xor_sync(0xffffffffu, best, d);
+                const int r = __shfl_xor_sync(0xffffffffu, at, d);
+                if (v > best || (v == best && r < at)) { best = v; at = r; }
+            }
+            const bool ok = !nan && best != 0;
+            if (ok) {
+                const double2 inv = cdiv(make_double2(1.0, 0.0), aug[at * ld + k]);
+                if (threadIdx.x == 0) s_inv = inv;
+            }
+            if (threadIdx.x == 0) piv = ok ? at : -1;
         }
         __syncthreads();
-        if (bad) return false;
-        if (piv != k)
-            for (int c = threadIdx.x; c < ld; c += blockDim.x) {
-                const double2 t = aug[k * ld + c];
-                aug[k * ld + c] = aug[piv * ld + c];
-                aug[piv * ld + c] = t;
-            }
+        const int p = piv;
+        if (p < 0) return false;
+        const double2 inv = s_inv;
+        for (int c = k + threadIdx.x; c < ld; c += blockDim.x) {  // columns before k are unit vectors already
+            const double2 t = aug[k * ld + c], v = aug[p * ld + c];
+            aug[k * ld + c] = cmul(v, inv);
+            if (p != k) aug[p * ld + c] = t;
+        }
         __syncthreads();
-        const double2 inv = cdiv(make_double2(1.0, 0.0), aug[k * ld + k]);
-        __syncthreads();
-        for (int c = threadIdx.x; c < ld; c += blockDim.x) aug[k * ld + c] = cmul(aug[k * ld + c], inv);
-        __syncthreads();
-        for (int e = threadIdx.x; e < o * ld; e += blockDim.x) {
-            const int r = e / ld, c = e - r * ld;
+        const int m = ld - k - 1;
+        for (int e = threadIdx.x; e < o * m; e += blockDim.x) {
+            const int r = e / m, c = k + 1 + e - r * m;
             if (r == k) continue;
-            const double2 f = aug[r * ld + k];
-            if (c == k) continue;
-            aug[r * ld + c] = csub(aug[r * ld + c], cmul(f, aug[k * ld + c]));
+            aug[r * ld + c] = csub(aug[r * ld + c], cmul(aug[r * ld + k], aug[k * ld + c]));
         }
         __syncthreads();
         for (int r = threadIdx.x; r < o; r += blockDim.x)
@@ -287,9 +297,9 @@ __device__ bool gj_inverse(int o, double2* aug) {
 }
 
 // out[i, b] (+)= sum_c (X[i, c] + sum_d Y[i, d] P[d, c]) conj(N[b, c]),
-// i < n, rows staged RT at a time.  X[i, c] = XT ? X[c * n + i] : X[i * o + c].
+// i < n, rows staged RT at a time.  X[i, c] = XT ? X[c * n + i] : X[i * o + c]; YR: Y is real.
 constexpr int RT = 32;
-template <bool XT>
+template <bool XT, bool YR>
 __device__ void rows_phase(int n, int o, const double2* X, const double2* Y, const double2* P, int ldp,
                            const double2* N, int ldn, double2* out, bool accumulate, double2* zt) {
     for (int i0 = 0; i0 < n; i0 += RT) {
@@ -297,7 +307,10 @@ __device__ void rows_phase(int n, int o, const double2* X, const double2* Y, con
         for (int e = threadIdx.x; e < rows * o; e += blockDim.x) {
             const int r = e / o, c = e - r * o, i = i0 + r;
             double2 z = X ? (XT ? X[(size_t)c * n + i] : X[(size_t)i * o + c]) : make_double2(0.0, 0.0);
-            for (int d = 0; d < o; ++d) cfma(z, Y[(size_t)i * o + d], P[d * ldp + c]);
+            for (int d = 0; d < o; ++d) {
+                if (YR) rfma(z, Y[(size_t)i * o + d].x, P[d * ldp + c]);
+                else cfma(z, Y[(size_t)i * o + d], P[d * ldp + c]);
+            }
             zt[r * o + c] = z;
         }
         __syncthreads();
@@ -317,6 +330,7 @@ __device__ void rows_phase(int n, int o, const double2* X, const double2* Y, con
 //   Wb += [Gb^T + C (kappa I - conj(G) Gb^T)] m^-H,  kappa = 2 conj(ov) ovb,
 // with conj(G) Gb^T = m^-H (W^H Gb^T).  gbar (W, o, n) and (ov, ovbar) may
 // be null.  A singular m sets *err = AFQ_STATUS_SINGULAR and leaves Wb as is.
+// The trial is real.
 // =====================================================================
 __global__ void __launch_bounds__(256) k_green_adj(int n, int o, const double2* __restrict__ mo,
                                                    const double2* __restrict__ walkers,
@@ -331,15 +345,17 @@ __global__ void __launch_bounds__(256) k_green_adj(int n, int o, const double2* 
     const int w = blockIdx.x, no = n * o;
     const double2* Ww = walkers + (size_t)w * no;
     const double2* Gb = gbar ? gbar + (size_t)w * no : nullptr;
-    for (int e = threadIdx.x; e < o * o; e += blockDim.x) {
-        const int a = e / o, b = e - a * o;
-        double2 m = make_double2(0.0, 0.0), t = make_double2(0.0, 0.0);
-        for (int i = 0; i < n; ++i) {
-            cfma(m, cconj(mo[(size_t)i * o + a]), Ww[(size_t)i * o + b]);
-            if (Gb) cfma(t, cconj(Ww[(size_t)i * o + a]), Gb[(size_t)b * n + i]);
+    for (int e = threadIdx.x; e < 2 * o * o; e += blockDim.x) {
+        const int h = e >= o * o, q = e - h * o * o, a = q / o, b = q - a * o;
+        double2 v = make_double2(0.0, 0.0);
+        if (h) {
+            for (int i = 0; i < n; ++i) rfma(v, mo[(size_t)i * o + a].x, Ww[(size_t)i * o + b]);
+            aug[a * 2 * o + b] = v;  // m
+        } else {
+            if (Gb)
+                for (int i = 0; i < n; ++i) cfma(v, cconj(Ww[(size_t)i * o + a]), Gb[(size_t)b * n + i]);
+            T[q] = v;  // T[c, b] = sum_j conj(W[j, c]) Gb[b, j]
         }
-        aug[a * 2 * o + b] = m;
-        T[a * o + b] = t;  // T[c, b] = sum_j conj(W[j, c]) Gb[b, j]
     }
     __syncthreads();
     if (!gj_inverse(o, aug)) {
@@ -359,7 +375,7 @@ __global__ void __launch_bounds__(256) k_green_adj(int n, int o, const double2* 
         P[a * o + b] = p;
     }
     __syncthreads();
-    rows_phase<true>(n, o, Gb, mo, P, o, mi, 2 * o, wbar + (size_t)w * no, true, zt);
+    rows_phase<true, true>(n, o, Gb, mo, P, o, mi, 2 * o, wbar + (size_t)w * no, true, zt);
 }
 
 int launch_green_adj(int W, int n, int o, const double2* mo, const double2* walkers, const double2* gbar,
@@ -424,7 +440,7 @@ __global__ void __launch_bounds__(256) k_qr_adj(int n, int o, const double2* __r
         M[a * o + b] = csub(kb, B[a * o + b]);
     }
     __syncthreads();
-    rows_phase<false>(n, o, Qb, Qw, M, o, Ri, o, abar + (size_t)w * no, false, zt);
+    rows_phase<false, false>(n, o, Qb, Qw, M, o, Ri, o, abar + (size_t)w * no, false, zt);
 }
 
 int launch_qr_adj(int W, int n, int o, const double2* A, const double2* Q, const double2* qbar, double2* abar,
