@@ -526,12 +526,6 @@ __device__ __forceinline__ void oz_store8(const OzDst& o, long long b, int r, in
     *(uint4*)(d + 5 * plane) = oz_pack8<5>(y);
     *(uint4*)(d + 6 * plane) = oz_pack8<6>(y);
 }
-__device__ __forceinline__ int warp_max(int v) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(0xffffffffu, v, o));
-    return v;
-}
-
 // The largest of the values of the LN threads that share a row (LN <= 32 lanes of a warp, or the CTA's 256).
 template <int LN>
 __device__ __forceinline__ int row_max(int e, int* s_max) {
@@ -775,15 +769,19 @@ __device__ __forceinline__ void cfma2(double& re, double& im, double2 a, double2
 // The adjoint's outer products: row i of walker w over (k, c, part) is
 // conj(i sqrt_dt / k) tb_k[i, c] = (sqrt_dt / k) (tb.y, -tb.x), k = 1 .. K (A); the right
 // operand's rows (j, Re) [Re, Im] and (j, Im) [-Im, Re] of t_{k-1}[j, c] give
-// sum a conj(t).  One warp a row.
+// sum a conj(t).  LN lanes a row, eight entries a lane.
+template <int LN>
 __global__ void __launch_bounds__(256) k_oz_vbar(int W, int n, int o, int K, double sqrt_dt,
                                                  const double2* __restrict__ tbar, const double2* __restrict__ terms,
                                                  OzDst A, int* __restrict__ ea, OzDst B, int* __restrict__ eb) {
-    const int lane = threadIdx.x & 31, no = n * o, L = K * o;
+    constexpr int RC = 256 / LN;  // rows a CTA
+    const int t = threadIdx.x % LN, no = n * o, L = K * o;
     const long long rows = (long long)W * n;
-    for (long long r = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); r < 2 * rows; r += (long long)gridDim.x * 8) {
-        const bool right = r >= rows;
-        const long long x = right ? r - rows : r;
+    // every thread of a warp stays for the shuffles
+    for (long long r0 = (long long)blockIdx.x * RC; r0 < 2 * rows; r0 += (long long)gridDim.x * RC) {
+        const long long r = r0 + threadIdx.x / LN;
+        const bool in = r < 2 * rows, right = in && r >= rows;
+        const long long x = !in ? 0 : right ? r - rows : r;
         const int w = (int)(x / n), i = (int)(x - (long long)w * n);
         // entry l = (k - 1) o + c of the row
         const double2* src = right ? terms + (long long)w * K * no + (long long)i * o
@@ -798,16 +796,17 @@ __global__ void __launch_bounds__(256) k_oz_vbar(int W, int n, int o, int K, dou
             return v;
         };
         int e = 0;
-        for (int l = lane; l < L; l += 32) {
+        for (int l = t; in && l < L; l += LN) {
             const double2 v = at(l);
             e = max(e, max(oz_expo(v.x), oz_expo(v.y)));
         }
-        const int E = oz_scale(warp_max(e));
-        if (lane == 0) {
+        const int E = oz_scale(row_max<LN>(e, nullptr));
+        if (!in) continue;
+        if (t == 0) {
             if (right) eb[2 * x] = eb[2 * x + 1] = E;
             else ea[x] = E;
         }
-        for (int k = 8 * lane; k < 32 * A.nks; k += 256) {
+        for (int k = 8 * t; k < 32 * A.nks; k += 8 * LN) {
             long long y[8], z[8];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -1487,9 +1486,12 @@ int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tb
     const long long no = (long long)n * o, n2 = (long long)n * n;
     for (int w0 = 0; w0 < W; w0 += v.wc) {
         const int wc = W - w0 < v.wc ? W - w0 : v.wc;
-        k_oz_vbar<<<row_blocks(2LL * wc * n), 256, 0, s>>>(wc, n, o, K, sqrt_dt, tbar + (long long)w0 * (K + 1) * no,
-                                                          terms + (long long)w0 * K * no, dst_of(v.A, n, k2), v.A.ex,
-                                                          dst_of(v.B, 2 * n, k2), v.B.ex);
+        // eight lanes a row of up to 64 entries, sixteen of 128 (60 orbitals, 120 entries, 256 walkers: 106 -> 65 us)
+        const int lanes = k2 <= 64 ? 8 : k2 <= 128 ? 16 : 32;
+        const auto cut = lanes == 8 ? k_oz_vbar<8> : lanes == 16 ? k_oz_vbar<16> : k_oz_vbar<32>;
+        cut<<<row_blocks(2LL * wc * n, 256 / lanes), 256, 0, s>>>(
+            wc, n, o, K, sqrt_dt, tbar + (long long)w0 * (K + 1) * no, terms + (long long)w0 * K * no,
+            dst_of(v.A, n, k2), v.A.ex, dst_of(v.B, 2 * n, k2), v.B.ex);
         AFQ_LAUNCHED("k_oz_vbar");
         const OzOut out = {vbar + w0 * n2, n2, 0, 1, n, n, 0, nullptr};
         AFQ_TRY(oz_launch(n, 2 * n, k2, wc, 1, v.A, v.B, out, 1, (k2 + 255) / 256, nullptr, err, s));
