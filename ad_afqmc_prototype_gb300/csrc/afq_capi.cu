@@ -166,6 +166,7 @@ static bool oz_supported(const afq_dims* d) { return d->nocc <= 32 && d->norb <=
 static OzScratch take_oz(Arena& a, size_t bytes, int* status) {
     OzScratch z;
     z.p = a.take<char>(bytes);
+    z.bytes = bytes;
     z.err = status;
     return z;
 }
@@ -551,12 +552,11 @@ static int orthonormalize_refresh(const afq_problem* pb, const afq_state* st, cu
     double2* walk = (double2*)st->walkers;
     const bool keep = is_mixed(d->precision) && det_buf && (ws || green_kept);
     const StepWS* sw = ws ? ws : green_ws;
-    void* qr_scratch = sw ? sw->oz.p : nullptr;
     {
         AFQ_PHASE("qr", s);
         if (is_mixed(d->precision))
             AFQ_TRY(launch_cholqr2(d->n_walkers, d->norb, d->nocc, walk, walk, keep ? det_buf : nullptr, s));
-        else AFQ_TRY(launch_qr_auto(d->n_walkers, d->norb, d->nocc, walk, walk, nullptr, qr_scratch, s));
+        else AFQ_TRY(launch_qr_auto(d->n_walkers, d->norb, d->nocc, walk, walk, nullptr, sw ? sw->oz : OzScratch{}, s));
     }
     if (keep) {
         AFQ_PHASE("overlap_rescale", s);
@@ -841,8 +841,11 @@ int afq_orthogonalize_ws(const afq_dims* d, const double* walkers, double* walke
     AFQ_NOTNULL(walkers); AFQ_NOTNULL(walkers_out); AFQ_NOTNULL(workspace);
     if (workspace_bytes < need) return fail(AFQ_E_WORKSPACE, "workspace of %zu bytes < %zu needed", workspace_bytes, need);
     if (((uintptr_t)workspace) & 255) return fail(AFQ_E_INVALID_ARGUMENT, "workspace must be 256-byte aligned");
+    OzScratch oz;
+    oz.p = workspace;
+    oz.bytes = workspace_bytes;
     return launch_qr_auto(d->n_walkers, d->norb, d->nocc, (const double2*)walkers, (double2*)walkers_out,
-                          (double2*)det_r, workspace, as_stream(stream));
+                          (double2*)det_r, oz, as_stream(stream));
 }
 
 size_t afq_sr_workspace(int32_t n_walkers) {

@@ -119,10 +119,11 @@ GradWS layout_grad(Arena& a, const afq_dims* d, const afq_params* p, int ck) {
         const size_t z2 = (size_t)zgemm_splits((int)W, (int)no, (int)G) * W * no;
         g.zpart = a.take<double2>(z1 > z2 ? z1 : z2);
         const int Wi = (int)W, Gi = (int)G, n2 = (int)(n * n), noi = (int)no, oi = (int)o, ni = (int)n, wo = (int)(wc * o);
-        g.oz.p = a.take<char>(std::max({zgemm_oz_scratch(Wi, Gi, noi), zgemm_oz_scratch(Wi, n2, Gi),
+        g.oz.bytes = std::max({zgemm_oz_scratch(Wi, Gi, noi), zgemm_oz_scratch(Wi, n2, Gi),
                                         zgemm_oz_scratch(Wi, Gi, n2), zgemm_oz_scratch(Wi, noi, Gi),
                                         zgemm_oz_scratch(wo, Gi * oi, ni), zgemm_oz_scratch(wo, ni, Gi * oi),
-                                        green_oz_scratch(Wi, ni, oi), taylor_grad_oz_scratch(Wi, ni, oi), vbar_oz_scratch(Wi, ni, oi, (int)K)}));
+                                        green_oz_scratch(Wi, ni, oi), taylor_grad_oz_scratch(Wi, ni, oi), vbar_oz_scratch(Wi, ni, oi, (int)K)});
+        g.oz.p = a.take<char>(g.oz.bytes);
         g.oz.err = g.status;
     }
     g.wk = a.take<double2>(W * no);
@@ -201,7 +202,7 @@ T* slot(T* base, size_t per, int k) { return base + (size_t)k * per; }
 int zgemm_adj(const GradWS& g, int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B,
               int64_t ldb, bool b_trans, double2* C, cudaStream_t s) {
     if (zgemm_oz_pays(M, N, K))
-        return launch_zgemm_oz(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, N, g.oz.p, g.oz.err, s);
+        return launch_zgemm_oz(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, N, g.oz, s);
     return launch_zgemm_splitk(M, N, K, alpha, A, lda, B, ldb, false, b_trans, C, g.zpart, s);
 }
 
@@ -248,7 +249,7 @@ int step_adjoint(const Ctx& c, const BlockSnap& sn, int op, int st_i, uint64_t c
       AFQ_TRY(launch_ebar(W, n, o, g.tbar, (long long)(K + 1) * no, Wpre, no, g.ebar_part, s)); }
     // V = sum_g x~_g L_g: x~b = Vb . L^T
     { AFQ_PHASE("adj_vbar", s);
-      AFQ_TRY(launch_vbar_oz(W, n, o, K, pb->sqrt_dt, g.tbar, g.terms, g.V, g.oz.p, g.oz.err, s)); }
+      AFQ_TRY(launch_vbar_oz(W, n, o, K, pb->sqrt_dt, g.tbar, g.terms, g.V, g.oz, s)); }
     { AFQ_PHASE("adj_xbar_gemm", s);
       AFQ_TRY(zgemm_adj(g, W, G, n * n, 1.0, g.V, (int64_t)n * n, pb->chol, (int64_t)n * n, true, g.xtb, s)); }
     // field shifts, then the force bias fb = 2 L~ vec(G_half)

@@ -305,10 +305,12 @@ int launch_zgemm_splitk(int M, int N, int K, double alpha, const double2* A, int
                         int64_t ldb, bool b_complex, bool b_trans, double2* C, double2* part, cudaStream_t s);
 
 // k_ozgemm.cu : the binary64 form's contractions from integer digits on the
-// tensor cores.  Scratch of a call: *_oz_scratch bytes, 256-byte aligned; a
-// bounded wait that expires sets *err.
+// tensor cores.  Scratch of a call: *_oz_scratch bytes, 256-byte aligned (a
+// smaller region is refused before anything is launched); a bounded wait that
+// expires sets *err.
 struct OzScratch {
     void* p = nullptr;
+    size_t bytes = 0;
     int* err = nullptr;
     // a block's steps: digits of chol (n^2 rows over the vectors) and of rot_chol (vectors over nocc norb), or null
     void* chol = nullptr;
@@ -322,7 +324,7 @@ bool zgemm_oz_pays(int M, int N, int K);
 size_t zgemm_oz_scratch(int M, int N, int K);
 // launch_zgemm with a real right operand; alpha a power of two
 int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
-                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s,
+                    bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s,
                     const void* real = nullptr);
 // room for digits of the real operand kept over several products (`real` above and below); 0: not kept
 size_t oz_real_bytes(int N, int K);
@@ -330,11 +332,12 @@ bool trotter_oz_pays(int W, int n, int n_terms);
 bool green_oz_pays(int n, int o);
 size_t green_oz_scratch(int W, int n, int o);
 int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walkers, double2* ovlp_out,
-                    double2* green_out, int ov_square, void* scratch, int* err, cudaStream_t s);
+                    double2* green_out, int ov_square, const OzScratch& oz, cudaStream_t s);
+// grows with W: a call's last chunk of walkers is smaller than the chunk that the scratch was sized for
 size_t trotter_oz_scratch(int W, int n, int o, int ns);
-bool trotter_oz_whole(int W, int n);  // all walkers in one chunk of the scratch
+bool trotter_oz_whole(int W, int n, int o, int ns);  // all walkers in one chunk of the scratch
 int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
-                      const double2* win, double2* wout, int ns, long long ws, long long ss, void* scratch, int* err,
+                      const double2* win, double2* wout, int ns, long long ws, long long ss, const OzScratch& oz,
                       cudaStream_t s);
 // k_trotter_oz.cu : the same in one kernel a walker, n <= 64
 bool trotter_small_fits(int n, int oc, int n_terms);
@@ -347,14 +350,14 @@ int launch_taylor_adj_small(int W, int n, int o, int K, double sqrt_dt, const do
                             const double2* wbar_post, double2* tbar, double2* wbar_pre, cudaStream_t s);
 size_t taylor_grad_oz_scratch(int W, int n, int o);
 int launch_taylor_tape_oz(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
-                          const double2* win, double2* terms, double2* w2, void* scratch, int* err, cudaStream_t s);
+                          const double2* win, double2* terms, double2* w2, const OzScratch& oz, cudaStream_t s);
 int launch_taylor_adj_oz(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
-                         const double2* wbar_post, double2* tbar, double2* wbar_pre, void* scratch, int* err,
+                         const double2* wbar_post, double2* tbar, double2* wbar_pre, const OzScratch& oz,
                          cudaStream_t s);
 bool energy_oz_pays(int W, int n, int o, int G);
 size_t energy_oz_scratch(int W, int n, int o, int G);
 int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, const double* rot_chol,
-                             double* partial, void* scratch, int* err, cudaStream_t s);
+                             double* partial, const OzScratch& oz, cudaStream_t s);
 // the product by digits where that pays, else on the binary64 pipe
 int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B, int64_t ldb,
                       bool b_complex, bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s,
@@ -375,8 +378,10 @@ int launch_energy_partial_auto(int W, int n, int o, int G, const double2* green,
 // binary64 QR by digits with the Householder form for the walkers it does not suit; scratch bytes (0: not taken)
 bool qr_oz_pays(int W, int n, int o);
 size_t qr_oz_scratch(int W, int n, int o);
-int launch_qr_oz(int W, int n, int o, const double2* win, double2* wout, double2* det_r, void* scratch, cudaStream_t s);
-int launch_qr_auto(int W, int n, int o, const double2* win, double2* wout, double2* det_r, void* scratch, cudaStream_t s);
+int launch_qr_oz(int W, int n, int o, const double2* win, double2* wout, double2* det_r, const OzScratch& oz,
+                 cudaStream_t s);
+int launch_qr_auto(int W, int n, int o, const double2* win, double2* wout, double2* det_r, const OzScratch& oz,
+                   cudaStream_t s);
 // k_qr_oz.cu : its small kernels
 int launch_qr_factor(int W, int o, const double2* gram, double2* tinv, double* det, int* flag, cudaStream_t s);
 int launch_qr_finish(int W, int n, int o, const double2* q1, const double2* gram, const double* det, const int* err,
@@ -534,7 +539,7 @@ int launch_taylor_adj(int W, int n, int o, int K, double sqrt_dt, const double* 
 // Vb_w = sum_{k = 1 .. K} conj(i sqrt_dt / k) tb_k t_{k-1}^H by digits on the tensor cores (k_ozgemm.cu)
 size_t vbar_oz_scratch(int W, int n, int o, int K);
 int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms,
-                   double2* vbar, void* scratch, int* err, cudaStream_t s);
+                   double2* vbar, const OzScratch& oz, cudaStream_t s);
 int ebar_splits(int W);
 int launch_ebar(int W, int n, int o, const double2* X, long long xs, const double2* Y, long long ys, double* partial,
                 cudaStream_t s);

@@ -128,12 +128,13 @@ UWS layout_u(Arena& a, const afq_dims* d, int n_chunks, bool block = false) {
     u.ov_new = a.take<double2>(W);
     const int wc = chunk_of(d->n_walkers, n_chunks);
     u.V = a.take<double2>((size_t)wc * n * n);
-    u.oz.p = a.take<char>(oz_most({green_oz_scratch(2 * d->n_walkers, d->norb, d->nocc),
+    u.oz.bytes = oz_most({green_oz_scratch(2 * d->n_walkers, d->norb, d->nocc),
                                    zgemm_oz_scratch(2 * d->n_walkers, d->nchol, (int)no),
                                    zgemm_oz_scratch(wc, (int)(n * n), d->nchol),
                                    trotter_oz_scratch(wc, d->norb, d->nocc, 2),
                                    qr_oz_scratch(2 * d->n_walkers, d->norb, d->nocc),
-                                   energy_oz_scratch(2 * d->n_walkers, d->norb, d->nocc, d->nchol)}));
+                                   energy_oz_scratch(2 * d->n_walkers, d->norb, d->nocc, d->nchol)});
+    u.oz.p = a.take<char>(u.oz.bytes);
     u.oz.err = u.status;
     u.partial = (double*)a.take<double2>(energy_partial_count(2 * d->n_walkers, d->nocc, d->nchol));
     u.energy = a.take<double2>(W);
@@ -238,7 +239,7 @@ int step_u(const afq_problem* pb, const afq_params* p, const afq_state* st, cons
 int orthonormalize_u(const afq_problem* pb, const afq_state* st, const UWS& u, double2* green, cudaStream_t s) {
     const afq_dims* d = &pb->dims;
     double2* walk = (double2*)st->walkers;
-    { AFQ_PHASE("qr", s); AFQ_TRY(launch_qr_auto(2 * d->n_walkers, d->norb, d->nocc, walk, walk, nullptr, u.oz.p, s)); }
+    { AFQ_PHASE("qr", s); AFQ_TRY(launch_qr_auto(2 * d->n_walkers, d->norb, d->nocc, walk, walk, nullptr, u.oz, s)); }
     AFQ_PHASE(green ? "green" : "overlap", s);
     return overlap_u(d, (const double2*)pb->mo_coeff, walk, (double2*)st->overlaps, green, u, s);
 }
@@ -304,10 +305,11 @@ GWS layout_g(Arena& a, const afq_dims* d, int n_chunks) {
     g.gsum = a.take<double2>(W * o * n);
     const int wc = chunk_of(d->n_walkers, n_chunks);
     g.V = a.take<double2>((size_t)wc * n * n);
-    g.oz.p = a.take<char>(oz_most({green_oz_scratch(d->n_walkers, 2 * d->norb, 2 * d->nocc),
+    g.oz.bytes = oz_most({green_oz_scratch(d->n_walkers, 2 * d->norb, 2 * d->nocc),
                                    zgemm_oz_scratch(d->n_walkers, d->nchol, (int)(n * o)),
                                    zgemm_oz_scratch(wc, (int)(n * n), d->nchol),
-                                   trotter_oz_scratch(wc, d->norb, 2 * d->nocc, 2)}));
+                                   trotter_oz_scratch(wc, d->norb, 2 * d->nocc, 2)});
+    g.oz.p = a.take<char>(g.oz.bytes);
     g.oz.err = g.status;
     return g;
 }

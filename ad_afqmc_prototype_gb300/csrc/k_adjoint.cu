@@ -78,7 +78,7 @@ int launch_taylor_tape(int W, int n, int o, int K, double sqrt_dt, const double*
     const size_t smem = 2 * sizeof(double2) * (size_t)n * o;
     if (smem > 227 * 1024)
         return fail(AFQ_E_UNSUPPORTED, "Taylor adjoint: norb %d x nocc %d needs %zu bytes of shared memory", n, o, smem);
-    if (trotter_oz_pays(W, n, K)) return launch_taylor_tape_oz(W, n, o, K, sqrt_dt, E, V, win, terms, w2, oz.p, oz.err, s);
+    if (trotter_oz_pays(W, n, K)) return launch_taylor_tape_oz(W, n, o, K, sqrt_dt, E, V, win, terms, w2, oz, s);
     AFQ_TRY(allow_smem(k_taylor_tape, smem));
     k_taylor_tape<<<W, 256, smem, s>>>(n, o, K, sqrt_dt, E, V, win, terms, w2);
     AFQ_LAUNCHED("k_taylor_tape");
@@ -147,7 +147,7 @@ int launch_taylor_adj(int W, int n, int o, int K, double sqrt_dt, const double* 
     if (smem > 227 * 1024)
         return fail(AFQ_E_UNSUPPORTED, "Taylor adjoint: norb %d x nocc %d needs %zu bytes of shared memory", n, o, smem);
     if (trotter_oz_pays(W, n, K))
-        return launch_taylor_adj_oz(W, n, o, K, sqrt_dt, E, V, wbar_post, tbar, wbar_pre, oz.p, oz.err, s);
+        return launch_taylor_adj_oz(W, n, o, K, sqrt_dt, E, V, wbar_post, tbar, wbar_pre, oz, s);
     AFQ_TRY(allow_smem(k_taylor_adj, smem));
     k_taylor_adj<<<W, 256, smem, s>>>(n, o, K, sqrt_dt, E, V, wbar_post, tbar, wbar_pre);
     AFQ_LAUNCHED("k_taylor_adj");

@@ -276,7 +276,7 @@ int launch_green_det(int W, int n, int o, const double2* mo, int trial_real, con
 int launch_green_auto(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
                       double2* ovlp_out, double2* green_out, int ov_square, const OzScratch& oz, cudaStream_t s) {
     if (trial_real && oz.p && green_oz_pays(n, o))
-        return launch_green_oz(W, n, o, mo, walkers, ovlp_out, green_out, ov_square, oz.p, oz.err, s);
+        return launch_green_oz(W, n, o, mo, walkers, ovlp_out, green_out, ov_square, oz, s);
     return launch_green_sq(W, n, o, mo, trial_real, walkers, ovlp_out, green_out, ov_square, s);
 }
 

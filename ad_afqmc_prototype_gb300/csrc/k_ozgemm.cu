@@ -1003,6 +1003,12 @@ int even_chunk(int W, long long most) {
     return (int)((W + n - 1) / n);
 }
 
+// a call's layout in the region that it was given
+int oz_room(const Arena& a) {
+    if (!a.base || !a.ok()) return fail(AFQ_E_WORKSPACE, "digit scratch of %zu bytes < %zu needed", a.cap, a.used);
+    return AFQ_OK;
+}
+
 constexpr int OZ_TILE_SMS = 152;
 
 struct ZLayout {
@@ -1102,13 +1108,14 @@ static int oz_real_split(int N, int K, const double* B, int64_t ldb, bool b_tran
 
 // sn > 0: the V-build over sn orbitals, whose symmetric vectors' rows are in SymRows's order (asym: the flag of `real`)
 static int zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
-                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s, const void* real,
+                    bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s, const void* real,
                     int sn, const int* asym) {
     if (M <= 0 || N <= 0) return AFQ_OK;
     int ae = 0;
     if (frexp(alpha, &ae) != 0.5) return fail(AFQ_E_UNSUPPORTED, "digit GEMM: alpha=%g is no power of two", alpha);
-    Arena ar(scratch, (size_t)-1);
+    Arena ar(oz.p, oz.bytes);
     ZLayout z = z_layout(ar, M, N, K);
+    AFQ_TRY(oz_room(ar));
     if (real) {
         Arena a((void*)real, (size_t)-1);
         z.A = take_digits(a, N, K);
@@ -1132,15 +1139,15 @@ static int zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t
             const long long tiles = (long long)((nc + OZ_ROWS - 1) / OZ_ROWS) * ((2 * mc + OZ_TN - 1) / OZ_TN);
             int splits, cps;
             oz_splits(tiles, K, sms < OZ_TILE_SMS ? sms : OZ_TILE_SMS, splits, cps);
-            AFQ_TRY(oz_launch(nc, 2 * mc, K, 1, 0, z.A, z.B, out, splits, cps, z.raw, err, s, sn ? sym : SymRows{}));
+            AFQ_TRY(oz_launch(nc, 2 * mc, K, 1, 0, z.A, z.B, out, splits, cps, z.raw, oz.err, s, sn ? sym : SymRows{}));
         }
     }
     return AFQ_OK;
 }
 
 int launch_zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
-                    bool b_trans, double2* C, int64_t ldc, void* scratch, int* err, cudaStream_t s, const void* real) {
-    return zgemm_oz(M, N, K, alpha, A, lda, B, ldb, b_trans, C, ldc, scratch, err, s, real, 0, nullptr);
+                    bool b_trans, double2* C, int64_t ldc, const OzScratch& oz, cudaStream_t s, const void* real) {
+    return zgemm_oz(M, N, K, alpha, A, lda, B, ldb, b_trans, C, ldc, oz, s, real, 0, nullptr);
 }
 
 // ---------------------------------------------------------------- Taylor --
@@ -1150,12 +1157,16 @@ struct TrLayout {
     OzDigits E, V, T, X;  // E_half, V rows, right operands of V T, walker columns
     double2 *Y, *U;
 };
-// W walkers of ns blocks (n x o) each
-TrLayout tr_layout(Arena& a, int W, int n, int o, int ns) {
+// walkers of ns blocks (n x o) each in a chunk: their digits and blocks take at most OZ_CAP
+long long tr_most(int n, int o, int ns) {
+    const long long per = (round_up(n, 8) + round_up(2 * ns * o, 8)) * digit_row_bytes(2 * n) +
+                          2LL * ns * o * (digit_row_bytes(n) + 16LL * n);
+    return OZ_CAP / per > 1 ? OZ_CAP / per : 1;
+}
+// a chunk of wc walkers
+TrLayout tr_layout(Arena& a, int wc, int n, int o, int ns) {
     TrLayout t;
-    const long long per = round_up(n, 8) * digit_row_bytes(2 * n);  // digits of one V
-    long long wc = OZ_CAP / per;                                    // walkers whose V digits fit
-    t.wc = even_chunk(W, wc);
+    t.wc = wc;
     const size_t nb = (size_t)t.wc * ns;
     t.E = take_digits(a, n, n);
     t.V = take_digits(a, n, 2 * n, t.wc);
@@ -1181,15 +1192,19 @@ int launch_term(int W, int n, int o, double s, const double2* Y, const double2* 
 }
 }  // namespace
 
+// The largest chunk of up to W walkers, not the even one that a call of W takes: where W walkers are two chunks of half
+// of them, W - 1 can be one.
 size_t trotter_oz_scratch(int W, int n, int o, int ns) {
-    Arena a;
-    tr_layout(a, W, n, o, ns);
-    return a.used + 256;
+    size_t most = 0;
+    for (int k = 1; k <= ns; ++k) {  // the spins together, or one at a time
+        Arena a;
+        const long long m = tr_most(n, o, k);
+        tr_layout(a, W < m ? W : (int)m, n, o, k);
+        most = std::max(most, a.used);
+    }
+    return most + 256;
 }
-bool trotter_oz_whole(int W, int n) {
-    Arena a;
-    return tr_layout(a, W, n, 1, 1).wc == W;
-}
+bool trotter_oz_whole(int W, int n, int o, int ns) { return W <= tr_most(n, o, ns); }
 
 // E_half . sum_{k <= K} (i sqrt_dt V)^k / k! . E_half . X, n_terms >= 1, of the
 // ns blocks X of each walker, which share its V: block p of walker w is n x o at
@@ -1198,11 +1213,13 @@ bool trotter_oz_whole(int W, int n) {
 // E_half X is formed as X + (E_half - I) X: E_half is close to the identity,
 // and a digit product's error scales with its operands' largest entries.
 int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
-                      const double2* win, double2* wout, int ns, long long ws, long long ss, void* scratch, int* err,
+                      const double2* win, double2* wout, int ns, long long ws, long long ss, const OzScratch& oz,
                       cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
-    Arena ar(scratch, (size_t)-1);
-    const TrLayout t = tr_layout(ar, W, n, o, ns);
+    Arena ar(oz.p, oz.bytes);
+    const TrLayout t = tr_layout(ar, even_chunk(W, tr_most(n, o, ns)), n, o, ns);
+    AFQ_TRY(oz_room(ar));
+    int* err = oz.err;
     AFQ_TRY(split_rows(n, n, n, E, n, t.E, s, 1));
     const size_t no = (size_t)n * o;
     for (int w0 = 0; w0 < W; w0 += t.wc) {
@@ -1253,7 +1270,8 @@ struct TgLayout {
 };
 TgLayout tg_layout(Arena& a, int W, int n, int o) {
     TgLayout t;
-    const long long n2 = (long long)n * n, per = round_up(n, 8) * digit_row_bytes(2 * n) + 16 * n2;
+    const long long n2 = (long long)n * n, per = (round_up(n, 8) + round_up(2 * o, 8)) * digit_row_bytes(2 * n) + 16 * n2 +
+                                                 2LL * o * (digit_row_bytes(n) + 16LL * n);
     const long long most = OZ_CAP / per;
     t.wc = even_chunk(W, most < 65535 ? most : 65535);
     t.E = take_digits(a, n, n);
@@ -1275,9 +1293,11 @@ size_t taylor_grad_oz_scratch(int W, int n, int o) {
 }
 
 int launch_taylor_tape_oz(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
-                          const double2* win, double2* terms, double2* w2, void* scratch, int* err, cudaStream_t s) {
-    Arena ar(scratch, (size_t)-1);
+                          const double2* win, double2* terms, double2* w2, const OzScratch& oz, cudaStream_t s) {
+    Arena ar(oz.p, oz.bytes);
     const TgLayout t = tg_layout(ar, W, n, o);
+    AFQ_TRY(oz_room(ar));
+    int* err = oz.err;
     const size_t no = (size_t)n * o;
     AFQ_TRY(split_rows(n, n, n, E, n, t.E, s, 1));
     const OzOut xo = {t.Y, 0, (long long)no, 1, o, o, 0, nullptr}, to = {t.Y, (long long)no, 0, 1, o, o, 0, nullptr};
@@ -1299,10 +1319,12 @@ int launch_taylor_tape_oz(int W, int n, int o, int K, double sqrt_dt, const doub
 }
 
 int launch_taylor_adj_oz(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
-                         const double2* wbar_post, double2* tbar, double2* wbar_pre, void* scratch, int* err,
+                         const double2* wbar_post, double2* tbar, double2* wbar_pre, const OzScratch& oz,
                          cudaStream_t s) {
-    Arena ar(scratch, (size_t)-1);
+    Arena ar(oz.p, oz.bytes);
     const TgLayout t = tg_layout(ar, W, n, o);
+    AFQ_TRY(oz_room(ar));
+    int* err = oz.err;
     const size_t no = (size_t)n * o;
     const unsigned nt = (n + 31) / 32;
     k_oz_adjoint<double><<<dim3(nt, nt, 1), 256, 0, s>>>(n, E, t.et);
@@ -1362,10 +1384,12 @@ size_t green_oz_scratch(int W, int n, int o) {
 
 // m = C^T W of all walkers as one product, its factorisations, and G_half[b, i] = sum_a W[i, a] m^-1[a, b] a walker
 int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walkers, double2* ovlp_out,
-                    double2* green_out, int ov_square, void* scratch, int* err, cudaStream_t s) {
+                    double2* green_out, int ov_square, const OzScratch& oz, cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
-    Arena ar(scratch, (size_t)-1);
+    Arena ar(oz.p, oz.bytes);
     const GrLayout g = gr_layout(ar, W, n, o);
+    AFQ_TRY(oz_room(ar));
+    int* err = oz.err;
     const size_t no = (size_t)n * o;
     AFQ_TRY(split_cols(o, n, (const double*)mo, 2LL * o, g.C, s, 2));
     for (int w0 = 0; w0 < W; w0 += g.wc) {
@@ -1420,10 +1444,12 @@ size_t qr_oz_scratch(int W, int n, int o) {
     return a.used + 256;
 }
 
-int launch_qr_oz(int W, int n, int o, const double2* win, double2* wout, double2* det_r, void* scratch, cudaStream_t s) {
+int launch_qr_oz(int W, int n, int o, const double2* win, double2* wout, double2* det_r, const OzScratch& oz,
+                 cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
-    Arena ar(scratch, (size_t)-1);
+    Arena ar(oz.p, oz.bytes);
     const QrLayout g = qr_layout(ar, W, n, o);
+    AFQ_TRY(oz_room(ar));
     const size_t no = (size_t)n * o;
     const OzOut gout = {g.gram, 2LL * o * o, 2 * o, 0, 1, 1, 0, nullptr};      // gram[b][2 a + part]
     const OzOut qout = {g.q1, (long long)no, 1, 0, o, 1, 0, nullptr};          // q1[i][c]
@@ -1445,8 +1471,9 @@ int launch_qr_oz(int W, int n, int o, const double2* win, double2* wout, double2
     return launch_qr(W, n, o, win, wout, det_r, s, g.flag);
 }
 
-int launch_qr_auto(int W, int n, int o, const double2* win, double2* wout, double2* det_r, void* scratch, cudaStream_t s) {
-    if (scratch && qr_oz_pays(W, n, o)) return launch_qr_oz(W, n, o, win, wout, det_r, scratch, s);
+int launch_qr_auto(int W, int n, int o, const double2* win, double2* wout, double2* det_r, const OzScratch& oz,
+                   cudaStream_t s) {
+    if (oz.p && qr_oz_pays(W, n, o)) return launch_qr_oz(W, n, o, win, wout, det_r, oz, s);
     return launch_qr(W, n, o, win, wout, det_r, s);
 }
 
@@ -1474,14 +1501,15 @@ size_t vbar_oz_scratch(int W, int n, int o, int K) {
 
 // Vb_w = sum_{k = 1 .. K} conj(i sqrt_dt / k) tb_k t_{k-1}^H
 int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms,
-                   double2* vbar, void* scratch, int* err, cudaStream_t s) {
+                   double2* vbar, const OzScratch& oz, cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
     if (K == 0) {
         AFQ_CUDA(cudaMemsetAsync(vbar, 0, sizeof(double2) * (size_t)W * n * n, s));
         return AFQ_OK;
     }
-    Arena ar(scratch, (size_t)-1);
+    Arena ar(oz.p, oz.bytes);
     const VbLayout v = vb_layout(ar, W, n, o, K);
+    AFQ_TRY(oz_room(ar));
     const int k2 = 2 * K * o;
     const long long no = (long long)n * o, n2 = (long long)n * n;
     for (int w0 = 0; w0 < W; w0 += v.wc) {
@@ -1494,7 +1522,7 @@ int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tb
             dst_of(v.A, n, k2), v.A.ex, dst_of(v.B, 2 * n, k2), v.B.ex);
         AFQ_LAUNCHED("k_oz_vbar");
         const OzOut out = {vbar + w0 * n2, n2, 0, 1, n, n, 0, nullptr};
-        AFQ_TRY(oz_launch(n, 2 * n, k2, wc, 1, v.A, v.B, out, 1, (k2 + 255) / 256, nullptr, err, s));
+        AFQ_TRY(oz_launch(n, 2 * n, k2, wc, 1, v.A, v.B, out, 1, (k2 + 255) / 256, nullptr, oz.err, s));
     }
     return AFQ_OK;
 }
@@ -1524,10 +1552,11 @@ size_t energy_oz_scratch(int W, int n, int o, int G) {
 }
 
 int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, const double* rot_chol,
-                             double* partial_d, void* scratch, int* err, cudaStream_t s) {
+                             double* partial_d, const OzScratch& oz, cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
-    Arena ar(scratch, (size_t)-1);
+    Arena ar(oz.p, oz.bytes);
     const EnLayout e = en_layout(ar, W, n, o, G);
+    AFQ_TRY(oz_room(ar));
     const int nchunk = energy_partial_chunks(o, G), ng = (G + nchunk - 1) / nchunk;
     const int smem = ng * o * (o + 1) * (int)sizeof(double2);
     if (smem > OZ_XSMEM || W > 65535) return fail(AFQ_E_UNSUPPORTED, "digit energy: nocc=%d W=%d", o, W);
@@ -1538,7 +1567,7 @@ int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, c
         AFQ_TRY(split_crows((long long)wc * o, n, green + (size_t)w0 * o * n, n, e.X, s));
         const OzOut out = {e.F, 0, (long long)G * o, 0, 1, 1, 0, nullptr};
         AFQ_TRY(oz_launch(G * o, 2 * wc * o, n, 1, 0, e.L, e.X, out, 1, (n + 255) / 256,
-                          nullptr, err, s));
+                          nullptr, oz.err, s));
         k_oz_exchange<<<dim3(nchunk, wc), 256, smem, s>>>(o, G, ng, e.F, (double2*)partial_d + (size_t)w0 * nchunk * 2);
         AFQ_LAUNCHED("k_oz_exchange");
     }
@@ -1570,7 +1599,7 @@ int launch_zgemm_auto(int M, int N, int K, double alpha, const double2* A, int64
     if (!b_complex && zgemm_small_pays(M, N, K))
         return launch_zgemm_small(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, ldc, s);
     if (!b_complex && zgemm_oz_pays(M, N, K))
-        return launch_zgemm_oz(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, ldc, oz.p, oz.err, s, real);
+        return launch_zgemm_oz(M, N, K, alpha, A, lda, (const double*)B, ldb, b_trans, C, ldc, oz, s, real);
     return launch_zgemm(M, N, K, alpha, A, lda, B, ldb, b_complex, b_trans, C, ldc, s);
 }
 
@@ -1579,7 +1608,7 @@ int launch_vbuild(int W, int n, int G, const double2* xs, const double* chol, do
     const int n2 = n * n, sn = (oz.chol ? oz.asym != nullptr : vbuild_sym_pays(W, n)) ? n : 0;
     if (zgemm_small_pays(W, n2, G)) return launch_zgemm_small(W, n2, G, 1.0, xs, G, chol, n2, false, V, n2, s);
     if (zgemm_oz_pays(W, n2, G))
-        return zgemm_oz(W, n2, G, 1.0, xs, G, chol, n2, false, V, n2, oz.p, oz.err, s, oz.chol, sn, oz.asym);
+        return zgemm_oz(W, n2, G, 1.0, xs, G, chol, n2, false, V, n2, oz, s, oz.chol, sn, oz.asym);
     return launch_zgemm(W, n2, G, 1.0, xs, G, chol, n2, false, false, V, n2, s);
 }
 
@@ -1590,7 +1619,7 @@ int launch_trotter_auto(int W, int n, int o, int n_terms, double sqrt_dt, const 
     if (trotter_small_pays(wp, n, o * vdiv, n_terms))
         return launch_trotter_small(wp, n, o, n_terms, sqrt_dt, E, V, win, wout, vdiv, vdiv * no, no, s);
     if (trotter_oz_pays(W, n, n_terms))
-        return launch_trotter_oz(wp, n, o, n_terms, sqrt_dt, E, V, win, wout, vdiv, vdiv * no, no, oz.p, oz.err, s);
+        return launch_trotter_oz(wp, n, o, n_terms, sqrt_dt, E, V, win, wout, vdiv, vdiv * no, no, oz, s);
     return launch_trotter(W, n, o, n_terms, sqrt_dt, E, V, win, wout, s, vdiv);
 }
 
@@ -1599,8 +1628,8 @@ int launch_trotter_spins(int W, int n, int o, int n_terms, double sqrt_dt, const
     const long long no = (long long)n * o;
     if (trotter_small_pays(W, n, 2 * o, n_terms))
         return launch_trotter_small(W, n, o, n_terms, sqrt_dt, E, V, win, wout, 2, no, (long long)half, s);
-    if (trotter_oz_pays(W, n, n_terms) && (long long)half == W * no && trotter_oz_whole(W, n))
-        return launch_trotter_oz(W, n, o, n_terms, sqrt_dt, E, V, win, wout, 2, no, W * no, oz.p, oz.err, s);
+    if (trotter_oz_pays(W, n, n_terms) && (long long)half == W * no && trotter_oz_whole(W, n, o, 2))
+        return launch_trotter_oz(W, n, o, n_terms, sqrt_dt, E, V, win, wout, 2, no, W * no, oz, s);
     for (int spin = 0; spin < 2; ++spin)
         AFQ_TRY(launch_trotter_auto(W, n, o, n_terms, sqrt_dt, E, V, win + spin * half, wout + spin * half, 1, oz, s));
     return AFQ_OK;
@@ -1609,7 +1638,7 @@ int launch_trotter_spins(int W, int n, int o, int n_terms, double sqrt_dt, const
 int launch_energy_partial_auto(int W, int n, int o, int G, const double2* green, const void* rot_chol, int trial_real,
                                double* partial, const OzScratch& oz, cudaStream_t s) {
     if (trial_real && energy_oz_pays(W, n, o, G))
-        return launch_energy_partial_oz(W, n, o, G, green, (const double*)rot_chol, partial, oz.p, oz.err, s);
+        return launch_energy_partial_oz(W, n, o, G, green, (const double*)rot_chol, partial, oz, s);
     return launch_energy_partial(W, n, o, G, green, rot_chol, trial_real, partial, s);
 }
 
