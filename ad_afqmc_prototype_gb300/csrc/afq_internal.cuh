@@ -540,6 +540,9 @@ int launch_taylor_adj(int W, int n, int o, int K, double sqrt_dt, const double* 
 size_t vbar_oz_scratch(int W, int n, int o, int K);
 int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms,
                    double2* vbar, const OzScratch& oz, cudaStream_t s);
+// the same on the binary64 pipe: sums that the digits do not take
+int launch_vbar(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms, double2* vbar,
+                cudaStream_t s);
 int ebar_splits(int W);
 int launch_ebar(int W, int n, int o, const double2* X, long long xs, const double2* Y, long long ys, double* partial,
                 cudaStream_t s);

@@ -155,11 +155,63 @@ int launch_taylor_adj(int W, int n, int o, int K, double sqrt_dt, const double* 
 }
 
 // =====================================================================
-// Sum of outer products over (walker, column): 32 x 32 output tiles, 256
+// Sums of outer products over (batch, column): 32 x 32 output tiles, 256
 // threads with 2 x 2 outputs each, 16 columns staged at a time.
+//   k_vbar:  Vb_w = sum_{k=1..K} conj(a/k) tb_k t_{k-1}^H     (walkers over grid.z; sums the digits do not take)
 //   k_ebar:  Eb[split] += Re sum_{w in split} X_w Y_w^H       (real, per split)
 // =====================================================================
 constexpr int OT = 32, OC = 16;
+
+__global__ void __launch_bounds__(256) k_vbar(int W, int n, int o, int K, double sqrt_dt,
+                                              const double2* __restrict__ tbar, const double2* __restrict__ terms,
+                                              double2* __restrict__ vbar) {
+    __shared__ double2 As[OC][OT + 1], Bs[OC][OT + 1];
+    const int no = n * o, i0 = blockIdx.y * OT, j0 = blockIdx.x * OT;
+    const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+    for (int w = blockIdx.z; w < W; w += gridDim.z) {
+        double2 acc[2][2] = {};
+        for (int k = 1; k <= K; ++k) {
+            const double2* X = tbar + ((size_t)w * (K + 1) + k) * no;
+            const double2* Y = terms + ((size_t)w * K + (k - 1)) * no;
+            const double c = sqrt_dt / k;  // conj(a/k) = -i c
+            for (int a0 = 0; a0 < o; a0 += OC) {
+                for (int e = threadIdx.x; e < OC * OT; e += 256) {
+                    const int r = e / OC, cc = e - r * OC;
+                    const int i = i0 + r, j = j0 + r, a = a0 + cc;
+                    const double2 x = (i < n && a < o) ? X[i * o + a] : make_double2(0.0, 0.0);
+                    As[cc][r] = make_double2(c * x.y, -c * x.x);
+                    Bs[cc][r] = (j < n && a < o) ? cconj(Y[j * o + a]) : make_double2(0.0, 0.0);
+                }
+                __syncthreads();
+                const int cn = min(OC, o - a0);
+                for (int cc = 0; cc < cn; ++cc) {
+                    const double2 a_0 = As[cc][ty], a_1 = As[cc][ty + 16];
+                    const double2 b_0 = Bs[cc][tx], b_1 = Bs[cc][tx + 16];
+                    cfma(acc[0][0], a_0, b_0); cfma(acc[0][1], a_0, b_1);
+                    cfma(acc[1][0], a_1, b_0); cfma(acc[1][1], a_1, b_1);
+                }
+                __syncthreads();
+            }
+        }
+        double2* Vb = vbar + (size_t)w * n * n;
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+            for (int c2 = 0; c2 < 2; ++c2) {
+                const int i = i0 + ty + 16 * r, j = j0 + tx + 16 * c2;
+                if (i < n && j < n) Vb[(size_t)i * n + j] = acc[r][c2];
+            }
+    }
+}
+
+int launch_vbar(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms, double2* vbar,
+                cudaStream_t s) {
+    if (W <= 0) return AFQ_OK;
+    const int t = (n + OT - 1) / OT;
+    k_vbar<<<dim3(t, t, W < 65535 ? W : 65535), 256, 0, s>>>(W, n, o, K, sqrt_dt, tbar, terms, vbar);
+    AFQ_LAUNCHED("k_vbar");
+    return AFQ_OK;
+}
 
 // X_w at X + w xs, Y_w at Y + w ys (each n x o); walkers [split*per, ...).
 __global__ void __launch_bounds__(256) k_ebar(int W, int n, int o, int per, const double2* __restrict__ X,

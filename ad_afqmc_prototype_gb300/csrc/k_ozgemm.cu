@@ -27,9 +27,9 @@
 // 4 and the last one (drained every 512) pass 2^24 only in sums of hundreds of
 // extremal digits of one sign; what truncation loses there is below 2^-45 of
 // such a sum's value and nothing otherwise.  The drained values are summed in
-// 64-bit integers (d <= 4; units of 2^-46 of the largest product, so that
-// 2^17 of them cannot overflow) and in fp32 (the last accumulator), and
-// converted once to binary64.  Rows holding inf or nan give nan.
+// 64-bit integers (d <= 4; units of 2^-46 of the largest product, which
+// leave room for the 2^62 of fewer than 2^16 of them, OZ_KMAX) and in fp32
+// (the last accumulator), and converted once to binary64.  Rows holding inf or nan give nan.
 //
 // Kernel: persistent CTAs with 128 x 64 tiles, so that all six accumulators
 // stay in tensor memory and each digit tile is read once for its 34 products.
@@ -1053,7 +1053,7 @@ ZLayout z_layout(Arena& a, int M, int N, int K) {
 //            10 140 -> 193 at 200, 1595 -> 2469 at 4096.
 //   energy   n = 8, o = 2, 40 vectors: 12 -> 24 us at 200 walkers, 64 -> 55 at 2048; n = 12, o = 6, 60 vectors: 27 ->
 //            29 at 8, 51 -> 34 at 200; n = 20, o = 5, 100 vectors: 41 -> 30 at 8, 547 -> 185 at 2048.
-bool zgemm_oz_pays(int M, int N, int K) { return M > 0 && N > 0 && K >= 1 && K <= 1 << 17 && M <= 65535 * 64; }
+bool zgemm_oz_pays(int M, int N, int K) { return M > 0 && N > 0 && K >= 1 && K <= OZ_KMAX && M <= 65535 * 64; }
 int launch_asym(int n, int G, const double* chol, int* asym, cudaStream_t s) {
     AFQ_CUDA(cudaMemsetAsync(asym, 0, sizeof(int), s));
     const int nt = (n + 31) / 32, pairs = nt * (nt + 1) / 2, gy = (152 * 8 + pairs - 1) / pairs;
@@ -1084,6 +1084,7 @@ bool energy_oz_pays(int W, int n, int o, int G) {
 }
 
 size_t zgemm_oz_scratch(int M, int N, int K) {
+    if (!zgemm_oz_pays(M, N, K)) return 0;
     Arena a;
     z_layout(a, M, N, K);
     return a.used + 256;
@@ -1493,9 +1494,12 @@ VbLayout vb_layout(Arena& a, int W, int n, int o, int K) {
 }
 }  // namespace
 
+// Where the sums are too long for the digits the adjoint's binary64 kernel (k_adjoint.cu) forms them.
+bool vbar_oz_pays(int o, int K) { return K >= 1 && 2LL * K * o <= OZ_KMAX; }
 size_t vbar_oz_scratch(int W, int n, int o, int K) {
+    if (!vbar_oz_pays(o, K)) return 0;
     Arena a;
-    vb_layout(a, W, n, o, K > 0 ? K : 1);
+    vb_layout(a, W, n, o, K);
     return a.used + 256;
 }
 
@@ -1503,10 +1507,7 @@ size_t vbar_oz_scratch(int W, int n, int o, int K) {
 int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms,
                    double2* vbar, const OzScratch& oz, cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
-    if (K == 0) {
-        AFQ_CUDA(cudaMemsetAsync(vbar, 0, sizeof(double2) * (size_t)W * n * n, s));
-        return AFQ_OK;
-    }
+    if (!vbar_oz_pays(o, K)) return launch_vbar(W, n, o, K, sqrt_dt, tbar, terms, vbar, s);
     Arena ar(oz.p, oz.bytes);
     const VbLayout v = vb_layout(ar, W, n, o, K);
     AFQ_TRY(oz_room(ar));

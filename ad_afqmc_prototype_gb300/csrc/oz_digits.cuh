@@ -7,6 +7,7 @@ namespace afq {
 
 constexpr int OZ_S = 7;             // digits
 constexpr int OZ_NAN = 0x7fffffff;  // scale of a row holding inf or nan
+constexpr int OZ_KMAX = 65535;      // longest product: below 2^16 its integer sum stays below 2^62
 
 __device__ __forceinline__ int oz_expo(double x) {  // biased binary64 exponent
     return (int)(((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ffu);
