@@ -293,6 +293,10 @@ int launch_sum_spin_blocks(int n, const double2* rdm1, double2* dm, cudaStream_t
 int launch_zgemm(int M, int N, int K, double alpha, const double2* A, int64_t lda,
                  const void* B, int64_t ldb, bool b_complex, bool b_trans, double2* C,
                  int64_t ldc, cudaStream_t s);
+// the rows of a real-B product that the digits cannot be left to (oz_digits.cuh), found on the device
+int launch_zgemm_lost(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
+                      bool b_trans, double2* C, int64_t ldc, const int* amax, const int* ex, int aexp,
+                      cudaStream_t s);
 // a real B; pays: where the digits' launches would take longer
 bool zgemm_small_pays(int M, int N, int K);
 int launch_zgemm_small(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
@@ -390,9 +394,9 @@ int launch_qr_finish(int W, int n, int o, const double2* q1, const double2* gram
 // k_green.cu
 int launch_green(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
                  double2* ovlp_out, double2* green_out, cudaStream_t s);
-// det(C^H W) per walker (not squared: the unrestricted overlap's per-spin factor)
-int launch_green_det(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,
-                     double2* det_out, double2* green_out, cudaStream_t s);
+// with det(C^H W) unsquared where !ov_square (the unrestricted overlap's per-spin factor); only (optional): the walkers it marks
+int launch_green_sq(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers, double2* ovlp_out,
+                    double2* green_out, int ov_square, cudaStream_t s, const int* only = nullptr);
 // determinants (squared: ov_square) and, with inv_out, inverses of given m (W x o x o)
 int launch_lu(int W, int o, const double2* m, double2* ovlp_out, double2* inv_out, int ov_square, cudaStream_t s);
 // either of the above, m and G_half by digits where that pays (real trial, scratch given)
@@ -400,9 +404,10 @@ int launch_green_auto(int W, int n, int o, const double2* mo, int trial_real, co
                       double2* ovlp_out, double2* green_out, int ov_square, const OzScratch& oz, cudaStream_t s);
 
 // k_walker.cu
-// vdiv walkers share each V (2: the top and bottom halves of generalized walkers)
+// vdiv walkers share each V (2: the top and bottom halves of generalized walkers); only (optional): the V's it marks
 int launch_trotter(int W, int n, int o, int n_terms, double sqrt_dt, const double* E,
-                   const double2* V, const double2* win, double2* wout, cudaStream_t s, int vdiv = 1);
+                   const double2* V, const double2* win, double2* wout, cudaStream_t s, int vdiv = 1,
+                   const int* only = nullptr);
 int launch_field_shift(int W, int G, double sqrt_dt, const double* x, const double2* fb,
                        const double2* mf, double2* xs, double2* shift_term, double2* fb_term,
                        cudaStream_t s);
@@ -540,9 +545,13 @@ int launch_taylor_adj(int W, int n, int o, int K, double sqrt_dt, const double* 
 size_t vbar_oz_scratch(int W, int n, int o, int K);
 int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms,
                    double2* vbar, const OzScratch& oz, cudaStream_t s);
-// the same on the binary64 pipe: sums that the digits do not take
+// the same on the binary64 pipe, for all walkers or those that `only` marks
 int launch_vbar(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms, double2* vbar,
-                cudaStream_t s);
+                const int* only, cudaStream_t s);
+int launch_taylor_tape_plain(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                             const double2* win, double2* terms, double2* w2, const int* only, cudaStream_t s);
+int launch_taylor_adj_plain(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                            const double2* wbar_post, double2* tbar, double2* wbar_pre, const int* only, cudaStream_t s);
 int ebar_splits(int W);
 int launch_ebar(int W, int n, int o, const double2* X, long long xs, const double2* Y, long long ys, double* partial,
                 cudaStream_t s);

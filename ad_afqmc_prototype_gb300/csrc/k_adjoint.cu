@@ -34,7 +34,9 @@ __device__ __forceinline__ void set_err(int* err, int code) {
 // =====================================================================
 __global__ void __launch_bounds__(256) k_taylor_tape(int n, int o, int K, double sqrt_dt, const double* __restrict__ E,
                                                      const double2* __restrict__ V, const double2* __restrict__ win,
-                                                     double2* __restrict__ terms, double2* __restrict__ w2) {
+                                                     double2* __restrict__ terms, double2* __restrict__ w2,
+                                                     const int* __restrict__ only) {
+    if (only && !only[blockIdx.x]) return;
     extern __shared__ double2 sm2[];
     const int w = blockIdx.x, no = n * o;
     double2* cur = sm2;
@@ -79,8 +81,14 @@ int launch_taylor_tape(int W, int n, int o, int K, double sqrt_dt, const double*
     if (smem > 227 * 1024)
         return fail(AFQ_E_UNSUPPORTED, "Taylor adjoint: norb %d x nocc %d needs %zu bytes of shared memory", n, o, smem);
     if (trotter_oz_pays(W, n, K)) return launch_taylor_tape_oz(W, n, o, K, sqrt_dt, E, V, win, terms, w2, oz, s);
+    return launch_taylor_tape_plain(W, n, o, K, sqrt_dt, E, V, win, terms, w2, nullptr, s);
+}
+
+int launch_taylor_tape_plain(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                             const double2* win, double2* terms, double2* w2, const int* only, cudaStream_t s) {
+    const size_t smem = 2 * sizeof(double2) * (size_t)n * o;
     AFQ_TRY(allow_smem(k_taylor_tape, smem));
-    k_taylor_tape<<<W, 256, smem, s>>>(n, o, K, sqrt_dt, E, V, win, terms, w2);
+    k_taylor_tape<<<W, 256, smem, s>>>(n, o, K, sqrt_dt, E, V, win, terms, w2, only);
     AFQ_LAUNCHED("k_taylor_tape");
     return AFQ_OK;
 }
@@ -94,7 +102,9 @@ int launch_taylor_tape(int W, int n, int o, int K, double sqrt_dt, const double*
 // =====================================================================
 __global__ void __launch_bounds__(256) k_taylor_adj(int n, int o, int K, double sqrt_dt, const double* __restrict__ E,
                                                     const double2* __restrict__ V, const double2* wbar_post,
-                                                    double2* __restrict__ tbar, double2* wbar_pre) {
+                                                    double2* __restrict__ tbar, double2* wbar_pre,
+                                                    const int* __restrict__ only) {
+    if (only && !only[blockIdx.x]) return;
     extern __shared__ double2 sm2[];
     const int w = blockIdx.x, no = n * o;
     double2* cur = sm2;
@@ -148,8 +158,14 @@ int launch_taylor_adj(int W, int n, int o, int K, double sqrt_dt, const double* 
         return fail(AFQ_E_UNSUPPORTED, "Taylor adjoint: norb %d x nocc %d needs %zu bytes of shared memory", n, o, smem);
     if (trotter_oz_pays(W, n, K))
         return launch_taylor_adj_oz(W, n, o, K, sqrt_dt, E, V, wbar_post, tbar, wbar_pre, oz, s);
+    return launch_taylor_adj_plain(W, n, o, K, sqrt_dt, E, V, wbar_post, tbar, wbar_pre, nullptr, s);
+}
+
+int launch_taylor_adj_plain(int W, int n, int o, int K, double sqrt_dt, const double* E, const double2* V,
+                            const double2* wbar_post, double2* tbar, double2* wbar_pre, const int* only, cudaStream_t s) {
+    const size_t smem = 2 * sizeof(double2) * (size_t)n * o;
     AFQ_TRY(allow_smem(k_taylor_adj, smem));
-    k_taylor_adj<<<W, 256, smem, s>>>(n, o, K, sqrt_dt, E, V, wbar_post, tbar, wbar_pre);
+    k_taylor_adj<<<W, 256, smem, s>>>(n, o, K, sqrt_dt, E, V, wbar_post, tbar, wbar_pre, only);
     AFQ_LAUNCHED("k_taylor_adj");
     return AFQ_OK;
 }
@@ -157,18 +173,19 @@ int launch_taylor_adj(int W, int n, int o, int K, double sqrt_dt, const double* 
 // =====================================================================
 // Sums of outer products over (batch, column): 32 x 32 output tiles, 256
 // threads with 2 x 2 outputs each, 16 columns staged at a time.
-//   k_vbar:  Vb_w = sum_{k=1..K} conj(a/k) tb_k t_{k-1}^H     (walkers over grid.z; sums the digits do not take)
+//   k_vbar:  Vb_w = sum_{k=1..K} conj(a/k) tb_k t_{k-1}^H     (walkers over grid.z; those and the sums that the digits do not take)
 //   k_ebar:  Eb[split] += Re sum_{w in split} X_w Y_w^H       (real, per split)
 // =====================================================================
 constexpr int OT = 32, OC = 16;
 
 __global__ void __launch_bounds__(256) k_vbar(int W, int n, int o, int K, double sqrt_dt,
                                               const double2* __restrict__ tbar, const double2* __restrict__ terms,
-                                              double2* __restrict__ vbar) {
+                                              double2* __restrict__ vbar, const int* __restrict__ only) {
     __shared__ double2 As[OC][OT + 1], Bs[OC][OT + 1];
     const int no = n * o, i0 = blockIdx.y * OT, j0 = blockIdx.x * OT;
     const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
     for (int w = blockIdx.z; w < W; w += gridDim.z) {
+        if (only && !only[w]) continue;
         double2 acc[2][2] = {};
         for (int k = 1; k <= K; ++k) {
             const double2* X = tbar + ((size_t)w * (K + 1) + k) * no;
@@ -205,10 +222,10 @@ __global__ void __launch_bounds__(256) k_vbar(int W, int n, int o, int K, double
 }
 
 int launch_vbar(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms, double2* vbar,
-                cudaStream_t s) {
+                const int* only, cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
     const int t = (n + OT - 1) / OT;
-    k_vbar<<<dim3(t, t, W < 65535 ? W : 65535), 256, 0, s>>>(W, n, o, K, sqrt_dt, tbar, terms, vbar);
+    k_vbar<<<dim3(t, t, W < 65535 ? W : 65535), 256, 0, s>>>(W, n, o, K, sqrt_dt, tbar, terms, vbar, only);
     AFQ_LAUNCHED("k_vbar");
     return AFQ_OK;
 }

@@ -6,6 +6,7 @@
 // so the kernel is a register-blocked SIMT GEMM: 64x64 tile, 4x4 complex
 // outputs per thread, K staged through shared memory 16 at a time.
 #include "afq_internal.cuh"
+#include "oz_digits.cuh"
 
 namespace afq {
 
@@ -24,25 +25,17 @@ __device__ __forceinline__ void load_b(double& dst, const double* p, bool ok) { 
 __device__ __forceinline__ void load_b(double2& dst, const double2* p, bool ok) { dst = ok ? *p : zero2(); }
 __device__ __forceinline__ void mac(double2& acc, double2 a, double b) { rfma(acc, b, a); }
 __device__ __forceinline__ void mac(double2& acc, double2 a, double2 b) { cfma(acc, a, b); }
-}  // namespace
 
-// grid.z > 1 (split K): CTA layer z sums k in [z kc, min(K, (z + 1) kc)) into
-// C + z cs (the caller adds the layers in a fixed order).
+// One 64 x 64 tile by 256 threads, sums over k in [kbeg, kend).
 template <bool BC, bool BT>
-__global__ void __launch_bounds__(256) k_zgemm(int M, int N, int K, double alpha,
-                                               const double2* __restrict__ A, int64_t lda,
-                                               const void* __restrict__ Bv, int64_t ldb,
-                                               double2* __restrict__ C, int64_t ldc, int kc, int64_t cs) {
+__device__ __forceinline__ void zgemm_tile(int M, int N, int kbeg, int kend, double alpha, const double2* __restrict__ A,
+                                           int64_t lda, const typename BElem<BC>::T* __restrict__ B, int64_t ldb,
+                                           double2* __restrict__ C, int64_t ldc, int m0, int n0) {
     using TB = typename BElem<BC>::T;
-    const TB* B = (const TB*)Bv;
-    const int kbeg = blockIdx.z * kc;
-    const int kend = min(K, kbeg + kc);
-    C += (int64_t)blockIdx.z * cs;
     __shared__ double2 As[BK][BM + 1];
     __shared__ TB Bs[BK][BN + 1];
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
 
     double2 acc[4][4];
 #pragma unroll
@@ -103,6 +96,60 @@ __global__ void __launch_bounds__(256) k_zgemm(int M, int N, int K, double alpha
             if (gn < N) C[(int64_t)gm * ldc + gn] = cscale(acc[i][j], alpha);
         }
     }
+}
+}  // namespace
+
+// grid.z > 1 (split K): CTA layer z sums k in [z kc, min(K, (z + 1) kc)) into
+// C + z cs (the caller adds the layers in a fixed order).
+template <bool BC, bool BT>
+__global__ void __launch_bounds__(256) k_zgemm(int M, int N, int K, double alpha,
+                                               const double2* __restrict__ A, int64_t lda,
+                                               const void* __restrict__ Bv, int64_t ldb,
+                                               double2* __restrict__ C, int64_t ldc, int kc, int64_t cs) {
+    const int kbeg = blockIdx.z * kc;
+    zgemm_tile<BC, BT>(M, N, kbeg, min(K, kbeg + kc), alpha, A, lda, (const typename BElem<BC>::T*)Bv, ldb,
+                       C + (int64_t)blockIdx.z * cs, ldc, blockIdx.y * BM, blockIdx.x * BN);
+}
+
+// The rows of C (tiles of 64) among which the digits (scales ex of the rows' parts) lost too much (oz_lost).  A CTA checks its tile's rows and, mostly,
+// ends.
+template <bool BT>
+__global__ void __launch_bounds__(256) k_zgemm_lost(int M, int N, int K, double alpha, const double2* __restrict__ A,
+                                                    int64_t lda, const double* __restrict__ B, int64_t ldb,
+                                                    double2* __restrict__ C, int64_t ldc, const int* __restrict__ amax,
+                                                    const int* __restrict__ ex, int aexp) {
+    const int m0 = blockIdx.y * BM, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // eight rows a warp: mostly one of a row's first 32 results tells that it is sound
+    constexpr int R = BM / 8;
+    int key[R], bmax[R];
+    bool lost = false;
+    const int am = *amax;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int m = min(m0 + R * wid + r, M - 1);
+        key[r] = lane < N ? oz_key(C[(int64_t)m * ldc + lane]) : 0;
+        bmax[r] = max(ex[2 * m], ex[2 * m + 1]);
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const int m = min(m0 + R * wid + r, M - 1), bm = bmax[r], to = oz_reach(am, bm);
+        const bool any = __any_sync(0xffffffffu, oz_key_expo(key[r]) - aexp >= to);
+        lost = lost || oz_lost(am, bm, any || oz_scan(C + (int64_t)m * ldc, N, to == OZ_NAN ? to : to + aexp));
+    }
+    if (!__syncthreads_or(lost)) return;
+    for (int n0 = blockIdx.x * BN; n0 < N; n0 += gridDim.x * BN)
+        zgemm_tile<false, BT>(M, N, 0, K, alpha, A, lda, B, ldb, C, ldc, m0, n0);
+}
+
+int launch_zgemm_lost(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
+                      bool b_trans, double2* C, int64_t ldc, const int* amax, const int* ex, int aexp,
+                      cudaStream_t s) {
+    const int mt = (M + BM - 1) / BM, nt = (N + BN - 1) / BN, per = 304 / mt;  // two CTAs an SM
+    const dim3 grid(per < 1 ? 1 : per < nt ? per : nt, mt);
+    if (b_trans) k_zgemm_lost<true><<<grid, 256, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, C, ldc, amax, ex, aexp);
+    else k_zgemm_lost<false><<<grid, 256, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, C, ldc, amax, ex, aexp);
+    AFQ_LAUNCHED("k_zgemm_lost");
+    return AFQ_OK;
 }
 
 int launch_zgemm(int M, int N, int K, double alpha, const double2* A, int64_t lda, const void* B,

@@ -14,7 +14,8 @@
 //
 // k_green<., INV = false> (overlaps only) skips the rows that are done.
 // Where m and G_half are large products of their own they go by digits on
-// the tensor cores (launch_green_oz) and this kernel only factorises.
+// the tensor cores (launch_green_oz) and this kernel only factorises.  only
+// (optional): the walkers it marks.
 #include "afq_internal.cuh"
 
 namespace afq {
@@ -50,7 +51,9 @@ template <int NE, bool CR, bool INV>
 __global__ void __launch_bounds__(GR_T) k_green(int n, int o, const double2* __restrict__ mo,
                                                 const double2* __restrict__ walkers, const double2* __restrict__ m_in,
                                                 double2* __restrict__ ovlp_out, double2* __restrict__ green_out,
-                                                double2* __restrict__ inv_out, int ov_square) {
+                                                double2* __restrict__ inv_out, int ov_square,
+                                                const int* __restrict__ only) {
+    if (only && !only[blockIdx.x]) return;
     extern __shared__ double2 sm[];
     __shared__ double2 s_col[2][64], s_row[64], s_piv[64];
     __shared__ unsigned long long s_key[2][64];
@@ -216,22 +219,22 @@ __global__ void __launch_bounds__(GR_T) k_green(int n, int o, const double2* __r
 
 template <int NE, bool CR, bool INV>
 int run(int W, int n, int o, const double2* mo, const double2* walkers, const double2* m_in, double2* ovlp_out,
-        double2* green_out, double2* inv_out, int ov_square, cudaStream_t s) {
+        double2* green_out, double2* inv_out, int ov_square, cudaStream_t s, const int* only) {
     static DeviceOnce once;
     const size_t wp = o | 1, stage = m_in ? 0 : GR_IC * wp * (sizeof(double2) + (CR ? sizeof(double) : sizeof(double2)));
     const size_t gsm = green_out ? ((size_t)o * o + GR_IC * wp) * sizeof(double2) : 0;
     const size_t smem = stage > gsm ? stage : gsm;
     AFQ_TRY(raise_smem_once(once, k_green<NE, CR, INV>, (64 * 64 + GR_IC * 65) * (int)sizeof(double2)));
-    k_green<NE, CR, INV><<<W, GR_T, smem, s>>>(n, o, mo, walkers, m_in, ovlp_out, green_out, inv_out, ov_square);
+    k_green<NE, CR, INV><<<W, GR_T, smem, s>>>(n, o, mo, walkers, m_in, ovlp_out, green_out, inv_out, ov_square, only);
     AFQ_LAUNCHED("k_green");
     return AFQ_OK;
 }
 template <bool CR, bool INV>
 int run_ne(int W, int n, int o, const double2* mo, const double2* walkers, const double2* m_in, double2* ovlp_out,
-           double2* green_out, double2* inv_out, int ov_square, cudaStream_t s) {
+           double2* green_out, double2* inv_out, int ov_square, cudaStream_t s, const int* only = nullptr) {
     const int ne = (o * o + GR_T - 1) / GR_T;
 #define AFQ_GR(NE) \
-    if (ne <= NE) return run<NE, CR, INV>(W, n, o, mo, walkers, m_in, ovlp_out, green_out, inv_out, ov_square, s)
+    if (ne <= NE) return run<NE, CR, INV>(W, n, o, mo, walkers, m_in, ovlp_out, green_out, inv_out, ov_square, s, only)
     AFQ_GR(1);
     AFQ_GR(2);
     AFQ_GR(4);
@@ -253,24 +256,19 @@ int launch_lu(int W, int o, const double2* m, double2* ovlp_out, double2* inv_ou
 }
 
 int launch_green_sq(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers, double2* ovlp_out,
-                    double2* green_out, int ov_square, cudaStream_t s) {
+                    double2* green_out, int ov_square, cudaStream_t s, const int* only) {
     if (W <= 0) return AFQ_OK;
     if (trial_real) {
-        if (green_out) return run_ne<true, true>(W, n, o, mo, walkers, nullptr, ovlp_out, green_out, nullptr, ov_square, s);
-        return run_ne<true, false>(W, n, o, mo, walkers, nullptr, ovlp_out, nullptr, nullptr, ov_square, s);
+        if (green_out) return run_ne<true, true>(W, n, o, mo, walkers, nullptr, ovlp_out, green_out, nullptr, ov_square, s, only);
+        return run_ne<true, false>(W, n, o, mo, walkers, nullptr, ovlp_out, nullptr, nullptr, ov_square, s, only);
     }
-    if (green_out) return run_ne<false, true>(W, n, o, mo, walkers, nullptr, ovlp_out, green_out, nullptr, ov_square, s);
-    return run_ne<false, false>(W, n, o, mo, walkers, nullptr, ovlp_out, nullptr, nullptr, ov_square, s);
+    if (green_out) return run_ne<false, true>(W, n, o, mo, walkers, nullptr, ovlp_out, green_out, nullptr, ov_square, s, only);
+    return run_ne<false, false>(W, n, o, mo, walkers, nullptr, ovlp_out, nullptr, nullptr, ov_square, s, only);
 }
 
 int launch_green(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers, double2* ovlp_out,
                  double2* green_out, cudaStream_t s) {
     return launch_green_sq(W, n, o, mo, trial_real, walkers, ovlp_out, green_out, 1, s);
-}
-
-int launch_green_det(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers, double2* det_out,
-                     double2* green_out, cudaStream_t s) {
-    return launch_green_sq(W, n, o, mo, trial_real, walkers, det_out, green_out, 0, s);
 }
 
 int launch_green_auto(int W, int n, int o, const double2* mo, int trial_real, const double2* walkers,

@@ -29,7 +29,16 @@
 // such a sum's value and nothing otherwise.  The drained values are summed in
 // 64-bit integers (d <= 4; units of 2^-46 of the largest product, which
 // leave room for the 2^62 of fewer than 2^16 of them, OZ_KMAX) and in fp32
-// (the last accumulator), and converted once to binary64.  Rows holding inf or nan give nan.
+// (the last accumulator), and converted once to binary64.
+//
+// A product is held to its operands' largest entries, where a binary64 chain's
+// error goes with the terms.  So each is checked by its results (oz_lost in
+// oz_digits.cuh) and, where those are too small for that (or with inf and nan),
+// formed again on the binary64 pipe: k_zgemm_lost's tiles, the walkers marked for
+// k_trotter, k_green and the adjoint's kernels, k_oz_exchange's blocks by itself.
+// Where all is sound, which the first 32 results mostly tell, that costs a launch
+// of 3-4 us a product: a step of 30 orbitals and 200 walkers 144 -> 153 us, of 120 x
+// 20, 600 vectors and 2048 walkers 5.43 -> 5.51 ms.
 //
 // Kernel: persistent CTAs with 128 x 64 tiles, so that all six accumulators
 // stay in tensor memory and each digit tile is read once for its 34 products.
@@ -96,6 +105,8 @@ struct OzOut {
     long long bs, ms1, ms0, rs;
     int md, aexp;
     const double2* add;
+    const int* skip;  // blocks m / md whose walker (m / md / sd) % sm it marks are not written
+    int sd, sm;
 };
 
 struct OzArgs {
@@ -234,8 +245,8 @@ __device__ __forceinline__ void oz_stage(int P, uint32_t smem, uint32_t tmem, in
     oz_commit(smem + OZ_BAR0 + 8 * (OZB_EB + P));
 }
 
-// SYM: the real operand's rows may be those of symmetric vectors (sym_blocks.cuh).
-template <bool SYM>
+// SYM: the real operand's rows may be those of symmetric vectors (sym_blocks.cuh).  SKIP: out.skip is looked at.
+template <bool SYM, bool SKIP>
 __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
     extern __shared__ uint8_t smem_raw[];
     const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -427,6 +438,7 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
                     const int mh = a.out.md == 1 ? m : m / a.out.md;
                     const long long e = at + (long long)mh * a.out.ms1 + (long long)(m - mh * a.out.md) * a.out.ms0;
                     if (a.out.add) v = cadd(v, a.out.add[e]);
+                    if (SKIP && a.out.skip[mh / a.out.sd % a.out.sm]) continue;
                     a.out.C[e] = v;
                     if (SYM && mirror) a.out.C[e + mirror] = v;
                 }
@@ -543,13 +555,15 @@ __device__ __forceinline__ int row_max(int e, int* s_max) {
 // Real rows with K contiguous (row r at src + r ld), LN threads a row: a lane
 // cuts eight entries, so a warp takes four rows of up to 64 entries, and a CTA
 // takes one where rows are few and long.  `per` rows a batch; one: minus the
-// identity.  Every split writes zeros from K up to a multiple of 32.
-template <int LN>
+// identity.  Every split writes zeros from K up to a multiple of 32.  AMAX: of
+// one batch, whose largest scale amax is raised to.
+template <int LN, bool AMAX>
 __global__ void __launch_bounds__(256) k_oz_rows(long long rows, int per, int K, const double* __restrict__ src,
-                                                 long long ld, int one, OzDst dst, int* __restrict__ ex) {
+                                                 long long ld, int one, OzDst dst, int* __restrict__ ex, int* amax) {
     __shared__ int s_max[8];
     const int t = threadIdx.x % LN;  // place in the row's threads
     constexpr int RC = 256 / LN;     // rows a CTA
+    int most = OZ_EMPTY;
     // every thread of a warp stays for the shuffles
     for (long long r0 = (long long)blockIdx.x * RC; r0 < rows; r0 += (long long)gridDim.x * RC) {
         const long long r = r0 + threadIdx.x / LN;
@@ -559,11 +573,12 @@ __global__ void __launch_bounds__(256) k_oz_rows(long long rows, int per, int K,
         int e = 0;
         if (in) {
 #pragma unroll 4
-            for (int k = t; k < K; k += LN) e = max(e, oz_expo(k == rd ? x[k] - 1.0 : x[k]));
+            for (int k = t; k < K; k += LN) e = max(e, oz_key(k == rd ? x[k] - 1.0 : x[k]));
         }
         const int E = oz_scale(row_max<LN>(e, s_max));
         if (!in) continue;
         if (t == 0) ex[r] = E;
+        if (AMAX) most = max(most, E);
         const long long b = r / per;
         for (int k = 8 * t; k < 32 * dst.nks; k += 8 * LN) {
             long long y[8];
@@ -572,14 +587,20 @@ __global__ void __launch_bounds__(256) k_oz_rows(long long rows, int per, int K,
             oz_store8(dst, b, (int)(r - b * per), k, y);
         }
     }
+    if (AMAX) {
+        most = __reduce_max_sync(0xffffffffu, most);
+        if ((threadIdx.x & 31) == 0) atomicMax(amax, most);
+    }
 }
 
 // Complex rows with K contiguous: digit rows 2 r (real parts) and 2 r + 1.
+// amax (optional): set for the other operand's cut to raise.
 template <int LN>
 __global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const double2* __restrict__ src, long long ld,
-                                                  OzDst dst, int* __restrict__ ex) {
+                                                  OzDst dst, int* __restrict__ ex, int* __restrict__ amax) {
     __shared__ int s_max[2][8];
     const int t = threadIdx.x % LN;
+    if (amax && blockIdx.x == 0 && threadIdx.x == 0) *amax = OZ_EMPTY;
     for (long long r = (long long)blockIdx.x * (256 / LN) + threadIdx.x / LN; r < rows;
          r += (long long)gridDim.x * (256 / LN)) {
         const double2* x = src + r * ld;
@@ -587,8 +608,8 @@ __global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const d
 #pragma unroll 4
         for (int k = t; k < K; k += LN) {
             const double2 v = x[k];
-            e0 = max(e0, oz_expo(v.x));
-            e1 = max(e1, oz_expo(v.y));
+            e0 = max(e0, oz_key(v.x));
+            e1 = max(e1, oz_key(v.y));
         }
         const int E0 = oz_scale(row_max<LN>(e0, s_max[0])), E1 = oz_scale(row_max<LN>(e1, s_max[1]));
         if (t == 0) {
@@ -614,10 +635,10 @@ __global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const d
 // would leave SMs idle), transposed through shared memory.
 template <int RB>
 __global__ void __launch_bounds__(256) k_oz_cols(int nrows, int K, const double* __restrict__ src, long long ld, int es,
-                                                 OzDst dst, int* __restrict__ ex, SymRows sym) {
+                                                 OzDst dst, int* __restrict__ ex, SymRows sym, int* amax) {
     constexpr int TY = 256 / RB, KT = 8 * TY;  // threads a row; k at a time
     __shared__ double tile[RB][KT + 1];
-    __shared__ int se[RB];
+    __shared__ int se[RB], s_most;
     const int tx = threadIdx.x % RB, ty = threadIdx.x / RB, r0 = blockIdx.x * RB;
     const bool sy = sym_on(sym);
     const int rows = sym_rows(sym, sy, nrows);
@@ -632,16 +653,20 @@ __global__ void __launch_bounds__(256) k_oz_cols(int nrows, int K, const double*
         at += sym.r0;
     }
     if (threadIdx.x < RB) se[threadIdx.x] = 0;
+    if (threadIdx.x == 0) s_most = OZ_EMPTY;
     __syncthreads();
     int e = 0;
     if (in) {
 #pragma unroll 8
-        for (int k = ty; k < K; k += TY) e = max(e, oz_expo(src[(long long)k * ld + at]));
+        for (int k = ty; k < K; k += TY) e = max(e, oz_key(src[(long long)k * ld + at]));
     }
     atomicMax(&se[tx], e);
     __syncthreads();
     const int rr = threadIdx.x / TY, kq = (threadIdx.x % TY) * 8, E = oz_scale(se[rr]);
-    if (threadIdx.x % TY == 0 && r0 + rr < rows) ex[r0 + rr] = E;
+    if (threadIdx.x % TY == 0 && r0 + rr < rows) {
+        ex[r0 + rr] = E;
+        atomicMax(&s_most, E);
+    }
     for (int k0 = 0; k0 < 32 * dst.nks; k0 += KT) {
         __syncthreads();
 #pragma unroll
@@ -657,6 +682,7 @@ __global__ void __launch_bounds__(256) k_oz_cols(int nrows, int K, const double*
             oz_store8(dst, 0, r0 + rr, k0 + kq, y);
         }
     }
+    if (amax && threadIdx.x == 0) atomicMax(amax, s_most);  // every row's is in: the loop above has barriers
 }
 
 // Walker-shaped blocks (j, c), c fastest, `ws` entries apart, eight columns c
@@ -672,13 +698,19 @@ __global__ void __launch_bounds__(256) k_oz_cols(int nrows, int K, const double*
 //   COLS  as WALK, a batch a walker (both operands of its Gram matrix)
 //   BACK  T = U - i s Y; digits of T as the right operand of V T
 //   BACKL T = U = U - i s Y; digits of U as WALK's
-// tp (optional): T also there, tw entries a walker apart.
+// tp (optional): T also there, tw entries a walker apart.  mx.p (optional):
+// raised, at the walker (w / mx.div) % mx.mod, to the largest scale of the cut
+// entries times 2^mx.add.
+struct OzMax {
+    int *p, div, mod, add;
+};
 enum { OZ_WALK, OZ_PLAIN, OZ_INIT, OZ_TERM, OZ_LAST, OZ_COLS, OZ_BACK, OZ_BACKL };
 constexpr int OZ_CB = 8;
 template <int MODE>
-__global__ void __launch_bounds__(256) k_oz_term(int n, int o, int on, long long ws, long long ss, int ncg, double s, const double2* __restrict__ Y,
+__global__ void __launch_bounds__(256, MODE == OZ_WALK || MODE == OZ_LAST || MODE == OZ_COLS || MODE == OZ_BACKL ? 4 : 3)
+    k_oz_term(int n, int o, int on, long long ws, long long ss, int ncg, double s, const double2* __restrict__ Y,
                                                  const double2* __restrict__ W, double2* __restrict__ U, OzDst dst, int* __restrict__ ex,
-                                                 double2* __restrict__ tp, long long tw) {
+                                                 double2* __restrict__ tp, long long tw, OzMax mx) {
     constexpr bool SERIES = MODE == OZ_INIT || MODE == OZ_TERM || MODE == OZ_LAST || MODE == OZ_BACK || MODE == OZ_BACKL;
     extern __shared__ double2 sh[];  // OZ_CB x (n + 1)
     __shared__ int se[2 * OZ_CB];
@@ -706,14 +738,18 @@ __global__ void __launch_bounds__(256) k_oz_term(int n, int o, int on, long long
             }
             if (SERIES && MODE != OZ_LAST && tp) tp[w * tw + (long long)j * on + c0 + c] = t;
             sh[c * pitch + j] = t;
-            e0 = max(e0, oz_expo(t.x));
-            e1 = max(e1, oz_expo(t.y));
+            e0 = max(e0, oz_key(t.x));
+            e1 = max(e1, oz_key(t.y));
         }
     }
     atomicMax(&se[2 * c], e0);
     atomicMax(&se[2 * c + 1], e1);
     __syncthreads();
     const int cn = min(OZ_CB, o - c0);
+    if (MODE != OZ_COLS && MODE != OZ_PLAIN && mx.p && tid < 32) {
+        const int E = oz_scale(__reduce_max_sync(0xffffffffu, tid < 2 * cn ? se[tid] : 0));
+        if (tid == 0) atomicMax(mx.p + w / mx.div % mx.mod, E == OZ_NAN || E == OZ_ZERO ? E : E + mx.add);
+    }
     if (MODE == OZ_WALK || MODE == OZ_LAST || MODE == OZ_COLS || MODE == OZ_BACKL) {
         const int nq = 4 * dst.nks;
         for (int it = tid; it < cn * nq; it += 256) {
@@ -798,7 +834,7 @@ __global__ void __launch_bounds__(256) k_oz_vbar(int W, int n, int o, int K, dou
         int e = 0;
         for (int l = t; in && l < L; l += LN) {
             const double2 v = at(l);
-            e = max(e, max(oz_expo(v.x), oz_expo(v.y)));
+            e = max(e, max(oz_key(v.x), oz_key(v.y)));
         }
         const int E = oz_scale(row_max<LN>(e, nullptr));
         if (!in) continue;
@@ -827,18 +863,36 @@ __global__ void __launch_bounds__(256) k_oz_vbar(int W, int n, int o, int K, dou
     }
 }
 
+__device__ __forceinline__ int warp_max(const int* x, int n) {
+    int m = OZ_EMPTY;
+    for (int i = threadIdx.x & 31; i < n; i += 32) m = max(m, x[i]);
+    return __reduce_max_sync(0xffffffffu, m);
+}
+
 // Coulomb and exchange partials of a chunk of ng Cholesky vectors from F
 // (rows (w, k), columns (g, i): f_g[i, k]), as launch_energy_partial's:
 // partial[w, chunk] = (sum_g (tr f_g)^2, sum_g sum_ik f_g[i, k] f_g[k, i]).
-// Its floor is the binary64 pipe: four FMAs a pair i < k.
-__global__ void __launch_bounds__(256) k_oz_exchange(int o, int G, int NG, const double2* __restrict__ F,
-                                                     double2* __restrict__ partial) {
+// Its floor is the binary64 pipe: four FMAs a pair i < k.  F's blocks are
+// checked (oz_lost; scales ea of L~'s rows (g, i) and eb of G_half's) and, where
+// they have lost too much, formed here from L~ and G_half.
+__global__ void __launch_bounds__(256) k_oz_exchange(int n, int o, int G, int NG, const double2* __restrict__ F,
+                                                     double2* __restrict__ partial, const int* __restrict__ ea,
+                                                     const int* __restrict__ eb,
+                                                     const double* __restrict__ rot, const double2* __restrict__ green) {
     extern __shared__ double2 sh[];  // NG blocks of o x (o + 1)
     const int nchunk = gridDim.x, w = blockIdx.y, g0 = blockIdx.x * NG, ng = min(NG, G - g0), tid = threadIdx.x;
     const int lane = tid & 31, wid = tid >> 5;
     const int pitch = o + 1, gi = ng * o;
     const double2* Fw = F + (long long)w * o * G * o + (long long)g0 * o;
     const float io = 1.0f / o;  // quotients of small integers below: (x + 0.5) / o is never within rounding of an integer
+    __shared__ int s_max[2];
+    if (wid == 7) {  // which mostly has no column below
+        const int am = warp_max(ea + g0 * o, gi), bm = warp_max(eb + (long long)w * 2 * o, 2 * o);
+        if (lane == 0) {
+            s_max[0] = am;
+            s_max[1] = bm;
+        }
+    }
     for (int x = tid; x < gi; x += 256) {
         const int g = (int)((x + 0.5f) * io), i = x - g * o;
         const double2* src = Fw + x;
@@ -847,6 +901,26 @@ __global__ void __launch_bounds__(256) k_oz_exchange(int o, int G, int NG, const
         for (int k = 0; k < o; ++k) dst[k * pitch] = src[(long long)k * G * o];
     }
     __syncthreads();
+    const int am = s_max[0], bm = s_max[1];
+    const int reach = oz_reach(am, bm);
+    bool lost = oz_lost(am, bm, oz_scan(sh, pitch - 1, reach));  // a row of the first block tells enough, mostly
+    if (lost) {
+        bool any = false;
+        for (int x = tid; x < gi; x += 256)
+            for (int k = 0; k < o; ++k) any |= oz_key_expo(oz_key(sh[(x / o * o + k) * pitch + x % o])) >= reach;
+        lost = oz_lost(am, bm, __syncthreads_or(any));
+    }
+    if (lost) {
+        for (int e = tid; e < gi * o; e += 256) {
+            const int k = e / gi, x = e - k * gi, g = x / o;
+            const double* l = rot + ((long long)g0 * o + x) * n;
+            const double2* gk = green + ((long long)w * o + k) * n;
+            double2 f = make_double2(0.0, 0.0);
+            for (int j = 0; j < n; ++j) rfma(f, l[j], gk[j]);
+            sh[(g * o + k) * pitch + x - g * o] = f;
+        }
+        __syncthreads();
+    }
     double cr = 0.0, ci = 0.0, xr = 0.0, xi = 0.0;
     // sum over i < k of f[i, k] f[k, i], doubled below, a warp a vector: rows k = r and o - 1 - r hold o - 1 such pairs
     // together (the middle row of an odd o half of that)
@@ -887,8 +961,50 @@ __global__ void __launch_bounds__(256) k_oz_exchange(int o, int G, int NG, const
     }
 }
 
+// flag[w]: one of walker w's two products (at most) has lost too much (oz_lost): scales of its `rows` rows (shared: of
+// all) and `cols` columns, its `results` results.  A warp a walker.
+struct OzWalk {
+    const int *a, *b;
+    const double2* c;
+    int results, rows, cols, shared;
+};
+__global__ void __launch_bounds__(128) k_oz_flags(int W, OzWalk g, OzWalk h, int* __restrict__ flag) {
+    const int w = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (w >= W) return;
+    auto lost = [&](const OzWalk& p) {
+        if (!p.c) return false;
+        const int a = warp_max(p.a + (p.shared ? 0 : (long long)w * p.rows), p.rows);
+        const int b = warp_max(p.b + (long long)w * p.cols, p.cols);
+        return oz_lost(a, b, oz_scan(p.c + (long long)w * p.results, p.results, oz_reach(a, b)));
+    };
+    const bool l = lost(g) || lost(h);
+    if ((threadIdx.x & 31) == 0) flag[w] = l;
+}
+
+// The same of a Taylor series, whose products are to be judged by its sum U (E_half X and its last product are X + (E -
+// I) X): largest scales of E - I (e) and X, of the terms times their coefficients (t), of U (u), and those of V's n rows.
+struct OzSeries {
+    int *e, *x, *t, *u, *flag;
+};
+__global__ void __launch_bounds__(128) k_oz_series_flags(int W, int n, OzSeries g, const int* __restrict__ v) {
+    const int w = blockIdx.x * 4 + (threadIdx.x >> 5);
+    if (w >= W) return;
+    const int a = warp_max(v + (long long)w * n, n);
+    if ((threadIdx.x & 31) != 0) return;
+    auto lost = [&](int a, int b) { return oz_lost(a, b, g.u[w] - 1 >= oz_reach(a, b)); };
+    g.flag[w] = lost(*g.e, g.x[w]) || lost(a, g.t[w]);
+}
+
 constexpr int OZ_XSMEM = 96 * 1024;  // the exchange kernel's F blocks
-DeviceOnce g_oz, g_ozsym, g_ozterm[8], g_ozx;
+DeviceOnce g_ozterm[8], g_ozx;
+template <bool SYM, bool SKIP>
+int run_ozgemm(const OzArgs& a, int grid, cudaStream_t s) {
+    static DeviceOnce once;
+    AFQ_TRY(raise_smem_once(once, k_ozgemm<SYM, SKIP>, OZ_GSMEM));
+    k_ozgemm<SYM, SKIP><<<grid, OZ_GT, OZ_GSMEM, s>>>(a);
+    AFQ_LAUNCHED("k_ozgemm");
+    return AFQ_OK;
+}
 
 int nks_of(int K) { return (K + OZ_BK - 1) / OZ_BK; }
 long long digit_row_bytes(int K) { return 64LL * OZ_S * nks_of(K); }
@@ -931,14 +1047,9 @@ int oz_launch(int rows, int cols, int K, int batch, int adiv, const OzDigits& A,
     const long long tiles = (long long)mt * nt * batch * splits;
     if (tiles > 0x7fffffffLL) return fail(AFQ_E_UNSUPPORTED, "digit GEMM: %lld tiles", tiles);
     const int grid = tiles < sms ? (int)tiles : sms;
-    if (sym.asym) {
-        AFQ_TRY(raise_smem_once(g_ozsym, k_ozgemm<true>, OZ_GSMEM));
-        k_ozgemm<true><<<grid, OZ_GT, OZ_GSMEM, s>>>(a);
-    } else {
-        AFQ_TRY(raise_smem_once(g_oz, k_ozgemm<false>, OZ_GSMEM));
-        k_ozgemm<false><<<grid, OZ_GT, OZ_GSMEM, s>>>(a);
-    }
-    AFQ_LAUNCHED("k_ozgemm");
+    if (sym.asym) AFQ_TRY((run_ozgemm<true, false>(a, grid, s)));
+    else if (out.skip) AFQ_TRY((run_ozgemm<false, true>(a, grid, s)));
+    else AFQ_TRY((run_ozgemm<false, false>(a, grid, s)));
     if (splits > 1) {
         long long blocks = ((long long)rows * (cols >> 1) + 255) / 256;
         if (blocks > 152 * 16) blocks = 152 * 16;
@@ -957,26 +1068,34 @@ unsigned row_blocks(long long rows, int per_cta = 8) {
 // A warp a row leaves SMs idle below some 16 warps an SM; a row of a few hundred k is short for a CTA.
 bool row_cta(long long rows, int K) { return rows < 16 * 152 && K >= 512; }
 int split_rows(long long rows, int per, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s,
-               int one = 0) {
+               int* amax = nullptr, int one = 0) {
     const OzDst dst = dst_of(D, per, K);
-    if (row_cta(rows, K)) k_oz_rows<256><<<row_blocks(rows, 1), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
-    else if (K <= 64) k_oz_rows<8><<<row_blocks(rows, 32), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
-    else if (K <= 128) k_oz_rows<16><<<row_blocks(rows, 16), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
-    else k_oz_rows<32><<<row_blocks(rows), 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex);
+#define AFQ_OZR(LN, BLOCKS)                                                                                       \
+    do {                                                                                                          \
+        if (amax) k_oz_rows<LN, true><<<BLOCKS, 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex, amax);        \
+        else k_oz_rows<LN, false><<<BLOCKS, 256, 0, s>>>(rows, per, K, src, ld, one, dst, D.ex, nullptr);         \
+    } while (0)
+    if (row_cta(rows, K)) AFQ_OZR(256, row_blocks(rows, 1));
+    else if (K <= 64) AFQ_OZR(8, row_blocks(rows, 32));
+    else if (K <= 128) AFQ_OZR(16, row_blocks(rows, 16));
+    else AFQ_OZR(32, row_blocks(rows));
+#undef AFQ_OZR
     AFQ_LAUNCHED("k_oz_rows");
     return AFQ_OK;
 }
-int split_crows(long long rows, int K, const double2* src, long long ld, const OzDigits& D, cudaStream_t s) {
+int split_crows(long long rows, int K, const double2* src, long long ld, const OzDigits& D, cudaStream_t s,
+                int* amax = nullptr) {
     const OzDst dst = dst_of(D, 2 * rows, K);
-    if (row_cta(rows, K)) k_oz_crows<256><<<row_blocks(rows, 1), 256, 0, s>>>(rows, K, src, ld, dst, D.ex);
-    else k_oz_crows<32><<<row_blocks(rows), 256, 0, s>>>(rows, K, src, ld, dst, D.ex);
+    if (row_cta(rows, K)) k_oz_crows<256><<<row_blocks(rows, 1), 256, 0, s>>>(rows, K, src, ld, dst, D.ex, amax);
+    else k_oz_crows<32><<<row_blocks(rows), 256, 0, s>>>(rows, K, src, ld, dst, D.ex, amax);
     AFQ_LAUNCHED("k_oz_crows");
     return AFQ_OK;
 }
-int split_cols(int rows, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s, int es = 1,
+int split_cols(int rows, int K, const double* src, long long ld, const OzDigits& D, cudaStream_t s, int* amax, int es = 1,
                const SymRows& sym = {}) {
-    if (rows <= 32 * 152) k_oz_cols<8><<<(rows + 7) / 8, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex, sym);
-    else k_oz_cols<32><<<(rows + 31) / 32, 256, 0, s>>>(rows, K, src, ld, es, dst_of(D, rows, K), D.ex, sym);
+    const OzDst dst = dst_of(D, rows, K);
+    if (rows <= 32 * 152) k_oz_cols<8><<<(rows + 7) / 8, 256, 0, s>>>(rows, K, src, ld, es, dst, D.ex, sym, amax);
+    else k_oz_cols<32><<<(rows + 31) / 32, 256, 0, s>>>(rows, K, src, ld, es, dst, D.ex, sym, amax);
     AFQ_LAUNCHED("k_oz_cols");
     return AFQ_OK;
 }
@@ -1015,7 +1134,7 @@ struct ZLayout {
     int mc, nc;
     OzDigits A, B;
     long long* raw;
-    int* asym;
+    int *asym, *amax;
 };
 ZLayout z_layout(Arena& a, int M, int N, int K) {
     ZLayout z;
@@ -1028,6 +1147,7 @@ ZLayout z_layout(Arena& a, int M, int N, int K) {
     const size_t nch = (K + 255) / 256, most = (size_t)OZ_TILE_SMS * OZ_ROWS * OZ_TN, all = nch * 2 * z.mc * z.nc;
     z.raw = a.take<long long>((nch > 1 ? (all < most ? all : most) : 0) * 3 / 2);  // 64-bit sums, 32-bit tails
     z.asym = a.take<int>(64);
+    z.amax = a.take<int>(1);
     return z;
 }
 
@@ -1093,18 +1213,29 @@ size_t zgemm_oz_scratch(int M, int N, int K) {
 // Digits of a real operand kept by the caller (a block's steps share theirs): bytes, 0 where they would take more
 // than OZ_KEEP.
 constexpr long long OZ_KEEP = 640LL << 20;
+struct ZKept {
+    OzDigits D;
+    int* amax;
+};
+static ZKept kept_layout(Arena& a, int N, int K) {
+    ZKept k;
+    k.D = take_digits(a, N, K);
+    k.amax = a.take<int>(1);
+    return k;
+}
 size_t oz_real_bytes(int N, int K) {
     if (!zgemm_oz_pays(1, N, K) || round_up(N, 8) * digit_row_bytes(K) > OZ_KEEP) return 0;
     Arena a;
-    take_digits(a, N, K);
+    kept_layout(a, N, K);
     return a.used + 256;
 }
 
 static int oz_real_split(int N, int K, const double* B, int64_t ldb, bool b_trans, void* real, cudaStream_t s,
                          const SymRows& sym = {}) {
     Arena a(real, (size_t)-1);
-    const OzDigits D = take_digits(a, N, K);
-    return b_trans ? split_rows(N, N, K, B, ldb, D, s) : split_cols(N, K, B, ldb, D, s, 1, sym);
+    const ZKept k = kept_layout(a, N, K);
+    AFQ_CUDA(cudaMemsetAsync(k.amax, 0x80, sizeof(int), s));
+    return b_trans ? split_rows(N, N, K, B, ldb, k.D, s, k.amax) : split_cols(N, K, B, ldb, k.D, s, k.amax, 1, sym);
 }
 
 // sn > 0: the V-build over sn orbitals, whose symmetric vectors' rows are in SymRows's order (asym: the flag of `real`)
@@ -1117,9 +1248,12 @@ static int zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t
     Arena ar(oz.p, oz.bytes);
     ZLayout z = z_layout(ar, M, N, K);
     AFQ_TRY(oz_room(ar));
+    const int* amax = z.amax;
     if (real) {
         Arena a((void*)real, (size_t)-1);
-        z.A = take_digits(a, N, K);
+        const ZKept k = kept_layout(a, N, K);
+        z.A = k.D;
+        amax = k.amax;
         z.nc = N;
     } else if (sn) {
         AFQ_TRY(launch_asym(sn, K, B, z.asym, s));
@@ -1129,18 +1263,24 @@ static int zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t
     AFQ_TRY(device_sms(&sms));
     for (int m0 = 0; m0 < M; m0 += z.mc) {
         const int mc = M - m0 < z.mc ? M - m0 : z.mc;
-        AFQ_TRY(split_crows(mc, K, A + (int64_t)m0 * lda, lda, z.B, s));
+        AFQ_TRY(split_crows(mc, K, A + (int64_t)m0 * lda, lda, z.B, s, z.amax));
         for (int n0 = 0; n0 < N; n0 += z.nc) {
             const int nc = N - n0 < z.nc ? N - n0 : z.nc;
             const SymRows sym = {sn ? asym : nullptr, sn, n0};  // the chunk's first row
             if (real) {}
-            else if (b_trans) AFQ_TRY(split_rows(nc, nc, K, B + (int64_t)n0 * ldb, ldb, z.A, s));
-            else AFQ_TRY(split_cols(nc, K, B, ldb, z.A, s, 1, sym));
+            else if (b_trans) AFQ_TRY(split_rows(nc, nc, K, B + (int64_t)n0 * ldb, ldb, z.A, s, z.amax));
+            else AFQ_TRY(split_cols(nc, K, B, ldb, z.A, s, z.amax, 1, sym));
             const OzOut out = {C + (int64_t)m0 * ldc + (sn ? 0 : n0), 0, ldc, 0, 1, 1, ae - 1, nullptr};
             const long long tiles = (long long)((nc + OZ_ROWS - 1) / OZ_ROWS) * ((2 * mc + OZ_TN - 1) / OZ_TN);
             int splits, cps;
             oz_splits(tiles, K, sms < OZ_TILE_SMS ? sms : OZ_TILE_SMS, splits, cps);
             AFQ_TRY(oz_launch(nc, 2 * mc, K, 1, 0, z.A, z.B, out, splits, cps, z.raw, oz.err, s, sn ? sym : SymRows{}));
+            // a chunk's columns of C, or all where its rows are symmetric vectors' blocks
+            const bool all = sn != 0;
+            AFQ_TRY(launch_zgemm_lost(mc, all ? N : nc, K, alpha, A + (int64_t)m0 * lda, lda,
+                                      all ? B : b_trans ? B + (int64_t)n0 * ldb : B + n0, ldb, b_trans,
+                                      C + (int64_t)m0 * ldc + (all ? 0 : n0), ldc, amax, z.B.ex, ae - 1, s));
+            if (n0 + nc < N) AFQ_CUDA(cudaMemsetAsync(z.amax, 0x80, sizeof(int), s));  // the next is judged by itself
         }
     }
     return AFQ_OK;
@@ -1157,11 +1297,31 @@ struct TrLayout {
     int wc;
     OzDigits E, V, T, X;  // E_half, V rows, right operands of V T, walker columns
     double2 *Y, *U;
+    OzSeries g;
 };
+// a chunk's scales and marks (x, t, u and flag), and that of E - I
+constexpr int OZ_SERIES = 4;
+OzSeries take_series(Arena& a, int wc) {
+    int* p = a.take<int>(OZ_SERIES * (size_t)wc + 1);
+    if (!p) return {};
+    return {p + OZ_SERIES * (size_t)wc, p, p + wc, p + 2 * (size_t)wc, p + 3 * (size_t)wc};
+}
+// all maxima of nothing yet
+int clear_series(const OzSeries& g, cudaStream_t s) {
+    AFQ_CUDA(cudaMemsetAsync(g.x, 0x80, (size_t)(g.flag - g.x) * sizeof(int), s));
+    return AFQ_OK;
+}
+int series_flags(const OzSeries& g, int wc, int n, const OzDigits& V, cudaStream_t s) {
+    k_oz_series_flags<<<(wc + 3) / 4, 128, 0, s>>>(wc, n, g, V.ex);
+    AFQ_LAUNCHED("k_oz_series_flags");
+    return AFQ_OK;
+}
+// the power of two above a coefficient
+int coef(double s) { return s == 0.0 ? -1100 : ilogb(s) + 1; }
 // walkers of ns blocks (n x o) each in a chunk: their digits and blocks take at most OZ_CAP
 long long tr_most(int n, int o, int ns) {
     const long long per = (round_up(n, 8) + round_up(2 * ns * o, 8)) * digit_row_bytes(2 * n) +
-                          2LL * ns * o * (digit_row_bytes(n) + 16LL * n);
+                          2LL * ns * o * (digit_row_bytes(n) + 16LL * n) + 4 * OZ_SERIES;
     return OZ_CAP / per > 1 ? OZ_CAP / per : 1;
 }
 // a chunk of wc walkers
@@ -1175,19 +1335,21 @@ TrLayout tr_layout(Arena& a, int wc, int n, int o, int ns) {
     t.X = take_digits(a, nb * 2 * o, n);
     t.Y = a.take<double2>(nb * n * o);
     t.U = a.take<double2>(nb * n * o);
+    t.g = take_series(a, t.wc);
     return t;
 }
 // W blocks of o columns, ns of them taken together (block strides ws, ss)
 template <int MODE>
 int launch_term(int W, int n, int o, double s, const double2* Y, const double2* X, double2* U, const OzDigits& D,
-                cudaStream_t st, int ns = 1, long long ws = 0, long long ss = 0, double2* tp = nullptr, long long tw = 0) {
+                cudaStream_t st, OzMax mx = {nullptr, 1, 1, 0}, int ns = 1, long long ws = 0, long long ss = 0,
+                double2* tp = nullptr, long long tw = 0) {
     const int oc = o * ns, ncg = (oc + OZ_CB - 1) / OZ_CB, smem = OZ_CB * (n + 1) * (int)sizeof(double2);
     if (ns == 1) ws = (long long)n * o;
     AFQ_TRY(raise_smem_once(g_ozterm[MODE], k_oz_term<MODE>, OZ_CB * 513 * (int)sizeof(double2)));
     const OzDst dst = MODE == OZ_WALK || MODE == OZ_LAST || MODE == OZ_BACKL ? dst_of(D, 2LL * W * oc, n)
                       : MODE == OZ_COLS                                      ? dst_of(D, 2 * oc, n)
                                                                              : dst_of(D, 2 * oc, 2 * n);
-    k_oz_term<MODE><<<(unsigned)W * ncg, 256, smem, st>>>(n, oc, o, ws, ss, ncg, s, Y, X, U, dst, D.ex, tp, tw);
+    k_oz_term<MODE><<<(unsigned)W * ncg, 256, smem, st>>>(n, oc, o, ws, ss, ncg, s, Y, X, U, dst, D.ex, tp, tw, mx);
     AFQ_LAUNCHED("k_oz_term");
     return AFQ_OK;
 }
@@ -1221,24 +1383,39 @@ int launch_trotter_oz(int W, int n, int o, int n_terms, double sqrt_dt, const do
     const TrLayout t = tr_layout(ar, even_chunk(W, tr_most(n, o, ns)), n, o, ns);
     AFQ_TRY(oz_room(ar));
     int* err = oz.err;
-    AFQ_TRY(split_rows(n, n, n, E, n, t.E, s, 1));
+    AFQ_CUDA(cudaMemsetAsync(t.g.e, 0x80, sizeof(int), s));
+    AFQ_TRY(split_rows(n, n, n, E, n, t.E, s, t.g.e, 1));
     const size_t no = (size_t)n * o;
     for (int w0 = 0; w0 < W; w0 += t.wc) {
         const int wc = W - w0 < t.wc ? W - w0 : t.wc, nb = wc * ns;  // the chunk's blocks are contiguous
+        const int bd = ws == (long long)no ? 1 : ns;                 // block b is walker b / bd % wc's
         const double2* x = win + (size_t)w0 * ns * no;
+        AFQ_TRY(clear_series(t.g, s));
         AFQ_TRY(split_rows((long long)wc * n, n, 2 * n, (const double*)(V + (size_t)w0 * n * n), 2 * n, t.V, s));
-        AFQ_TRY(launch_term<OZ_WALK>(nb, n, o, 0.0, x, nullptr, nullptr, t.X, s));
+        AFQ_TRY(launch_term<OZ_WALK>(nb, n, o, 0.0, x, nullptr, nullptr, t.X, s, {t.g.x, bd, wc, 0}));
         const OzOut xo = {t.Y, 0, (long long)no, 1, o, o, 0, nullptr};
         AFQ_TRY(oz_launch(n, 2 * nb * o, n, 1, 0, t.E, t.X, xo, 1, (n + 255) / 256, nullptr, err, s));
-        AFQ_TRY(launch_term<OZ_INIT>(wc, n, o, 0.0, t.Y, x, t.U, t.T, s, ns, ws, ss));
+        AFQ_TRY(launch_term<OZ_INIT>(wc, n, o, 0.0, t.Y, x, t.U, t.T, s, {t.g.t, 1, wc, coef(sqrt_dt)}, ns, ws, ss));
         for (int k = 1; k <= n_terms; ++k) {
             const OzOut to = {t.Y, ns == 1 ? (long long)no : ws, ss, 1, o, o, 0, nullptr};
             AFQ_TRY(oz_launch(n, 2 * ns * o, 2 * n, wc, 1, t.V, t.T, to, 1, (2 * n + 255) / 256, nullptr, err, s));
-            if (k < n_terms) AFQ_TRY(launch_term<OZ_TERM>(wc, n, o, sqrt_dt / k, t.Y, nullptr, t.U, t.T, s, ns, ws, ss));
-            else AFQ_TRY(launch_term<OZ_LAST>(nb, n, o, sqrt_dt / k, t.Y, nullptr, t.U, t.X, s));
+            if (k < n_terms)
+                AFQ_TRY(launch_term<OZ_TERM>(wc, n, o, sqrt_dt / k, t.Y, nullptr, t.U, t.T, s,
+                                             {t.g.t, 1, wc, coef(sqrt_dt / (k + 1))}, ns, ws, ss));
+            else AFQ_TRY(launch_term<OZ_LAST>(nb, n, o, sqrt_dt / k, t.Y, nullptr, t.U, t.X, s, {t.g.u, bd, wc, 0}));
         }
-        const OzOut wo = {wout + (size_t)w0 * ns * no, 0, (long long)no, 1, o, o, 0, t.U};
+        AFQ_TRY(series_flags(t.g, wc, n, t.V, s));
+        double2* y = wout + (size_t)w0 * ns * no;
+        const OzOut wo = {y, 0, (long long)no, 1, o, o, 0, t.U, t.g.flag, bd, wc};
         AFQ_TRY(oz_launch(n, 2 * nb * o, n, 1, 0, t.E, t.X, wo, 1, (n + 255) / 256, nullptr, err, s));
+        // the marked walkers, whose input is still in place where wout is win
+        const double2* v = V + (size_t)w0 * n * n;
+        if (bd == ns) {
+            AFQ_TRY(launch_trotter(nb, n, o, n_terms, sqrt_dt, E, v, x, y, s, ns, t.g.flag));
+        } else {
+            for (int p = 0; p < ns; ++p)
+                AFQ_TRY(launch_trotter(wc, n, o, n_terms, sqrt_dt, E, v, x + p * ss, y + p * ss, s, 1, t.g.flag));
+        }
     }
     return AFQ_OK;
 }
@@ -1268,11 +1445,12 @@ struct TgLayout {
     OzDigits E, V, T, X;
     double2 *Y, *U, *vh;
     double* et;
+    OzSeries g;
 };
 TgLayout tg_layout(Arena& a, int W, int n, int o) {
     TgLayout t;
     const long long n2 = (long long)n * n, per = (round_up(n, 8) + round_up(2 * o, 8)) * digit_row_bytes(2 * n) + 16 * n2 +
-                                                 2LL * o * (digit_row_bytes(n) + 16LL * n);
+                                                 2LL * o * (digit_row_bytes(n) + 16LL * n) + 4 * OZ_SERIES;
     const long long most = OZ_CAP / per;
     t.wc = even_chunk(W, most < 65535 ? most : 65535);
     t.E = take_digits(a, n, n);
@@ -1283,6 +1461,7 @@ TgLayout tg_layout(Arena& a, int W, int n, int o) {
     t.U = a.take<double2>((size_t)t.wc * n * o);
     t.vh = a.take<double2>(t.wc * n2);
     t.et = a.take<double>(n2);
+    t.g = take_series(a, t.wc);
     return t;
 }
 }  // namespace
@@ -1300,21 +1479,27 @@ int launch_taylor_tape_oz(int W, int n, int o, int K, double sqrt_dt, const doub
     AFQ_TRY(oz_room(ar));
     int* err = oz.err;
     const size_t no = (size_t)n * o;
-    AFQ_TRY(split_rows(n, n, n, E, n, t.E, s, 1));
+    AFQ_CUDA(cudaMemsetAsync(t.g.e, 0x80, sizeof(int), s));
+    AFQ_TRY(split_rows(n, n, n, E, n, t.E, s, t.g.e, 1));
     const OzOut xo = {t.Y, 0, (long long)no, 1, o, o, 0, nullptr}, to = {t.Y, (long long)no, 0, 1, o, o, 0, nullptr};
     for (int w0 = 0; w0 < W; w0 += t.wc) {
         const int wc = W - w0 < t.wc ? W - w0 : t.wc;
         const double2* x = win + w0 * no;
         double2 *u = w2 + w0 * no, *tp = terms + w0 * K * no;
+        AFQ_TRY(clear_series(t.g, s));
         AFQ_TRY(split_rows((long long)wc * n, n, 2 * n, (const double*)(V + (size_t)w0 * n * n), 2 * n, t.V, s));
-        AFQ_TRY(launch_term<OZ_WALK>(wc, n, o, 0.0, x, nullptr, nullptr, t.X, s));
+        AFQ_TRY(launch_term<OZ_WALK>(wc, n, o, 0.0, x, nullptr, nullptr, t.X, s, {t.g.x, 1, wc, 0}));
         AFQ_TRY(oz_launch(n, 2 * wc * o, n, 1, 0, t.E, t.X, xo, 1, (n + 255) / 256, nullptr, err, s));
-        AFQ_TRY(launch_term<OZ_INIT>(wc, n, o, 0.0, t.Y, x, u, t.T, s, 1, 0, 0, tp, K * no));
+        AFQ_TRY(launch_term<OZ_INIT>(wc, n, o, 0.0, t.Y, x, u, t.T, s, {t.g.t, 1, wc, coef(sqrt_dt)}, 1, 0, 0, tp, K * no));
         for (int k = 1; k <= K; ++k) {
             AFQ_TRY(oz_launch(n, 2 * o, 2 * n, wc, 1, t.V, t.T, to, 1, (2 * n + 255) / 256, nullptr, err, s));
-            if (k < K) AFQ_TRY(launch_term<OZ_TERM>(wc, n, o, sqrt_dt / k, t.Y, nullptr, u, t.T, s, 1, 0, 0, tp + k * no, K * no));
-            else AFQ_TRY(launch_term<OZ_LAST>(wc, n, o, sqrt_dt / k, t.Y, nullptr, u, t.X, s));
+            if (k < K)
+                AFQ_TRY(launch_term<OZ_TERM>(wc, n, o, sqrt_dt / k, t.Y, nullptr, u, t.T, s,
+                                             {t.g.t, 1, wc, coef(sqrt_dt / (k + 1))}, 1, 0, 0, tp + k * no, K * no));
+            else AFQ_TRY(launch_term<OZ_LAST>(wc, n, o, sqrt_dt / k, t.Y, nullptr, u, t.X, s, {t.g.u, 1, wc, 0}));
         }
+        AFQ_TRY(series_flags(t.g, wc, n, t.V, s));
+        AFQ_TRY(launch_taylor_tape_plain(wc, n, o, K, sqrt_dt, E, V + (size_t)w0 * n * n, x, tp, u, t.g.flag, s));
     }
     return AFQ_OK;
 }
@@ -1330,7 +1515,8 @@ int launch_taylor_adj_oz(int W, int n, int o, int K, double sqrt_dt, const doubl
     const unsigned nt = (n + 31) / 32;
     k_oz_adjoint<double><<<dim3(nt, nt, 1), 256, 0, s>>>(n, E, t.et);
     AFQ_LAUNCHED("k_oz_adjoint");
-    AFQ_TRY(split_rows(n, n, n, t.et, n, t.E, s, 1));
+    AFQ_CUDA(cudaMemsetAsync(t.g.e, 0x80, sizeof(int), s));
+    AFQ_TRY(split_rows(n, n, n, t.et, n, t.E, s, t.g.e, 1));
     const OzOut xo = {t.Y, 0, (long long)no, 1, o, o, 0, nullptr}, to = {t.Y, (long long)no, 0, 1, o, o, 0, nullptr};
     for (int w0 = 0; w0 < W; w0 += t.wc) {
         const int wc = W - w0 < t.wc ? W - w0 : t.wc;
@@ -1338,18 +1524,26 @@ int launch_taylor_adj_oz(int W, int n, int o, int K, double sqrt_dt, const doubl
         double2* tp = tbar + w0 * (K + 1) * no;
         k_oz_adjoint<double2><<<dim3(nt, nt, wc), 256, 0, s>>>(n, V + (size_t)w0 * n * n, t.vh);
         AFQ_LAUNCHED("k_oz_adjoint");
+        AFQ_TRY(clear_series(t.g, s));
         AFQ_TRY(split_rows((long long)wc * n, n, 2 * n, (const double*)t.vh, 2 * n, t.V, s));
-        AFQ_TRY(launch_term<OZ_WALK>(wc, n, o, 0.0, x, nullptr, nullptr, t.X, s));
+        AFQ_TRY(launch_term<OZ_WALK>(wc, n, o, 0.0, x, nullptr, nullptr, t.X, s, {t.g.x, 1, wc, 0}));
         AFQ_TRY(oz_launch(n, 2 * wc * o, n, 1, 0, t.E, t.X, xo, 1, (n + 255) / 256, nullptr, err, s));
-        AFQ_TRY(launch_term<OZ_INIT>(wc, n, o, 0.0, t.Y, x, t.U, t.T, s, 1, 0, 0, tp + K * no, (K + 1) * no));
+        AFQ_TRY(launch_term<OZ_INIT>(wc, n, o, 0.0, t.Y, x, t.U, t.T, s, {t.g.t, 1, wc, coef(sqrt_dt / K)}, 1, 0, 0,
+                                     tp + K * no, (K + 1) * no));
         for (int k = K - 1; k >= 0; --k) {
             AFQ_TRY(oz_launch(n, 2 * o, 2 * n, wc, 1, t.V, t.T, to, 1, (2 * n + 255) / 256, nullptr, err, s));
             const double c = sqrt_dt / (k + 1);
-            if (k > 0) AFQ_TRY(launch_term<OZ_BACK>(wc, n, o, c, t.Y, nullptr, t.U, t.T, s, 1, 0, 0, tp + k * no, (K + 1) * no));
-            else AFQ_TRY(launch_term<OZ_BACKL>(wc, n, o, c, t.Y, nullptr, t.U, t.X, s, 1, 0, 0, tp, (K + 1) * no));
+            if (k > 0)
+                AFQ_TRY(launch_term<OZ_BACK>(wc, n, o, c, t.Y, nullptr, t.U, t.T, s, {t.g.t, 1, wc, coef(sqrt_dt / k)}, 1, 0,
+                                             0, tp + k * no, (K + 1) * no));
+            else AFQ_TRY(launch_term<OZ_BACKL>(wc, n, o, c, t.Y, nullptr, t.U, t.X, s, {t.g.u, 1, wc, 0}, 1, 0, 0, tp,
+                                               (K + 1) * no));
         }
-        const OzOut wo = {wbar_pre + w0 * no, 0, (long long)no, 1, o, o, 0, t.U};
+        AFQ_TRY(series_flags(t.g, wc, n, t.V, s));
+        const OzOut wo = {wbar_pre + w0 * no, 0, (long long)no, 1, o, o, 0, t.U, t.g.flag, 1, wc};
         AFQ_TRY(oz_launch(n, 2 * wc * o, n, 1, 0, t.E, t.X, wo, 1, (n + 255) / 256, nullptr, err, s));
+        AFQ_TRY(launch_taylor_adj_plain(wc, n, o, K, sqrt_dt, E, V + (size_t)w0 * n * n, x, tp, wbar_pre + w0 * no, t.g.flag,
+                                        s));
     }
     return AFQ_OK;
 }
@@ -1360,11 +1554,12 @@ struct GrLayout {
     int wc;
     OzDigits C, X, A, B;  // trial columns, walker columns, walker rows, right operands W^T m^-1
     double2 *m, *inv;
+    int* flag;  // walkers whose product has lost too much
 };
 GrLayout gr_layout(Arena& a, int W, int n, int o) {
     GrLayout g;
     const long long per = 2LL * o * digit_row_bytes(n) + round_up(n, 8) * digit_row_bytes(2 * o) +
-                          round_up(2 * o, 8) * digit_row_bytes(2 * o) + 32LL * o * o;
+                          round_up(2 * o, 8) * digit_row_bytes(2 * o) + 32LL * o * o + 4;
     long long wc = OZ_CAP / per;
     g.wc = even_chunk(W, wc);
     g.C = take_digits(a, o, n);
@@ -1373,6 +1568,7 @@ GrLayout gr_layout(Arena& a, int W, int n, int o) {
     g.B = take_digits(a, 2 * o, 2 * o, g.wc);
     g.m = a.take<double2>((size_t)g.wc * o * o);
     g.inv = a.take<double2>((size_t)g.wc * o * o);
+    g.flag = a.take<int>(g.wc);
     return g;
 }
 }  // namespace
@@ -1392,19 +1588,25 @@ int launch_green_oz(int W, int n, int o, const double2* mo, const double2* walke
     AFQ_TRY(oz_room(ar));
     int* err = oz.err;
     const size_t no = (size_t)n * o;
-    AFQ_TRY(split_cols(o, n, (const double*)mo, 2LL * o, g.C, s, 2));
+    AFQ_TRY(split_cols(o, n, (const double*)mo, 2LL * o, g.C, s, nullptr, 2));
     for (int w0 = 0; w0 < W; w0 += g.wc) {
         const int wc = W - w0 < g.wc ? W - w0 : g.wc;
         const double2* w = walkers + w0 * no;
+        double2 *ov = ovlp_out ? ovlp_out + w0 : nullptr, *gr = green_out ? green_out + w0 * no : nullptr;
         AFQ_TRY(launch_term<OZ_WALK>(wc, n, o, 0.0, w, nullptr, nullptr, g.X, s));
         const OzOut mout = {g.m, 0, (long long)o * o, 1, o, o, 0, nullptr};
         AFQ_TRY(oz_launch(o, 2 * wc * o, n, 1, 0, g.C, g.X, mout, 1, (n + 255) / 256, nullptr, err, s));
-        AFQ_TRY(launch_lu(wc, o, g.m, ovlp_out ? ovlp_out + w0 : nullptr, green_out ? g.inv : nullptr, ov_square, s));
-        if (!green_out) continue;
-        AFQ_TRY(split_rows((long long)wc * n, n, 2 * o, (const double*)w, 2 * o, g.A, s));
-        AFQ_TRY(launch_term<OZ_PLAIN>(wc, o, o, 0.0, g.inv, nullptr, nullptr, g.B, s));
-        const OzOut gout = {green_out + w0 * no, (long long)no, 0, n, 1, 2 * o, 0, nullptr};
-        AFQ_TRY(oz_launch(n, 2 * o, 2 * o, wc, 1, g.A, g.B, gout, 1, (2 * o + 255) / 256, nullptr, err, s));
+        AFQ_TRY(launch_lu(wc, o, g.m, ov, gr ? g.inv : nullptr, ov_square, s));
+        if (gr) {
+            AFQ_TRY(split_rows((long long)wc * n, n, 2 * o, (const double*)w, 2 * o, g.A, s));
+            AFQ_TRY(launch_term<OZ_PLAIN>(wc, o, o, 0.0, g.inv, nullptr, nullptr, g.B, s));
+            const OzOut gout = {gr, (long long)no, 0, n, 1, 2 * o, 0, nullptr};
+            AFQ_TRY(oz_launch(n, 2 * o, 2 * o, wc, 1, g.A, g.B, gout, 1, (2 * o + 255) / 256, nullptr, err, s));
+        }
+        const OzWalk gm = {g.C.ex, g.X.ex, g.m, o * o, o, 2 * o, 1}, gg = {g.A.ex, g.B.ex, gr, (int)no, n, 2 * o, 0};
+        k_oz_flags<<<(wc + 3) / 4, 128, 0, s>>>(wc, gm, gg, g.flag);
+        AFQ_LAUNCHED("k_oz_flags");
+        AFQ_TRY(launch_green_sq(wc, n, o, mo, 1, w, ov, gr, ov_square, s, g.flag));
     }
     return AFQ_OK;
 }
@@ -1483,6 +1685,7 @@ namespace {
 struct VbLayout {
     int wc;
     OzDigits A, B;
+    int* flag;
 };
 VbLayout vb_layout(Arena& a, int W, int n, int o, int K) {
     VbLayout v;
@@ -1490,6 +1693,7 @@ VbLayout vb_layout(Arena& a, int W, int n, int o, int K) {
     v.wc = even_chunk(W, OZ_CAP / (3 * round_up(n, 8) * digit_row_bytes(k2)));
     v.A = take_digits(a, n, k2, v.wc);
     v.B = take_digits(a, 2 * n, k2, v.wc);
+    v.flag = a.take<int>(v.wc);
     return v;
 }
 }  // namespace
@@ -1507,7 +1711,7 @@ size_t vbar_oz_scratch(int W, int n, int o, int K) {
 int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tbar, const double2* terms,
                    double2* vbar, const OzScratch& oz, cudaStream_t s) {
     if (W <= 0) return AFQ_OK;
-    if (!vbar_oz_pays(o, K)) return launch_vbar(W, n, o, K, sqrt_dt, tbar, terms, vbar, s);
+    if (!vbar_oz_pays(o, K)) return launch_vbar(W, n, o, K, sqrt_dt, tbar, terms, vbar, nullptr, s);
     Arena ar(oz.p, oz.bytes);
     const VbLayout v = vb_layout(ar, W, n, o, K);
     AFQ_TRY(oz_room(ar));
@@ -1518,12 +1722,15 @@ int launch_vbar_oz(int W, int n, int o, int K, double sqrt_dt, const double2* tb
         // eight lanes a row of up to 64 entries, sixteen of 128 (60 orbitals, 120 entries, 256 walkers: 106 -> 65 us)
         const int lanes = k2 <= 64 ? 8 : k2 <= 128 ? 16 : 32;
         const auto cut = lanes == 8 ? k_oz_vbar<8> : lanes == 16 ? k_oz_vbar<16> : k_oz_vbar<32>;
-        cut<<<row_blocks(2LL * wc * n, 256 / lanes), 256, 0, s>>>(
-            wc, n, o, K, sqrt_dt, tbar + (long long)w0 * (K + 1) * no, terms + (long long)w0 * K * no,
-            dst_of(v.A, n, k2), v.A.ex, dst_of(v.B, 2 * n, k2), v.B.ex);
+        const double2 *tb = tbar + (long long)w0 * (K + 1) * no, *tm = terms + (long long)w0 * K * no;
+        cut<<<row_blocks(2LL * wc * n, 256 / lanes), 256, 0, s>>>(wc, n, o, K, sqrt_dt, tb, tm, dst_of(v.A, n, k2), v.A.ex,
+                                                                  dst_of(v.B, 2 * n, k2), v.B.ex);
         AFQ_LAUNCHED("k_oz_vbar");
         const OzOut out = {vbar + w0 * n2, n2, 0, 1, n, n, 0, nullptr};
         AFQ_TRY(oz_launch(n, 2 * n, k2, wc, 1, v.A, v.B, out, 1, (k2 + 255) / 256, nullptr, oz.err, s));
+        k_oz_flags<<<(wc + 3) / 4, 128, 0, s>>>(wc, {v.A.ex, v.B.ex, out.C, (int)n2, n, 2 * n, 0}, {}, v.flag);
+        AFQ_LAUNCHED("k_oz_flags");
+        AFQ_TRY(launch_vbar(wc, n, o, K, sqrt_dt, tb, tm, vbar + w0 * n2, v.flag, s));
     }
     return AFQ_OK;
 }
@@ -1565,11 +1772,13 @@ int launch_energy_partial_oz(int W, int n, int o, int G, const double2* green, c
     AFQ_TRY(split_rows((long long)G * o, G * o, n, rot_chol, n, e.L, s));
     for (int w0 = 0; w0 < W; w0 += e.wc) {
         const int wc = W - w0 < e.wc ? W - w0 : e.wc;
-        AFQ_TRY(split_crows((long long)wc * o, n, green + (size_t)w0 * o * n, n, e.X, s));
+        const double2* g = green + (size_t)w0 * o * n;
+        AFQ_TRY(split_crows((long long)wc * o, n, g, n, e.X, s));
         const OzOut out = {e.F, 0, (long long)G * o, 0, 1, 1, 0, nullptr};
         AFQ_TRY(oz_launch(G * o, 2 * wc * o, n, 1, 0, e.L, e.X, out, 1, (n + 255) / 256,
                           nullptr, oz.err, s));
-        k_oz_exchange<<<dim3(nchunk, wc), 256, smem, s>>>(o, G, ng, e.F, (double2*)partial_d + (size_t)w0 * nchunk * 2);
+        k_oz_exchange<<<dim3(nchunk, wc), 256, smem, s>>>(n, o, G, ng, e.F, (double2*)partial_d + (size_t)w0 * nchunk * 2,
+                                                          e.L.ex, e.X.ex, rot_chol, g);
         AFQ_LAUNCHED("k_oz_exchange");
     }
     return AFQ_OK;

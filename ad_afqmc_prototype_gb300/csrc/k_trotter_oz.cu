@@ -55,9 +55,9 @@ struct TsGeo {
 
 // Digits of A's rows: eight k a lane, GL lanes a row, the scale from a max over
 // the row's lanes.  ONE: A = E - I with E real (its Im parts zero).  ADJ: of
-// the conjugate transpose.
+// the conjugate transpose.  s_amax is raised to the largest scale.
 template <bool ONE, bool ADJ>
-__device__ void ts_load_a(const TsGeo& g, int n, const void* __restrict__ src, __nv_bfloat16* As, int* s_ea) {
+__device__ void ts_load_a(const TsGeo& g, int n, const void* __restrict__ src, __nv_bfloat16* As, int* s_ea, int* s_amax) {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int l8 = g.kp / 8, gl = l8 <= 2 ? 2 : l8 <= 4 ? 4 : l8 <= 8 ? 8 : 16;  // lanes a row
     const int rw = 32 / gl, sub = lane / gl, k = 8 * (lane % gl);
@@ -79,10 +79,13 @@ __device__ void ts_load_a(const TsGeo& g, int n, const void* __restrict__ src, _
         }
         int e = 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) e = max(e, oz_expo(x[i]));
+        for (int i = 0; i < 8; ++i) e = max(e, oz_key(x[i]));
         for (int o = gl / 2; o > 0; o >>= 1) e = max(e, __shfl_xor_sync(0xffffffffu, e, o));
         const int E = oz_scale(e);
-        if (k == 0 && r < 16 * g.mt) s_ea[r] = E;
+        if (k == 0 && r < 16 * g.mt) {
+            s_ea[r] = E;
+            atomicMax(s_amax, E);
+        }
         if (k < g.kp && r < 16 * g.mt) {
             long long y[8];
 #pragma unroll
@@ -115,6 +118,63 @@ __device__ __forceinline__ void ts_put(uint32_t* d, size_t plane, int pw, long l
 //   TS_ADJ   the reverse: b = E^T W, t_K = b, t_k = b + conj(i sqrt_dt / (k + 1)) V^H
 //            t_{k+1} to `terms` (W, K + 1, n, o), wout = E^T t_0
 enum { TS_STEP, TS_TAPE, TS_ADJ };
+
+// The walker's series on the binary64 pipe, for the one that the digits cannot be left to (oz_lost): its input is still
+// in place, the digits' shared memory (at least 28 n (n + 4 oc) bytes) holds two terms and the sum.
+template <int MODE>
+__device__ __forceinline__ void ts_plain(int n, int o, int oc, long long ws, long long ss, int n_terms, double sqrt_dt,
+                                      const double* E, const double2* V, const double2* win, double2* wout, double2* terms,
+                                      double2* sm) {
+    const int w = blockIdx.x, no = n * oc;
+    const double2* Vw = V + (size_t)w * n * n;
+    double2 *cur = sm, *nxt = sm + no, *sum = sm + 2 * no;
+    auto at = [&](int e) {
+        const int i = e / oc, c = e - i * oc, p = c >= o;
+        return w * ws + (long long)i * o + (c - p * o) + p * ss;
+    };
+    auto keep = [&](int slot, int e, double2 t) {  // ns = 1: oc = o
+        if (MODE != TS_STEP) terms[((size_t)w * (MODE == TS_ADJ ? n_terms + 1 : n_terms) + slot) * no + e] = t;
+    };
+    auto e_times = [&](const double2* x, int e) {  // (E x)[e], E^T in the adjoint
+        const int i = e / oc, c = e - i * oc;
+        double2 a = make_double2(0.0, 0.0);
+        for (int j = 0; j < n; ++j) rfma(a, E[MODE == TS_ADJ ? j * n + i : i * n + j], x[j * oc + c]);
+        return a;
+    };
+    for (int e = threadIdx.x; e < no; e += blockDim.x) nxt[e] = win[at(e)];
+    __syncthreads();
+    for (int e = threadIdx.x; e < no; e += blockDim.x) {
+        cur[e] = sum[e] = e_times(nxt, e);
+        keep(MODE == TS_ADJ ? n_terms : 0, e, cur[e]);
+    }
+    __syncthreads();
+    for (int k = 1; k <= n_terms; ++k) {
+        const double s = sqrt_dt / (MODE == TS_ADJ ? n_terms + 1 - k : k);
+        for (int e = threadIdx.x; e < no; e += blockDim.x) {
+            const int i = e / oc, c = e - i * oc;
+            double2 a = make_double2(0.0, 0.0);
+            for (int j = 0; j < n; ++j) {
+                const double2 v = Vw[MODE == TS_ADJ ? (size_t)j * n + i : (size_t)i * n + j];
+                cfma(a, MODE == TS_ADJ ? make_double2(v.x, -v.y) : v, cur[j * oc + c]);
+            }
+            if (MODE == TS_ADJ) {
+                nxt[e] = make_double2(sum[e].x + s * a.y, sum[e].y - s * a.x);
+                keep(n_terms - k, e, nxt[e]);
+            } else {
+                nxt[e] = make_double2(-s * a.y, s * a.x);
+                sum[e] = cadd(sum[e], nxt[e]);
+                if (k < n_terms) keep(k, e, nxt[e]);
+            }
+        }
+        __syncthreads();
+        double2* t = cur;
+        cur = nxt;
+        nxt = t;
+    }
+    for (int e = threadIdx.x; e < no; e += blockDim.x)
+        wout[at(e)] = MODE == TS_TAPE ? sum[e] : e_times(MODE == TS_ADJ ? cur : sum, e);
+}
+
 template <int NT, int MODE>
 __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long long ws, long long ss, int n_terms,
                                                     double sqrt_dt, const double* __restrict__ E,
@@ -125,7 +185,7 @@ __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long l
     const TsGeo g(n, oc);
     __nv_bfloat16* As = (__nv_bfloat16*)smem_raw;
     __nv_bfloat16* Bs = (__nv_bfloat16*)(smem_raw + g.a_bytes);
-    __shared__ int s_ea[TS_NMAX], s_eb[2][TS_NMAX];
+    __shared__ int s_ea[TS_NMAX], s_eb[2][TS_NMAX], s_amax[2], s_most[2];  // s_amax: of E - I, V
     const int w = blockIdx.x, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int mt = wid % g.mt, n0 = wid / g.mt * NT;  // this warp's row tile and first column tile
     const int r0 = 16 * mt + (lane >> 2), q = lane & 3;
@@ -133,8 +193,13 @@ __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long l
     const size_t plane_b = (size_t)8 * g.nt * pw;      // words a digit plane
 
     for (int e = tid; e < 2 * TS_NMAX; e += blockDim.x) s_eb[0][e] = 0;
+    if (tid == 0) {
+        s_amax[0] = s_amax[1] = s_most[0] = OZ_EMPTY;
+        s_most[1] = 0;
+    }
     for (int e = tid; e < (int)(g.b_bytes / 16); e += blockDim.x) ((uint4*)Bs)[e] = make_uint4(0, 0, 0, 0);
-    ts_load_a<true, MODE == TS_ADJ>(g, n, E, As, s_ea);
+    __syncthreads();
+    ts_load_a<true, MODE == TS_ADJ>(g, n, E, As, s_ea, &s_amax[0]);
 
     // entry (t, h): row r0 + 8 h, column c = 4 (n0 + t) + q
     double2 U[NT][2], T[NT][2];
@@ -159,11 +224,12 @@ __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long l
             }
     };
     int buf = 0;
-    // T's digits into Bs (after every warp has read the last ones)
-    auto put = [&]() {
+    // T's digits into Bs (after every warp has read the last ones); the product to come is A's (s_amax[v]) by a
+    // coefficient below 2^ce
+    auto put = [&](int v, int ce) {
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
-            int e = max(max(oz_expo(T[t][0].x), oz_expo(T[t][0].y)), max(oz_expo(T[t][1].x), oz_expo(T[t][1].y)));
+            int e = max(max(oz_key(T[t][0].x), oz_key(T[t][0].y)), max(oz_key(T[t][1].x), oz_key(T[t][1].y)));
             e = max(e, __shfl_xor_sync(0xffffffffu, e, 4));
             e = max(e, __shfl_xor_sync(0xffffffffu, e, 8));
             e = max(e, __shfl_xor_sync(0xffffffffu, e, 16));
@@ -171,6 +237,11 @@ __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long l
             if (lane < 4 && c < oc) atomicMax(&s_eb[buf][c], e);
         }
         __syncthreads();
+        if (tid < oc) {
+            const int Ea = s_amax[v], Eb = oz_scale(s_eb[buf][tid]);
+            if (Ea == OZ_NAN || Eb == OZ_NAN) atomicMax(&s_most[0], OZ_NAN);
+            else if (Ea > OZ_ZERO && Eb > OZ_ZERO) atomicMax(&s_most[0], Ea + Eb + ce);
+        }
         for (int e = tid; e < TS_NMAX; e += blockDim.x) s_eb[buf ^ 1][e] = 0;
 #pragma unroll
         for (int t = 0; t < NT; ++t) {
@@ -246,21 +317,21 @@ __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long l
         buf ^= 1;
     };
 
-    put();
+    put(0, 0);
     mul();
 #pragma unroll
     for (int t = 0; t < NT; ++t)
 #pragma unroll
         for (int h = 0; h < 2; ++h) U[t][h] = T[t][h] = cadd(U[t][h], T[t][h]);
     __syncthreads();
-    ts_load_a<false, MODE == TS_ADJ>(g, n, V + (size_t)w * n * n, As, s_ea);
+    ts_load_a<false, MODE == TS_ADJ>(g, n, V + (size_t)w * n * n, As, s_ea, &s_amax[1]);
     if (MODE == TS_TAPE) keep((size_t)w * n_terms);
     if (MODE == TS_ADJ) keep((size_t)w * (n_terms + 1) + n_terms);
     for (int k = 1; k <= n_terms; ++k) {
-        put();
-        mul();
         // (i sqrt_dt / k) z = s (-z.y, z.x); the adjoint's coefficient is conj(i sqrt_dt / (K + 1 - k))
         const double s = sqrt_dt / (MODE == TS_ADJ ? n_terms + 1 - k : k);
+        put(1, oz_scale(oz_key(s)));
+        mul();
 #pragma unroll
         for (int t = 0; t < NT; ++t)
 #pragma unroll
@@ -277,7 +348,7 @@ __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long l
     }
     if (MODE != TS_TAPE) {
         __syncthreads();
-        ts_load_a<true, MODE == TS_ADJ>(g, n, E, As, s_ea);
+        ts_load_a<true, MODE == TS_ADJ>(g, n, E, As, s_ea, &s_amax[0]);
 #pragma unroll
         for (int t = 0; t < NT; ++t)
 #pragma unroll
@@ -285,8 +356,22 @@ __global__ void __launch_bounds__(256) k_trotter_oz(int n, int o, int ns, long l
                 if (MODE == TS_ADJ) U[t][h] = T[t][h];
                 else T[t][h] = U[t][h];
             }
-        put();
+        put(0, -4000);  // judged with the first one, by the same E
         mul();
+    }
+    // the products' scales against the sum's (oz_lost)
+    int top = 0;
+#pragma unroll
+    for (int t = 0; t < NT; ++t)
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (r0 + 8 * h < n && 4 * (n0 + t) + q < oc) top = max(top, max(oz_key(U[t][h].x), oz_key(U[t][h].y)));
+    top = __reduce_max_sync(0xffffffffu, top);
+    if (lane == 0) atomicMax(&s_most[1], top);
+    __syncthreads();
+    if (s_most[0] != OZ_EMPTY && oz_lost(s_most[0], 0, (s_most[1] >> 20) - 1023 >= oz_reach(s_most[0], 0))) {
+        ts_plain<MODE>(n, o, oc, ws, ss, n_terms, sqrt_dt, E, V, win, wout, terms, (double2*)smem_raw);
+        return;
     }
 #pragma unroll
     for (int t = 0; t < NT; ++t)

@@ -57,7 +57,9 @@ template <int NR>
 __global__ void __launch_bounds__(TR_THREADS) k_trotter(int n, int o, int n_terms, double sqrt_dt,
                                                         const double* __restrict__ E,
                                                         const double2* __restrict__ V,
-                                                        const double2* win, double2* wout, int vdiv) {
+                                                        const double2* win, double2* wout, int vdiv,
+                                                        const int* __restrict__ only) {
+    if (only && !only[blockIdx.y / vdiv]) return;
     extern __shared__ double2 sm[];
     double2* T = sm;                    // n x OC
     double2* Ms = sm + (size_t)n * TR_OC;  // n x BJ
@@ -108,7 +110,7 @@ __global__ void __launch_bounds__(TR_THREADS) k_trotter(int n, int o, int n_term
 }
 
 int launch_trotter(int W, int n, int o, int n_terms, double sqrt_dt, const double* E, const double2* V,
-                   const double2* win, double2* wout, cudaStream_t s, int vdiv) {
+                   const double2* win, double2* wout, cudaStream_t s, int vdiv, const int* only) {
     if (W <= 0) return AFQ_OK;
     const int nr = (n + TR_NRG - 1) / TR_NRG;
     size_t smem = (size_t)n * (TR_OC + TR_BJ) * sizeof(double2);
@@ -117,7 +119,7 @@ int launch_trotter(int W, int n, int o, int n_terms, double sqrt_dt, const doubl
 #define AFQ_TR(NRV)                                                                   \
     do {                                                                              \
         AFQ_TRY(set_smem(k_trotter<NRV>, smem));                                      \
-        k_trotter<NRV><<<grid, TR_THREADS, smem, s>>>(n, o, n_terms, sqrt_dt, E, V, win, wout, vdiv); \
+        k_trotter<NRV><<<grid, TR_THREADS, smem, s>>>(n, o, n_terms, sqrt_dt, E, V, win, wout, vdiv, only); \
     } while (0)
     if (nr <= 1) AFQ_TR(1);
     else if (nr <= 2) AFQ_TR(2);

@@ -8,12 +8,15 @@ namespace afq {
 constexpr int OZ_S = 7;             // digits
 constexpr int OZ_NAN = 0x7fffffff;  // scale of a row holding inf or nan
 constexpr int OZ_KMAX = 65535;      // longest product: below 2^16 its integer sum stays below 2^62
+constexpr int OZ_ZERO = -1022;      // scale of a row of zeros
+constexpr int OZ_EMPTY = (int)0x80808080u;  // a maximum of nothing yet (bytes of one value: a memset makes it)
 
-__device__ __forceinline__ int oz_expo(double x) {  // biased binary64 exponent
-    return (int)(((unsigned long long)__double_as_longlong(x) >> 52) & 0x7ffu);
+// a key that orders as |x| does (0 below 2^-1042)
+__device__ __forceinline__ int oz_key(double x) { return __double2hiint(x) & 0x7fffffff; }
+// scale of a row whose largest key is given: |x| < 2^E
+__device__ __forceinline__ int oz_scale(int key) {
+    return key >= 0x7ff00000 ? OZ_NAN : key == 0 ? OZ_ZERO : max(key >> 20, 1) - 1022;
 }
-// scale of a row whose largest biased exponent is eb: |x| < 2^E
-__device__ __forceinline__ int oz_scale(int eb) { return eb == 0x7ff ? OZ_NAN : eb - 1022; }
 
 // x 2^(55 - E) rounded to an integer, |.| <= 2^55, plus 0x808080808080, whose
 // low six bytes are then the lower digits plus 128 (zero for subnormal x and
@@ -50,6 +53,35 @@ template <int S>
 __device__ __forceinline__ uint4 oz_pack8(const long long (&y)[8]) {
     return make_uint4(oz_pack(oz_dig<S>(y[0]), oz_dig<S>(y[1])), oz_pack(oz_dig<S>(y[2]), oz_dig<S>(y[3])),
                       oz_pack(oz_dig<S>(y[4]), oz_dig<S>(y[5])), oz_pack(oz_dig<S>(y[6]), oz_dig<S>(y[7])));
+}
+
+// What a product by digits may lose.  Its rows are held to 2^-55 of their largest entries, so its error scales with
+// the largest entries of both operands, that of a binary64 chain with the terms: where large entries meet small ones
+// only (rows graded in opposite directions, a sum that cancels) the chain is the better one.  Checked by its
+// results, a walker (or a column) at a time: amax and bmax are the operands' largest scales there, and the product
+// stands where some result reaches 2^-OZ_LOSS of 2^(amax + bmax), so that its error stays within about 2^-49 of
+// the largest result, a chain's of a few hundred terms.  Otherwise, and with inf, nan or scales whose products come near
+// the subnormals, the caller forms it again on the binary64 pipe.
+constexpr int OZ_LOSS = 6;
+// the larger part's key, and the exponent of a key
+__device__ __forceinline__ int oz_key(double2 v) { return max(oz_key(v.x), oz_key(v.y)); }
+__device__ __forceinline__ int oz_key_expo(int key) { return (key >> 20) - 1023; }
+// the exponent that one result has to reach
+__device__ __forceinline__ int oz_reach(int amax, int bmax) {
+    return amax == OZ_NAN || bmax == OZ_NAN ? OZ_NAN : amax + bmax - OZ_LOSS;
+}
+__device__ __forceinline__ bool oz_lost(int amax, int bmax, bool reached) {
+    if (amax == OZ_NAN || bmax == OZ_NAN) return true;
+    if (amax <= OZ_ZERO || bmax <= OZ_ZERO) return false;  // zeros: so are the results
+    return amax + bmax < -880 || !reached;
+}
+// whether one of n results, over the warp's lanes, reaches: mostly one of the first 32
+__device__ __forceinline__ bool oz_scan(const double2* x, long long n, int reach) {
+    for (long long i0 = 0; i0 < n; i0 += 32) {
+        const long long i = i0 + (threadIdx.x & 31);
+        if (__any_sync(0xffffffffu, i < n && oz_key_expo(oz_key(x[i])) >= reach)) return true;
+    }
+    return false;
 }
 
 // (acc 2^-32 + tail) 2^ex in binary64, rounded to nearest even, by integer

@@ -42,7 +42,10 @@ extern "C" {
 #define AFQ_E_WORKSPACE (-4)        /* workspace smaller than the query says */
 #define AFQ_E_DEVICE_CHECK (-5)     /* a device-side bounded wait or check failed */
 
-#define AFQ_PREC_FP64 0  /* every product in binary64 (large ones from integer digits, no larger error) */
+/* Every product in binary64.  Large ones come from integer digits: each walker's is held to 2^-49 or so of its largest
+ * result (norm-wise, a chain of a few hundred terms' error), and formed on the binary64 pipe where the digits cannot
+ * hold that. */
+#define AFQ_PREC_FP64 0
 #define AFQ_PREC_MIXED 1 /* tensor-core / FP32 products, FP64 overlaps, QR, weights */
 #define AFQ_PREC_MIXED_FAST 2 /* as MIXED with two-piece bf16 operands (~2^-17 products): half the GEMM work */
 
