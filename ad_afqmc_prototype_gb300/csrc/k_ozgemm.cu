@@ -56,6 +56,7 @@
 // the conversion of six accumulators a tile, in single tiles the chain of both
 // (18-25 us).
 #include "afq_internal.cuh"
+#include "copy_ring.h"
 #include "oz_digits.cuh"
 #include "sym_blocks.cuh"
 #include "tc_common.cuh"
@@ -191,6 +192,9 @@ __device__ __forceinline__ void oz_wait(uint32_t bar, uint32_t parity, volatile 
     __syncwarp();
 }
 
+// the whole warp gives up where one of its lanes does: what follows a wait is the warp's together
+__device__ __forceinline__ bool oz_all(bool ok) { return __all_sync(0xffffffffu, ok); }
+
 // shared-memory offsets of the barriers (8 bytes each) after the tiles
 constexpr int OZ_BAR0 = OZ_STG * OZ_S * (OZ_A_SL + OZ_B_SL);
 enum {
@@ -279,7 +283,8 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
 
     if (warp == 0) {
         if (lane == 0) {
-            unsigned c = 0;     // stages issued
+            unsigned c = 0;  // stages issued
+            int na = 0;      // A tiles issued of the next one
             bool ok = true;
             for (int t = blockIdx.x; ok && t < ntiles; t += gridDim.x) {
                 int z, mb, nb;
@@ -298,6 +303,7 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
                         if (!mbar_wait_inl(bars + 8 * (OZB_EA + i), par, abort_flag)) { ok = false; break; }
                         mbar_expect_tx(fa, ab);
                         oz_copy(smem + i * OZ_A_SL, ga + (OZ_S - 1 - j) * pa, ab, fa);
+                        na = j + 1;
                     }
                     if (!ok || !mbar_wait_inl(bars + 8 * (OZB_EB + p), par, abort_flag)) { ok = false; break; }
                     for (int j = 0; j < OZ_S; ++j) {
@@ -305,6 +311,7 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
                         mbar_expect_tx(fb, bb);
                         oz_copy(smem + OZ_STG * OZ_S * OZ_A_SL + i * OZ_B_SL, gb + j * pb, bb, fb);
                     }
+                    na = 0;
                     ga += OZ_S * pa;
                     gb += OZ_S * pb;
                 }
@@ -313,17 +320,15 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
                 atomicExch(a.err, 1);
                 *abort_flag = 1;
             }
-            // every copy this thread issued lands before the CTA exits
-            if (ok) {
-                for (unsigned v = c > OZ_STG ? c - OZ_STG : 0; v < c; ++v)
-                    for (int j = 0; j < OZ_S; ++j) {
-                        mbar_wait(bars + 8 * (OZB_FA + (v & 1) * OZ_S + j), (v >> 1) & 1, nullptr);
-                        mbar_wait(bars + 8 * (OZB_FB + (v & 1) * OZ_S + j), (v >> 1) & 1, nullptr);
-                    }
-            } else {
-                const unsigned long long t0 = now_ns();  // copies in flight land within microseconds
-                while (now_ns() - t0 < 1000000ull) {}
-            }
+            // every copy this thread issued lands before the CTA exits, also where it gave up in the middle of a stage
+            // (a stage's B tiles are issued together, with its last A tile behind them)
+            static_assert(OZ_STG == 2, "ring_last");
+            for (int p = 0; p < OZ_STG; ++p)
+                for (int j = 0; j < OZ_S; ++j) {
+                    const int va = ring_last(c, na, j, p), vb = ring_last(c, 0, j, p);
+                    if (va >= 0) mbar_wait(bars + 8 * (OZB_FA + p * OZ_S + j), (va >> 1) & 1, nullptr);
+                    if (vb >= 0) mbar_wait(bars + 8 * (OZB_FB + p * OZ_S + j), (vb >> 1) & 1, nullptr);
+                }
         }
     } else if (warp == 1) {
         OzMmaState m = {0, 0, 0};
@@ -384,7 +389,7 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
             for (int i = OZ_CHUNK; ok; i += OZ_CHUNK) {
                 const bool end = i >= ni;
                 if (end || i % (2 * OZ_CHUNK) == 0) {
-                    if (!mbar_wait_inl(bars + 8 * OZB_TFS, ns & 1, abort_flag)) { ok = false; break; }
+                    if (!oz_all(mbar_wait_inl(bars + 8 * OZB_TFS, ns & 1, abort_flag))) { ok = false; break; }
                     tc_fence_after();
                     take(5, OZ_D5);
                     take(4, OZ_D4);
@@ -392,7 +397,7 @@ __global__ void __launch_bounds__(OZ_GT, 1) k_ozgemm(const OzArgs a) {
                     take(0, OZ_D0);
                     ++ns;
                 }
-                if (!mbar_wait_inl(bars + 8 * (OZB_TFD + (nd & 1)), (nd >> 1) & 1, abort_flag)) { ok = false; break; }
+                if (!oz_all(mbar_wait_inl(bars + 8 * (OZB_TFD + (nd & 1)), (nd >> 1) & 1, abort_flag))) { ok = false; break; }
                 tc_fence_after();
                 take(3, OZ_D3 + (int)(nd & 1));
                 take(2, OZ_D2 + (int)(nd & 1));

@@ -35,7 +35,8 @@ print = partial(print, flush=True)
 def make_run_blocks(block, engine_args: dict | None = None):
     """run_blocks(state, n_blocks) -> (state, energies (n,), weights (n,)).
     engine_args (keyword arguments of afqmc_block) selects the graph-replayed
-    engine loop."""
+    engine loop.  Raises EngineError where a bounded wait on the device expired
+    (the energies are lost then)."""
 
     def run_blocks(state0: prop_state, *, n_blocks: int):
         if engine_args is not None:
@@ -54,13 +55,16 @@ def make_run_blocks(block, engine_args: dict | None = None):
                 new = prop_state(walkers=st.walkers, weights=st.weights, overlaps=st.overlaps, rng_key=key,
                                  pop_control_ene_shift=st.pop_shift.reshape(()),
                                  e_estimate=st.e_estimate.reshape(()))
-                return new, e.cpu(), w.cpu()
+                e, w = e.cpu(), w.cpu()
+                engine.check_waits()
+                return new, e, w
         es, ws = [], []
         state = state0
         for _ in range(n_blocks):
             state, obs = block(state)
             es.append(float(obs.scalars["energy"]))
             ws.append(float(obs.scalars["weight"]))
+        engine.check_waits()
         return state, torch.tensor(es, dtype=torch.float64), torch.tensor(ws, dtype=torch.float64)
 
     return run_blocks

@@ -345,6 +345,14 @@ def workspace_status():
     return v.value
 
 
+def check_waits():
+    """Raises EngineError if a bounded device-side wait expired in a call since the word was last read (its results are
+    lost then); other marks stay for workspace_counters.  Reads one word of the step / block workspace."""
+    b = _arena.buf.get(torch.cuda.current_device()) if _arena.buf else None
+    if b is not None and int(b[:4].view(torch.int32).item()) == _lib.AFQ_STATUS_WAIT_EXPIRED:
+        workspace_status()
+
+
 def workspace_counters():
     """(status, nonfinite): the status word of the step / block workspace and
     the number of walker updates that produced a NaN or infinite overlap or
