@@ -106,17 +106,28 @@ struct LowpBufs {
     __nv_bfloat16* Bf;  // G x Kt_F     right operand of rot_chol_flat
     __nv_bfloat16* Le;  // G o x Kt_E   left operand [hi hi lo] of rot_chol
     int* asym;          // Bv's rows are in the order of symmetric vectors unless *asym (null: n^2 rows)
+    __nv_bfloat16* Bp;  // Bv as the vectors come, for few walkers (null: none)
 };
 
-// Half a V-build over symmetric vectors, where the mirrored writes are whole 16-byte vectors and the 8 x 8 blocks
-// cover at most four fifths of n^2 (n >= 32; not a function of the walkers, the operand is laid out once).  The split
-// form's blocks cost a second kernel, so its V needs tiles enough that few walkers, one row tile, gain as well.  V-build of
+// Half a V-build over symmetric vectors, where the mirrored writes are whole 16-byte vectors, the 8 x 8 blocks
+// cover at most four fifths of n^2 and the sums are long enough to cost more than the writes.  The split form's blocks cost a second kernel, so its V needs tiles enough that few walkers, one row tile, gain as well.  V-build of
 // 120 orbitals, 600 vectors, 2048 walkers, six sections: 0.58 -> 0.39 ms; 200, 1000, 4096, three sections: 1.79 -> 1.30.
 // Blocks of ten steps, three sections, 120 orbitals: 2.61 -> 2.73 ms at 8 walkers and 9.88 -> 9.83 at 1024 with it; at
 // 160 and 200 orbitals no size was slower.
 static bool lowp_sym(const afq_dims* d) {
     const int n = d->norb;
-    return n % 4 == 0 && 5 * sym_total(n) <= 4 * n * n && (n >= 160 || !tc_taylor_form(d, lowp_dims(d)));
+    const LowpDims L = lowp_dims(d);
+    return n % 4 == 0 && 5 * sym_total(n) <= 4 * n * n && L.Kt_V >= 1024 && (n >= 160 || !tc_taylor_form(d, L));
+}
+// Below 160 orbitals both orders are laid out (the operand does not know the walkers), and the half is taken where the
+// whole is more than a wave of 128 x 256 tiles: in one wave fewer tiles save nothing and their scattered writes cost.
+// Whole -> half, six sections, 4 n vectors, in us: 48 orbitals 26.8 -> 34.3 at 64 walkers, 87.9 -> 86.5 at 4096; 80: 34.8 ->
+// 41.3 at 64, 93.9 -> 81.7 at 1024; 120: 47.2 -> 53.2 at 64, 86.0 -> 55.2 at 256; 160: 59.7 -> 65.6 at 64 (of a step of
+// 1 ms), 156 -> 123 at 256.  Sums shorter than 1024 (32 orbitals 38.9 -> 47.2 at 4096; three sections, 60 orbitals 109 ->
+// 113) take all of V.
+static bool lowp_both(const afq_dims* d) { return lowp_sym(d) && d->norb < 160; }
+static bool vbuild_half_pays(int wc, int n) {
+    return (2LL * wc + 127) / 128 * (((long long)n * n + 255) / 256) > 152;
 }
 
 static LowpBufs layout_lowp(Arena& a, const afq_dims* d) {
@@ -127,6 +138,7 @@ static LowpBufs layout_lowp(Arena& a, const afq_dims* d) {
     b.Bf = a.take<__nv_bfloat16>(G * L.Kt_F);
     b.Le = a.take<__nv_bfloat16>(G * L.Pe * L.Kt_E);
     b.asym = lowp_sym(d) ? a.take<int>(64) : nullptr;
+    b.Bp = lowp_both(d) ? a.take<__nv_bfloat16>(n * n * L.Kt_V) : nullptr;
     (void)o;
     return b;
 }
@@ -407,9 +419,10 @@ static int step_mixed(const afq_problem* pb, const afq_params* p, const afq_stat
     AFQ_TRY(launch_e_minus_i(n, pb->exp_h1_half, ws.emi, s));
     for (int w0 = 0; w0 < W; w0 += Wc) {
         const int wc = W - w0 < Wc ? W - w0 : Wc;
+        const bool whole = lb.Bp && !vbuild_half_pays(wc, n);
         { AFQ_PHASE("vbuild_gemm", s);
-          AFQ_TRY(launch_tc_vbuild(2 * wc, n, L.Kt_V, ws.Av + (size_t)2 * w0 * L.Kt_V, L.Kt_V, lb.Bv, L.Kt_V, lb.asym,
-                                   ws.Vm, nullptr, nullptr, nullptr, L.ldv, ws.status, s)); }
+          AFQ_TRY(launch_tc_vbuild(2 * wc, n, L.Kt_V, ws.Av + (size_t)2 * w0 * L.Kt_V, L.Kt_V, whole ? lb.Bp : lb.Bv,
+                                   L.Kt_V, whole ? nullptr : lb.asym, ws.Vm, nullptr, nullptr, nullptr, L.ldv, ws.status, s)); }
         { AFQ_PHASE("trotter", s);
           AFQ_TRY(launch_trotter_mixed(wc, n, o, p->n_exp_terms, pb->sqrt_dt, ws.emi, ws.Vm, L.ldv,
                                        walk + (size_t)w0 * n * o, walk + (size_t)w0 * n * o, ws.tsum, s)); }
@@ -712,6 +725,7 @@ int afq_prepare_lowp(const afq_dims* d, const double* chol, const double* rot_ch
     // chol^T: row j = (i, k) of L_g[i, k] over g   (right operand of the V-build)
     if (b.asym) AFQ_TRY(launch_asym((int)n, (int)G, chol, b.asym, s));
     AFQ_TRY(launch_split_rows(n * n, (int)G, L.S_V, L.Kt_V, chol, 1, n * n, b.Bv, 0, L.sec, s, 0, 0, b.asym, (int)n));
+    if (b.Bp) AFQ_TRY(launch_split_rows(n * n, (int)G, L.S_V, L.Kt_V, chol, 1, n * n, b.Bp, 0, L.sec, s));
     // rot_chol_flat: row g over (p, j)              (right operand of the force bias)
     AFQ_TRY(launch_split_rows(G, (int)(o * n), L.S_F, L.Kt_F, rot_chol, o * n, 1, b.Bf, 0, L.sec, s));
     // rot_chol rows (g, p) over j                   (left operand of the energy);

@@ -132,7 +132,8 @@ int afq_build_meas_ctx(int32_t norb, int32_t nocc, int32_t nchol, const double* 
 /* Low-precision copies of chol / rot_chol for AFQ_PREC_MIXED / MIXED_FAST
  * (bf16 splits in six or three K sections, tensor-core operand order; the
  * layout depends on d->precision, and that of chol on whether its matrices
- * are symmetric, bit for bit: then half of the V-build's rows are laid out).
+ * are symmetric, bit for bit: then half of the V-build's rows are laid out,
+ * below 160 orbitals beside all of them).
  * `out` must hold afq_lowp_bytes(). */
 size_t afq_lowp_bytes(const afq_dims* d);
 int afq_prepare_lowp(const afq_dims* d, const double* chol, const double* rot_chol,
