@@ -1112,7 +1112,7 @@ OzDigits take_digits(Arena& a, size_t rows, int K, size_t batch = 1) {
 }
 
 // Digit scratch is bounded: operands whose digits take more than this are
-// processed in row chunks.
+// processed in row chunks (but the energy's rotated vectors, cut whole).
 constexpr long long OZ_CAP = 1LL << 30;
 int cap_rows(long long rows, long long bytes_per_row) {
     long long c = OZ_CAP / (bytes_per_row > 0 ? bytes_per_row : 1) / OZ_ROWS * OZ_ROWS;
