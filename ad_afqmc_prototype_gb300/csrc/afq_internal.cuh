@@ -295,8 +295,8 @@ int launch_zgemm(int M, int N, int K, double alpha, const double2* A, int64_t ld
                  int64_t ldc, cudaStream_t s);
 // the rows of a real-B product that the digits cannot be left to (oz_digits.cuh), found on the device
 int launch_zgemm_lost(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
-                      bool b_trans, double2* C, int64_t ldc, const int* amax, const int* ex, int aexp,
-                      cudaStream_t s);
+                      bool b_trans, double2* C, int64_t ldc, const int* amax, const int* ex, int aexp, int* arrived,
+                      int* err, cudaStream_t s);
 // a real B; pays: where the digits' launches would take longer
 bool zgemm_small_pays(int M, int N, int K);
 int launch_zgemm_small(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,

@@ -26,6 +26,12 @@ __device__ __forceinline__ void load_b(double2& dst, const double2* p, bool ok) 
 __device__ __forceinline__ void mac(double2& acc, double2 a, double b) { rfma(acc, b, a); }
 __device__ __forceinline__ void mac(double2& acc, double2 a, double2 b) { cfma(acc, a, b); }
 
+__device__ __forceinline__ unsigned long long now_ns() {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
 // One 64 x 64 tile by 256 threads, sums over k in [kbeg, kend).
 template <bool BC, bool BT>
 __device__ __forceinline__ void zgemm_tile(int M, int N, int kbeg, int kend, double alpha, const double2* __restrict__ A,
@@ -111,13 +117,14 @@ __global__ void __launch_bounds__(256) k_zgemm(int M, int N, int K, double alpha
                        C + (int64_t)blockIdx.z * cs, ldc, blockIdx.y * BM, blockIdx.x * BN);
 }
 
-// The rows of C (tiles of 64) among which the digits (scales ex of the rows' parts) lost too much (oz_lost).  A CTA checks its tile's rows and, mostly,
-// ends.
+// The rows of C (tiles of 64) among which the digits (scales ex of the rows' parts) lost too much (oz_lost).  A tile's
+// CTAs all check its rows and, mostly, end.  Otherwise they all see it, and wait for one another (arrived[tile], a
+// cooperative launch) before the first of them writes what another one may still be reading.
 template <bool BT>
 __global__ void __launch_bounds__(256) k_zgemm_lost(int M, int N, int K, double alpha, const double2* __restrict__ A,
                                                     int64_t lda, const double* __restrict__ B, int64_t ldb,
                                                     double2* __restrict__ C, int64_t ldc, const int* __restrict__ amax,
-                                                    const int* __restrict__ ex, int aexp) {
+                                                    const int* __restrict__ ex, int aexp, int* arrived, int* err) {
     const int m0 = blockIdx.y * BM, wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // eight rows a warp: mostly one of a row's first 32 results tells that it is sound
     constexpr int R = BM / 8;
@@ -137,17 +144,34 @@ __global__ void __launch_bounds__(256) k_zgemm_lost(int M, int N, int K, double 
         lost = lost || oz_lost(am, bm, any || oz_scan(C + (int64_t)m * ldc, N, to == OZ_NAN ? to : to + aexp));
     }
     if (!__syncthreads_or(lost)) return;
+    if (gridDim.x > 1) {
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(arrived + blockIdx.y, 1);
+            const unsigned long long t0 = now_ns();
+            while (*(volatile int*)(arrived + blockIdx.y) < (int)gridDim.x)
+                if (now_ns() - t0 > 1000000000ull) {
+                    atomicExch(err, AFQ_STATUS_WAIT_EXPIRED);
+                    break;
+                }
+        }
+        __syncthreads();
+    }
     for (int n0 = blockIdx.x * BN; n0 < N; n0 += gridDim.x * BN)
         zgemm_tile<false, BT>(M, N, 0, K, alpha, A, lda, B, ldb, C, ldc, m0, n0);
 }
 
 int launch_zgemm_lost(int M, int N, int K, double alpha, const double2* A, int64_t lda, const double* B, int64_t ldb,
-                      bool b_trans, double2* C, int64_t ldc, const int* amax, const int* ex, int aexp,
-                      cudaStream_t s) {
-    const int mt = (M + BM - 1) / BM, nt = (N + BN - 1) / BN, per = 304 / mt;  // two CTAs an SM
+                      bool b_trans, double2* C, int64_t ldc, const int* amax, const int* ex, int aexp, int* arrived,
+                      int* err, cudaStream_t s) {
+    int sms = 0;
+    AFQ_TRY(device_sms(&sms));
+    const int mt = (M + BM - 1) / BM, nt = (N + BN - 1) / BN, per = sms / mt;  // at most a CTA an SM where they wait
     const dim3 grid(per < 1 ? 1 : per < nt ? per : nt, mt);
-    if (b_trans) k_zgemm_lost<true><<<grid, 256, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, C, ldc, amax, ex, aexp);
-    else k_zgemm_lost<false><<<grid, 256, 0, s>>>(M, N, K, alpha, A, lda, B, ldb, C, ldc, amax, ex, aexp);
+    void* args[] = {&M, &N, &K, &alpha, &A, &lda, &B, &ldb, &C, &ldc, &amax, &ex, &aexp, &arrived, &err};
+    const void* kernel = b_trans ? (const void*)k_zgemm_lost<true> : (const void*)k_zgemm_lost<false>;
+    AFQ_CUDA(grid.x > 1 ? cudaLaunchCooperativeKernel(kernel, grid, dim3(256), args, 0, s)
+                        : cudaLaunchKernel(kernel, grid, dim3(256), args, 0, s));
     AFQ_LAUNCHED("k_zgemm_lost");
     return AFQ_OK;
 }

@@ -599,10 +599,11 @@ __global__ void __launch_bounds__(256) k_oz_rows(long long rows, int per, int K,
 }
 
 // Complex rows with K contiguous: digit rows 2 r (real parts) and 2 r + 1.
-// amax (optional): set for the other operand's cut to raise.
+// amax (optional): set for the other operand's cut to raise; arrived, one a 64 rows, too (k_zgemm_lost).
 template <int LN>
 __global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const double2* __restrict__ src, long long ld,
-                                                  OzDst dst, int* __restrict__ ex, int* __restrict__ amax) {
+                                                  OzDst dst, int* __restrict__ ex, int* __restrict__ amax,
+                                                  int* __restrict__ arrived) {
     __shared__ int s_max[2][8];
     const int t = threadIdx.x % LN;
     if (amax && blockIdx.x == 0 && threadIdx.x == 0) *amax = OZ_EMPTY;
@@ -620,6 +621,7 @@ __global__ void __launch_bounds__(256) k_oz_crows(long long rows, int K, const d
         if (t == 0) {
             ex[2 * r] = E0;
             ex[2 * r + 1] = E1;
+            if (amax && r % 64 == 0) arrived[r / 64] = 0;
         }
         for (int k = 8 * t; k < 32 * dst.nks; k += 8 * LN) {
             long long y[8], w[8];
@@ -1089,10 +1091,10 @@ int split_rows(long long rows, int per, int K, const double* src, long long ld, 
     return AFQ_OK;
 }
 int split_crows(long long rows, int K, const double2* src, long long ld, const OzDigits& D, cudaStream_t s,
-                int* amax = nullptr) {
+                int* amax = nullptr, int* arrived = nullptr) {
     const OzDst dst = dst_of(D, 2 * rows, K);
-    if (row_cta(rows, K)) k_oz_crows<256><<<row_blocks(rows, 1), 256, 0, s>>>(rows, K, src, ld, dst, D.ex, amax);
-    else k_oz_crows<32><<<row_blocks(rows), 256, 0, s>>>(rows, K, src, ld, dst, D.ex, amax);
+    if (row_cta(rows, K)) k_oz_crows<256><<<row_blocks(rows, 1), 256, 0, s>>>(rows, K, src, ld, dst, D.ex, amax, arrived);
+    else k_oz_crows<32><<<row_blocks(rows), 256, 0, s>>>(rows, K, src, ld, dst, D.ex, amax, arrived);
     AFQ_LAUNCHED("k_oz_crows");
     return AFQ_OK;
 }
@@ -1135,11 +1137,12 @@ int oz_room(const Arena& a) {
 
 constexpr int OZ_TILE_SMS = 152;
 
+constexpr int OZ_LOST = 64;  // rows a tile of k_zgemm_lost
 struct ZLayout {
     int mc, nc;
     OzDigits A, B;
     long long* raw;
-    int *asym, *amax;
+    int *asym, *amax, *arrived;
 };
 ZLayout z_layout(Arena& a, int M, int N, int K) {
     ZLayout z;
@@ -1153,6 +1156,7 @@ ZLayout z_layout(Arena& a, int M, int N, int K) {
     z.raw = a.take<long long>((nch > 1 ? (all < most ? all : most) : 0) * 3 / 2);  // 64-bit sums, 32-bit tails
     z.asym = a.take<int>(64);
     z.amax = a.take<int>(1);
+    z.arrived = a.take<int>((z.mc + OZ_LOST - 1) / OZ_LOST);
     return z;
 }
 
@@ -1268,7 +1272,7 @@ static int zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t
     AFQ_TRY(device_sms(&sms));
     for (int m0 = 0; m0 < M; m0 += z.mc) {
         const int mc = M - m0 < z.mc ? M - m0 : z.mc;
-        AFQ_TRY(split_crows(mc, K, A + (int64_t)m0 * lda, lda, z.B, s, z.amax));
+        AFQ_TRY(split_crows(mc, K, A + (int64_t)m0 * lda, lda, z.B, s, z.amax, z.arrived));
         for (int n0 = 0; n0 < N; n0 += z.nc) {
             const int nc = N - n0 < z.nc ? N - n0 : z.nc;
             const SymRows sym = {sn ? asym : nullptr, sn, n0};  // the chunk's first row
@@ -1284,8 +1288,12 @@ static int zgemm_oz(int M, int N, int K, double alpha, const double2* A, int64_t
             const bool all = sn != 0;
             AFQ_TRY(launch_zgemm_lost(mc, all ? N : nc, K, alpha, A + (int64_t)m0 * lda, lda,
                                       all ? B : b_trans ? B + (int64_t)n0 * ldb : B + n0, ldb, b_trans,
-                                      C + (int64_t)m0 * ldc + (all ? 0 : n0), ldc, amax, z.B.ex, ae - 1, s));
-            if (n0 + nc < N) AFQ_CUDA(cudaMemsetAsync(z.amax, 0x80, sizeof(int), s));  // the next is judged by itself
+                                      C + (int64_t)m0 * ldc + (all ? 0 : n0), ldc, amax, z.B.ex, ae - 1, z.arrived,
+                                      oz.err, s));
+            if (n0 + nc < N) {  // the next is judged by itself
+                AFQ_CUDA(cudaMemsetAsync(z.amax, 0x80, sizeof(int), s));
+                AFQ_CUDA(cudaMemsetAsync(z.arrived, 0, (size_t)(mc + OZ_LOST - 1) / OZ_LOST * sizeof(int), s));
+            }
         }
     }
     return AFQ_OK;
