@@ -85,6 +85,25 @@ def test_green_of_graded_columns(n, o):
     assert _rel(g, O.half_green(w, mo)) < RTOL and _rel(ov, O.overlap_r(w, mo)) < 10 * RTOL
 
 
+@pytest.mark.parametrize("n,o,W", [(60, 20, 5), (130, 17, 70)])
+def test_force_bias_from_a_graded_green(n, o, W):
+    """The same, where m and G_half are products by digits (n o^2 from 24000 on); every third walker is of one size."""
+    rng = np.random.default_rng(6)
+    s = 10.0 ** (10 * np.arange(n) / n)
+    mo = rng.normal(size=(n, o)) / s[:, None]
+    w = (rng.normal(size=(n, o)) + 0.3 * _crandn(rng, W, n, o)) * s[:, None]
+    w[::3] /= s[:, None]
+    rot = rng.normal(size=(40, o, n)) / s
+    got = engine.force_bias(_cdev(w), _cdev(mo), _dev(rot), True).cpu().numpy()
+    ctx = O.MeasCtx(rot_h1=None, rot_chol=rot, rot_chol_flat=rot.reshape(40, -1))
+    want = O.force_bias_r(w, ctx, mo)
+    # conditions of m: below 3e3 in the graded walkers, 1e6 in those of one size (the trial's first rows are all they
+    # meet); 30 roundings each
+    each = np.linalg.norm(got - want, axis=1) / np.linalg.norm(want, axis=1)
+    graded = np.arange(W) % 3 != 0
+    assert each[graded].max() < 1e-11 and each[~graded].max() < 3e-9
+
+
 @pytest.mark.parametrize("n,o,G,W,sym", [(40, 7, 200, 9, False), (40, 7, 900, 9, False), (120, 8, 40, 70, True),
                                          (36, 5, 64, 700, True)])
 def test_vectors_and_fields_graded_in_opposite_directions(n, o, G, W, sym):
